@@ -1,0 +1,105 @@
+// edges.cuh -- passes over the entries of a CSR in tiles of consecutive
+// entries, with the row of every entry at hand.
+//
+// A warp per row leaves a hub row of tens of thousands of entries to one
+// warp, and the kernel waits for it (R-MAT 20 directed, writing one 12-byte
+// pair per entry: 642 us with a warp per row).  A tile has the same work
+// whatever the row lengths: a block finds the row of its first entry by a
+// 32-way search of the offsets, marks the position where each later row
+// starts with that row's id, and an inclusive max-scan of the marks gives
+// every entry its row.
+#pragma once
+#include "common.cuh"
+
+namespace apspie {
+
+constexpr int kEdgeThreads = 256;
+constexpr int kEdgeItems = 8;                          // entries per thread
+constexpr int kEdgeTile = kEdgeThreads * kEdgeItems;  // entries per tile
+
+// Largest r with ptr[r] <= k, given ptr[m] > k.  Warp-collective.
+__device__ __forceinline__ int row_of_entry(const int *__restrict__ ptr, int m, int k) {
+  const int lane = lane_id();
+  int lo = 0, hi = m;  // ptr[lo] <= k < ptr[hi]
+  while (hi - lo > 1) {
+    const long long span = hi - lo;
+    const int piv = lo + (int)(span * lane / 32);
+    const unsigned b = __ballot_sync(kFull, __ldg(ptr + piv) <= k);  // lane 0 always
+    const int last = 31 - __clz(b);
+    const int nlo = lo + (int)(span * last / 32);
+    const int nhi = last == 31 ? hi : lo + (int)(span * (last + 1) / 32);
+    lo = nlo;
+    hi = max(nhi, nlo + 1);
+  }
+  return lo;
+}
+
+// s_row[t] = row of entry k0 + t for t in [0, n), n <= kEdgeTile.  Called by
+// all kEdgeThreads threads; s_row is ready when it returns.
+__device__ __forceinline__ void edge_tile_rows(const int *__restrict__ ptr, int m, int k0, int n,
+                                               int *s_row) {
+  __shared__ int s_warp[kEdgeThreads / 32];
+  __shared__ int s_r0;
+  const int t = threadIdx.x, lane = lane_id(), w = warp_in_block();
+  if (w == 0) {
+    const int r = row_of_entry(ptr, m, k0);
+    if (lane == 0) s_r0 = r;
+  }
+  for (int i = t; i < kEdgeTile; i += kEdgeThreads) s_row[i] = -1;
+  __syncthreads();
+  const int r0 = s_r0;
+  // empty rows start where the next non-empty one does: the largest id wins
+  for (unsigned r = (unsigned)(r0 + 1 + t); r < (unsigned)m; r += kEdgeThreads) {
+    const int at = __ldg(ptr + r) - k0;
+    if (at >= n) break;
+    atomicMax(s_row + at, (int)r);
+  }
+  __syncthreads();
+  // inclusive max-scan, kEdgeItems consecutive entries per thread
+  int4 *q4 = reinterpret_cast<int4 *>(s_row) + t * (kEdgeItems / 4);
+  int v[kEdgeItems];
+#pragma unroll
+  for (int i = 0; i < kEdgeItems / 4; ++i) {
+    const int4 x = q4[i];
+    v[4 * i] = x.x, v[4 * i + 1] = x.y, v[4 * i + 2] = x.z, v[4 * i + 3] = x.w;
+  }
+#pragma unroll
+  for (int i = 1; i < kEdgeItems; ++i) v[i] = max(v[i], v[i - 1]);
+  int incl = v[kEdgeItems - 1];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl = max(incl, y);
+  }
+  if (lane == 31) s_warp[w] = incl;
+  int before = __shfl_up_sync(kFull, incl, 1);
+  if (lane == 0) before = -1;
+  __syncthreads();
+  before = max(before, r0);
+  for (int x = 0; x < w; ++x) before = max(before, s_warp[x]);
+#pragma unroll
+  for (int i = 0; i < kEdgeItems / 4; ++i)
+    q4[i] = make_int4(max(before, v[4 * i]), max(before, v[4 * i + 1]), max(before, v[4 * i + 2]),
+                      max(before, v[4 * i + 3]));
+  __syncthreads();
+}
+
+// The lanes of a warp that hold entries of this lane's row, for entries in
+// CSR order (equal rows are adjacent); leader: the first of them.  Lanes
+// past the end pass row -1.  Warp-collective.
+__device__ __forceinline__ unsigned row_peers(int row, int *leader) {
+  const int lane = lane_id();
+  const int prev = __shfl_up_sync(kFull, row, 1);
+  const unsigned heads = __ballot_sync(kFull, lane == 0 || row != prev);
+  const unsigned upto = lane == 31 ? kFull : (2u << lane) - 1u;
+  *leader = 31 - __clz(heads & upto);
+  const unsigned after = heads & ~upto;
+  const unsigned below_next = after ? (1u << (__ffs(after) - 1)) - 1u : kFull;
+  return below_next & ~((1u << *leader) - 1u);
+}
+
+inline unsigned edge_tiles(long long nnz) {
+  return (unsigned)((nnz + kEdgeTile - 1) / kEdgeTile);
+}
+
+}  // namespace apspie

@@ -12,6 +12,7 @@
 
 #include "common.cuh"
 #include "context.h"
+#include "edges.cuh"
 #include "gen_common.h"
 #include "primitives.cuh"
 
@@ -138,25 +139,43 @@ __global__ void key_rows(const unsigned long long *k, long long n, int dbits, in
   }
 }
 
-// key of edge k = (row u -> col ind[k]) for the transpose: (col, row); value k
-__global__ void transpose_keys(int m, const int *ptr, const int *ind, int rbits,
-                               unsigned long long *keys, int *vals) {
-  const int lane = threadIdx.x & 31;
-  for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < m;
-       u += (gridDim.x * blockDim.x) >> 5)
-    for (int k = ptr[u] + lane; k < ptr[u + 1]; k += 32) {
-      keys[k] = ((unsigned long long)ind[k] << rbits) | (unsigned)u;
-      vals[k] = k;
-    }
+// rv[k] = (value bits << 32 | row) of entry k, so that the transpose's last
+// step gathers both with one 8-byte load; equal work per block (edges.cuh)
+__global__ void __launch_bounds__(kEdgeThreads)
+transpose_rows(int m, int nnz, const int *__restrict__ ptr, const float *__restrict__ val,
+               unsigned long long *rv) {
+  __shared__ __align__(16) int s_row[kEdgeTile];
+  const int k0 = (int)blockIdx.x * kEdgeTile;
+  const int n = min(kEdgeTile, nnz - k0);
+  edge_tile_rows(ptr, m, k0, n, s_row);
+  for (int t = threadIdx.x; t < n; t += kEdgeThreads) {
+    const float v = val ? __ldg(val + k0 + t) : 1.0f;
+    rv[k0 + t] = ((unsigned long long)__float_as_uint(v) << 32) | (unsigned)s_row[t];
+  }
 }
 
-__global__ void transpose_emit(long long n, int rbits, const unsigned long long *keys,
-                               const int *vals, const float *val, int *tind, float *tval) {
-  const unsigned long long mask = (1ull << rbits) - 1ull;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    tind[i] = (int)(keys[i] & mask);
-    if (tval) tval[i] = val ? val[vals[i]] : 1.0f;
+// Sorted (column, entry) pairs -> the transpose's rows and values and each
+// column's length: +(i + 1) at a column's last pair and -i at its first, two
+// adds per column.  The pairs of a sort that gave up (reported by the
+// caller) may hold any entry or column: both are bounds-checked.
+__global__ void transpose_emit(int n, int ncols, const unsigned *__restrict__ keys,
+                               const int *__restrict__ ids,
+                               const unsigned long long *__restrict__ rv, int *tcnt, int *tind,
+                               float *tval) {
+  const unsigned stride = gridDim.x * blockDim.x;
+  for (unsigned j = blockIdx.x * blockDim.x + threadIdx.x; j < (unsigned)n; j += stride) {
+    const int i = (int)j;
+    const unsigned c = keys[i];
+    const int k = ids[i];
+    const unsigned long long x = (unsigned)k < (unsigned)n ? __ldg(rv + k) : 0ull;
+    tind[i] = (int)(unsigned)x;
+    if (tval) tval[i] = __uint_as_float((unsigned)(x >> 32));
+    if (c < (unsigned)ncols) {
+      if (i == 0 || keys[i - 1] != c) {
+        if (i) atomicAdd(tcnt + c, -i);
+      }
+      if (i == n - 1 || keys[i + 1] != c) atomicAdd(tcnt + c, i + 1);
+    }
   }
 }
 
@@ -314,29 +333,31 @@ int apspie_csr_transpose(apspie_ctx ctx, int m, int n, int64_t nnz, const int *d
   fill_int<<<gg(ctx, (long long)n + 1), 256, 0, st>>>(n + 1, 0, d_tptr);
   int rc = check_launch(ctx, "fill_int");
   if (rc || nnz == 0) return rc;
-  const int rbits = std::max(1, bits_for(m)), cbits = std::max(1, bits_for(n));
-  auto *ka = (unsigned long long *)workspace(ctx, kSlotSortKeysA, 8 * (size_t)nnz);
-  auto *kb = (unsigned long long *)workspace(ctx, kSlotSortKeysB, 8 * (size_t)nnz);
+  // The entries in row order, stably sorted by column: rows come out
+  // ascending within a column, so only the column's bits are sorted (R-MAT 20
+  // directed, 16 M entries: three passes of 8-byte pairs instead of five of
+  // 12-byte ones on packed (column, row) keys).
+  const int cbits = std::max(1, bits_for(n));
+  auto *ka = (unsigned *)workspace(ctx, kSlotSortKeysA, 4 * (size_t)nnz);
+  auto *kb = (unsigned *)workspace(ctx, kSlotSortKeysB, 4 * (size_t)nnz);
   auto *va = (int *)workspace(ctx, kSlotSortValsA, 4 * (size_t)nnz);
   auto *vb = (int *)workspace(ctx, kSlotSortValsB, 4 * (size_t)nnz);
-  if (!ka || !kb || !va || !vb) return APSPIE_ERR_OOM;
-  transpose_keys<<<gg(ctx, (long long)m * 32), 256, 0, st>>>(m, d_ptr, d_ind, rbits, ka, va);
-  rc = check_launch(ctx, "transpose_keys");
+  auto *rv = (unsigned long long *)workspace(ctx, kSlotMisc0, 8 * (size_t)nnz);
+  if (!ka || !kb || !va || !vb || !rv) return APSPIE_ERR_OOM;
+  transpose_rows<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, (int)nnz, d_ptr, d_val, rv);
+  rc = check_launch(ctx, "transpose_rows");
   if (rc) return rc;
-  // rows within a column come out ascending: the keys hold them, and the
-  // sort only needs the column bits above them (stable LSD on all bits)
   bool in_b = false;
-  rc = device_radix_sort<unsigned long long, int>(ctx, ka, va, kb, vb, nnz, rbits + cbits, &in_b);
+  rc = device_radix_sort<unsigned, int>(ctx, ka, va, kb, vb, nnz, cbits, &in_b,
+                                        reinterpret_cast<const unsigned *>(d_ind));
   if (rc) return rc;
-  rc = radix_sort_check(ctx);  // before the sorted keys index anything
+  transpose_emit<<<gg(ctx, nnz), 256, 0, st>>>((int)nnz, n, in_b ? kb : ka, in_b ? vb : va, rv,
+                                               d_tptr, d_tind, d_tval);
+  rc = check_launch(ctx, "transpose_emit");
   if (rc) return rc;
-  const unsigned long long *k = in_b ? kb : ka;
-  const int *v = in_b ? vb : va;
-  key_rows<<<gg(ctx, nnz), 256, 0, st>>>(k, nnz, rbits, d_tptr);
-  transpose_emit<<<gg(ctx, nnz), 256, 0, st>>>(nnz, rbits, k, v, d_val, d_tind, d_tval);
-  rc = check_launch(ctx, "transpose_emit", 2);
+  rc = device_exclusive_scan<int>(ctx, d_tptr, d_tptr, (long long)n + 1, nullptr);
   if (rc) return rc;
-  return device_exclusive_scan<int>(ctx, d_tptr, d_tptr, (long long)n + 1, nullptr);
+  return radix_sort_check(ctx);
 }
 
 int apspie_gen_weights_u32_device(apspie_ctx ctx, int m, const int *d_ptr, const int *d_ind,

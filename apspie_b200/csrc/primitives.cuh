@@ -342,14 +342,15 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
     const unsigned long long at = gbase[sdig[t]] + t;
     if (at < (unsigned long long)n) keys_out[at] = skeys[t];
   }
-  if (vals_in) {  // keys-only sorts pass no values
+  if (vals_out) {  // keys-only sorts pass no values
     if (vdone > 0) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
     V *svals = reinterpret_cast<V *>(skeys);
 #pragma unroll
     for (int i = 0; i < kSortItems; ++i) {
       const int t = wofs + i * 32 + lane;
-      if (t < tlen) svals[pos[i]] = t < vdone ? svin[t] : vals_in[tbase + t];
+      if (t < tlen)
+        svals[pos[i]] = t < vdone ? svin[t] : (vals_in ? vals_in[tbase + t] : (V)(tbase + t));
     }
     __syncthreads();
     for (int t = threadIdx.x; t < tlen; t += kSortThreads) {
@@ -395,13 +396,18 @@ inline int radix_sort_check(apspie_context *ctx) {
 
 // Stable sort of n (key, value) pairs on the low `bits` bits of the key
 // (va == vb == nullptr sorts keys only).  Ping-pongs between (ka, va) and
-// (kb, vb); *result_in_b tells where the sorted data ended up.  Scratch:
-// slot kSlotSortHist (histograms, tile counters, status words).
+// (kb, vb); *result_in_b tells where the sorted data ended up.  With kfirst
+// the first pass reads its keys there instead (an array that must stay as it
+// is) and each key's value is its index, so neither is copied first; va and
+// vb must be given.  Scratch: slot kSlotSortHist (histograms, tile counters,
+// status words).
 template <typename K, typename V>
 int device_radix_sort(apspie_context *ctx, K *ka, V *va, K *kb, V *vb, long long n, int bits,
-                      bool *result_in_b) {
+                      bool *result_in_b, const K *kfirst = nullptr) {
   *result_in_b = false;
-  if (n <= 1 || bits <= 0) return APSPIE_OK;
+  if (!kfirst && (n <= 1 || bits <= 0)) return APSPIE_OK;
+  if (kfirst && (n < 1 || bits < 1))
+    return set_error(ctx, APSPIE_ERR_INVALID, "radix sort: %lld keys of %d bits", n, bits);
   const int npass = (bits + kRadixBits - 1) / kRadixBits;
   if (npass > kMaxPasses || n >= (1ll << 40))
     return set_error(ctx, APSPIE_ERR_OVERFLOW, "radix sort: %lld keys of %d bits", n, bits);
@@ -422,7 +428,7 @@ int device_radix_sort(apspie_context *ctx, K *ka, V *va, K *kb, V *vb, long long
   cudaMemsetAsync(ws, 0, bytes, st);
   const int hgrid = (int)std::max(1ll, std::min((n + kSortThreads * 8 - 1) / (kSortThreads * 8),
                                                 (long long)ctx->num_sms * 4));
-  radix_histograms<K><<<hgrid, kSortThreads, 0, st>>>(ka, n, npass, ghist);
+  radix_histograms<K><<<hgrid, kSortThreads, 0, st>>>(kfirst ? kfirst : ka, n, npass, ghist);
   radix_digit_offsets<kRadix><<<1, kRadix, 0, st>>>(ghist, npass);
   int rc = check_launch(ctx, "radix_histograms", 2);
   if (rc) return rc;
@@ -433,9 +439,10 @@ int device_radix_sort(apspie_context *ctx, K *ka, V *va, K *kb, V *vb, long long
     cudaFuncSetAttribute(radix_onesweep<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)vdyn);
   for (int p = 0; p < npass; ++p) {
-    radix_onesweep<K, V><<<(unsigned)tiles, kSortThreads, vdyn, st>>>(kin, vin, kout, vout, n, p,
-                                                                      ghist, status, counters + p,
-                                                                      err, (int *)(counters + 15));
+    const bool first = kfirst && p == 0;
+    radix_onesweep<K, V><<<(unsigned)tiles, kSortThreads, vdyn, st>>>(
+        first ? kfirst : kin, first ? nullptr : vin, kout, vout, n, p, ghist, status,
+        counters + p, err, (int *)(counters + 15));
     rc = check_launch(ctx, "radix_onesweep");
     if (rc) return rc;
     std::swap(kin, kout);

@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "context.h"
+#include "edges.cuh"
 #include "gen_common.h"
 #include "primitives.cuh"
 
@@ -298,36 +299,43 @@ __global__ void rank_to_perm(int m, const int *order, int *perm) {
 }
 
 // Per vertex v of new id r: how many neighbours rank below r (the length
-// of L's row r) and how many above (v's entries in L's columns).  A warp
-// per vertex, both counts from one read of the row.  The same pass sums a
+// of L's row r) and how many above (v's entries in L's columns), added to
+// zeroed lcnt / ucnt by warp and row from one pass over the edges in tiles of
+// equal size (a warp per vertex waited for the hubs' warps: R-MAT 18, 7.6 M
+// edges, 221 us).  The same pass sums a
 // 64-bit hash of every edge (v, u) and of its reverse (u, v) into hsum[0] and
 // hsum[1] (wrapping): the edge multiset equals its transpose -- the graph is
 // symmetric -- exactly when the multisets of hashed pairs agree, which the two
 // sums confirm up to a 2^-64 chance.
-__global__ void split_counts(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
-                            const int *__restrict__ perm, int *lcnt, int *ucnt,
-                            unsigned long long *hsum) {
+__global__ void __launch_bounds__(kEdgeThreads)
+split_counts(int m, int nnz, const int *__restrict__ ptr, const int *__restrict__ ind,
+             const int *__restrict__ perm, int *lcnt, int *ucnt, unsigned long long *hsum) {
+  __shared__ __align__(16) int s_row[kEdgeTile];
+  const int k0 = (int)blockIdx.x * kEdgeTile;
+  const int n = min(kEdgeTile, min(nnz, __ldg(ptr + m)) - k0);
+  if (n <= 0) return;
+  edge_tile_rows(ptr, m, k0, n, s_row);
   const int lane = lane_id();
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
   unsigned long long h_fwd = 0, h_rev = 0;
-  for (int v = gwarp; v < m; v += nwarps) {
-    const int r = __ldg(perm + v);
-    const int s = __ldg(ptr + v), e = __ldg(ptr + v + 1);
-    int lo = 0, hi = 0;
-    for (int k = s + lane; k < e; k += 32) {
-      const int u = __ldg(ind + k);
-      const int pu = __ldg(perm + u);
-      lo += pu < r;
-      hi += pu > r;
+  for (int t0 = (int)threadIdx.x - lane; t0 < n; t0 += kEdgeThreads) {
+    const int t = t0 + lane;
+    int v = -1, r = 0, pu = 0;
+    if (t < n) {
+      v = s_row[t];
+      const int u = __ldg(ind + k0 + t);
+      r = __ldg(perm + v);
+      pu = __ldg(perm + u);
       h_fwd += apspie_gen::mix64(((unsigned long long)(unsigned)v << 32) | (unsigned)u);
       h_rev += apspie_gen::mix64(((unsigned long long)(unsigned)u << 32) | (unsigned)v);
     }
-    lo = warp_sum(lo);
-    hi = warp_sum(hi);
-    if (lane == 0) {
-      lcnt[r] = lo;
-      ucnt[r] = hi;
+    const unsigned below = __ballot_sync(kFull, t < n && pu < r);
+    const unsigned above = __ballot_sync(kFull, t < n && pu > r);
+    int leader;
+    const unsigned peers = row_peers(v, &leader);
+    if (lane == leader && v >= 0) {
+      const int lo = __popc(below & peers), hi = __popc(above & peers);
+      if (lo) atomicAdd(lcnt + r, lo);
+      if (hi) atomicAdd(ucnt + r, hi);
     }
   }
   h_fwd = warp_sum(h_fwd);
@@ -339,29 +347,38 @@ __global__ void split_counts(int m, const int *__restrict__ ptr, const int *__re
 }
 
 // L's entries as (row new(u), column r) pairs, grouped by column r in
-// ascending order (segment uoff[r]): a stable sort by row then leaves each
-// row's columns ascending.  A warp per vertex, lanes compacted by ballot.
-__global__ void upper_pairs(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
-                            const int *__restrict__ perm, const int *__restrict__ uoff,
-                            unsigned *rows, int *cols) {
+// ascending order (segment uoff[r], which counts up as the pairs are
+// written): a stable sort by row then leaves each row's columns ascending.
+// Within a column the pairs may come in any order, since their rows differ
+// (equal pairs are the same pair), so a warp reserves its places in a
+// column with one add.
+__global__ void __launch_bounds__(kEdgeThreads)
+upper_pairs(int m, int nnz, const int *__restrict__ ptr, const int *__restrict__ ind,
+            const int *__restrict__ perm, int *uoff, unsigned *rows, int *cols) {
+  __shared__ __align__(16) int s_row[kEdgeTile];
+  const int k0 = (int)blockIdx.x * kEdgeTile;
+  const int n = min(kEdgeTile, min(nnz, __ldg(ptr + m)) - k0);
+  if (n <= 0) return;
+  edge_tile_rows(ptr, m, k0, n, s_row);
   const int lane = lane_id();
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int v = gwarp; v < m; v += nwarps) {
-    const int r = __ldg(perm + v);
-    const int s = __ldg(ptr + v), e = __ldg(ptr + v + 1);
-    int out = __ldg(uoff + r);
-    for (int k0 = s; k0 < e; k0 += 32) {
-      const int k = k0 + lane;
-      const int pu = k < e ? __ldg(perm + __ldg(ind + k)) : -1;
-      const bool keep = pu > r;
-      const unsigned mask = __ballot_sync(kFull, keep);
-      if (keep) {
-        const int at = out + __popc(mask & ((1u << lane) - 1u));
-        rows[at] = (unsigned)pu;
-        cols[at] = r;
-      }
-      out += __popc(mask);
+  for (int t0 = (int)threadIdx.x - lane; t0 < n; t0 += kEdgeThreads) {
+    const int t = t0 + lane;
+    int v = -1, r = 0, pu = 0;
+    if (t < n) {
+      v = s_row[t];
+      r = __ldg(perm + v);
+      pu = __ldg(perm + __ldg(ind + k0 + t));
+    }
+    const bool keep = t < n && pu > r;
+    int leader;
+    const unsigned mine = row_peers(v, &leader) & __ballot_sync(kFull, keep);
+    int base = 0;
+    if (lane == leader && mine) base = atomicAdd(uoff + r, __popc(mine));
+    base = __shfl_sync(kFull, base, leader);
+    if (keep) {
+      const int at = base + __popc(mine & ((1u << lane) - 1u));
+      rows[at] = (unsigned)pu;
+      cols[at] = r;
     }
   }
 }
@@ -414,14 +431,16 @@ int apspie_tc_prepare(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr, cons
   auto *lcnt = d_Lptr;
   auto *uoff = (int *)workspace(ctx, kSlotMisc0, sizeof(int) * ((size_t)m + 1));
   if (!uoff) return APSPIE_ERR_OOM;
-  cudaMemsetAsync(lcnt + m, 0, sizeof(int), st);
-  cudaMemsetAsync(uoff + m, 0, sizeof(int), st);
+  cudaMemsetAsync(lcnt, 0, sizeof(int) * ((size_t)m + 1), st);
+  cudaMemsetAsync(uoff, 0, sizeof(int) * ((size_t)m + 1), st);
   // small[0]: the largest degree; small + 8 bytes .. + 24: the two edge hashes
   auto *hsum = reinterpret_cast<unsigned long long *>(small) + 1;
-  split_counts<<<tgrid(ctx, (long long)m * 32, 256), 256, 0, st>>>(m, d_ptr, d_ind, d_perm, lcnt,
-                                                                   uoff, hsum);
-  rc = check_launch(ctx, "split_counts");
-  if (rc) return rc;
+  if (nnz > 0) {
+    split_counts<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, (int)nnz, d_ptr, d_ind, d_perm,
+                                                           lcnt, uoff, hsum);
+    rc = check_launch(ctx, "split_counts");
+    if (rc) return rc;
+  }
   // exclusive scans of the m + 1 entries (entry m is 0): offsets + totals
   rc = device_exclusive_scan<int>(ctx, lcnt, d_Lptr, (long long)m + 1, nullptr);
   if (rc) return rc;
@@ -454,8 +473,8 @@ int apspie_tc_prepare(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr, cons
     auto *kb = (unsigned *)workspace(ctx, kSlotMisc2, sizeof(unsigned) * (size_t)lnnz);
     auto *va = (int *)workspace(ctx, kSlotMisc3, sizeof(int) * (size_t)lnnz);
     if (!ka || !kb || !va) return APSPIE_ERR_OOM;
-    upper_pairs<<<tgrid(ctx, (long long)m * 32, 256), 256, 0, st>>>(m, d_ptr, d_ind, d_perm,
-                                                                    uoff, ka, va);
+    upper_pairs<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, (int)nnz, d_ptr, d_ind, d_perm,
+                                                          uoff, ka, va);
     rc = check_launch(ctx, "upper_pairs");
     if (rc) return rc;
     in_b = false;

@@ -73,3 +73,55 @@ def test_csr_transpose_matches_host(ctx, m, n):
     np.testing.assert_array_equal(tp.cpu().numpy(), c.indptr)
     np.testing.assert_array_equal(ti.cpu().numpy(), c.indices)
     np.testing.assert_array_equal(tv.cpu().numpy(), c.data)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,nnz", [(1, 1, 1), (5, 3, 31), (4000, 70, 2047), (3, 5000, 2048),
+                                     (300000, 257, 2049), (700, 300, 40961)])
+def test_csr_transpose_rows_across_tiles(ctx, m, n, nnz):
+    """Rows that span tiles of 2,048 entries (one row holds half of them), long
+    runs of empty rows, entry counts at and around a tile, 1 to 2 sort passes;
+    columns may repeat in a row (their order is then the input's)."""
+    import torch
+    rng = np.random.default_rng(nnz)
+    rows = np.sort(np.concatenate([np.full(nnz // 2, m // 2),
+                                   rng.integers(0, m, size=nnz - nnz // 2)]))
+    ind = rng.integers(0, n, size=nnz).astype(np.int32)
+    val = rng.random(nnz, dtype=np.float32)
+    ptr = np.searchsorted(rows, np.arange(m + 1)).astype(np.int32)
+    t = lambda x: torch.from_numpy(x).cuda()
+    tp, ti, tv = ap.csr_transpose(ctx, m, n, t(ptr), t(ind), t(val))
+    order = np.argsort(ind, kind="stable")
+    assert np.array_equal(tp.cpu().numpy(), np.searchsorted(ind[order], np.arange(n + 1)))
+    assert np.array_equal(ti.cpu().numpy(), rows[order])
+    assert np.array_equal(tv.cpu().numpy(), val[order])
+    _, _, ones = ap.csr_transpose(ctx, m, n, t(ptr), t(ind))
+    assert bool((ones == 1.0).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("leaves,extra", [(1, 0), (2047, 0), (2049, 64), (9000, 20000)])
+def test_tc_prepare_hub_rows_across_tiles(ctx, leaves, extra):
+    """L of a star with random edges among its leaves: the hub's row spans
+    tiles, and isolated vertices leave empty rows."""
+    import torch
+    rng = np.random.default_rng(leaves)
+    m = leaves + 50
+    hub = m // 3
+    others = np.setdiff1d(rng.permutation(m)[:leaves + 1], [hub])
+    e = np.concatenate([np.stack([np.full(len(others), hub), others]),
+                        rng.choice(others, size=(2, extra))], axis=1)
+    e = e[:, e[0] != e[1]]
+    keys = np.unique(np.concatenate([e[0] * m + e[1], e[1] * m + e[0]]))
+    rows, cols = keys // m, keys % m
+    ptr = np.searchsorted(rows, np.arange(m + 1)).astype(np.int32)
+    g = ap.DeviceGraph(m, len(cols), torch.from_numpy(ptr).cuda(),
+                       torch.from_numpy(cols.astype(np.int32)).cuda(), symmetric=True)
+    perm, lp, li = ap.tc_prepare(ctx, g)
+    want = np.empty(m, np.int64)
+    want[np.lexsort((np.arange(m), np.diff(ptr)))] = np.arange(m)
+    assert np.array_equal(perm.cpu().numpy(), want)
+    r, c = want[rows], want[cols]
+    low = np.sort((r * m + c)[c < r])
+    assert np.array_equal(lp.cpu().numpy(), np.searchsorted(low // m, np.arange(m + 1)))
+    assert np.array_equal(li.cpu().numpy(), low % m)

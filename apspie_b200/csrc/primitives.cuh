@@ -145,21 +145,66 @@ constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
 constexpr int kMaxPasses = 8;
-constexpr unsigned long long kStAgg = 1ull << 62, kStIncl = 2ull << 62;
-constexpr unsigned long long kStCountMask = (1ull << 40) - 1;
 
-// all passes' digit counts in one read of the keys
+// Status words.  32 bits for sorts of fewer than 2^27 keys: flag 2 bits, pass
+// tag 3 bits, count 27 bits; else 64 bits (flag 2, tag 22, count 40).  The
+// tag tells a pass's words from those an earlier pass left, so all passes
+// share one zeroed array.  A tile loads kWindow predecessors' words at once:
+// the look-back moves on by that many tiles per L2 round trip (about 0.35 us),
+// which bounds the tiles finished per microsecond -- with 4 words a pass over
+// 16 M pairs took 170 us whether the pairs had 8 or 12 bytes.
+template <typename S>
+struct SortStatus;
+template <>
+struct SortStatus<unsigned> {
+  static constexpr unsigned kAgg = 1u << 30, kIncl = 2u << 30, kFlags = 3u << 30;
+  static constexpr unsigned kTag = 7u << 27, kCount = (1u << 27) - 1u;
+  static constexpr int kWindow = 16;
+  __device__ __forceinline__ static unsigned tag(int pass) { return (unsigned)pass << 27; }
+  __device__ __forceinline__ static unsigned load(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+  }
+};
+template <>
+struct SortStatus<unsigned long long> {
+  static constexpr unsigned long long kAgg = 1ull << 62, kIncl = 2ull << 62, kFlags = 3ull << 62;
+  static constexpr unsigned long long kTag = 0x3FFFFFull << 40, kCount = (1ull << 40) - 1ull;
+  static constexpr int kWindow = 8;
+  __device__ __forceinline__ static unsigned long long tag(int pass) {
+    return (unsigned long long)pass << 40;
+  }
+  __device__ __forceinline__ static unsigned long long load(const unsigned long long *p) {
+    return ld_relaxed64(p);
+  }
+};
+
+// All passes' digit counts in one read of the keys, kHistKeys loads in
+// flight per thread (one at a time the kernel waited for each: 64 us for
+// 16 M 4-byte keys).
+constexpr int kHistKeys = 8;
+
 template <typename K>
 __global__ void __launch_bounds__(kSortThreads)
 radix_histograms(const K *keys, long long n, int npass, unsigned long long *ghist) {
   __shared__ unsigned hist[kMaxPasses][kRadix];
   for (int t = threadIdx.x; t < kMaxPasses * kRadix; t += blockDim.x) hist[t / kRadix][t % kRadix] = 0;
   __syncthreads();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const K k = keys[i];
+  constexpr long long kStep = (long long)kSortThreads * kHistKeys;
+  for (long long b = blockIdx.x * kStep; b < n; b += gridDim.x * kStep) {
+    K k[kHistKeys];
+#pragma unroll
+    for (int q = 0; q < kHistKeys; ++q) {
+      const long long i = b + q * kSortThreads + threadIdx.x;
+      k[q] = i < n ? keys[i] : K(0);
+    }
+    const int cnt = (int)min((long long)kHistKeys,
+                             (n - b - threadIdx.x + kSortThreads - 1) / kSortThreads);
     for (int p = 0; p < npass; ++p)
-      atomicAdd(&hist[p][(unsigned)(k >> (p * kRadixBits)) & (kRadix - 1)], 1u);
+#pragma unroll
+      for (int q = 0; q < kHistKeys; ++q)
+        if (q < cnt) atomicAdd(&hist[p][(unsigned)(k[q] >> (p * kRadixBits)) & (kRadix - 1)], 1u);
   }
   __syncthreads();
   for (int t = threadIdx.x; t < npass * kRadix; t += blockDim.x) {
@@ -184,12 +229,11 @@ __global__ void radix_digit_offsets(unsigned long long *ghist, int npass) {
 // Polls of a look-back wait before it gives up (a predecessor normally
 // publishes within microseconds; about half a second with the back-off).
 constexpr unsigned kLookbackSpinLimit = 1u << 20;
-constexpr int kLookbackWindow = 4;  // predecessors whose status words are loaded at once
 
-template <typename K, typename V>
+template <typename K, typename V, typename S>
 __global__ void __launch_bounds__(kSortThreads, 3)
 radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, long long n,
-               int pass, const unsigned long long *goff, unsigned long long *status,
+               int pass, const unsigned long long *goff, S *status,
                unsigned *tile_counter, int *err, int *gaveup) {
   constexpr int kWarps = kSortThreads / 32;
   static_assert(sizeof(V) <= sizeof(K), "values are staged in the keys' shared array");
@@ -200,7 +244,7 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
   __shared__ unsigned char sdig[kSortTile];
   __shared__ unsigned whist[kWarps][kRadix];
   __shared__ unsigned long long gbase[kRadix];
-  __shared__ unsigned long long s_scan[33];
+  __shared__ unsigned s_scan[33];
   __shared__ unsigned s_tile;
   __shared__ int s_withhold;
   // the tile's values, copied in by cp.async while the keys are ranked
@@ -209,7 +253,9 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
   V *svin = reinterpret_cast<V *>(sort_dyn);
   const int lane = lane_id(), w = warp_in_block();
   const int shift = pass * kRadixBits;
-  const unsigned long long tag = (unsigned long long)(pass + 1) << 40;
+  using St = SortStatus<S>;
+  constexpr int kWindow = St::kWindow;
+  const S tag = St::tag(pass);
   if (threadIdx.x == 0) {
     s_tile = atomicAdd(tile_counter, 1u);
     // test hook (apspie_debug_inject): err[1] set makes tile 0 of the next
@@ -273,40 +319,42 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
     whist[ww][d] = run;
     run += c;
   }
-  unsigned long long tot;
-  const unsigned long long loc = block_excl_scan((unsigned long long)run, s_scan, &tot);
-  unsigned long long *mine = status + (size_t)tile * kRadix + d;
-  unsigned long long excl = 0;
+  unsigned tot;
+  const unsigned loc = block_excl_scan(run, s_scan, &tot);
+  S *mine = status + (size_t)tile * kRadix + d;
+  S excl = 0;
   if (tile == 0) {
-    if (!s_withhold) __stcg(mine, kStIncl | tag | (unsigned long long)run);
+    if (!s_withhold) __stcg(mine, St::kIncl | tag | (S)run);
   } else {
-    __stcg(mine, kStAgg | tag | (unsigned long long)run);
-    // Look back kLookbackWindow predecessors at a time (their status words
-    // loaded together, relaxed: a word's count is all that is read), adding
-    // counts from the nearest one back until an inclusive word; a word not
-    // yet published stops the window and is polled again.
+    __stcg(mine, St::kAgg | tag | (S)run);
+    // Look back kWindow predecessors at a time (their status words loaded
+    // together, relaxed: a word's count is all that is read), adding counts
+    // from the nearest one back until an inclusive word; a word not yet
+    // published stops the window and is polled again.
     long long t = (long long)tile - 1;
     unsigned spins = 0;
     while (t >= 0) {
-      unsigned long long sv[kLookbackWindow];
+      S sv[kWindow];
 #pragma unroll
-      for (int k = 0; k < kLookbackWindow; ++k)
-        sv[k] = t - k >= 0 ? ld_relaxed64(status + (size_t)(t - k) * kRadix + d) : 0ull;
+      for (int k = 0; k < kWindow; ++k)
+        sv[k] = t - k >= 0 ? St::load(status + (size_t)(t - k) * kRadix + d) : S(0);
       bool done = false, stalled = false;
+      int adv = 0;
 #pragma unroll
-      for (int k = 0; k < kLookbackWindow; ++k) {
-        if (done || stalled || t < 0) continue;
-        const unsigned long long w = sv[k];
-        if ((w & (0x3FFFFFull << 40)) != tag || (w >> 62) == 0ull) {
-          stalled = true;
+      for (int k = 0; k < kWindow; ++k) {
+        if (done || stalled) continue;
+        const S x = sv[k];
+        if ((x & St::kFlags) == 0 || (x & St::kTag) != tag) {
+          stalled = true;  // not published (or before tile 0, when t < k)
           continue;
         }
-        excl += w & kStCountMask;
-        if ((w >> 62) == 2ull) done = true;  // inclusive: everything before is in it
-        else --t;
+        excl += x & St::kCount;
+        ++adv;
+        if ((x & St::kFlags) == St::kIncl) done = true;  // everything before is in it
       }
       if (done) break;
-      if (stalled) {
+      t -= adv;
+      if (stalled && t >= 0) {
         // a predecessor has not published: give up after kLookbackSpinLimit
         // polls, or at once when another tile of this sort already gave up
         // (checked every 256; *gaveup is zeroed with the sort's status words)
@@ -319,10 +367,10 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
         if ((spins & 15u) == 0u) __nanosleep(64);
       }
     }
-    __stcg(mine, kStIncl | tag | (excl + run));
+    __stcg(mine, St::kIncl | tag | (S)(excl + run));
   }
-  gbase[d] = goff[pass * kRadix + d] + excl - loc;
-  for (int ww = 0; ww < kWarps; ++ww) whist[ww][d] += (unsigned)loc;
+  gbase[d] = goff[pass * kRadix + d] + (unsigned long long)excl - loc;
+  for (int ww = 0; ww < kWarps; ++ww) whist[ww][d] += loc;
   __syncthreads();
   // tile position of every key: its digit's start + the warps before it + its rank
 #pragma unroll
@@ -413,21 +461,23 @@ int device_radix_sort(apspie_context *ctx, K *ka, V *va, K *kb, V *vb, long long
     return set_error(ctx, APSPIE_ERR_OVERFLOW, "radix sort: %lld keys of %d bits", n, bits);
   const long long tiles = (n + kSortTile - 1) / kSortTile;
   // [histograms: npass x 256 u64][tile counters: 8 x u32, padded; the
-  // sort's give-up word at u32 15][status: tiles x 256 u64]
+  // sort's give-up word at u32 15][status: tiles x 256 words]
   const size_t hist_bytes = sizeof(unsigned long long) * kMaxPasses * kRadix;
   const size_t head = hist_bytes + 64;
-  const size_t bytes = head + sizeof(unsigned long long) * (size_t)tiles * kRadix;
+  const bool narrow = n < (1ll << 27);
+  const size_t bytes = head + (narrow ? 4 : 8) * (size_t)tiles * kRadix;
   int *err = radix_sort_err(ctx);
   auto *ws = (unsigned char *)workspace(ctx, kSlotSortHist, bytes);
   if (!ws || !err) return APSPIE_ERR_OOM;
   auto *ghist = (unsigned long long *)ws;
   auto *counters = (unsigned *)(ws + hist_bytes);
-  auto *status = (unsigned long long *)(ws + head);
+  void *status = ws + head;
   cudaStream_t st = ctx->stream;
   // zero the histograms, counters and every status word
   cudaMemsetAsync(ws, 0, bytes, st);
-  const int hgrid = (int)std::max(1ll, std::min((n + kSortThreads * 8 - 1) / (kSortThreads * 8),
-                                                (long long)ctx->num_sms * 4));
+  const int hgrid = (int)std::max(
+      1ll, std::min((n + kSortThreads * kHistKeys - 1) / (kSortThreads * kHistKeys),
+                    (long long)ctx->num_sms * 8));
   radix_histograms<K><<<hgrid, kSortThreads, 0, st>>>(kfirst ? kfirst : ka, n, npass, ghist);
   radix_digit_offsets<kRadix><<<1, kRadix, 0, st>>>(ghist, npass);
   int rc = check_launch(ctx, "radix_histograms", 2);
@@ -435,14 +485,25 @@ int device_radix_sort(apspie_context *ctx, K *ka, V *va, K *kb, V *vb, long long
   K *kin = ka, *kout = kb;
   V *vin = va, *vout = vb;
   const size_t vdyn = va ? sizeof(V) * kSortTile : 0;
-  if (vdyn)
-    cudaFuncSetAttribute(radix_onesweep<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)vdyn);
+  auto pass32 = radix_onesweep<K, V, unsigned>;
+  auto pass64 = radix_onesweep<K, V, unsigned long long>;
+  if (vdyn) {
+    cudaFuncSetAttribute(pass32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vdyn);
+    cudaFuncSetAttribute(pass64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vdyn);
+  }
   for (int p = 0; p < npass; ++p) {
     const bool first = kfirst && p == 0;
-    radix_onesweep<K, V><<<(unsigned)tiles, kSortThreads, vdyn, st>>>(
-        first ? kfirst : kin, first ? nullptr : vin, kout, vout, n, p, ghist, status,
-        counters + p, err, (int *)(counters + 15));
+    const K *kp = first ? kfirst : kin;
+    const V *vp = first ? nullptr : vin;
+    int *gave = (int *)(counters + 15);
+    if (narrow)
+      pass32<<<(unsigned)tiles, kSortThreads, vdyn, st>>>(kp, vp, kout, vout, n, p, ghist,
+                                                          (unsigned *)status, counters + p, err,
+                                                          gave);
+    else
+      pass64<<<(unsigned)tiles, kSortThreads, vdyn, st>>>(kp, vp, kout, vout, n, p, ghist,
+                                                          (unsigned long long *)status,
+                                                          counters + p, err, gave);
     rc = check_launch(ctx, "radix_onesweep");
     if (rc) return rc;
     std::swap(kin, kout);

@@ -347,7 +347,7 @@ __device__ __forceinline__ void msbfs_relax_n(BatchJob *j, const unsigned long l
 #pragma unroll
   for (int r = 0; r < K; ++r) nb[r] = u[r] >= 0 ? f[r] & ~__ldcg(j->visited + u[r]) : 0ull;
 #pragma unroll
-  for (int r = 0; r < K; ++r) old[r] = nb[r] ? atomicOr(j->visited + u[r], nb[r]) : ~0ull;
+  for (int r = 0; r < K; ++r) old[r] = or_if(nb[r] != 0, j->visited + u[r], nb[r], ~0ull);
   unsigned long long mine[K], fo[K];
 #pragma unroll
   for (int r = 0; r < K; ++r) {
@@ -358,7 +358,7 @@ __device__ __forceinline__ void msbfs_relax_n(BatchJob *j, const unsigned long l
     }
   }
 #pragma unroll
-  for (int r = 0; r < K; ++r) fo[r] = mine[r] ? atomicOr(Fn + u[r], mine[r]) : 1ull;
+  for (int r = 0; r < K; ++r) fo[r] = or_if(mine[r] != 0, Fn + u[r], mine[r], 1ull);
 #pragma unroll
   for (int r = 0; r < K; ++r) found[r] = mine[r] != 0ull && fo[r] == 0ull;
 }
@@ -554,7 +554,7 @@ __device__ __forceinline__ bool mssp_relax(BatchJob *j, int ue, unsigned we, int
   // and the ballots need not wait for the atomics
 #pragma unroll
   for (int i = 0; i < kSsspSlots; ++i)
-    if (act[i] && nd[i] < cur[i]) atomicMin(dist + (size_t)uu[i] * sw + src, nd[i]);
+    min_if(act[i] && nd[i] < cur[i], dist + (size_t)uu[i] * sw + src, nd[i]);
   unsigned mybal = 0;
 #pragma unroll
   for (int i = 0; i < kSsspSlots; ++i) {

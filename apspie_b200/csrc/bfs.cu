@@ -19,6 +19,14 @@
 // than m/beta vertices.  Discovered vertices are appended to the next queue
 // with one atomic per warp; the per-level counters rotate over three slots so
 // no block reads a counter while another resets it.
+//
+// Graphs of few edges per vertex (meshes, road networks) have hundreds of
+// thin levels, and each costs the whole grid 7 us or more whatever its size
+// (barrier 1.4 us, the rest the hand-over of the frontier through L2).  One
+// cluster of blocks runs their levels first (bfs_thin): the frontier in
+// distributed shared memory, one hardware cluster barrier per level.  The
+// persistent kernel takes over at the first level that is not thin.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -33,6 +41,26 @@ namespace apspie {
 namespace {
 
 constexpr int kBfsThreads = 512;
+
+// Thin levels: at most kThinEdges out-edges, or kThinHubEdges when a vertex
+// has more than kBigDeg of them (a warp takes all of a vertex's edges).  A
+// single SM gets through one scattered edge per 4.5 cycles (1024 x 1024 grid
+// on one block: 16,800 cycles a level of 1,020 vertices), so kThinBlocks SMs
+// need about 3.5 us for the largest thin level, half of what the whole grid
+// needs for the smallest.
+constexpr int kThinThreads = 512;
+constexpr int kThinBlocks = 16;    // blocks of the cluster (8 where 16 do not fit)
+constexpr int kThinQueue = 4096;   // frontier entries a block can append per level
+constexpr unsigned kThinEdges = 24576;
+constexpr unsigned kThinHubEdges = 4096;
+// Graphs of at most this many edges per vertex start with bfs_thin.  Denser
+// ones have a few levels in all, and the extra launches (about 4 us) cost
+// more than their first and last levels gain.
+constexpr long long kThinMeanDegree = 5;
+
+__device__ __forceinline__ bool thin_fits(bool hub, unsigned long long mf) {
+  return mf <= (hub ? kThinHubEdges : kThinEdges);
+}
 constexpr int kProbe = 1;         // in-neighbours a lane probes per round in a pull level
 constexpr int kTraceLevels = 64;  // levels recorded in the per-run trace
 
@@ -70,6 +98,11 @@ struct BfsState {
   unsigned long long reached;
   unsigned long long edges;
   unsigned long long t_start;
+  // where the persistent kernel starts after a separate initialisation: the
+  // level of the frontier in c[0] and the totals before it
+  int start_level;
+  unsigned start_over;  // bfs_thin: vertices found past a block's kThinQueue
+  unsigned long long start_prev_nf, start_reached, start_explored;
   LevelTrace trace[kTraceLevels];
 };
 
@@ -79,8 +112,9 @@ struct BfsVisit {
   int next;
   int32_t *depth;
   __device__ __forceinline__ bool two_way() const { return false; }
-  __device__ __forceinline__ bool check(unsigned, int, int u, unsigned &) const {
-    return __ldcg(depth + u) == -1;
+  __device__ __forceinline__ bool check(bool on, unsigned, int, int u, unsigned &) const {
+    const int du = on ? __ldcg(depth + u) : 0;
+    return du == -1;
   }
   template <int N>
   __device__ __forceinline__ void commit_n(const unsigned (&)[N], const int (&)[N],
@@ -88,7 +122,7 @@ struct BfsVisit {
                                            const bool (&ok)[N], int (&cls)[N]) const {
     int old[N];
 #pragma unroll
-    for (int r = 0; r < N; ++r) old[r] = ok[r] ? atomicCAS(depth + u[r], -1, next) : 0;
+    for (int r = 0; r < N; ++r) old[r] = cas_if(ok[r], depth + u[r], -1, next, 0);
 #pragma unroll
     for (int r = 0; r < N; ++r) cls[r] = (ok[r] && old[r] == -1) ? 1 : 0;
   }
@@ -116,6 +150,9 @@ __device__ __forceinline__ void bfs_clear(int m, int src, int32_t *depth,
       st->pull_levels = 0;
       st->reached = 0;
       st->edges = 0;
+      st->start_level = 0;
+      st->start_over = 0;
+      st->start_prev_nf = st->start_reached = st->start_explored = 0;
     }
     for (int i = threadIdx.x; i < kTraceLevels; i += blockDim.x) {
       st->trace[i].queued = 0;
@@ -130,6 +167,240 @@ __global__ void bfs_init(int m, int src, int32_t *depth, const int *__restrict__
                          int *queue, int2 *chunks, BfsState *st) {
   bfs_clear(m, src, depth, ptr, queue, chunks, st, true);
   if (blockIdx.x == 0 && threadIdx.x == 0) st->par = -1;
+}
+
+// Appends the found candidates (4 per lane) to the block's next frontier, or
+// past kThinQueue to `over`; adds their out-degrees to *edges and flags a hub.
+// Warp-collective.
+__device__ __forceinline__ void thin_append(const bool (&found)[4], const int (&u)[4],
+                                            const int *__restrict__ ptr, int *q, unsigned *count,
+                                            int *over, unsigned *nover,
+                                            unsigned long long *edges, bool *hub) {
+  unsigned mask[4], tot = 0;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    mask[r] = __ballot_sync(kFull, found[r]);
+    tot += __popc(mask[r]);
+  }
+  if (!tot) return;
+  // the offsets of all candidates in flight while the slots are reserved
+  int d[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) d[r] = found[r] ? __ldg(ptr + u[r] + 1) - __ldg(ptr + u[r]) : 0;
+  unsigned at = 0;
+  if (lane_id() == 0) at = atomicAdd(count, tot);
+  at = __shfl_sync(kFull, at, 0);
+  const unsigned below = (1u << lane_id()) - 1u;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const unsigned i = at + __popc(mask[r] & below);
+    if (found[r]) {
+      if (i < (unsigned)kThinQueue) q[i] = u[r];
+      else over[atomicAdd(nover, 1u)] = u[r];
+    }
+    at += __popc(mask[r]);
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    *edges += (unsigned long long)d[r];
+    *hub |= d[r] > kBigDeg;
+  }
+}
+
+// What a block found in a level, told to every block of the cluster.
+struct __align__(16) ThinInfo {
+  unsigned n;      // entries of its next frontier
+  unsigned flags;  // 1: one of them is a hub, 2: some are past kThinQueue
+  unsigned long long edges;
+};
+
+// The levels from the source on, by one cluster, until the frontier is empty
+// or not thin, the next level would pull or is the last one.  Every block
+// appends what it finds to its own shared queue and tells the others its
+// count; the blocks then take equal shares of the queues laid end to end,
+// read through distributed shared memory.  Bound by the chain of a level:
+// remote queue entry, offsets, indices, CAS, append, cluster barrier, and by
+// the scattered accesses of one SM per share.  Levels of 24 to 240 vertices
+// of the 1024 x 1024 grid take 2.7 to 3.2 us (7.2 to 7.9 by the whole grid),
+// its BFS 5.3 ms instead of 13.2.  Leaves the frontier in (qa, ca, st->c[0])
+// for the persistent kernel.
+__global__ void __launch_bounds__(kThinThreads)
+bfs_thin(long long nnz, const int *__restrict__ ptr, const int *__restrict__ ind, int32_t *depth,
+         int src, int *qa, int2 *ca, int *over, BfsState *st, int max_levels, int alpha, int mode) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ int s_q[2][kThinQueue];
+  __shared__ ThinInfo s_info[2][kThinBlocks];
+  __shared__ unsigned s_n[3], s_hub[3];
+  __shared__ unsigned long long s_e[3];
+  const int lane = lane_id(), w = warp_in_block();
+  const unsigned rank = cluster.block_rank(), nb = cluster.num_blocks();
+  constexpr unsigned kWarps = kThinThreads / 32;
+  const int deg0 = __ldg(ptr + src + 1) - __ldg(ptr + src);
+  unsigned long long nf = 1, mf = (unsigned long long)deg0, prev_nf = 0, reached = 0,
+                     explored = 0;
+  bool hub = deg0 > kBigDeg, spilt = false;
+  int L = 0;
+  auto stop = [&]() {
+    return nf == 0 || spilt || !thin_fits(hub, mf) || (max_levels > 0 && L + 1 >= max_levels) ||
+           mode == 2 ||
+           (mode == 0 && (long long)mf * alpha > nnz - (long long)(explored + mf));
+  };
+  if (rank == 0 && threadIdx.x == 0) st->t_start = globaltimer();
+  if (stop()) return;  // the same for every block; bfs_init's frontier stands
+  if (threadIdx.x < 3) {
+    s_n[threadIdx.x] = 0;
+    s_hub[threadIdx.x] = 0;
+    s_e[threadIdx.x] = 0;
+  }
+  if (threadIdx.x < kThinBlocks) s_info[0][threadIdx.x] = ThinInfo{threadIdx.x == 0 ? 1u : 0u, 0, 0};
+  if (threadIdx.x == 0) s_q[0][0] = src;
+  cluster.sync();
+  // lane b: block b's entries of the current frontier and those before them
+  unsigned have = lane < (int)nb ? s_info[0][lane].n : 0u;
+  unsigned first = (unsigned)warp_incl_scan((int)have) - have;
+  int p = 0, step = 0;
+  for (;; ++step) {
+    reached += nf;
+    explored += mf;
+    const int a = (step + 1) % 3;
+    const int *qc = s_q[p];
+    int *qn = s_q[p ^ 1];
+    const unsigned lo = (unsigned)(nf * rank / nb), hi = (unsigned)(nf * (rank + 1) / nb);
+    const unsigned cnt = hi - lo;
+    unsigned long long edges = 0;
+    bool hubs = false;
+    // a small share is spread over all warps
+    const unsigned per = cnt >= (unsigned)kThinThreads ? 32u : (cnt + kWarps - 1u) / kWarps;
+    for (unsigned base = 0; base < cnt; base += kThinThreads) {
+      const unsigned i = base + (unsigned)w * per + (unsigned)lane;
+      const bool on = (unsigned)lane < per && i < cnt;
+      if (!__any_sync(kFull, on)) continue;
+      // the block that holds entry lo + i: the last with first <= lo + i
+      unsigned b = 0;
+#pragma unroll
+      for (unsigned h = kThinBlocks / 2; h > 0; h >>= 1) {
+        const unsigned f = __shfl_sync(kFull, first, b + h);
+        if (b + h < nb && f <= lo + i) b += h;
+      }
+      const unsigned fb = __shfl_sync(kFull, first, b);
+      int s = 0, d = 0;
+      if (on) {
+        const int v = *cluster.map_shared_rank(qc + (lo + i - fb), b);
+        s = __ldg(ptr + v);
+        d = __ldg(ptr + v + 1) - s;
+      }
+      if (!__any_sync(kFull, d > 4)) {
+        // a vertex per lane
+        int u[4], old[4];
+        bool f[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) u[r] = r < d ? __ldg(ind + s + r) : -1;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) old[r] = cas_if(u[r] >= 0, depth + u[r], -1, L + 1, 0);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) f[r] = u[r] >= 0 && old[r] == -1;
+        thin_append(f, u, ptr, qn, &s_n[a], over, &st->start_over, &edges, &hubs);
+      } else {
+        // the warp's edges dealt over its lanes
+        const int incl = warp_incl_scan(d), excl = incl - d;
+        const int total = __shfl_sync(kFull, incl, 31);
+        for (int e0 = 0; e0 < total; e0 += 128) {
+          int u[4], old[4];
+          bool f[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const int e = e0 + r * 32 + lane;
+            const int owner = warp_owner(excl, e);
+            const int at = __shfl_sync(kFull, s - excl, owner) + e;
+            u[r] = e < total ? __ldg(ind + at) : -1;
+          }
+#pragma unroll
+          for (int r = 0; r < 4; ++r) old[r] = u[r] >= 0 ? __ldcg(depth + u[r]) : 0;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) f[r] = old[r] == -1;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) old[r] = cas_if(f[r], depth + u[r], -1, L + 1, 0);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) f[r] = f[r] && old[r] == -1;
+          thin_append(f, u, ptr, qn, &s_n[a], over, &st->start_over, &edges, &hubs);
+        }
+      }
+    }
+    // 24 bits at a time through the warp's 32-bit adder
+    const unsigned e_lo = __reduce_add_sync(kFull, (unsigned)(edges & 0xffffffull));
+    const unsigned e_hi = __reduce_add_sync(kFull, (unsigned)(edges >> 24));
+    hubs = __any_sync(kFull, hubs);
+    if (lane == 0) {
+      if (e_lo | e_hi) atomicAdd(&s_e[a], ((unsigned long long)e_hi << 24) + e_lo);
+      if (hubs) s_hub[a] = 1;
+    }
+    __syncthreads();
+    if (w == 0 && lane < (int)nb) {
+      const unsigned n = s_n[a];
+      *cluster.map_shared_rank(&s_info[p ^ 1][rank], lane) =
+          ThinInfo{min(n, (unsigned)kThinQueue),
+                   s_hub[a] | (n > (unsigned)kThinQueue ? 2u : 0u), s_e[a]};
+    }
+    if (threadIdx.x == kThinThreads - 1) {
+      // the slots the next step adds to; last read two barriers ago
+      const int z = (step + 2) % 3;
+      s_n[z] = 0;
+      s_hub[z] = 0;
+      s_e[z] = 0;
+      if (rank == 0 && L < kTraceLevels) {
+        const unsigned long long t = globaltimer();
+        LevelTrace &tr = st->trace[L];
+        tr.mode = 1;
+        tr.nf = nf;
+        tr.mf = mf;
+        tr.expanded = mf;
+        tr.t_first = tr.t_last = tr.t_end = t;
+      }
+    }
+    cluster.sync();
+    ThinInfo in{0, 0, 0};
+    if (lane < (int)nb) in = s_info[p ^ 1][lane];
+    have = in.n;
+    const unsigned incl = (unsigned)warp_incl_scan((int)have);
+    first = incl - have;
+    prev_nf = nf;
+    nf = __shfl_sync(kFull, incl, 31);
+    mf = ((unsigned long long)__reduce_add_sync(kFull, (unsigned)(in.edges >> 24)) << 24) +
+         __reduce_add_sync(kFull, (unsigned)(in.edges & 0xffffffull));
+    const unsigned flags = __reduce_or_sync(kFull, in.flags);
+    hub = (flags & 1u) != 0;
+    spilt = (flags & 2u) != 0;
+    ++L;
+    p ^= 1;
+    if (stop()) break;
+  }
+  // the frontier in the persistent kernel's form: queue and big list
+  LevelCounters *c0 = &st->c[0];
+  if (rank == 0 && threadIdx.x == 0) {
+    *c0 = LevelCounters{0ull, 0, 0, 0ull};
+    c0->edges = mf;
+    st->start_level = L;
+    st->start_prev_nf = prev_nf;
+    st->start_reached = reached;
+    st->start_explored = explored;
+  }
+  cluster.sync();
+  const unsigned mine = __shfl_sync(kFull, have, rank);
+  const unsigned nover = rank == 0 && spilt ? __ldcg(&st->start_over) : 0u;
+  for (unsigned base = 0; base < mine + nover; base += kThinThreads) {
+    const unsigned i = base + threadIdx.x;
+    const int v = i < mine ? s_q[p][i] : (i < mine + nover ? __ldcg(over + (i - mine)) : -1);
+    const int d = v >= 0 ? __ldg(ptr + v + 1) - __ldg(ptr + v) : 0;
+    const unsigned slot = warp_append(v >= 0 && d <= kBigDeg, &c0->q);
+    if (v >= 0 && d <= kBigDeg) qa[slot] = v;
+    if (d > kBigDeg) {
+      // one word for both, so that list order is chunk order
+      const unsigned nc = (unsigned)((d + kChunk - 1) / kChunk);
+      const unsigned long long at = atomicAdd(&c0->bc, ((unsigned long long)nc << 32) | 1ull);
+      ca[bc_big(at)] = make_int2(v, (int)bc_chunks(at));
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kBfsThreads, 3)
@@ -169,16 +440,23 @@ bfs_persistent(int m, long long nnz, const int *__restrict__ ptr, const int *__r
     bfs_clear(m, src, depth, ptr, qa, ca, st, false);
     if (!grid_barrier(bar, err)) return;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->t_start = globaltimer();
   bool pull = false;
   int pull_levels = 0;
   unsigned long long prev_nf = 0;
   unsigned long long reached = 0, explored = 0;
   int L = 0;
-  for (;; ++L) {
-    LevelCounters *cur = &st->c[L % 3];
-    LevelCounters *nxt = &st->c[(L + 1) % 3];
-    LevelCounters *clr = &st->c[(L + 2) % 3];
+  if (init_par < 0) {
+    L = st->start_level;
+    prev_nf = st->start_prev_nf;
+    reached = st->start_reached;
+    explored = st->start_explored;
+  }
+  if (L == 0 && blockIdx.x == 0 && threadIdx.x == 0) st->t_start = globaltimer();
+  // ci counts this launch's levels
+  for (int ci = 0;; ++ci, ++L) {
+    LevelCounters *cur = &st->c[ci % 3];
+    LevelCounters *nxt = &st->c[(ci + 1) % 3];
+    LevelCounters *clr = &st->c[(ci + 2) % 3];
     if (threadIdx.x == 0) {
       const unsigned long long bc = __ldcg(&cur->bc);
       s_q = __ldcg(&cur->q);
@@ -191,7 +469,7 @@ bfs_persistent(int m, long long nnz, const int *__restrict__ ptr, const int *__r
       s_next = 0;
       if (blockIdx.x == 0) {
         *clr = LevelCounters{0ull, 0, 0, 0ull};
-        st->comp[(L + 1) & 1] = LevelCounters{0ull, 0, 0, 0ull};
+        st->comp[(ci + 1) & 1] = LevelCounters{0ull, 0, 0, 0ull};
       }
     }
     __syncthreads();
@@ -216,10 +494,10 @@ bfs_persistent(int m, long long nnz, const int *__restrict__ ptr, const int *__r
     } else if ((long long)nf * beta < (long long)m) {
       pull = false;
     }
-    int *qin = (L & 1) ? qb : qa;
-    int *qout = (L & 1) ? qa : qb;
-    int2 *cin = (L & 1) ? cb : ca;
-    int2 *cout = (L & 1) ? ca : cb;
+    int *qin = (ci & 1) ? qb : qa;
+    int *qout = (ci & 1) ? qa : qb;
+    int2 *cin = (ci & 1) ? cb : ca;
+    int2 *cout = (ci & 1) ? ca : cb;
     const int next = L + 1;
 
     if (!pull) {
@@ -248,16 +526,16 @@ bfs_persistent(int m, long long nnz, const int *__restrict__ ptr, const int *__r
             bool f[1] = {bits != 0u};
             int u[1] = {f[0] ? (int)(gw * 32u) + __ffs(bits) - 1 : 0};
             bits &= bits - 1u;
-            discover_n<1, false>(f, u, ptr, qin, cin, &st->comp[L & 1], acc);
+            discover_n<1, false>(f, u, ptr, qin, cin, &st->comp[ci & 1], acc);
             if (lane == 0 && L < kTraceLevels)
               atomicAdd(&st->trace[L].queued, (unsigned long long)__popc(fm));
           }
         }
-        flush_acc(acc, &st->comp[L & 1]);
+        flush_acc(acc, &st->comp[ci & 1]);
         if (!grid_barrier(bar, err)) return;
         if (threadIdx.x == 0) {
-          const unsigned long long bc = __ldcg(&st->comp[L & 1].bc);
-          s_q = __ldcg(&st->comp[L & 1].q);
+          const unsigned long long bc = __ldcg(&st->comp[ci & 1].bc);
+          s_q = __ldcg(&st->comp[ci & 1].q);
           s_chunks = bc_chunks(bc);
           s_nbig = bc_big(bc);
         }
@@ -437,6 +715,35 @@ int bfs_grid(apspie_context *ctx) {
   return occupancy_grid(ctx, (const void *)bfs_persistent, kBfsThreads);
 }
 
+// Blocks of bfs_thin's cluster on a device: kThinBlocks, or 8 where a
+// cluster that large does not fit, or 0 where none does; asked once.
+int thin_blocks(int device) {
+  constexpr int kDevices = 64;
+  static std::mutex mu;
+  static int known[kDevices];  // 0: not asked, else blocks + 1
+  if (device < 0 || device >= kDevices) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  if (known[device]) return known[device] - 1;
+  cudaFuncSetAttribute(bfs_thin, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  int found = 0;
+  for (int nb = kThinBlocks; nb >= 8 && !found; nb /= 2) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)nb;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)nb);
+    cfg.blockDim = dim3(kThinThreads);
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, bfs_thin, &cfg) == cudaSuccess && fit > 0) found = nb;
+  }
+  cudaGetLastError();
+  known[device] = found + 1;
+  return found;
+}
+
 }  // namespace
 }  // namespace apspie
 
@@ -479,14 +786,34 @@ int apspie_bfs(apspie_ctx ctx, int src, int64_t nnz, int m, const int *d_ptr,
   long long nnz_ll = (long long)nnz;
   int alpha = ctx->bfs_alpha, beta = ctx->bfs_beta, mode = ctx->bfs_mode;
   if (!d_tptr) mode = 1;  // no in-adjacency: push only
-  int par = ctx->bfs_par;
+  const int thin = (long long)nnz <= kThinMeanDegree * m && mode != 2 ? thin_blocks(ctx->device) : 0;
+  if (thin) {
+    bfs_init<<<std::min((m + 255) / 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+        m, src, d_depth, d_ptr, qa, ca, st);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)thin;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)thin);
+    cfg.blockDim = dim3(kThinThreads);
+    cfg.stream = ctx->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t et = cudaLaunchKernelEx(&cfg, bfs_thin, nnz_ll, d_ptr, d_ind, d_depth, src, qa, ca,
+                                        qb, st, max_levels, alpha, mode);
+    if (et != cudaSuccess) return check_cuda(ctx, et, "bfs_thin");
+    int rc = check_launch(ctx, "bfs_thin", 2);
+    if (rc) return rc;
+  }
+  int par = thin ? -1 : ctx->bfs_par;
   void *args[] = {&m,  &nnz_ll, (void *)&d_ptr, (void *)&d_ind, (void *)&d_tptr, (void *)&d_tind,
                   &d_depth, &qa, &qb, &ca, &cb, &st, &max_levels, &alpha, &beta, &mode,
                   &gmask, &src, &par};
   cudaError_t e = cudaLaunchCooperativeKernel((const void *)bfs_persistent, dim3(grid),
                                               dim3(kBfsThreads), args, 0, ctx->stream);
   if (e != cudaSuccess) return check_cuda(ctx, e, "bfs_persistent");
-  ctx->bfs_par ^= 1;
+  if (!thin) ctx->bfs_par ^= 1;
   ctx->launches += 1;
   return APSPIE_OK;
 }

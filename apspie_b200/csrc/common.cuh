@@ -87,6 +87,45 @@ __device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long l
   return v;
 }
 
+// Atomics of the lanes with `on` set, as one predicated instruction each: a
+// batch of them is in flight together.  `on ? atomicCAS(..) : x` becomes a
+// branch around the atomic, and the next one of the batch is issued only
+// when this one has returned (four independent CAS and an append: 4,280
+// cycles with branches, 2,170 predicated).  The lanes without `on` get
+// `other`.
+__device__ __forceinline__ int cas_if(bool on, int *p, int cmp, int val, int other) {
+  int r;
+  asm volatile(
+      "{ .reg .pred q; setp.ne.s32 q, %4, 0; mov.b32 %0, %5;\n"
+      "@q atom.relaxed.gpu.global.cas.b32 %0, [%1], %2, %3; }"
+      : "=&r"(r) : "l"(p), "r"(cmp), "r"(val), "r"((int)on), "r"(other) : "memory");
+  return r;
+}
+__device__ __forceinline__ int exch_if(bool on, int *p, int val, int other) {
+  int r;
+  asm volatile(
+      "{ .reg .pred q; setp.ne.s32 q, %3, 0; mov.b32 %0, %4;\n"
+      "@q atom.relaxed.gpu.global.exch.b32 %0, [%1], %2; }"
+      : "=&r"(r) : "l"(p), "r"(val), "r"((int)on), "r"(other) : "memory");
+  return r;
+}
+__device__ __forceinline__ unsigned long long or_if(bool on, unsigned long long *p,
+                                                    unsigned long long val,
+                                                    unsigned long long other) {
+  unsigned long long r;
+  asm volatile(
+      "{ .reg .pred q; setp.ne.s32 q, %3, 0; mov.b64 %0, %4;\n"
+      "@q atom.relaxed.gpu.global.or.b64 %0, [%1], %2; }"
+      : "=&l"(r) : "l"(p), "l"(val), "r"((int)on), "l"(other) : "memory");
+  return r;
+}
+__device__ __forceinline__ void min_if(bool on, unsigned *p, unsigned val) {
+  asm volatile(
+      "{ .reg .pred q; setp.ne.s32 q, %2, 0;\n"
+      "@q red.relaxed.gpu.global.min.u32 [%0], %1; }"
+      :: "l"(p), "r"(val), "r"((int)on) : "memory");
+}
+
 // Grid barrier for cooperatively launched kernels, on one 64-bit arrival
 // counter that only grows (bar must be 8-byte aligned and zero at launch):
 // the k-th barrier of every block waits until the counter reaches

@@ -18,7 +18,8 @@
 // Rounds are issued kUnroll at a time: all index loads of the batch, then all
 // visitor checks (the random loads), then the atomic commits, so each lane
 // keeps several independent loads in flight.  A visitor provides
-//   check(payload, k, u, &aux) -> bool   (plain loads only)
+//   check(on, payload, k, u, &aux) -> bool   (plain loads only, selected by
+//     `on` and not branched around, so that a batch's are in flight together)
 //   commit_n<N>(payload[], k[], u[], aux[], ok[], cls[])   (the atomics of
 //     the N candidates for which ok[r], issued together -- each class of
 //     atomic for all N before the next class -- so a batch waits for one or
@@ -363,7 +364,7 @@ __device__ __forceinline__ void expand_chunks(const int *__restrict__ ptr,
         }
 #pragma unroll
         for (int r = 0; r < kUnroll; ++r)
-          ok[r] = uu[r] >= 0 && visit.check(pay, k0 + r * 32 + lane, uu[r], aux[r]);
+          ok[r] = visit.check(uu[r] >= 0, pay, k0 + r * 32 + lane, uu[r], aux[r]);
         bool f[kUnroll], g[kUnroll];
         int cls[kUnroll], kk[kUnroll];
         unsigned pp[kUnroll];
@@ -473,7 +474,7 @@ __device__ __forceinline__ void expand_push(const int *__restrict__ ptr,
       for (int r = 0; r < kUnroll; ++r) uu[r] = kk[r] >= 0 ? __ldg(ind + kk[r]) : -1;
 #pragma unroll
       for (int r = 0; r < kUnroll; ++r)
-        ok[r] = uu[r] >= 0 && visit.check(pp[r], kk[r], uu[r], aux[r]);
+        ok[r] = visit.check(uu[r] >= 0, pp[r], kk[r], uu[r], aux[r]);
       bool f[kUnroll], g[kUnroll];
       int cls[kUnroll];
       visit.template commit_n<kUnroll>(pp, kk, uu, aux, ok, cls);
@@ -570,7 +571,7 @@ __device__ __forceinline__ void expand_chunks_direct(const int *__restrict__ ptr
         }
 #pragma unroll
         for (int r = 0; r < kUnroll; ++r)
-          ok[r] = uu[r] >= 0 && visit.check(pay, k0 + r * 32 + lane, uu[r], aux[r]);
+          ok[r] = visit.check(uu[r] >= 0, pay, k0 + r * 32 + lane, uu[r], aux[r]);
         bool f[kUnroll], g[kUnroll];
         int cls[kUnroll], kk[kUnroll];
         unsigned pp[kUnroll];
@@ -663,7 +664,7 @@ __device__ __forceinline__ void expand_push_direct(const int *__restrict__ ptr,
       for (int r = 0; r < kUnroll; ++r) uu[r] = kk[r] >= 0 ? __ldg(ind + kk[r]) : -1;
 #pragma unroll
       for (int r = 0; r < kUnroll; ++r)
-        ok[r] = uu[r] >= 0 && visit.check(pp[r], kk[r], uu[r], aux[r]);
+        ok[r] = visit.check(uu[r] >= 0, pp[r], kk[r], uu[r], aux[r]);
       bool f[kUnroll], g[kUnroll];
       int cls[kUnroll];
       visit.template commit_n<kUnroll>(pp, kk, uu, aux, ok, cls);

@@ -139,9 +139,12 @@ struct SsspVisit {
   unsigned *far_min;
   // far lists only exist under a finite threshold (near-far schedule)
   __device__ __forceinline__ bool two_way() const { return thresh != Arith<W>::kInf; }
-  __device__ __forceinline__ bool check(unsigned du, int k, int u, unsigned &nd) const {
-    nd = Arith<W>::add(du, __ldg(w + k));
-    return nd < __ldcg(dist + u);
+  __device__ __forceinline__ bool check(bool on, unsigned du, int k, int u, unsigned &nd) const {
+    // selected, not branched around: the batch's loads are in flight together
+    const W wk = on ? __ldg(w + k) : W(0);
+    const unsigned old = on ? __ldcg(dist + u) : 0u;
+    nd = Arith<W>::add(du, wk);
+    return nd < old;
   }
   template <int N>
   __device__ __forceinline__ void commit_n(const unsigned (&)[N], const int (&)[N],
@@ -157,13 +160,12 @@ struct SsspVisit {
     // R-MAT 20 u32 0.556 against 0.533 ms, R-MAT 22 3.13 against 2.93 ms.)
 #pragma unroll
     for (int r = 0; r < N; ++r)
-      if (ok[r]) atomicMin(dist + u[r], nd[r]);
+      min_if(ok[r], dist + u[r], nd[r]);
     int prev[N];
 #pragma unroll
     for (int r = 0; r < N; ++r) {
-      prev[r] = 0;
-      if (ok[r])
-        prev[r] = nd[r] < thresh ? atomicExch(stamp + u[r], round) : atomicExch(fstamp + u[r], phase);
+      const bool near = nd[r] < thresh;
+      prev[r] = exch_if(ok[r], (near ? stamp : fstamp) + u[r], near ? round : phase, 0);
     }
 #pragma unroll
     for (int r = 0; r < N; ++r) {

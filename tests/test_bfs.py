@@ -163,3 +163,64 @@ def test_bfs_prepared_in_adjacency(ctx, symmetric, mode):
             np.testing.assert_array_equal(ap.bfs(ctx, g, s).cpu().numpy(), ref)
     finally:
         ap.bfs_set_params(ctx, mode=0)
+
+
+def _tree(*fanouts):
+    """Undirected tree given the number of children of every vertex, level by
+    level (a number for all vertices of a level, or one per vertex)."""
+    parent, level, n = [], np.array([0]), 1
+    for f in fanouts:
+        kids = np.broadcast_to(np.asarray(f), level.shape)
+        parent.append(np.repeat(level, kids))
+        level = np.arange(n, n + int(kids.sum()))
+        n += len(level)
+    p, c = np.concatenate(parent), np.arange(1, n)
+    return np.concatenate([p, c]), np.concatenate([c, p]), n
+
+
+def _layers(*sizes):
+    """Undirected graph of layers; every vertex has an edge to a random vertex
+    of the layer before, so depth = layer from vertex 0."""
+    rng = np.random.default_rng(0)
+    first = np.concatenate([[0], np.cumsum(sizes)])
+    u = np.arange(1, first[-1])
+    layer = np.searchsorted(first, u, side="right") - 1
+    v = first[layer - 1] + (rng.random(len(u)) * np.asarray(sizes)[layer - 1]).astype(np.int64)
+    return np.concatenate([u, v]), np.concatenate([v, u]), int(first[-1])
+
+
+@pytest.mark.parametrize("edges", [
+    _layers(*[1] * 700),
+    _layers(1, 15, 16, 17, 511, 512, 513, 8191, 8192, 8193, 3),  # shares and warps
+    _layers(1, 1000, 5000, 24000, 24600, 30000, 200, 1, 1),      # thin, wide, thin
+    _layers(1, 40, 4000, 1, 5000, 7),                            # hubs below and above the limit
+    # one block finds 150 * 31 vertices, more than its queue holds
+    _tree(16, 150, np.repeat([31, 7], [150, 2250]), 1, 1),
+], ids=["path", "shares", "wide", "hubs", "spill"])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_bfs_thin_levels(ctx, edges, mode):
+    """Graphs of few edges per vertex, whose thin levels one cluster runs:
+    frontiers around a block's share, levels that are too wide or too
+    hub-heavy, a block's queue that overflows, and a level limit before and
+    after the hand-over."""
+    import apspie_b200 as ap
+    r, c, m = edges
+    h = ap.from_edges(m, r, c)
+    h.symmetric = True
+    g = h.to_device()
+    ap.bfs_set_params(ctx, mode=mode)
+    try:
+        for src in (0, m - 1, m // 2):
+            ref, depth = oracle.bfs(h.m, h.ptr, h.ind, src)
+            np.testing.assert_array_equal(ap.bfs(ctx, g, src).cpu().numpy(), ref)
+            st = ap.bfs_stats(ctx)
+            assert st["levels"] == depth
+            assert st["vertices_reached"] == int((ref >= 0).sum())
+            assert st["edges_traversed"] == int(h.degrees()[ref >= 0].sum())
+            for lim in (1, 2, 4, depth - 1, depth, depth + 1):
+                if lim < 1:
+                    continue
+                d = ap.bfs(ctx, g, src, max_levels=lim).cpu().numpy()
+                np.testing.assert_array_equal(d, np.where(ref < lim, ref, -1))
+    finally:
+        ap.bfs_set_params(ctx)

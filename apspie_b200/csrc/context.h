@@ -157,6 +157,7 @@ enum SlotId : int {
   kSlotMisState,
   kSlotMisQueueA,
   kSlotMisQueueB,
+  kSlotMisWord,  // key while undecided, then the decision
   kSlotSortKeysA,
   kSlotSortKeysB,
   kSlotSortValsA,

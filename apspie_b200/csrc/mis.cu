@@ -8,26 +8,34 @@
 // joins when its priority beats that maximum (updateMis :64), and the
 // neighbours of joiners leave (updateNeighbor :71) -- with a full D->H copy of
 // the candidate vector every round (:240).  Here one persistent kernel runs
-// the rounds, one pass and one bounded grid barrier each: every undecided
-// vertex v scans its neighbours' states (the max-priority SpMSpV with the
-// comparison fused in) and
-//   * leaves (OUT) when a neighbour is IN;
-//   * else joins (IN), if it is a candidate of the round, when no
-//     neighbour of larger key is still undecided, and at once marks its
-//     undecided neighbours OUT (they would leave next round anyway; doing
-//     it now lets their other neighbours decide a round earlier);
-//   * else stays, and is compacted into the next round's queue (a queued
+// the rounds, one pass and one bounded grid barrier each.  A word per vertex
+// holds its key while it is undecided, and 0 (OUT) or all ones (IN) after.
+// Every undecided vertex v scans its neighbours' words (the max-priority
+// SpMSpV with the comparison fused in) until one stops it:
+//   * a neighbour that is IN: v leaves (OUT);
+//   * an undecided neighbour of larger key: v stays, and is compacted into
+//     the next round's queue with the position it stopped at;
+//   * none left, and v is a candidate of the round: v joins (IN) and at once
+//     marks its neighbours OUT (they would leave next round anyway; doing it
+//     now lets their other neighbours decide a round earlier; a queued
 //     vertex marked OUT meanwhile is dropped next round).
-// States change in place during the pass, so a neighbour's state may be
-// read before or after its own update in the same pass; the stale value is
-// always "undecided" (IN and OUT are final), which only delays a decision.
+// A neighbour passed over was OUT, or smaller and undecided; the first is
+// final and the second cannot join before v is decided, so the next round
+// goes on from where this one stopped and a vertex reads each of its edges
+// once over all rounds, plus the stopping one once per round.  (Scanning
+// every edge of every undecided vertex each round, state and priority apart:
+// 188 us on 2^20 vertices of mean degree 8, half of it waiting for loads
+// issued one edge at a time.)
+// Words change in place during the pass, so a neighbour's word may be read
+// before or after its own update in the same pass; the stale value is always
+// "undecided" (IN and OUT are final), which only delays a decision.
 // v is IN exactly when no neighbour of larger key is IN, so the set is the
 // greedy MIS in descending key order for any delta, whatever the timing.
-// key(v) = (prio[v] << 32) | v, so ties in priority go to the larger id and
-// every round decides at least the undecided vertex of largest key.
-// Self-loops are ignored.  Work per round is spread over warps with the same scan-based
-// edge dealing as the traversal kernels; a per-warp shared flag array
-// collects the per-vertex OR of the edge predicates.
+// key(v) = (prio[v] << 32) | (v + 1), so ties in priority go to the larger id
+// and every round decides at least the undecided vertex of largest key.
+// Self-loops are ignored.  A lane scans its own vertex's next edges four at a
+// time; the few scans longer than that are taken by the whole warp, one
+// vertex after the other.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,15 +56,14 @@ struct MisState {
   int rounds;
 };
 
-__device__ __forceinline__ unsigned long long mis_key(const uint32_t *prio, int v) {
-  return ((unsigned long long)__ldg(prio + v) << 32) | (unsigned)v;
-}
+constexpr unsigned long long kOutWord = 0ull, kInWord = ~0ull;
+constexpr int kLaneScans = 4;  // batches of four edges a lane scans by itself
+constexpr unsigned kLaneMarks = 32;  // joiners of more edges are marked by the warp
 
-__global__ void mis_init(int m, int32_t *state, int *queue, MisState *st) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x) {
-    state[v] = kUndecided;
-    queue[v] = v;
-  }
+__global__ void mis_init(int m, const uint32_t *__restrict__ prio, unsigned long long *word,
+                         MisState *st) {
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x)
+    word[v] = ((unsigned long long)prio[v] << 32) | (unsigned)(v + 1);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->q[0] = (unsigned)m;
     st->q[1] = st->q[2] = 0;
@@ -66,45 +73,16 @@ __global__ void mis_init(int m, int32_t *state, int *queue, MisState *st) {
   }
 }
 
-// Deals the edges of 32 queued vertices to the lanes of a warp.  code(v, u)
-// is evaluated per edge (v = owner vertex, u = neighbour); lane j gets the
-// OR of the codes over the edges of the warp's j-th vertex.
-template <typename Code>
-__device__ __forceinline__ unsigned warp_or_edges(int v, int s, int d, const int *__restrict__ ind,
-                                                  unsigned *flags, Code code) {
-  const int lane = lane_id();
-  flags[lane] = 0u;
-  __syncwarp();
-  int incl = warp_incl_scan(d);
-  int excl = incl - d;
-  int total = __shfl_sync(kFull, incl, 31);
-  for (int e0 = 0; e0 < total; e0 += 32) {
-    int e = e0 + lane;
-    int owner = warp_owner(excl, e);
-    int so = __shfl_sync(kFull, s, owner);
-    int eo = __shfl_sync(kFull, excl, owner);
-    int vo = __shfl_sync(kFull, v, owner);
-    if (e < total) {
-      const unsigned c = code(vo, __ldg(ind + so + (e - eo)));
-      if (c) atomicOr(flags + owner, c);
-    }
-  }
-  __syncwarp();
-  return flags[lane];
-}
+enum { kScanning = 0, kStopped, kLeaves, kFree };
 
-constexpr unsigned kHitIn = 1u, kHitLarger = 2u;
-
-__global__ void __launch_bounds__(kMisThreads)
+__global__ void __launch_bounds__(kMisThreads, 3)
 mis_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
-               const uint32_t *__restrict__ prio, int32_t *state, int *qa, int *qb, MisState *st,
+               unsigned long long *word, int32_t *out, int2 *qa, int2 *qb, MisState *st,
                double delta, int max_rounds) {
   const int lane = lane_id();
   const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  __shared__ unsigned s_flags[kMisThreads];
   __shared__ unsigned s_q;
-  unsigned *flags = s_flags + 32 * warp_in_block();
   int r = 0;
   for (;; ++r) {
     if (threadIdx.x == 0) {
@@ -117,47 +95,122 @@ mis_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
     // candidates of this round: prio > threshold (the reference's minimum)
     double level = 1.0 - (double)(r + 1) * delta;
     unsigned long long thr = level <= 0.0 ? 0ull : (unsigned long long)(level * 4294967296.0);
-    const int *qin = (r & 1) ? qb : qa;
-    int *qout = (r & 1) ? qa : qb;
+    const int2 *qin = (r & 1) ? qb : qa;
+    int2 *qout = (r & 1) ? qa : qb;
     for (unsigned base = (unsigned)gwarp * 32u; base < nq; base += (unsigned)nwarps * 32u) {
       const unsigned idx = base + lane;
-      int v = -1, s = 0, d = 0;
+      int v = -1;
+      unsigned pos = 0, e = 0;  // unsigned: a batch past the last edge of 2^31 does not wrap
+      unsigned long long my = kOutWord;
       if (idx < nq) {
-        v = __ldcg(qin + idx);
-        if (__ldcg(state + v) == kUndecided) {
-          s = __ldg(ptr + v);
-          d = __ldg(ptr + v + 1) - s;
+        if (r == 0) {  // every vertex, from its first edge
+          v = (int)idx;
+          pos = (unsigned)__ldg(ptr + v);
         } else {
-          v = -1;  // marked OUT by a neighbour that joined after it was queued
+          const int2 q = __ldcg(qin + idx);
+          v = q.x;
+          pos = (unsigned)q.y;
+        }
+        e = (unsigned)__ldg(ptr + v + 1);
+        my = __ldcg(word + v);
+      }
+      int st_v = my == kOutWord ? kLeaves : (pos < e ? kScanning : kFree);
+#pragma unroll 1
+      for (int b = 0; b < kLaneScans; ++b) {
+        if (!__any_sync(kFull, st_v == kScanning)) break;
+        int u[4];
+        unsigned long long k[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          u[i] = st_v == kScanning && pos + i < e ? __ldg(ind + pos + i) : -1;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) k[i] = u[i] >= 0 ? __ldcg(word + u[i]) : kOutWord;
+        int stop = 4;
+#pragma unroll
+        for (int i = 3; i >= 0; --i)
+          if (k[i] > my && u[i] != v) stop = i;
+        if (st_v == kScanning) {
+          const unsigned long long ks =
+              stop == 0 ? k[0] : (stop == 1 ? k[1] : (stop == 2 ? k[2] : k[3]));
+          pos += (unsigned)stop;
+          if (stop < 4) st_v = ks == kInWord ? kLeaves : kStopped;
+          else if (pos >= e) st_v = kFree;
         }
       }
-      const unsigned hit = warp_or_edges(v, s, d, ind, flags, [&](int vo, int u) -> unsigned {
-        if (u == vo) return 0u;
-        const int su = __ldcg(state + u);
-        if (su == kIn) return kHitIn;
-        return (su == kUndecided && mis_key(prio, u) > mis_key(prio, vo)) ? kHitLarger : 0u;
-      });
-      bool survive = false, joined = false;
-      if (v >= 0) {
-        const bool cand = (thr == 0ull) || ((unsigned long long)__ldg(prio + v) >= thr);
-        if (hit & kHitIn) {
-          state[v] = kOut;
-        } else if (cand && !(hit & kHitLarger)) {
-          state[v] = kIn;
-          joined = true;
-        } else {
-          survive = true;
+      // the scans that are not over: the warp, 128 edges at a time
+      for (unsigned left = __ballot_sync(kFull, st_v == kScanning); left; left &= left - 1) {
+        const int j = __ffs(left) - 1;
+        const int vj = __shfl_sync(kFull, v, j);
+        const unsigned ej = __shfl_sync(kFull, e, j);
+        const unsigned long long mj = __shfl_sync(kFull, my, j);
+        unsigned pj = __shfl_sync(kFull, pos, j);
+        int sj = kFree;
+        for (; pj < ej; pj += 128) {
+          int u[4];
+          unsigned long long k[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const unsigned p = pj + 32u * i + (unsigned)lane;
+            u[i] = p < ej ? __ldg(ind + p) : -1;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) k[i] = u[i] >= 0 ? __ldcg(word + u[i]) : kOutWord;
+          unsigned in = 0, at = 128;
+#pragma unroll
+          for (int i = 3; i >= 0; --i) {
+            const bool big = k[i] > mj && u[i] != vj;
+            const unsigned bm = __ballot_sync(kFull, big);
+            in |= __ballot_sync(kFull, big && k[i] == kInWord);
+            if (bm) at = 32u * i + (unsigned)__ffs(bm) - 1u;
+          }
+          if (at < 128u) {
+            pj += at;
+            sj = in ? kLeaves : kStopped;
+            break;
+          }
+        }
+        if (lane == j) {
+          st_v = sj;
+          pos = pj;
         }
       }
-      if (__ballot_sync(kFull, joined))
-        warp_or_edges(v, s, joined ? d : 0, ind, flags, [&](int vo, int u) -> unsigned {
-          if (u != vo && __ldcg(state + u) == kUndecided) state[u] = kOut;
-          return 0u;
-        });
-      unsigned slot = warp_append(survive, &st->q[(r + 1) % 3]);
-      if (survive) qout[slot] = v;
+      const bool joins = v >= 0 && st_v == kFree && (my >> 32) >= thr;
+      // (v + 1 keeps an undecided word above kOutWord; a vertex marked OUT
+      // while it scanned keeps that word: it cannot have come out free)
+      if (v >= 0 && st_v == kLeaves && my != kOutWord) word[v] = kOutWord;
+      unsigned s = 0;
+      if (joins) {
+        word[v] = kInWord;
+        s = (unsigned)__ldg(ptr + v);
+        if (e - s <= kLaneMarks)
+          for (unsigned p = s; p < e; p += 4) {
+            int u[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) u[i] = p + i < e ? __ldg(ind + p + i) : v;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (u[i] != v) word[u[i]] = kOutWord;
+          }
+      }
+      for (unsigned wide = __ballot_sync(kFull, joins && e - s > kLaneMarks); wide;
+           wide &= wide - 1) {
+        const int j = __ffs(wide) - 1;
+        const int vj = __shfl_sync(kFull, v, j);
+        const unsigned ej = __shfl_sync(kFull, e, j);
+        for (unsigned p = __shfl_sync(kFull, s, j) + (unsigned)lane; p < ej; p += 32) {
+          const int u = __ldg(ind + p);
+          if (u != vj) word[u] = kOutWord;
+        }
+      }
+      const bool stays = v >= 0 && (st_v == kStopped || (st_v == kFree && !joins));
+      const unsigned slot = warp_append(stays, &st->q[(r + 1) % 3]);
+      if (stays) qout[slot] = make_int2(v, (int)pos);
     }
     if (!grid_barrier(st->bar, &st->err)) return;
+  }
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x) {
+    const unsigned long long k = __ldcg(word + v);
+    out[v] = k == kInWord ? kIn : (k == kOutWord ? kOut : kUndecided);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) st->rounds = r;
 }
@@ -208,22 +261,23 @@ int apspie_mis(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr, const int *
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_mis: null pointer");
   if (!(delta > 0.0f)) delta = 1.0f;
   auto *st = (MisState *)workspace(ctx, kSlotMisState, sizeof(MisState));
-  auto *qa = (int *)workspace(ctx, kSlotMisQueueA, sizeof(int) * (size_t)m);
-  auto *qb = (int *)workspace(ctx, kSlotMisQueueB, sizeof(int) * (size_t)m);
-  if (!st || !qa || !qb) return APSPIE_ERR_OOM;
+  auto *qa = (int2 *)workspace(ctx, kSlotMisQueueA, sizeof(int2) * (size_t)m);
+  auto *qb = (int2 *)workspace(ctx, kSlotMisQueueB, sizeof(int2) * (size_t)m);
+  auto *word = (unsigned long long *)workspace(ctx, kSlotMisWord, 8 * (size_t)m);
+  if (!st || !qa || !qb || !word) return APSPIE_ERR_OOM;
   ctx->mis_state = st;
   int grid = clamp_grid(ctx, mis_grid(ctx));
   if (grid <= 0) return set_error(ctx, APSPIE_ERR_CUDA, "apspie_mis: occupancy query failed");
   int init_grid = std::min((m + 255) / 256, ctx->num_sms * 8);
-  mis_init<<<init_grid, 256, 0, ctx->stream>>>(m, d_mis, qa, st);
+  mis_init<<<init_grid, 256, 0, ctx->stream>>>(m, d_prio, word, st);
   int rc = check_launch(ctx, "mis_init");
   if (rc) return rc;
   double dd = (double)delta;
   // the round cap only guards against a stalled device loop: every round
   // decides at least one vertex, so m + 1 rounds always suffice
   int max_rounds = (int)std::min(2.0e9, (double)m + 1.0 + 1.0 / dd);
-  void *args[] = {&m, (void *)&d_ptr, (void *)&d_ind, (void *)&d_prio, &d_mis, &qa, &qb, &st,
-                  &dd, &max_rounds};
+  void *args[] = {&m, (void *)&d_ptr, (void *)&d_ind, &word, &d_mis, &qa, &qb, &st, &dd,
+                  &max_rounds};
   cudaError_t e = cudaLaunchCooperativeKernel((const void *)mis_persistent, dim3(grid),
                                               dim3(kMisThreads), args, 0, ctx->stream);
   if (e != cudaSuccess) return check_cuda(ctx, e, "mis_persistent");

@@ -100,3 +100,29 @@ def test_mis_full_size_configs(ctx, which):
     h = ap.gen_er(1 << 20, 8, seed=1) if which == "er" else ap.gen_grid(1024, 1024)
     rounds = _check(ctx, h, ap.mt19937(5489, h.m))
     assert rounds < 100
+
+
+@pytest.mark.parametrize("delta", [1.0, 0.1])
+@pytest.mark.parametrize("leaves", [1, 3, 4, 7, 8, 9, 31, 32, 33, 127, 128, 129, 136, 137, 5000])
+def test_mis_scan_lengths(ctx, leaves, delta):
+    """Stars whose hub's scan ends in a lane's batches of four, at their end,
+    or in the warp's batches of 128, with the hub's key the largest, the
+    smallest and in between; leaves are paired up, one has a self-loop."""
+    import apspie_b200 as ap
+    hub = leaves // 2
+    others = np.setdiff1d(np.arange(leaves + 1), [hub])
+    r = np.concatenate([np.full(leaves, hub), others])
+    c = np.concatenate([others, np.full(leaves, hub)])
+    pair = others[: 2 * (leaves // 2)].reshape(-1, 2)
+    r = np.concatenate([r, pair[:, 0], pair[:, 1], others[-1:]])
+    c = np.concatenate([c, pair[:, 1], pair[:, 0], others[-1:]])
+    order = np.lexsort((c, r))
+    h = ap.from_edges(leaves + 1, r[order], c[order])
+    prio = ap.mt19937(leaves, h.m)
+    for hp in (0, 0xFFFFFFFF, 1 << 31, 0xFFFFFFFF - (1 << 24)):
+        p = prio.copy()
+        p[hub] = hp
+        got, _, _ = _run(ctx, h, p, delta)
+        np.testing.assert_array_equal(got, oracle.mis(h.m, h.ptr, h.ind, p))
+    got, _, _ = _run(ctx, h, np.zeros(h.m, np.uint32), delta)
+    np.testing.assert_array_equal(got, oracle.mis(h.m, h.ptr, h.ind, np.zeros(h.m, np.uint32)))

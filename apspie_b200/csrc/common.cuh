@@ -109,6 +109,14 @@ __device__ __forceinline__ int exch_if(bool on, int *p, int val, int other) {
       : "=&r"(r) : "l"(p), "r"(val), "r"((int)on), "r"(other) : "memory");
   return r;
 }
+__device__ __forceinline__ int add_if(bool on, int *p, int val, int other) {
+  int r;
+  asm volatile(
+      "{ .reg .pred q; setp.ne.s32 q, %3, 0; mov.b32 %0, %4;\n"
+      "@q atom.relaxed.gpu.global.add.s32 %0, [%1], %2; }"
+      : "=&r"(r) : "l"(p), "r"(val), "r"((int)on), "r"(other) : "memory");
+  return r;
+}
 __device__ __forceinline__ unsigned long long or_if(bool on, unsigned long long *p,
                                                     unsigned long long val,
                                                     unsigned long long other) {

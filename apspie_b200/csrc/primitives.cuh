@@ -2,8 +2,9 @@
 // (key, value) pairs, written for this library (the reference uses moderngpu
 // Scan and cub::DeviceRadixSort, src/mXv.cuh:142,191-193).
 //
-// Scan: reduce-then-scan in three launches (tile sums, scan of tile sums in
-// one block, tile scans seeded by the scanned sums).  No inter-block waits.
+// Scan: reduce-then-scan: tile sums, then tile scans that each add up the
+// sums before them; from kScanFewTiles tiles on the sums are scanned by one
+// block in between; short inputs take one launch.  No inter-block waits.
 //
 // Radix sort: 8-bit digits, only as many passes as the key's significant
 // bits need (ceil(log2 m) bits for row indices), in the onesweep form: one
@@ -88,9 +89,23 @@ __global__ void scan_single_block(T *sums, int n, T *total) {
   if (threadIdx.x == 0 && total) *total = carry;
 }
 
-template <typename T>
-__global__ void scan_tiles(const T *in, long long n, const T *sums, T *out) {
+// kSumsScanned: sums are exclusive prefixes already; else every tile adds up
+// the plain sums before it (at most kScanFewTiles, a coalesced read from L2
+// instead of a launch) and the last one writes the total.
+constexpr int kScanFewTiles = 1024;
+
+template <typename T, bool kSumsScanned>
+__global__ void scan_tiles(const T *in, long long n, const T *sums, T *out, T *total) {
   __shared__ T sw[33];
+  T before = 0;
+  if (kSumsScanned) {
+    before = sums[blockIdx.x];
+  } else {
+    for (unsigned i = threadIdx.x; i < blockIdx.x; i += kScanThreads) before += sums[i];
+    T all;
+    block_excl_scan(before, sw, &all);
+    before = all;
+  }
   long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
   T v[kScanItems];
   T acc = 0;
@@ -101,7 +116,9 @@ __global__ void scan_tiles(const T *in, long long n, const T *sums, T *out) {
     acc += v[i];
   }
   T tot;
-  T run = block_excl_scan(acc, sw, &tot) + sums[blockIdx.x];
+  T run = block_excl_scan(acc, sw, &tot) + before;
+  if (!kSumsScanned && total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+    *total = before + tot;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     long long idx = base + i;
@@ -110,12 +127,43 @@ __global__ void scan_tiles(const T *in, long long n, const T *sums, T *out) {
   }
 }
 
+// A short scan in one launch instead of three (about 2 us each): one block,
+// kScanItems values per thread.  (Twice the values in two steps: no faster
+// than the three launches.)
+constexpr int kSmallScanThreads = 1024;
+constexpr int kSmallScanMax = kSmallScanThreads * kScanItems;
+
+template <typename T>
+__global__ void __launch_bounds__(kSmallScanThreads)
+scan_small(const T *in, int n, T *out, T *total) {
+  __shared__ T sw[33];
+  const int first = (int)threadIdx.x * kScanItems;
+  T v[kScanItems];
+  T acc = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) {
+    v[i] = first + i < n ? in[first + i] : T(0);
+    acc += v[i];
+  }
+  T tot;
+  T run = block_excl_scan(acc, sw, &tot);
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) {
+    if (first + i < n) out[first + i] = run;
+    run += v[i];
+  }
+  if (threadIdx.x == 0 && total) *total = tot;
+}
+
 // Exclusive scan in[0..n) -> out[0..n) (may alias); *d_total gets the sum.
 // Scratch: slot kSlotScan.  Returns a status.
 template <typename T>
 int device_exclusive_scan(apspie_context *ctx, const T *in, T *out, long long n, T *d_total) {
+  if (n <= kSmallScanMax) {
+    scan_small<T><<<1, kSmallScanThreads, 0, ctx->stream>>>(in, (int)n, out, d_total);
+    return check_launch(ctx, "scan_small");
+  }
   long long tiles = (n + kScanTile - 1) / kScanTile;
-  if (tiles < 1) tiles = 1;
   // the tile sums are scanned by one block in a loop: fine up to 2^20 tiles
   // (2^32 elements); T must hold the total
   if (tiles > (1ll << 20))
@@ -124,8 +172,14 @@ int device_exclusive_scan(apspie_context *ctx, const T *in, T *out, long long n,
   if (!sums) return APSPIE_ERR_OOM;
   // tile sums are computed from `in` before `out` is written, so in == out works
   scan_tile_sums<T><<<(unsigned)tiles, kScanThreads, 0, ctx->stream>>>(in, n, sums);
+  if (tiles <= kScanFewTiles) {
+    scan_tiles<T, false><<<(unsigned)tiles, kScanThreads, 0, ctx->stream>>>(in, n, sums, out,
+                                                                            d_total);
+    return check_launch(ctx, "device_exclusive_scan", 2);
+  }
   scan_single_block<T><<<1, kScanThreads, 0, ctx->stream>>>(sums, (int)tiles, d_total);
-  scan_tiles<T><<<(unsigned)tiles, kScanThreads, 0, ctx->stream>>>(in, n, sums, out);
+  scan_tiles<T, true><<<(unsigned)tiles, kScanThreads, 0, ctx->stream>>>(in, n, sums, out,
+                                                                         nullptr);
   return check_launch(ctx, "device_exclusive_scan", 3);
 }
 
@@ -408,6 +462,90 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
   }
 }
 
+// A sort of at most kSmallSortItems<K> x kSortThreads keys: one block, every
+// pass in shared memory (in one launch; a pass of one tile and its status
+// words take 9 us, the histograms, offsets and the memset 7 us more).  The
+// ranking is radix_onesweep's.
+template <typename K>
+constexpr int kSmallSortItems = sizeof(K) <= 4 ? 16 : 8;
+
+template <typename K, typename V>
+__global__ void __launch_bounds__(kSortThreads)
+radix_small(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, int n, int npass) {
+  constexpr int kWarps = kSortThreads / 32;
+  constexpr int kItems = kSmallSortItems<K>;
+  constexpr int kTile = kItems * kSortThreads;
+  __shared__ __align__(16) K skeys[kTile];
+  __shared__ __align__(16) V svals[kTile];
+  __shared__ unsigned whist[kWarps][kRadix];
+  __shared__ unsigned s_scan[33];
+  const int lane = lane_id(), w = warp_in_block();
+  const int wofs = w * 32 * kItems;
+  K kv[kItems];
+  V vv[kItems];
+  unsigned pos[kItems];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int t = wofs + i * 32 + lane;
+    kv[i] = t < n ? keys_in[t] : K(0);
+    vv[i] = t < n && vals_in ? vals_in[t] : (V)t;
+  }
+  for (int p = 0; p < npass; ++p) {
+    const int shift = p * kRadixBits;
+    for (int d = lane; d < kRadix; d += 32) whist[w][d] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const bool valid = wofs + i * 32 + lane < n;
+      const unsigned d = valid ? (unsigned)(kv[i] >> shift) & (kRadix - 1) : (unsigned)kRadix;
+      const unsigned peers = __match_any_sync(kFull, d);
+      const int leader = __ffs(peers) - 1;
+      unsigned prev = 0;
+      if (valid && lane == leader) {
+        prev = whist[w][d];
+        whist[w][d] = prev + __popc(peers);
+      }
+      prev = __shfl_sync(kFull, prev, leader);
+      pos[i] = prev + __popc(peers & ((1u << lane) - 1u));
+      __syncwarp();
+    }
+    __syncthreads();
+    unsigned run = 0, tot;
+    for (int ww = 0; ww < kWarps; ++ww) {
+      const unsigned c = whist[ww][threadIdx.x];
+      whist[ww][threadIdx.x] = run;
+      run += c;
+    }
+    const unsigned loc = block_excl_scan(run, s_scan, &tot);
+    for (int ww = 0; ww < kWarps; ++ww) whist[ww][threadIdx.x] += loc;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kItems; ++i)
+      if (wofs + i * 32 + lane < n) {
+        const unsigned at = pos[i] + whist[w][(unsigned)(kv[i] >> shift) & (kRadix - 1)];
+        skeys[at] = kv[i];
+        svals[at] = vv[i];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+      const int t = wofs + i * 32 + lane;
+      if (t < n) {
+        kv[i] = skeys[t];
+        vv[i] = svals[t];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int t = wofs + i * 32 + lane;
+    if (t < n) {
+      keys_out[t] = kv[i];
+      if (vals_out) vals_out[t] = vv[i];
+    }
+  }
+}
+
 // The context's radix-sort give-up word: set by a tile whose look-back
 // waited kLookbackSpinLimit polls for a predecessor (the output is then in
 // bounds but neither sorted nor a permutation of the input: some slots keep
@@ -459,6 +597,13 @@ int device_radix_sort(apspie_context *ctx, K *ka, V *va, K *kb, V *vb, long long
   const int npass = (bits + kRadixBits - 1) / kRadixBits;
   if (npass > kMaxPasses || n >= (1ll << 40))
     return set_error(ctx, APSPIE_ERR_OVERFLOW, "radix sort: %lld keys of %d bits", n, bits);
+  if (n <= kSmallSortItems<K> * kSortThreads) {
+    radix_small<K, V><<<1, kSortThreads, 0, ctx->stream>>>(kfirst ? kfirst : ka,
+                                                           kfirst ? nullptr : va, kb, vb, (int)n,
+                                                           npass);
+    *result_in_b = true;
+    return check_launch(ctx, "radix_small");
+  }
   const long long tiles = (n + kSortTile - 1) / kSortTile;
   // [histograms: npass x 256 u64][tile counters: 8 x u32, padded; the
   // sort's give-up word at u32 15][status: tiles x 256 words]

@@ -5,16 +5,16 @@
 // of the strict lower / upper triangles, cuSPARSE csrgemm U * L materialising
 // every wedge (src/tc.cuh:63-165), the ewiseMultTc merge-intersect
 // (src/tc.cuh:169-199) and a float mgpu::Reduce.  Here nothing but the count
-// is produced: for each row i of L, L(i,:) goes into a shared-memory hash
-// set, and every wedge j in L(k,:) for k in L(i,:) probes it; a hit is a
-// triangle (i > k > j).  Rows of up to 256 entries go one warp per row
-// (table 512).  Longer rows are cut into units of 512 of their k's, one
-// block per unit, so a hub row's wedges spread over many blocks; the unit's
-// set of L(i,:) is a bitmap over all vertex ids in shared memory when the
-// graph has at most kTcBitmapMaxVerts vertices (one bit probe per wedge),
-// else a hash table (rows up to 8192) or a binary search of the sorted row.
-// Per-warp partial counts are summed in 64-bit and added with one atomic per
-// warp.
+// is produced.  With U(j) = the rows that have j in L (L's column j), a
+// triangle i > k > j is an entry (k, j) of L and an i in both U(j) and U(k),
+// so the count is the sum of |U(j) ^ U(k)| over L's entries.  The columns are
+// gathered first (tc_scatter; their order does not matter).  An entry belongs
+// to the end with the longer column, whose column is a set in shared memory;
+// the other end's column, the shorter one, is read and probes it.  Under
+// tc_prepare's order by ascending degree the columns are short (R-MAT 18: at
+// most 413 entries, rows of L up to 25,224), so the probes are 321 M where
+// the products of L's rows are 660 M, and a set is built once per 256
+// entries of its end, or by a warp for itself.
 //
 // tc_prepare relabels vertices by ascending (degree, id) with the stable
 // radix sort, keeps the edges with new(col) < new(row), sorts them by
@@ -34,13 +34,22 @@
 namespace apspie {
 namespace {
 
-// rows of L up to kTcWarpMax entries are one warp's (R-MAT 18, timed side
-// by side: 256 -> 2.55 ms, 128 -> 2.26 ms, 64 -> 2.26 ms, 512 -> 17.9 ms);
-// longer ones are cut into units
-constexpr int kTcWarpMax = 128, kTcWarpTable = 512;
-constexpr int kTcBlockMax = 4096, kTcBlockTable = 8192;
+// Ends of at most kTcTinyCand entries (row and column together) and a column
+// of at most kTcTiny are a quarter warp's (2^20 vertices of mean degree 10:
+// 393 us with a warp each); up to kTcWarpCand entries and a column of
+// kTcWarpSet they are one warp's; longer ones are cut into units of
+// kTcUnit entries, a block each.  A block's set holds kTcPart entries at a
+// time (more: the unit's probes are repeated for each part): those among the
+// kTcTop largest ids in a bitmap, one shared-memory read per probe, the rest
+// in a hash table at most half full.
+constexpr int kTcTiny = 8, kTcTinyCand = 24;
+constexpr int kTcWarpCand = 128, kTcWarpSet = 128, kTcWarpTableBits = 8;
+constexpr int kTcUnit = 256;
+constexpr int kTcPart = 1024, kTcTableBits = 11;
+constexpr int kTcTop = 1 << 16;
 constexpr int kTcThreads = 256;
-constexpr int kTcWarps = 4;
+constexpr int kTcWarps = kTcThreads / 32;
+constexpr int kTcLong = 24;  // columns of this many entries are read by the whole warp
 constexpr int kNone = INT_MAX;
 
 __device__ __forceinline__ unsigned tc_hash(int j) { return (unsigned)j * 0x9E3779B1u; }
@@ -65,217 +74,265 @@ __device__ __forceinline__ bool set_has(const int *keys, int bits, int j) {
   return false;
 }
 
-__device__ __forceinline__ int tbits(int n, int cap) {
-  int b = 5;
-  while ((1 << b) < 2 * n && b < cap) ++b;
-  return b;
-}
-
 struct TcBins {
-  unsigned n[3];
-  unsigned pad;
+  unsigned n[3];  // tiny ends, warp ends, units
+  unsigned grab;  // units handed out
   unsigned long long count;
 };
 
-// k's of a long row per block unit: smaller units balance the blocks better
-// than the row's column set (rebuilt per unit) costs (R-MAT 18, timed
-// side by side: 512 -> 3.2 ms, 256 -> 2.8 ms, 128 -> 2.6 ms, 64 -> 2.55 ms)
-constexpr int kTcUnitK = 64;
-constexpr int kTcBitmapMaxVerts = 1 << 20;    // 128 KiB of shared bitmap
+// lengths of L's columns
+__global__ void tc_col_counts(int lnnz, const int *__restrict__ end, const int *__restrict__ Li,
+                              int *cnt) {
+  const unsigned stride = gridDim.x * blockDim.x;
+  const unsigned n = (unsigned)min(lnnz, __ldg(end));  // end: Lp + m
+  for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride)
+    atomicAdd(cnt + __ldg(Li + k), 1);
+}
 
-// warp rows -> lists[0..); long rows -> units (i, piece) in units[0..)
-__global__ void tc_bin(int m, const int *__restrict__ Lp, int *lists, int2 *units, TcBins *bins) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    int d = Lp[i + 1] - Lp[i];
-    if (d < 2) continue;  // a triangle needs two lower neighbours
-    if (d <= kTcWarpMax) {
-      lists[atomicAdd(&bins->n[0], 1u)] = i;
-    } else {
-      const int pieces = (d + kTcUnitK - 1) / kTcUnitK;
-      const unsigned s = atomicAdd(&bins->n[1], (unsigned)pieces);
-      for (int p = 0; p < pieces; ++p) units[s + p] = make_int2(i, p);
+// Every vertex's column as (start, length), a cursor for the scatter, and its
+// place among the tiny ends (lists from the front), the warp ends (lists from
+// the back) or its units (vertex, piece).
+__global__ void tc_bin(int m, const int *__restrict__ Lp, const int *__restrict__ Up,
+                       int2 *col, int *cursor, int *lists, int2 *units, TcBins *bins) {
+  const int lane = lane_id();
+  for (int v0 = blockIdx.x * blockDim.x + threadIdx.x - lane; v0 < m; v0 += gridDim.x * blockDim.x) {
+    const int v = v0 + lane;
+    int cand = 0, d = 0;
+    if (v < m) {
+      const int us = Up[v];
+      d = Up[v + 1] - us;
+      cand = Lp[v + 1] - Lp[v] + d;
+      col[v] = make_int2(us, d);
+      cursor[v] = us;
+    }
+    // an entry needs a set to probe and a column no longer than it
+    // (an end of one entry has nothing but the entry to its set's member)
+    const bool tiny = d > 0 && cand > 1 && cand <= kTcTinyCand && d <= kTcTiny;
+    const bool warp = d > 0 && !tiny && cand > 1 && cand <= kTcWarpCand && d <= kTcWarpSet;
+    const unsigned at0 = warp_append(tiny, &bins->n[0]);
+    if (tiny) lists[at0] = v;
+    const unsigned at1 = warp_append(warp, &bins->n[1]);
+    if (warp) lists[m - 1 - (int)at1] = v;
+    if (d > 0 && cand > kTcTinyCand && !warp) {
+      const int pieces = (cand - 1) / kTcUnit + 1;
+      const unsigned u = atomicAdd(&bins->n[2], (unsigned)pieces);
+      for (int p = 0; p < pieces; ++p) units[u + p] = make_int2(v, p);
     }
   }
 }
 
-// Wedges (k, j) for the k's at positions [a0, a1) of Li, dealt over a group
-// (warp or block): visit(j) per wedge.
-template <bool WARP, typename F>
-__device__ __forceinline__ void for_each_wedge_in(int a0, int a1, const int *__restrict__ Lp,
-                                                  const int *__restrict__ Li, int *s_off,
-                                                  int *s_bs, F visit) {
-  const int width = WARP ? 32 : (int)blockDim.x;
-  const int tid = WARP ? lane_id() : (int)threadIdx.x;
-  for (int c0 = a0; c0 < a1; c0 += width) {
-    int a = c0 + tid, bs = 0, d = 0;
-    if (a < a1) {
-      int k = __ldg(Li + a);
-      bs = __ldg(Lp + k);
-      d = __ldg(Lp + k + 1) - bs;
-    }
-    int excl, total;
-    if (WARP) {
-      int incl = warp_incl_scan(d);
-      excl = incl - d;
-      total = __shfl_sync(kFull, incl, 31);
-    } else {
-      __shared__ int sw[33];
-      excl = block_excl_scan(d, sw, &total);
-    }
-    s_off[tid] = excl;
-    s_bs[tid] = bs;
-    if (WARP) __syncwarp(); else __syncthreads();
-    const int n_a = min(width, a1 - c0);
-    if (!WARP) {
-      // block: runs of vt consecutive wedges per thread (vt grows with the
-      // chunk's wedges, up to 8): one binary search for the run's first
-      // owner (the largest t with s_off[t] <= p), then a linear walk
-      const int vt = max(1, min(8, total / width));
-      for (int p0 = tid * vt; p0 < total; p0 += width * vt) {
-        int lo = 0, hi = n_a - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (s_off[mid] <= p0) lo = mid; else hi = mid - 1;
-        }
-        int nxt = lo + 1 < n_a ? s_off[lo + 1] : INT_MAX;
-        const int pend = min(p0 + vt, total);
-        // the run's wedge positions first, then all its loads, then the
-        // visits: up to 8 independent loads in flight per thread
-        int pos[8];
+// L's entries into their columns, in any order within a column.
+__global__ void __launch_bounds__(kEdgeThreads)
+tc_scatter(int m, int lnnz, const int *__restrict__ Lp, const int *__restrict__ Li, int *cursor,
+           int *Ui) {
+  __shared__ __align__(16) int s_row[kEdgeTile];
+  const int k0 = (int)blockIdx.x * kEdgeTile;
+  const int n = min(kEdgeTile, min(lnnz, __ldg(Lp + m)) - k0);
+  if (n <= 0) return;
+  edge_tile_rows(Lp, m, k0, n, s_row);
+  int c[kEdgeItems], at[kEdgeItems];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int p = p0 + q;
-          pos[q] = -1;
-          if (p < pend) {
-            while (p >= nxt) {
-              ++lo;
-              nxt = lo + 1 < n_a ? s_off[lo + 1] : INT_MAX;
-            }
-            pos[q] = s_bs[lo] + (p - s_off[lo]);
-          }
-        }
-        int jv[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) jv[q] = pos[q] >= 0 ? __ldg(Li + pos[q]) : -1;
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (jv[q] >= 0) visit(jv[q]);
-      }
-      __syncthreads();
-      continue;
-    }
-    // warp: the k owning wedge p; a lane's p grows by 32 per step, so its
-    // owner only moves forward -- gallop from the previous one
-    int lo = 0;
-    for (int p = tid; p < total; p += width) {
-      if (lo + 1 < n_a && s_off[lo + 1] <= p) {
-        int step = 1, hi = lo + 1;
-        while (hi + step < n_a && s_off[hi + step] <= p) {
-          hi += step;
-          step <<= 1;
-        }
-        // owner in [hi, min(hi + step, n_a) - 1]
-        int l2 = hi, h2 = min(hi + step, n_a) - 1;
-        while (l2 < h2) {
-          int mid = (l2 + h2 + 1) >> 1;
-          if (s_off[mid] <= p) l2 = mid; else h2 = mid - 1;
-        }
-        lo = l2;
-      }
-      visit(__ldg(Li + s_bs[lo] + (p - s_off[lo])));
-    }
-    if (WARP) __syncwarp(); else __syncthreads();
+  for (int q = 0; q < kEdgeItems; ++q) {
+    const int t = (int)threadIdx.x + q * kEdgeThreads;
+    c[q] = t < n ? __ldg(Li + k0 + t) : -1;
   }
+#pragma unroll
+  for (int q = 0; q < kEdgeItems; ++q) at[q] = add_if(c[q] >= 0, cursor + c[q], 1, 0);
+#pragma unroll
+  for (int q = 0; q < kEdgeItems; ++q)
+    if (c[q] >= 0) Ui[at[q]] = s_row[threadIdx.x + q * kEdgeThreads];
 }
 
-// Wedges of row i.
-template <bool WARP, typename F>
-__device__ __forceinline__ void for_each_wedge(int i, const int *__restrict__ Lp,
-                                               const int *__restrict__ Li, int *s_off, int *s_bs,
-                                               F visit) {
-  for_each_wedge_in<WARP>(__ldg(Lp + i), __ldg(Lp + i + 1), Lp, Li, s_off, s_bs, visit);
+// Members of the set `has` among the columns (start, len) that the lanes
+// hold, one each.  Long columns one after the other with 128 entries in
+// flight, the entries of the short ones dealt flat over the lanes.
+template <typename Has>
+__device__ __forceinline__ unsigned tc_probe(int start, int len, const int *__restrict__ Ui,
+                                             Has has) {
+  const int lane = lane_id();
+  unsigned cnt = 0;
+  for (unsigned big = __ballot_sync(kFull, len >= kTcLong); big; big &= big - 1) {
+    const int j = __ffs(big) - 1;
+    const int a = __shfl_sync(kFull, start, j), n = __shfl_sync(kFull, len, j);
+    for (int t = lane; t < n; t += 128) {
+      int x[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = t + 32 * q < n ? __ldg(Ui + a + t + 32 * q) : -1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) cnt += x[q] >= 0 && has(x[q]) ? 1u : 0u;
+    }
+  }
+  const int d = len < kTcLong ? len : 0;
+  const int incl = warp_incl_scan(d), excl = incl - d;
+  const int total = __shfl_sync(kFull, incl, 31);
+  for (int e0 = 0; e0 < total; e0 += 64) {
+    int x[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int e = e0 + 32 * q + lane;
+      const int owner = warp_owner(excl, e);
+      const int at = __shfl_sync(kFull, start - excl, owner) + e;
+      x[q] = e < total ? __ldg(Ui + at) : -1;
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) cnt += x[q] >= 0 && has(x[q]) ? 1u : 0u;
+  }
+  return cnt;
 }
 
-__global__ void __launch_bounds__(32 * kTcWarps)
-tc_warp_rows(const int *list, TcBins *bins, const int *__restrict__ Lp, const int *__restrict__ Li) {
-  __shared__ int s_keys[kTcWarps][kTcWarpTable];
-  __shared__ int s_off[kTcWarps][32], s_bs[kTcWarps][32];
+// The column that this lane's entry number c of end s reads, (0, 0) when the
+// entry belongs to its other end: row entries own columns up to d, column
+// entries only shorter ones, so that equal lengths belong to one end.
+__device__ __forceinline__ int2 tc_entry(int c, int nc, int la, int ld, int us, int d,
+                                         const int *__restrict__ Li, const int *__restrict__ Ui,
+                                         const int2 *__restrict__ col) {
+  if (c >= nc) return make_int2(0, 0);
+  const int p = c < ld ? __ldg(Li + la + c) : __ldg(Ui + us + (c - ld));
+  const int2 x = __ldg(col + p);
+  return x.y <= (c < ld ? d : d - 1) ? x : make_int2(0, 0);
+}
+
+// A tiny end per eight lanes: its column's members one per lane, an entry per
+// lane, and each member of the entry's column compared with the end's by
+// eight shuffles.
+__device__ __forceinline__ unsigned tc_tiny_ends(const int *list, const TcBins *bins,
+                                                const int *__restrict__ Lp,
+                                                const int *__restrict__ Li,
+                                                const int2 *__restrict__ col,
+                                                const int *__restrict__ Ui) {
+  const int lane = lane_id(), sub = lane >> 3, l = lane & 7;
+  const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
+  const unsigned n = bins->n[0];
+  unsigned cnt = 0;
+  for (unsigned r = gwarp * 4; r < n; r += nwarps * 4) {
+    int la = 0, ld = 0, us = 0, d = 0, mine = -1;
+    if (r + sub < n) {
+      const int s = __ldg(list + r + sub);
+      la = __ldg(Lp + s);
+      ld = __ldg(Lp + s + 1) - la;
+      const int2 c = __ldg(col + s);
+      us = c.x;
+      d = c.y;
+      if (l < d) mine = __ldg(Ui + us + l);
+    }
+    const int nc = ld + d;
+    const int most = (int)__reduce_max_sync(kFull, (unsigned)nc);
+    const int dmax = (int)__reduce_max_sync(kFull, (unsigned)d);
+    for (int c0 = 0; c0 < most; c0 += 8) {
+      const int2 x = tc_entry(c0 + l, nc, la, ld, us, d, Li, Ui, col);
+      const int longest = (int)__reduce_max_sync(kFull, (unsigned)x.y);
+      for (int t = 0; t < longest; t += 4) {
+        int j[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) j[q] = t + q < x.y ? __ldg(Ui + x.x + t + q) : -2;
+        for (int e = 0; e < dmax; ++e) {
+          const int other = __shfl_sync(kFull, mine, e, 8);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) cnt += j[q] == other ? 1u : 0u;
+        }
+      }
+    }
+  }
+  return cnt;
+}
+
+// A warp end per warp, its set in the warp's part of the block's table.
+static_assert(kTcWarps << kTcWarpTableBits == 1 << kTcTableBits, "the warps share the table");
+
+__device__ __forceinline__ unsigned long long tc_warp_ends(const int *list_end,
+                                                           const TcBins *bins, int *s_keys,
+                                                           const int *__restrict__ Lp,
+                                                           const int *__restrict__ Li,
+                                                           const int2 *__restrict__ col,
+                                                           const int *__restrict__ Ui) {
   const int w = warp_in_block(), lane = lane_id();
-  int *keys = s_keys[w];
+  int *keys = s_keys + (w << kTcWarpTableBits);
   unsigned long long cnt = 0;
-  const unsigned nrows = bins->n[0];
-  for (unsigned r = blockIdx.x * kTcWarps + w; r < nrows; r += gridDim.x * kTcWarps) {
-    int i = list[r];
-    int a0 = __ldg(Lp + i), d = __ldg(Lp + i + 1) - a0;
-    int bits = tbits(d, 9);
+  const unsigned n = bins->n[1];
+  for (unsigned r = blockIdx.x * kTcWarps + w; r < n; r += gridDim.x * kTcWarps) {
+    const int s = list_end[-(int)r];
+    const int la = __ldg(Lp + s), ld = __ldg(Lp + s + 1) - la;
+    const int2 c = __ldg(col + s);
+    int bits = 5;
+    while ((1 << bits) < 2 * c.y) ++bits;
     for (int t = lane; t < (1 << bits); t += 32) keys[t] = kNone;
     __syncwarp();
-    for (int t = lane; t < d; t += 32) set_insert(keys, bits, __ldg(Li + a0 + t));
+    for (int t = lane; t < c.y; t += 32) set_insert(keys, bits, __ldg(Ui + c.x + t));
     __syncwarp();
-    for_each_wedge<true>(i, Lp, Li, s_off[w], s_bs[w],
-                         [&](int j) { cnt += set_has(keys, bits, j) ? 1 : 0; });
+    const int nc = ld + c.y;
+    for (int c0 = 0; c0 < nc; c0 += 32) {
+      const int2 x = tc_entry(c0 + lane, nc, la, ld, c.x, c.y, Li, Ui, col);
+      cnt += tc_probe(x.x, x.y, Ui, [&](int j) { return set_has(keys, bits, j); });
+    }
     __syncwarp();
   }
-  cnt = warp_sum(cnt);
-  if (lane == 0 && cnt) atomicAdd(&bins->count, cnt);
+  return cnt;
 }
 
-// One unit = the k's [piece * kTcUnitK, +kTcUnitK) of a long row i, one
-// block per unit.  MODE 0: L(i,:) as a bitmap over all vertex ids (dynamic
-// shared memory, zero between units: set bits are cleared again); MODE 1:
-// hash table (rows up to kTcBlockMax); MODE 2: binary search in the row.
-template <int MODE>
-__global__ void __launch_bounds__(kTcThreads)
-tc_units(const int2 *units, TcBins *bins, int m, const int *__restrict__ Lp,
-         const int *__restrict__ Li) {
-  extern __shared__ unsigned tc_smem[];
-  __shared__ int s_off[kTcThreads], s_bs[kTcThreads];
+// All ends in one launch: the units first, handed out on demand, then every
+// warp its share of the warp ends and of the tiny ends, which fill the time
+// that the last units take.
+__global__ void __launch_bounds__(kTcThreads, 8)
+tc_count(const int2 *units, const int *lists, TcBins *bins, int m, const int *__restrict__ Lp,
+         const int *__restrict__ Li, const int2 *__restrict__ col, const int *__restrict__ Ui) {
+  __shared__ unsigned s_bits[kTcTop / 32];
+  __shared__ int s_keys[1 << kTcTableBits];
+  __shared__ unsigned s_unit;
+  __shared__ int s_hashed;
+  const int t0 = threadIdx.x, w = warp_in_block(), lane = lane_id();
   unsigned long long cnt = 0;
-  const unsigned nunits = bins->n[1];
-  if (MODE != 2) {
-    const int words = MODE == 0 ? (m + 31) / 32 : kTcBlockTable;
-    for (int t = threadIdx.x; t < words; t += blockDim.x) tc_smem[t] = MODE == 0 ? 0u : (unsigned)kNone;
+  const unsigned nunits = bins->n[2];
+  const int top = max(0, m - kTcTop);
+  for (int t = t0; t < kTcTop / 32; t += kTcThreads) s_bits[t] = 0u;
+  for (int t = t0; t < (1 << kTcTableBits); t += kTcThreads) s_keys[t] = kNone;
+  if (t0 == 0) s_hashed = 0;
+  for (;;) {
+    if (t0 == 0) s_unit = atomicAdd(&bins->grab, 1u);
     __syncthreads();
-  }
-  for (unsigned u = blockIdx.x; u < nunits; u += gridDim.x) {
+    const unsigned u = s_unit;
+    if (u >= nunits) break;
     const int2 un = units[u];
-    const int i = un.x;
-    const int a0 = __ldg(Lp + i), a1 = __ldg(Lp + i + 1), d = a1 - a0;
-    const int k0 = a0 + un.y * kTcUnitK, k1 = min(k0 + kTcUnitK, a1);
-    if (MODE == 0) {
-      for (int t = threadIdx.x; t < d; t += blockDim.x) {
-        const int j = __ldg(Li + a0 + t);
-        atomicOr(tc_smem + (j >> 5), 1u << (j & 31));
+    const int s = un.x;
+    const int la = __ldg(Lp + s), ld = __ldg(Lp + s + 1) - la;
+    const int2 c = __ldg(col + s);
+    const int us = c.x, d = c.y;
+    const int c_beg = un.y * kTcUnit, nc = min(ld + d, c_beg + kTcUnit);
+    for (int part = 0; part < d; part += kTcPart) {
+      const int pe = min(d, part + kTcPart);
+      for (int t = part + t0; t < pe; t += kTcThreads) {
+        const int j = __ldg(Ui + us + t);
+        if (j >= top) {
+          atomicOr(s_bits + ((j - top) >> 5), 1u << ((j - top) & 31));
+        } else {
+          set_insert(s_keys, kTcTableBits, j);
+          s_hashed = 1;
+        }
       }
       __syncthreads();
-      for_each_wedge_in<false>(k0, k1, Lp, Li, s_off, s_bs,
-                               [&](int j) { cnt += (tc_smem[j >> 5] >> (j & 31)) & 1u; });
+      const bool hashed = s_hashed != 0;
+      for (int c0 = c_beg + w * 32; c0 < nc; c0 += kTcThreads) {
+        const int2 x = tc_entry(c0 + lane, nc, la, ld, us, d, Li, Ui, col);
+        cnt += tc_probe(x.x, x.y, Ui, [&](int j) -> bool {
+          if (j >= top) return (s_bits[(j - top) >> 5] >> ((j - top) & 31)) & 1u;
+          return hashed && set_has(s_keys, kTcTableBits, j);
+        });
+      }
       __syncthreads();
-      for (int t = threadIdx.x; t < d; t += blockDim.x) tc_smem[__ldg(Li + a0 + t) >> 5] = 0u;
+      for (int t = part + t0; t < pe; t += kTcThreads) {
+        const int j = __ldg(Ui + us + t);
+        if (j >= top) s_bits[(j - top) >> 5] = 0u;
+      }
+      if (hashed)
+        for (int t = t0; t < (1 << kTcTableBits); t += kTcThreads) s_keys[t] = kNone;
+      if (t0 == 0) s_hashed = 0;
       __syncthreads();
-    } else if (MODE == 1 && d <= kTcBlockMax) {
-      int *keys = reinterpret_cast<int *>(tc_smem);
-      const int bits = tbits(d, 13);
-      for (int t = threadIdx.x; t < (1 << bits); t += blockDim.x) keys[t] = kNone;
-      __syncthreads();
-      for (int t = threadIdx.x; t < d; t += blockDim.x) set_insert(keys, bits, __ldg(Li + a0 + t));
-      __syncthreads();
-      for_each_wedge_in<false>(k0, k1, Lp, Li, s_off, s_bs,
-                               [&](int j) { cnt += set_has(keys, bits, j) ? 1 : 0; });
-      __syncthreads();
-    } else {
-      for_each_wedge_in<false>(k0, k1, Lp, Li, s_off, s_bs, [&](int j) {
-        int lo = a0, hi = a1;
-        while (lo < hi) {
-          int mid = (lo + hi) >> 1;
-          if (__ldg(Li + mid) < j) lo = mid + 1; else hi = mid;
-        }
-        cnt += (lo < a1 && __ldg(Li + lo) == j) ? 1 : 0;
-      });
     }
   }
+  cnt += tc_warp_ends(lists + (m - 1), bins, s_keys, Lp, Li, col, Ui);
+  cnt += tc_tiny_ends(lists, bins, Lp, Li, col, Ui);
   cnt = warp_sum(cnt);
-  if (lane_id() == 0 && cnt) atomicAdd(&bins->count, cnt);
+  if (lane == 0 && cnt) atomicAdd(&bins->count, cnt);
 }
 
 // ------------------------------------------------------------- prepare ---
@@ -298,6 +355,8 @@ __global__ void rank_to_perm(int m, const int *order, int *perm) {
     perm[order[r]] = r;
 }
 
+constexpr int kSplit = 4;  // entries per thread in flight in the two passes over the edges
+
 // Per vertex v of new id r: how many neighbours rank below r (the length
 // of L's row r) and how many above (v's entries in L's columns), added to
 // zeroed lcnt / ucnt by warp and row from one pass over the edges in tiles of
@@ -317,25 +376,34 @@ split_counts(int m, int nnz, const int *__restrict__ ptr, const int *__restrict_
   edge_tile_rows(ptr, m, k0, n, s_row);
   const int lane = lane_id();
   unsigned long long h_fwd = 0, h_rev = 0;
-  for (int t0 = (int)threadIdx.x - lane; t0 < n; t0 += kEdgeThreads) {
-    const int t = t0 + lane;
-    int v = -1, r = 0, pu = 0;
-    if (t < n) {
-      v = s_row[t];
-      const int u = __ldg(ind + k0 + t);
-      r = __ldg(perm + v);
-      pu = __ldg(perm + u);
-      h_fwd += apspie_gen::mix64(((unsigned long long)(unsigned)v << 32) | (unsigned)u);
-      h_rev += apspie_gen::mix64(((unsigned long long)(unsigned)u << 32) | (unsigned)v);
+  for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kSplit * kEdgeThreads) {
+    int v[kSplit], u[kSplit], r[kSplit], pu[kSplit];
+#pragma unroll
+    for (int q = 0; q < kSplit; ++q) {
+      const int t = t0 + q * kEdgeThreads;
+      v[q] = t < n ? s_row[t] : -1;
+      u[q] = t < n ? __ldg(ind + k0 + t) : 0;
     }
-    const unsigned below = __ballot_sync(kFull, t < n && pu < r);
-    const unsigned above = __ballot_sync(kFull, t < n && pu > r);
-    int leader;
-    const unsigned peers = row_peers(v, &leader);
-    if (lane == leader && v >= 0) {
-      const int lo = __popc(below & peers), hi = __popc(above & peers);
-      if (lo) atomicAdd(lcnt + r, lo);
-      if (hi) atomicAdd(ucnt + r, hi);
+#pragma unroll
+    for (int q = 0; q < kSplit; ++q) {
+      r[q] = v[q] >= 0 ? __ldg(perm + v[q]) : 0;
+      pu[q] = v[q] >= 0 ? __ldg(perm + u[q]) : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kSplit; ++q) {
+      if (v[q] >= 0) {
+        h_fwd += apspie_gen::mix64(((unsigned long long)(unsigned)v[q] << 32) | (unsigned)u[q]);
+        h_rev += apspie_gen::mix64(((unsigned long long)(unsigned)u[q] << 32) | (unsigned)v[q]);
+      }
+      const unsigned below = __ballot_sync(kFull, pu[q] < r[q]);
+      const unsigned above = __ballot_sync(kFull, pu[q] > r[q]);
+      int leader;
+      const unsigned peers = row_peers(v[q], &leader);
+      if (lane == leader && v[q] >= 0) {
+        const int lo = __popc(below & peers), hi = __popc(above & peers);
+        if (lo) atomicAdd(lcnt + r[q], lo);
+        if (hi) atomicAdd(ucnt + r[q], hi);
+      }
     }
   }
   h_fwd = warp_sum(h_fwd);
@@ -361,24 +429,33 @@ upper_pairs(int m, int nnz, const int *__restrict__ ptr, const int *__restrict__
   if (n <= 0) return;
   edge_tile_rows(ptr, m, k0, n, s_row);
   const int lane = lane_id();
-  for (int t0 = (int)threadIdx.x - lane; t0 < n; t0 += kEdgeThreads) {
-    const int t = t0 + lane;
-    int v = -1, r = 0, pu = 0;
-    if (t < n) {
-      v = s_row[t];
-      r = __ldg(perm + v);
-      pu = __ldg(perm + __ldg(ind + k0 + t));
+  for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kSplit * kEdgeThreads) {
+    int v[kSplit], u[kSplit], r[kSplit], pu[kSplit], base[kSplit], leader[kSplit];
+    unsigned mine[kSplit];
+#pragma unroll
+    for (int q = 0; q < kSplit; ++q) {
+      const int t = t0 + q * kEdgeThreads;
+      v[q] = t < n ? s_row[t] : -1;
+      u[q] = t < n ? __ldg(ind + k0 + t) : 0;
     }
-    const bool keep = t < n && pu > r;
-    int leader;
-    const unsigned mine = row_peers(v, &leader) & __ballot_sync(kFull, keep);
-    int base = 0;
-    if (lane == leader && mine) base = atomicAdd(uoff + r, __popc(mine));
-    base = __shfl_sync(kFull, base, leader);
-    if (keep) {
-      const int at = base + __popc(mine & ((1u << lane) - 1u));
-      rows[at] = (unsigned)pu;
-      cols[at] = r;
+#pragma unroll
+    for (int q = 0; q < kSplit; ++q) {
+      r[q] = v[q] >= 0 ? __ldg(perm + v[q]) : 0;
+      pu[q] = v[q] >= 0 ? __ldg(perm + u[q]) : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kSplit; ++q) {
+      mine[q] = row_peers(v[q], &leader[q]) & __ballot_sync(kFull, pu[q] > r[q]);
+      base[q] = add_if(lane == leader[q] && mine[q] != 0u, uoff + r[q], __popc(mine[q]), 0);
+    }
+#pragma unroll
+    for (int q = 0; q < kSplit; ++q) {
+      base[q] = __shfl_sync(kFull, base[q], leader[q]);
+      if (pu[q] > r[q]) {
+        const int at = base[q] + __popc(mine[q] & ((1u << lane) - 1u));
+        rows[at] = (unsigned)pu[q];
+        cols[at] = r[q];
+      }
     }
   }
 }
@@ -424,7 +501,8 @@ int apspie_tc_prepare(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr, cons
   bool in_b = false;
   rc = device_radix_sort<unsigned, int>(ctx, dk, ids, dk2, ids2, m, dbits, &in_b);
   if (rc) return rc;
-  rc = radix_sort_check(ctx);  // before the sorted ids index anything
+  // before the sorted ids index anything (one tile never waits)
+  rc = m > kSortTile ? radix_sort_check(ctx) : APSPIE_OK;
   if (rc) return rc;
   rank_to_perm<<<tgrid(ctx, m, 256), 256, 0, st>>>(m, in_b ? ids2 : ids, d_perm);
   // 2. row lengths of L (indexed by new id) and each vertex's count above it
@@ -480,7 +558,7 @@ int apspie_tc_prepare(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr, cons
     in_b = false;
     rc = device_radix_sort<unsigned, int>(ctx, ka, va, kb, d_Lind, lnnz, cbits, &in_b);
     if (rc) return rc;
-    rc = radix_sort_check(ctx);
+    rc = lnnz > kSortTile ? radix_sort_check(ctx) : APSPIE_OK;
     if (rc) return rc;
     if (!in_b) {
       rc = check_cuda(ctx, cudaMemcpyAsync(d_Lind, va, sizeof(int) * (size_t)lnnz,
@@ -498,33 +576,36 @@ int apspie_tc(apspie_ctx ctx, int m, int64_t lnnz, const int *d_Lptr, const int 
   APSPIE_CHECK_CTX(ctx);
   if (m <= 0 || lnnz < 0 || !d_Lptr || (lnnz > 0 && !d_Lind) || !h_count)
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_tc: bad arguments");
+  if (lnnz >= (int64_t)INT32_MAX)
+    return set_error(ctx, APSPIE_ERR_OVERFLOW, "apspie_tc: nnz(L) %lld exceeds int32 offsets",
+                     (long long)lnnz);
+  *h_count = 0;
+  if (lnnz == 0) return APSPIE_OK;
   cudaStream_t st = ctx->stream;
   auto *lists = (int *)workspace(ctx, kSlotMisc0, sizeof(int) * (size_t)m);
-  // units: at most lnnz / kTcUnitK + (rows longer than kTcWarpMax) pieces
+  // an end with units has more than kTcWarpSet entries, or a column that is
+  // longer: at most 2 lnnz / kTcWarpSet such ends, 2 lnnz / kTcUnit full units
   auto *units = (int2 *)workspace(
-      ctx, kSlotMisc1, sizeof(int2) * ((size_t)lnnz / kTcUnitK + (size_t)lnnz / kTcWarpMax + 2));
-  auto *bins = (TcBins *)workspace(ctx, kSlotSmall, sizeof(TcBins));
-  if (!lists || !units || !bins) return APSPIE_ERR_OOM;
-  cudaMemsetAsync(bins, 0, sizeof(TcBins), st);
-  tc_bin<<<tgrid(ctx, m, 256), 256, 0, st>>>(m, d_Lptr, lists, units, bins);
-  tc_warp_rows<<<ctx->num_sms * 16, 32 * kTcWarps, 0, st>>>(lists, bins, d_Lptr, d_Lind);
-  // every resident block: the units are L2-latency bound, so occupancy is
-  // what hides the latency (the bitmap's shared memory sets the limit)
-  if (m <= kTcBitmapMaxVerts) {
-    const int smem = (int)(sizeof(unsigned) * (size_t)((m + 31) / 32));
-    cudaFuncSetAttribute(tc_units<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_units<0>, kTcThreads, smem);
-    tc_units<0><<<ctx->num_sms * std::max(1, per_sm), kTcThreads, smem, st>>>(units, bins, m,
-                                                                              d_Lptr, d_Lind);
-  } else {
-    const int smem = (int)(sizeof(int) * kTcBlockTable);
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc_units<1>, kTcThreads, smem);
-    tc_units<1><<<ctx->num_sms * std::max(1, per_sm), kTcThreads, smem, st>>>(units, bins, m,
-                                                                              d_Lptr, d_Lind);
-  }
-  int rc = check_launch(ctx, "apspie_tc", 3);
+      ctx, kSlotMisc1,
+      sizeof(int2) * (2 * (size_t)lnnz / kTcUnit + 2 * (size_t)lnnz / kTcWarpSet + 2));
+  static_assert(sizeof(TcBins) % sizeof(int) == 0, "the counters precede the column offsets");
+  auto *bins = (TcBins *)workspace(ctx, kSlotMisc2, sizeof(TcBins) + sizeof(int) * ((size_t)m + 1));
+  auto *Up = bins ? (int *)(bins + 1) : nullptr;
+  auto *cursor = (int *)workspace(ctx, kSlotMisc3, sizeof(int) * (size_t)m);
+  auto *col = (int2 *)workspace(ctx, kSlotSortValsA, sizeof(int2) * (size_t)m);
+  auto *Ui = (int *)workspace(ctx, kSlotSortKeysA, sizeof(int) * (size_t)lnnz);
+  if (!lists || !units || !Up || !cursor || !col || !Ui || !bins) return APSPIE_ERR_OOM;
+  cudaMemsetAsync(bins, 0, sizeof(TcBins) + sizeof(int) * ((size_t)m + 1), st);
+  tc_col_counts<<<tgrid(ctx, lnnz, 256), 256, 0, st>>>((int)lnnz, d_Lptr + m, d_Lind, Up);
+  int rc = check_launch(ctx, "tc_col_counts");
+  if (rc) return rc;
+  rc = device_exclusive_scan<int>(ctx, Up, Up, (long long)m + 1, nullptr);
+  if (rc) return rc;
+  tc_bin<<<tgrid(ctx, m, 256), 256, 0, st>>>(m, d_Lptr, Up, col, cursor, lists, units, bins);
+  tc_scatter<<<edge_tiles(lnnz), kEdgeThreads, 0, st>>>(m, (int)lnnz, d_Lptr, d_Lind, cursor, Ui);
+  tc_count<<<ctx->num_sms * 8, kTcThreads, 0, st>>>(units, lists, bins, m, d_Lptr, d_Lind, col,
+                                                    Ui);
+  rc = check_launch(ctx, "apspie_tc", 3);
   if (rc) return rc;
   auto *h = (TcBins *)pinned(ctx, sizeof(TcBins));
   if (!h) return APSPIE_ERR_OOM;

@@ -125,3 +125,41 @@ def test_tc_prepare_hub_rows_across_tiles(ctx, leaves, extra):
     low = np.sort((r * m + c)[c < r])
     assert np.array_equal(lp.cpu().numpy(), np.searchsorted(low // m, np.arange(m + 1)))
     assert np.array_equal(li.cpu().numpy(), low % m)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nnz", [1, 2, 33, 511, 512, 4095, 4096, 4097, 8191, 8192, 8193])
+@pytest.mark.parametrize("n", [3, 256, 257, 100000])
+def test_csr_transpose_small_sorts(ctx, nnz, n):
+    """Entry and column counts around the one-block sort and scan, one to
+    three digit passes, with columns that repeat."""
+    import torch
+    rng = np.random.default_rng(nnz + n)
+    m = 50
+    rows = np.sort(rng.integers(0, m, size=nnz))
+    ind = rng.integers(0, n, size=nnz).astype(np.int32)
+    ptr = np.searchsorted(rows, np.arange(m + 1)).astype(np.int32)
+    val = rng.random(nnz, dtype=np.float32)
+    t = lambda x: torch.from_numpy(x).cuda()
+    tp, ti, tv = ap.csr_transpose(ctx, m, n, t(ptr), t(ind), t(val))
+    order = np.argsort(ind, kind="stable")
+    assert np.array_equal(tp.cpu().numpy(), np.searchsorted(ind[order], np.arange(n + 1)))
+    assert np.array_equal(ti.cpu().numpy(), rows[order])
+    assert np.array_equal(tv.cpu().numpy(), val[order])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [8190, 8191, 8192, 12287, 12288, 1 << 22, (1 << 22) + 5])
+def test_offset_scan_sizes(ctx, n):
+    """The offset scan around its one-launch, few-tile and many-tile forms:
+    the offsets of a transpose with n columns."""
+    import torch
+    rng = np.random.default_rng(n)
+    ind = rng.integers(0, n, size=5000).astype(np.int32)
+    ind[:3] = (0, n - 1, n // 2)
+    t = lambda x: torch.from_numpy(x).cuda()
+    tp, ti, _ = ap.csr_transpose(ctx, 1, n, t(np.array([0, 5000], np.int32)), t(ind))
+    want = np.zeros(n + 1, np.int64)
+    np.add.at(want, ind + 1, 1)
+    assert np.array_equal(tp.cpu().numpy(), np.cumsum(want))
+    assert int(ti.abs().max()) == 0

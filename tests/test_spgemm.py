@@ -224,3 +224,41 @@ def test_tc_long_rows_both_set_forms(ctx, m):
     keep = src < r.ind
     spread = lambda v: v.astype(np.int64) * ((m - 1) // r.m)
     _tc(ctx, _sym(m, np.stack([spread(src[keep]), spread(r.ind[keep])], axis=1)))
+
+
+def _lower(rows, cols, m):
+    keys = np.unique(np.maximum(rows, cols).astype(np.int64) * m + np.minimum(rows, cols))
+    keys = keys[keys // m != keys % m]
+    return np.searchsorted(keys // m, np.arange(m + 1)).astype(np.int32), \
+        (keys % m).astype(np.int32)
+
+
+@pytest.mark.parametrize("m,case", [(300, "dense"), (129, "dense"), (4000, "hub"), (3000, "parts"),
+                                    (70000, "window"), (200000, "hash")])
+def test_tc_any_lower_triangle(ctx, m, case):
+    """L in no degree order: columns and rows around the warp limit of 128, a
+    hub whose row or column spans units, a column longer than a set's part
+    (1,024 entries below the bitmap's ids), ids on both sides of the 2^16
+    largest, against SciPy's sum of (L * L) .* L."""
+    import scipy.sparse as sp
+    import torch
+    import apspie_b200 as ap
+    rng = np.random.default_rng(m)
+    if case == "dense":
+        r, c = np.divmod(np.flatnonzero(rng.random(m * m) < 0.6), m)
+    else:
+        n = {"hub": 4000, "parts": 2600, "window": 3000, "hash": 2500}[case]
+        ids = rng.permutation(m)[:n]
+        r, c = rng.choice(ids, size=(2, 30 * n))
+        hubs = {"hub": [ids.min(), ids.max(), np.sort(ids)[n // 2]], "parts": [ids.min()],
+                "window": [ids.min(), ids.max()], "hash": [ids.min()]}[case]
+        for h in hubs:
+            r, c = np.concatenate([r, np.full(n, h)]), np.concatenate([c, ids])
+    if case == "parts":  # the same graph among the low ids of 200,000
+        m = 200000
+    lp, li = _lower(r, c, m)
+    L = sp.csr_matrix((np.ones(len(li), np.int64), li, lp), shape=(m, m))
+    want = int((L @ L).multiply(L).sum())
+    t = lambda x: torch.from_numpy(x).cuda()
+    assert ap.triangle_count(ctx, m, t(lp), t(li)) == want
+    assert want > 0

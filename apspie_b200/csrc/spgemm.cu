@@ -17,17 +17,20 @@
 //      (spgemm_bitmap_rows<0>), else a 16384-key table (<= 8192 products) or
 //      a dense accumulator in global memory; the distinct columns per row
 //      give nnz(C(i,:)), a scan gives C's row offsets;
-//   2. the block-row bins are re-binned by that exact output size
-//      (rebin_rows): <= 512 / 1024 / 2048 outputs on mid tables of 1024 /
-//      2048 / 4096 slots whose entries are put in column order by an
-//      in-shared bucket sort; longer rows (bitmap case) on the column bitmap,
-//      where a product's position in the column-ordered row is the prefix
-//      popcount of the bitmap up to its column (no sort), values staged in
-//      shared memory (rows of up to 4096 outputs at 512 threads, windows of
-//      16384 positions at 1024 threads for longer ones);
+//   2. numeric rows of up to 4096 products that are not mostly repeats are
+//      sorted: the products' columns and values are gathered into shared
+//      memory, put into column buckets (about one product each) and ranked
+//      inside their bucket, and equal columns are summed
+//      (spgemm_sort_warp_rows, spgemm_sort_rows).  The rest are re-binned by
+//      their exact output size (rebin_rows): <= 512 / 1024 / 2048 outputs on
+//      mid tables of 1024 / 2048 / 4096 slots whose entries are put in column
+//      order by an in-shared bucket sort; longer rows (bitmap case) on the
+//      column bitmap, where a product's position in the column-ordered row is
+//      the prefix popcount of the bitmap up to its column (no sort), values
+//      staged in shared memory (rows of up to 4096 outputs at 512 threads,
+//      windows of 16384 positions at 1024 threads for longer ones);
 //   3. the numeric pass accumulates in double (so the float result is the
-//      correctly rounded exact sum up to double error); warp rows compact
-//      their table and emit by rank in column order.
+//      correctly rounded exact sum up to double error).
 // The bin limits above are those of table load 2 (every table at most half
 // full); at load 4 (apspie_ctx_set_tuning, picked per matrix pair by
 // apspie_autotune_spgemm) each limit is halved and tables are sized to four
@@ -39,9 +42,11 @@
 
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 #include "common.cuh"
 #include "context.h"
+#include "edges.cuh"
 #include "primitives.cuh"
 
 namespace apspie {
@@ -97,31 +102,49 @@ __device__ __forceinline__ int table_insert(int *keys, int bits, int j, bool *fr
 }
 
 // ---------------------------------------------------------- row products ---
-// Eight lanes per row (four rows per warp in flight): most rows of A are
-// short, so a whole warp per row would leave most lanes idle.
-__global__ void row_products(int m, const int *__restrict__ Aptr, const int *__restrict__ Aind,
-                             const int *__restrict__ Bptr, long long *prod) {
-  const int sub = threadIdx.x & 7;
-  const int g = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 3);
-  const int ng = (int)((gridDim.x * blockDim.x) >> 3);
-  const int rounds = (m + ng - 1) / ng;  // the same for every lane: shuffles stay converged
-  for (int rr = 0; rr < rounds; ++rr) {
-    const int i = g + rr * ng;
-    long long acc = 0;
-    if (i < m) {
-      const int a1 = __ldg(Aptr + i + 1);
-      for (int a = __ldg(Aptr + i) + sub; a < a1; a += 8) {
-        const int k = __ldg(Aind + a);
-        acc += __ldg(Bptr + k + 1) - __ldg(Bptr + k);
-      }
+// Over A's entries in tiles of equal size (edges.cuh), the entries of a row in
+// a warp summed by a segmented scan and added to the zeroed prod with one
+// atomic.  (Eight lanes per row waited for the rows of thousands of entries:
+// 97 us for 4.2 M entries.)
+__global__ void __launch_bounds__(kEdgeThreads)
+row_products(int m, int nnz, const int *__restrict__ Aptr, const int *__restrict__ Aind,
+             const int *__restrict__ Bptr, unsigned long long *prod) {
+  __shared__ __align__(16) int s_row[kEdgeTile];
+  const int k0 = (int)blockIdx.x * kEdgeTile;
+  const int n = min(kEdgeTile, min(nnz, __ldg(Aptr + m)) - k0);
+  if (n <= 0) return;
+  edge_tile_rows(Aptr, m, k0, n, s_row);
+  const int lane = lane_id();
+  constexpr int kFly = 4;  // entries per thread in flight
+  for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kFly * kEdgeThreads) {
+    int k[kFly], d[kFly], row[kFly];
+#pragma unroll
+    for (int q = 0; q < kFly; ++q) {
+      const int t = t0 + q * kEdgeThreads;
+      row[q] = t < n ? s_row[t] : -1;
+      k[q] = t < n ? __ldg(Aind + k0 + t) : -1;
     }
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
-    if (i < m && sub == 0) prod[i] = acc;
+    for (int q = 0; q < kFly; ++q) d[q] = k[q] >= 0 ? __ldg(Bptr + k[q] + 1) - __ldg(Bptr + k[q]) : 0;
+#pragma unroll
+    for (int q = 0; q < kFly; ++q) {
+      int leader;
+      const unsigned peers = row_peers(row[q], &leader);
+      unsigned long long sum = (unsigned long long)d[q];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(kFull, sum, o);
+        if (lane - o >= leader) sum += y;
+      }
+      const int last = 31 - __clz(peers);
+      if (lane == last && row[q] >= 0 && sum) atomicAdd(prod + row[q], sum);
+    }
   }
 }
 
-// Row bins.  Symbolic phase, by products: warp rows, two sizes of
+// Row bins.  (The numeric phase sorts rows of up to 256 products a warp each,
+// and of up to 1024 / 2048 / 4096 products a block of 128 / 256 / 512 each.)
+// Symbolic phase, by products: warp rows, two sizes of
 // mid rows (hash tables of 2048 / 8192 keys), block rows (bitmap or a
 // 16384-key table), dense rows (hash mode only).  Numeric phase, by the
 // exact output size of the non-warp rows: three mid sizes (tables of
@@ -138,6 +161,9 @@ enum {
   kBinN3,
   kBinN4,
   kBinN5,
+  kBinS1,
+  kBinS2,
+  kBinS3,
   kNumBins
 };
 constexpr int kMid1MaxProd = 1024;
@@ -442,106 +468,311 @@ __device__ __forceinline__ void bitonic_sort(int *keys, double *vals, int n) {
 }
 
 // ------------------------------------------------------------ warp rows ---
-// Writes the warp's compacted row (keys[0..fill) distinct, keys[fill..fill4)
-// padded with kEmpty) to C in column order: lane l holds entries l, l + 32,
-// ..., (P of them) and counts, over the whole row read four keys at a time
-// (broadcast loads), the keys below each; that count is the entry's place.
-template <int P>
-__device__ __forceinline__ void rank_emit(const int *keys, const double *vals, int fill,
-                                          int fill4, int n, int *ci, float *cv) {
-  const int lane = lane_id();
-  int myk[P], rk[P];
-#pragma unroll
-  for (int q = 0; q < P; ++q) {
-    const int e = lane + 32 * q;
-    myk[q] = e < fill ? keys[e] : kEmpty;
-    rk[q] = 0;
-  }
-  const int4 *k4 = reinterpret_cast<const int4 *>(keys);
-  for (int f = 0; f < (fill4 >> 2); ++f) {
-    const int4 x = k4[f];
-#pragma unroll
-    for (int q = 0; q < P; ++q)
-      rk[q] += (x.x < myk[q]) + (x.y < myk[q]) + (x.z < myk[q]) + (x.w < myk[q]);
-  }
-#pragma unroll
-  for (int q = 0; q < P; ++q) {
-    const int e = lane + 32 * q;
-    if (e < fill && rk[q] < n) {
-      ci[rk[q]] = myk[q];
-      cv[rk[q]] = (float)vals[e];
-    }
-  }
-}
-
-template <bool NUMERIC>
 __global__ void __launch_bounds__(32 * kWarpsPerBlockSmall)
 spgemm_warp_rows(const int *list, const unsigned *nlist, const long long *prod,
                  const int *__restrict__ Aptr, const int *__restrict__ Aind,
-                 const float *__restrict__ Aval, const int *__restrict__ Bptr,
-                 const int *__restrict__ Bind, const float *__restrict__ Bval, int *cnt,
-                 const int *Cptr, int *Cind, float *Cval, int load) {
+                 const int *__restrict__ Bptr, const int *__restrict__ Bind, int *cnt, int load) {
   __shared__ int s_keys[kWarpsPerBlockSmall][kWarpTable];
-  __shared__ double s_vals[NUMERIC ? kWarpsPerBlockSmall : 1][NUMERIC ? kWarpTable : 1];
   __shared__ int s_off[kWarpsPerBlockSmall][32], s_bs[kWarpsPerBlockSmall][32];
   __shared__ float s_av[kWarpsPerBlockSmall][32];
   const int w = warp_in_block(), lane = lane_id();
   int *keys = s_keys[w];
-  double *vals = NUMERIC ? s_vals[w] : nullptr;
   const unsigned nrows = *nlist;
   for (unsigned r = blockIdx.x * kWarpsPerBlockSmall + w; r < nrows;
        r += gridDim.x * kWarpsPerBlockSmall) {
     int i = list[r];
     int bits = table_bits(prod[i], 9, load);
     int T = 1 << bits;
-    for (int t = lane; t < T; t += 32) {
-      keys[t] = kEmpty;
-      if (NUMERIC) vals[t] = 0.0;
-    }
+    for (int t = lane; t < T; t += 32) keys[t] = kEmpty;
     __syncwarp();
     int fresh_count = 0;
-    for_each_product<true>(i, Aptr, Aind, Aval, Bptr, Bind, Bval, s_off[w], s_bs[w], s_av[w],
-                           [&](int j, double v) {
+    for_each_product<true>(i, Aptr, Aind, nullptr, Bptr, Bind, nullptr, s_off[w], s_bs[w], s_av[w],
+                           [&](int j, double) {
                              bool fresh;
-                             int h = table_insert(keys, bits, j, &fresh);
+                             table_insert(keys, bits, j, &fresh);
                              fresh_count += fresh;
-                             if (NUMERIC && h >= 0) atomicAdd(vals + h, v);
                            });
     __syncwarp();
-    if (!NUMERIC) {
-      int c = warp_sum(fresh_count);
-      if (lane == 0) cnt[i] = c;
-    } else {
-      // compact the occupied slots to the front (in place: a slot moves
-      // only left, and each chunk of 32 is read before it is written), pad
-      // to a power of two and sort that instead of the whole table
-      int base = Cptr[i], n = Cptr[i + 1] - base;
-      int fill = 0;
-      for (int t0 = 0; t0 < T; t0 += 32) {
-        const int k = keys[t0 + lane];
-        const double v = vals[t0 + lane];
-        const unsigned occ = __ballot_sync(kFull, k != kEmpty);
-        __syncwarp();
-        if (k != kEmpty) {
-          const int d = fill + __popc(occ & ((1u << lane) - 1u));
-          keys[d] = k;
-          vals[d] = v;
-        }
-        fill += __popc(occ);
-        __syncwarp();
+    const int c = warp_sum(fresh_count);
+    if (lane == 0) cnt[i] = c;
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------- sorted rows ---
+// A row's products sorted by column: a warp (SIZE 32, up to 256 products) or
+// a block (SIZE threads, up to 8 x SIZE products) per row.  Bound by
+// instructions and shared-memory round trips: most products have a column of
+// their own, so a product costs its gather, one shared atomic that counts its
+// bucket and numbers it in it, a move, and about one comparison inside the
+// bucket.  (The hash tables cost a compare-and-swap insert, an emulated
+// double atomic, and passes over two to four slots per entry before their own
+// bucket sort: 390 thread instructions a product.)
+constexpr int kSortPer = 8;         // products per thread
+constexpr int kSortBucketMax = 48;  // fuller buckets: bitonic sort instead
+
+template <int SIZE>
+__device__ __forceinline__ void group_sync() {
+  if (SIZE == 32) __syncwarp(); else __syncthreads();
+}
+
+template <int SIZE>
+__device__ __forceinline__ int group_tid() {
+  return SIZE == 32 ? lane_id() : (int)threadIdx.x;
+}
+
+template <int SIZE>
+__device__ __forceinline__ int group_excl_scan(int v, int *sw, int *total) {
+  if (SIZE == 32) {
+    const int incl = warp_incl_scan(v);
+    *total = __shfl_sync(kFull, incl, 31);
+    return incl - v;
+  }
+  return block_excl_scan(v, sw, total);
+}
+
+template <int SIZE>
+__device__ __forceinline__ unsigned group_min(unsigned v, unsigned *sw) {
+  v = __reduce_min_sync(kFull, v);
+  if (SIZE == 32) return v;
+  if (lane_id() == 0) sw[warp_in_block()] = v;
+  __syncthreads();
+  v = sw[0];
+#pragma unroll
+  for (int w = 1; w < SIZE / 32; ++w) v = min(v, sw[w]);
+  __syncthreads();
+  return v;
+}
+
+// Sorts the np products (scol, sval)[0..np) by column, sums equal columns and
+// writes the row's n outputs to ci / cv.  scnt: 8 * SIZE + 1 ints.  The row's
+// length n from the symbolic phase bounds every write (it is the number of
+// distinct columns unless A or B changed structure in between).
+template <int SIZE>
+__device__ __forceinline__ void sort_row(int np, int n, int *scol, double *sval, int *scnt,
+                                         int *sw, int *__restrict__ ci, float *__restrict__ cv) {
+  const int tid = group_tid<SIZE>();
+  unsigned c[kSortPer];
+  double v[kSortPer];
+  int rk[kSortPer];
+  unsigned lo = ~0u, nhi = ~0u;
+#pragma unroll
+  for (int q = 0; q < kSortPer; ++q) {
+    const int e = q * SIZE + tid;
+    c[q] = e < np ? (unsigned)scol[e] : 0u;
+    v[q] = e < np ? sval[e] : 0.0;
+    if (e < np) {
+      lo = min(lo, c[q]);
+      nhi = min(nhi, ~c[q]);
+    }
+  }
+  lo = group_min<SIZE>(lo, (unsigned *)sw);
+  const unsigned range = ~group_min<SIZE>(nhi, (unsigned *)sw) - lo;
+  // buckets of 2^shift columns over the row's own range: as many buckets as
+  // products or up to twice that
+  int nb = SIZE;
+  while (nb < np) nb <<= 1;
+  int shift = 0;
+  while ((range >> shift) >= (unsigned)nb) ++shift;
+  for (int t = tid; t <= nb; t += SIZE) scnt[t] = 0;
+  group_sync<SIZE>();
+  bool full = false;
+#pragma unroll
+  for (int q = 0; q < kSortPer; ++q) {
+    rk[q] = 0;
+    if (q * SIZE + tid < np) rk[q] = atomicAdd(scnt + ((c[q] - lo) >> shift), 1);
+    full |= rk[q] >= kSortBucketMax;
+  }
+  bool sorted = true;
+  if (SIZE == 32 ? __any_sync(kFull, full) : __syncthreads_or(full)) {
+    int n2 = SIZE;
+    while (n2 < np) n2 <<= 1;
+    for (int e = np + tid; e < n2; e += SIZE) scol[e] = kEmpty;
+    group_sync<SIZE>();
+    bitonic_sort<SIZE == 32>(scol, sval, n2);
+  } else {
+    // bucket counts -> bucket starts, nb / SIZE consecutive buckets a thread
+    const int per = nb / SIZE;
+    int sum = 0;
+    group_sync<SIZE>();
+    for (int q = 0; q < per; ++q) sum += scnt[tid * per + q];
+    int total;
+    int run = group_excl_scan<SIZE>(sum, sw, &total);
+    for (int q = 0; q < per; ++q) {
+      const int x = scnt[tid * per + q];
+      scnt[tid * per + q] = run;
+      run += x;
+    }
+    if (tid == SIZE - 1) scnt[nb] = run;
+    group_sync<SIZE>();
+#pragma unroll
+    for (int q = 0; q < kSortPer; ++q)
+      if (q * SIZE + tid < np) {
+        const int at = scnt[(c[q] - lo) >> shift] + rk[q];
+        scol[at] = (int)c[q];
+        sval[at] = v[q];
       }
-      // pad to a multiple of four with keys that compare above every column
-      const int fill4 = (fill + 3) & ~3;
-      if (fill + lane < fill4) keys[fill + lane] = kEmpty;
-      __syncwarp();
-      // each entry's rank among the row's (distinct) columns is its place in C
-      const int per = (fill + 31) >> 5;
-      if (per <= 1) rank_emit<1>(keys, vals, fill, fill4, n, Cind + base, Cval + base);
-      else if (per <= 2) rank_emit<2>(keys, vals, fill, fill4, n, Cind + base, Cval + base);
-      else if (per <= 4) rank_emit<4>(keys, vals, fill, fill4, n, Cind + base, Cval + base);
-      else rank_emit<8>(keys, vals, fill, fill4, n, Cind + base, Cval + base);
+    group_sync<SIZE>();
+    // rank inside the bucket; the columns are in place when none repeats
+    sorted = false;
+#pragma unroll
+    for (int q = 0; q < kSortPer; ++q) {
+      const int e = q * SIZE + tid;
+      if (e < np) {
+        c[q] = (unsigned)scol[e];
+        v[q] = sval[e];
+        const int b = (int)((c[q] - lo) >> shift);
+        const int b0 = scnt[b], b1 = scnt[b + 1];
+        int r = b0;
+        for (int k = b0; k < b1; ++k) {
+          const unsigned x = (unsigned)scol[k];
+          r += (x < c[q] || (x == c[q] && k < e)) ? 1 : 0;
+        }
+        rk[q] = r;
+        if (np == n) {
+          ci[r] = (int)c[q];
+          cv[r] = (float)(0.0 + v[q]);
+        }
+      }
+    }
+  }
+  if (np != n || sorted) {
+    if (!sorted) {
+      group_sync<SIZE>();
+#pragma unroll
+      for (int q = 0; q < kSortPer; ++q)
+        if (q * SIZE + tid < np) {
+          scol[rk[q]] = (int)c[q];
+          sval[rk[q]] = v[q];
+        }
+      group_sync<SIZE>();
+    }
+    // runs of equal columns, kSortPer consecutive products a thread
+    const int e0 = tid * kSortPer;
+    int heads = 0;
+#pragma unroll
+    for (int q = 0; q < kSortPer; ++q) {
+      const int e = e0 + q;
+      heads += e < np && (e == 0 || scol[e] != scol[e - 1]) ? 1 : 0;
+    }
+    int total;
+    int at = group_excl_scan<SIZE>(heads, sw, &total);
+#pragma unroll 1
+    for (int q = 0; q < kSortPer; ++q) {
+      const int e = e0 + q;
+      if (e >= np || (e > 0 && scol[e] == scol[e - 1])) continue;
+      const int col = scol[e];
+      double sum = 0.0;
+      for (int k = e; k < np && scol[k] == col; ++k) sum += sval[k];
+      if (at < n) {
+        ci[at] = col;
+        cv[at] = (float)sum;
+      }
+      ++at;
+    }
+  }
+  group_sync<SIZE>();
+}
+
+constexpr int kSortWarps = 4;  // rows per block of the warp version
+constexpr int kSortWarpCap = 32 * kSortPer;
+
+__global__ void __launch_bounds__(32 * kSortWarps)
+spgemm_sort_warp_rows(const int *list, const unsigned *nlist, const long long *prod,
+                      const int *__restrict__ Aptr, const int *__restrict__ Aind,
+                      const float *__restrict__ Aval, const int *__restrict__ Bptr,
+                      const int *__restrict__ Bind, const float *__restrict__ Bval,
+                      const int *__restrict__ Cptr, int *Cind, float *Cval) {
+  __shared__ double s_val[kSortWarps][kSortWarpCap];
+  __shared__ int s_col[kSortWarps][kSortWarpCap], s_cnt[kSortWarps][kSortWarpCap + 1];
+  const int w = warp_in_block(), lane = lane_id();
+  int *scol = s_col[w];
+  double *sval = s_val[w];
+  const unsigned nrows = *nlist;
+  for (unsigned r = blockIdx.x * kSortWarps + w; r < nrows; r += gridDim.x * kSortWarps) {
+    const int i = __ldg(list + r);
+    const int a0 = __ldg(Aptr + i), a1 = __ldg(Aptr + i + 1);
+    const int base = __ldg(Cptr + i), n = __ldg(Cptr + i + 1) - base;
+    const int np = min((int)prod[i], kSortWarpCap);
+    int pb = 0;  // products of the row before this chunk of A's entries
+    for (int c0 = a0; c0 < a1; c0 += 32) {
+      int bs = 0, d = 0;
+      float av = 0.f;
+      if (c0 + lane < a1) {
+        const int k = __ldg(Aind + c0 + lane);
+        av = Aval ? __ldg(Aval + c0 + lane) : 1.0f;
+        bs = __ldg(Bptr + k);
+        d = __ldg(Bptr + k + 1) - bs;
+      }
+      const int incl = warp_incl_scan(d), excl = incl - d;
+      const int total = __shfl_sync(kFull, incl, 31);
+      for (int e0 = 0; e0 < total; e0 += 64) {
+        int b[2];
+        float x[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int e = e0 + 32 * q + lane;
+          const int owner = warp_owner(excl, e);
+          b[q] = __shfl_sync(kFull, bs - excl, owner) + e;
+          x[q] = __shfl_sync(kFull, av, owner);
+        }
+        int j[2];
+        float y[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const bool on = e0 + 32 * q + lane < total;
+          j[q] = on ? __ldg(Bind + b[q]) : 0;
+          y[q] = on && Bval ? __ldg(Bval + b[q]) : 1.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int e = e0 + 32 * q + lane;
+          if (e < total && pb + e < np) {
+            scol[pb + e] = j[q];
+            sval[pb + e] = (double)x[q] * (double)y[q];
+          }
+        }
+      }
+      pb += total;
     }
     __syncwarp();
+    sort_row<32>(np, n, scol, sval, s_cnt[w], nullptr, Cind + base, Cval + base);
+  }
+}
+
+template <int TPB>
+constexpr size_t sort_smem() {
+  return (size_t)TPB * kSortPer * (sizeof(double) + 2 * sizeof(int)) + 16;
+}
+
+template <int TPB>
+__global__ void __launch_bounds__(TPB, 1024 / TPB)
+spgemm_sort_rows(const int *list, const unsigned *nlist, const long long *prod,
+                 const int *__restrict__ Aptr, const int *__restrict__ Aind,
+                 const float *__restrict__ Aval, const int *__restrict__ Bptr,
+                 const int *__restrict__ Bind, const float *__restrict__ Bval,
+                 const int *__restrict__ Cptr, int *Cind, float *Cval) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  constexpr int CAP = TPB * kSortPer;
+  double *sval = (double *)dyn;
+  int *scol = (int *)(sval + CAP);
+  int *scnt = scol + CAP;  // CAP + 1
+  __shared__ int s_off[TPB], s_bs[TPB];
+  __shared__ float s_av[TPB];
+  __shared__ int sw[33];
+  const unsigned nrows = *nlist;
+  for (unsigned r = blockIdx.x; r < nrows; r += gridDim.x) {
+    const int i = __ldg(list + r);
+    const int base = __ldg(Cptr + i), n = __ldg(Cptr + i + 1) - base;
+    const int np = min((int)prod[i], CAP);
+    for_each_product_lbs<TPB>(i, Aptr, Aind, Aval, Bptr, Bind, Bval, s_off, s_bs, s_av,
+                              [&](int j, double v, int q) {
+                                if (q < np) {
+                                  scol[q] = j;
+                                  sval[q] = v;
+                                }
+                              });
+    sort_row<TPB>(np, n, scol, sval, scnt, sw, Cind + base, Cval + base);
   }
 }
 
@@ -995,7 +1226,13 @@ __global__ void rebin_rows(int m, int *lists, SpgState *st, const int *cnt, bool
     const unsigned k = r < n1 ? r : (r < n1 + n2 ? r - n1 : r - n1 - n2);
     const int i = lists[(size_t)src * m + k];
     const int c = cnt[i];
-    const int b = c <= lim.n1   ? kBinN1
+    const long long p = prod[i];
+    // sorted when the products fit a block and are not mostly repeats (a
+    // sorted repeat costs a slot and a comparison, a hashed one an add)
+    const int b = p <= 8 * 512 && p <= 2ll * c ? (p <= 8 * 128   ? kBinS1
+                                                  : p <= 8 * 256 ? kBinS2
+                                                                 : kBinS3)
+                  : c <= lim.n1   ? kBinN1
                   : c <= lim.n2 ? kBinN2
                   : c <= lim.n3 ? kBinN3
                   : (!bitmap || c <= kStageSmem) ? kBinN4
@@ -1067,8 +1304,11 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   int rc0 = check_cuda(ctx, cudaMemsetAsync(sst, 0, sizeof(SpgState), st), "spgemm bins");
   if (rc0) return rc0;
   if (m > 0) {
-    row_products<<<gridsz(ctx, (long long)m * 32, 256), 256, 0, st>>>(m, A->d_ptr, A->d_ind,
-                                                                      B->d_ptr, prod);
+    cudaMemsetAsync(prod, 0, sizeof(long long) * (size_t)m, st);
+    if (A->nnz > 0)
+      row_products<<<edge_tiles(A->nnz), kEdgeThreads, 0, st>>>(
+          m, (int)std::min<int64_t>(A->nnz, INT_MAX), A->d_ptr, A->d_ind, B->d_ptr,
+          (unsigned long long *)prod);
     bin_rows<<<gridsz(ctx, m, 256), 256, 0, st>>>(m, prod, lists, sst, cnt, bitmap, lim);
     int rc = check_launch(ctx, "spgemm bin", 2);
     if (rc) return rc;
@@ -1121,10 +1361,9 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   const unsigned *nb = sst->n;
   int launches = 0;
   if (hb.n[kBinWarp]) {
-    spgemm_warp_rows<false><<<gridsz(ctx, hb.n[kBinWarp], kWarpsPerBlockSmall, 64),
-                              32 * kWarpsPerBlockSmall, 0, st>>>(
-        L(kBinWarp), nb + kBinWarp, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
-        nullptr, cnt, nullptr, nullptr, nullptr, load);
+    spgemm_warp_rows<<<gridsz(ctx, hb.n[kBinWarp], kWarpsPerBlockSmall, 64),
+                       32 * kWarpsPerBlockSmall, 0, st>>>(
+        L(kBinWarp), nb + kBinWarp, prod, A->d_ptr, A->d_ind, B->d_ptr, B->d_ind, cnt, load);
     ++launches;
   }
   if (hb.n[kBinMid1]) {
@@ -1239,6 +1478,8 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
   auto L = [&](int b) { return lists + (size_t)b * m; };
   const unsigned *nb = sst->n;
   const size_t dyn_num = sizeof(double) * kBlockTable + sizeof(int) * kBlockTable;
+  cudaFuncSetAttribute(spgemm_sort_rows<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sort_smem<512>());
   cudaFuncSetAttribute(spgemm_block_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)dyn_num);
   cudaFuncSetAttribute(spgemm_bitmap_rows<1, kSpgThreads>,
@@ -1264,12 +1505,22 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
   int launches = 0;
   // ---- numeric ----
   if (hn[kBinWarp]) {
-    spgemm_warp_rows<true><<<gridsz(ctx, hn[kBinWarp], kWarpsPerBlockSmall, 32),
-                             32 * kWarpsPerBlockSmall, 0, st>>>(
+    spgemm_sort_warp_rows<<<gridsz(ctx, hn[kBinWarp], kSortWarps, 64), 32 * kSortWarps, 0, st>>>(
         L(kBinWarp), nb + kBinWarp, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
-        B->d_val, cnt, Cptr, Cind, Cval, load);
+        B->d_val, Cptr, Cind, Cval);
     ++launches;
   }
+  auto sort_rows = [&](auto tpb, int bin, int per_sm) {
+    constexpr int TPB = decltype(tpb)::value;
+    if (!hn[bin]) return;
+    spgemm_sort_rows<TPB><<<gridsz(ctx, hn[bin], 1, per_sm), TPB, sort_smem<TPB>(), st>>>(
+        L(bin), nb + bin, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind, B->d_val, Cptr,
+        Cind, Cval);
+    ++launches;
+  };
+  sort_rows(std::integral_constant<int, 512>{}, kBinS3, 4);
+  sort_rows(std::integral_constant<int, 256>{}, kBinS2, 8);
+  sort_rows(std::integral_constant<int, 128>{}, kBinS1, 16);
   if (hn[kBinN1]) {
     spgemm_mid_rows<true, 128, 10><<<gridsz(ctx, hn[kBinN1], 1, 12), 128,
                                      mid_smem<128, 10, true>(), st>>>(

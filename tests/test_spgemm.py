@@ -262,3 +262,43 @@ def test_tc_any_lower_triangle(ctx, m, case):
     t = lambda x: torch.from_numpy(x).cuda()
     assert ap.triangle_count(ctx, m, t(lp), t(li)) == want
     assert want > 0
+
+
+@pytest.mark.parametrize("kind", ["spread", "dense", "clustered", "overlap", "one_column"])
+def test_spgemm_sorted_row_sizes(ctx, kind):
+    """Rows with product counts around the sorted numeric kernels' limits (a
+    lane, a warp's 256, blocks of 1024 / 2048 / 4096, the hash and bitmap
+    rows beyond), with columns spread out, consecutive, in one bucket but for
+    one (the bitonic fallback), shared by two rows of B, or all equal."""
+    import apspie_b200 as ap
+    rng = np.random.default_rng(len(kind))
+    n = 60000
+    sizes = [1, 2, 31, 32, 33, 63, 64, 65, 255, 256, 257, 511, 513, 1023, 1024, 1025, 2047, 2048,
+             2049, 4095, 4096, 4097, 5000]
+    arows, acols, brows, bcols = [], [], [], []
+    nb = 0
+    for i, p in enumerate(sizes):
+        if kind == "one_column":  # p rows of B with the same single column
+            parts = [np.array([n // 3])] * p
+        elif kind == "overlap" and p > 1:
+            cols = rng.choice(n, size=3 * ((p + 3) // 4), replace=False)
+            parts = [cols[: p // 2], cols[len(cols) - (p - p // 2):]]
+        elif kind == "dense":
+            parts = [np.arange(p) + 7 * i]
+        elif kind == "clustered":
+            parts = [np.append(np.arange(p - 1), n - 1)]
+        else:
+            parts = [rng.choice(n, size=p, replace=False)]
+        for part in parts:
+            arows.append(i)
+            acols.append(nb)
+            brows.append(np.full(len(part), nb))
+            bcols.append(rng.permutation(part))  # rows of B need not be sorted
+            nb += 1
+    A = ap.from_edges(len(sizes), np.array(arows), np.array(acols))
+    A.ncols = nb
+    B = ap.from_edges(nb, np.concatenate(brows), np.concatenate(bcols))
+    B.ncols = n
+    A.w_f32 = rng.uniform(-1, 1, A.nnz).astype(np.float32)
+    B.w_f32 = rng.uniform(-1, 1, B.nnz).astype(np.float32)
+    _check_product(ctx, A, B)

@@ -91,7 +91,7 @@ struct apspie_context {
   const void *spgemm_plan_A = nullptr, *spgemm_plan_B = nullptr;
   int spgemm_plan_m = 0, spgemm_plan_n = 0;
   // row counts of the SpGEMM bins (symbolic and numeric) and, last, the
-  // largest output row staged in global memory
+  // largest output row of the numeric bitmap rows
   unsigned spgemm_plan_bins[16] = {};
   int spgemm_plan_words = 0;  // bitmap words per row (0: hash tables)
   long long spgemm_bitmap_max_cols = 1 << 18;
@@ -185,8 +185,7 @@ enum SlotId : int {
   kSlotSpgVals,
   kSlotSpgStoredBits,  // the symbolic pass's bitmaps of its bitmap rows
   kSlotSpgBitmapSlot,
-  kSlotSpgSpillPos,    // numeric bitmap rows longer than one window: spilled products
-  kSlotSpgSpillVal,
+  kSlotSpgScratch,     // numeric bitmap rows: a row of doubles per block
   kSlotCount
 };
 

@@ -27,8 +27,7 @@
 //      order by an in-shared bucket sort; longer rows (bitmap case) on the
 //      column bitmap, where a product's position in the column-ordered row is
 //      the prefix popcount of the bitmap up to its column (no sort), values
-//      staged in shared memory (rows of up to 4096 outputs at 512 threads,
-//      windows of 16384 positions at 1024 threads for longer ones);
+//      staged in a scratch row in L2;
 //   3. the numeric pass accumulates in double (so the float result is the
 //      correctly rounded exact sum up to double error).
 // The bin limits above are those of table load 2 (every table at most half
@@ -148,8 +147,8 @@ row_products(int m, int nnz, const int *__restrict__ Aptr, const int *__restrict
 // mid rows (hash tables of 2048 / 8192 keys), block rows (bitmap or a
 // 16384-key table), dense rows (hash mode only).  Numeric phase, by the
 // exact output size of the non-warp rows: three mid sizes (tables of
-// 1024 / 2048 / 4096 entries), block rows, bitmap rows staged in global
-// memory.  Bin b's rows are lists[b * m ...].
+// 1024 / 2048 / 4096 entries), block rows (bitmap or a 16384-slot table).
+// Bin b's rows are lists[b * m ...].
 enum {
   kBinWarp = 0,
   kBinMid1,
@@ -160,7 +159,6 @@ enum {
   kBinN2,
   kBinN3,
   kBinN4,
-  kBinN5,
   kBinS1,
   kBinS2,
   kBinS3,
@@ -190,8 +188,7 @@ BinLimits bin_limits(int load, int warp_max_prod) {
 // Device-side counters of one SpGEMM, read back by the host in one copy.
 struct SpgState {
   unsigned n[kNumBins];
-  unsigned maxc;  // largest output row of bin kBinN5
-  unsigned maxp;  // most products of a kBinN5 row longer than one staging window
+  unsigned maxc;  // largest output row of bin kBinN4 over the bitmap
   long long total;  // nnz(C)
 };
 
@@ -372,14 +369,17 @@ __device__ __forceinline__ int block_excl_max(int v, int *sw) {
 // window marks position 0), an inclusive max-scan turns the marks into the
 // owner of every position, and thread t handles positions t and t + TPB --
 // one shared-memory read for the owner, and the loads of B's rows coalesced.
-template <int TPB, int PER = kLbsPer, typename F>
-__device__ __forceinline__ void for_each_product_lbs(int i, const int *__restrict__ Aptr,
+// f(j, value, q, h) handles product q of the row as its thread's h-th of the
+// window; g(h) is called for every h after the block barrier that ends the
+// window.
+template <int TPB, int PER, typename F, typename G>
+__device__ __forceinline__ void for_each_product_window(int i, const int *__restrict__ Aptr,
                                                      const int *__restrict__ Aind,
                                                      const float *__restrict__ Aval,
                                                      const int *__restrict__ Bptr,
                                                      const int *__restrict__ Bind,
                                                      const float *__restrict__ Bval, int *s_off,
-                                                     int *s_bs, float *s_av, F f) {
+                                                        int *s_bs, float *s_av, F f, G g) {
   // PER products per thread per step: the owner map and its max-scan
   // (five block barriers) are paid once per PER * TPB products
   constexpr int CAP = PER * TPB;
@@ -430,14 +430,29 @@ __device__ __forceinline__ void for_each_product_lbs(int i, const int *__restric
           const int o = s_om[q];
           const int b = s_bs[o] + (w0 + q - s_off[o]);
           f(__ldg(Bind + b), (double)s_av[o] * (double)(Bval ? __ldg(Bval + b) : 1.0f),
-            pb + w0 + q);
+            pb + w0 + q, h);
         }
       }
       __syncthreads();
+#pragma unroll
+      for (int h = 0; h < PER; ++h) g(h);
     }
     pb += total;
     __syncthreads();
   }
+}
+
+template <int TPB, int PER = kLbsPer, typename F>
+__device__ __forceinline__ void for_each_product_lbs(int i, const int *__restrict__ Aptr,
+                                                     const int *__restrict__ Aind,
+                                                     const float *__restrict__ Aval,
+                                                     const int *__restrict__ Bptr,
+                                                     const int *__restrict__ Bind,
+                                                     const float *__restrict__ Bval, int *s_off,
+                                                     int *s_bs, float *s_av, F f) {
+  for_each_product_window<TPB, PER>(
+      i, Aptr, Aind, Aval, Bptr, Bind, Bval, s_off, s_bs, s_av,
+      [&](int j, double v, int q, int) { f(j, v, q); }, [](int) {});
 }
 
 // In-place bitonic sort of (keys, vals)[0..n), n a power of two, ascending.
@@ -556,8 +571,11 @@ __device__ __forceinline__ void sort_row(int np, int n, int *scol, double *sval,
   double v[kSortPer];
   int rk[kSortPer];
   unsigned lo = ~0u, nhi = ~0u;
+  // (the loops over a thread's products leave at the row's length, the same
+  // for the whole group: short rows do not issue the rest)
 #pragma unroll
   for (int q = 0; q < kSortPer; ++q) {
+    if (q * SIZE >= np) break;
     const int e = q * SIZE + tid;
     c[q] = e < np ? (unsigned)scol[e] : 0u;
     v[q] = e < np ? sval[e] : 0.0;
@@ -570,15 +588,14 @@ __device__ __forceinline__ void sort_row(int np, int n, int *scol, double *sval,
   const unsigned range = ~group_min<SIZE>(nhi, (unsigned *)sw) - lo;
   // buckets of 2^shift columns over the row's own range: as many buckets as
   // products or up to twice that
-  int nb = SIZE;
-  while (nb < np) nb <<= 1;
-  int shift = 0;
-  while ((range >> shift) >= (unsigned)nb) ++shift;
+  const int nb = max(SIZE, 1 << (32 - __clz(np - 1)));
+  const int shift = max(0, (32 - __clz((int)range)) - (31 - __clz(nb)));
   for (int t = tid; t <= nb; t += SIZE) scnt[t] = 0;
   group_sync<SIZE>();
   bool full = false;
 #pragma unroll
   for (int q = 0; q < kSortPer; ++q) {
+    if (q * SIZE >= np) break;
     rk[q] = 0;
     if (q * SIZE + tid < np) rk[q] = atomicAdd(scnt + ((c[q] - lo) >> shift), 1);
     full |= rk[q] >= kSortBucketMax;
@@ -606,17 +623,20 @@ __device__ __forceinline__ void sort_row(int np, int n, int *scol, double *sval,
     if (tid == SIZE - 1) scnt[nb] = run;
     group_sync<SIZE>();
 #pragma unroll
-    for (int q = 0; q < kSortPer; ++q)
+    for (int q = 0; q < kSortPer; ++q) {
+      if (q * SIZE >= np) break;
       if (q * SIZE + tid < np) {
         const int at = scnt[(c[q] - lo) >> shift] + rk[q];
         scol[at] = (int)c[q];
         sval[at] = v[q];
       }
+    }
     group_sync<SIZE>();
     // rank inside the bucket; the columns are in place when none repeats
     sorted = false;
 #pragma unroll
     for (int q = 0; q < kSortPer; ++q) {
+      if (q * SIZE >= np) break;
       const int e = q * SIZE + tid;
       if (e < np) {
         c[q] = (unsigned)scol[e];
@@ -624,10 +644,11 @@ __device__ __forceinline__ void sort_row(int np, int n, int *scol, double *sval,
         const int b = (int)((c[q] - lo) >> shift);
         const int b0 = scnt[b], b1 = scnt[b + 1];
         int r = b0;
-        for (int k = b0; k < b1; ++k) {
-          const unsigned x = (unsigned)scol[k];
-          r += (x < c[q] || (x == c[q] && k < e)) ? 1 : 0;
-        }
+        if (b1 - b0 > 1)
+          for (int k = b0; k < b1; ++k) {
+            const unsigned x = (unsigned)scol[k];
+            r += (x < c[q] || (x == c[q] && k < e)) ? 1 : 0;
+          }
         rk[q] = r;
         if (np == n) {
           ci[r] = (int)c[q];
@@ -640,11 +661,13 @@ __device__ __forceinline__ void sort_row(int np, int n, int *scol, double *sval,
     if (!sorted) {
       group_sync<SIZE>();
 #pragma unroll
-      for (int q = 0; q < kSortPer; ++q)
+      for (int q = 0; q < kSortPer; ++q) {
+        if (q * SIZE >= np) break;
         if (q * SIZE + tid < np) {
           scol[rk[q]] = (int)c[q];
           sval[rk[q]] = v[q];
         }
+      }
       group_sync<SIZE>();
     }
     // runs of equal columns, kSortPer consecutive products a thread
@@ -1056,93 +1079,111 @@ spgemm_dense_rows(const int *list, const unsigned *nlist, int n,
 
 // ---------------------------------------------------------- bitmap rows ---
 // One block per row over a bitmap of the W = ceil(ncols / 32) words of C's
-// columns in shared memory.  MODE 0 (symbolic): set a bit per product, the
-// row's size is the popcount.  MODE 1 (numeric): set the bits, then
-// woff[w] = popcount of words [0, w) (a scan over the words), so the product
-// in column j lands at woff[j / 32] + popcount(word & bits below j) of the
-// column-ordered row; its value is added there in a double staging row of
-// scap entries in shared memory and the row is emitted word by word.  A row
-// longer than scap is done in windows of scap positions, one pass over its
-// products per window (products outside the window are skipped), so no
-// value ever goes through a global atomic.  Staging values are cleared as
-// they are emitted and the bits after the last window, so each row starts
-// clean.
-// With gbm (symbolic: store; numeric: load), the symbolic pass keeps each
-// row's finished bitmap in global memory at slot r of its bin (bslot[i] = r)
-// and the numeric pass of a row of more than kStageSmem outputs (always a
-// bitmap row of the symbolic phase) loads it instead of setting the bits
-// again.  With sp_pos / sp_val (numeric, rows longer than one window), the
-// first window's pass also records every product's position and value in
-// the block's spill region of sp_cap entries, and the later windows stream
-// that list instead of gathering the products again.
-constexpr int kStageSmem = 4096;     // 512-thread numeric rows: nnz(C(i,:)) <= this
-constexpr int kStageBig = 16384;     // 1024-thread numeric rows: window of this many
+// columns in shared memory.  Symbolic: set a bit per product, the row's size
+// is the popcount; with gbm the finished bitmap is kept in global memory at
+// slot r of its bin (bslot[i] = r) for the numeric phase.  Numeric: load the
+// bitmap (or set the bits again), woff[w] = popcount of words [0, w) (a scan
+// over the words), so the product in column j belongs to position woff[j /
+// 32] + popcount(word & bits below j) of the column-ordered row.
+//
+// The first product of a position claims it by a bit and stores its value in
+// the block's scratch row in global memory (L2: a scattered 8-byte store);
+// the others, few in most rows, are added by double atomics after the
+// barrier that ends the window they were read in.  The row is then written
+// from the scratch and the bitmap, coalesced.  (A staging row of doubles in
+// shared memory took 128 KB, one block per SM, an emulated double atomic per
+// product, and for rows longer than the stage a pass over a list of spilled
+// products per window: 790 - 890 us on the rows of more than 4096 products
+// of 2^18 power-law A*A, at 35 % issue.)
 constexpr int kBitmapMaxWords = 8192;
-// device memory the symbolic pass may keep its bitmap rows' bitmaps in, and
-// the numeric pass its spilled products in (above: recomputed / re-gathered)
+// device memory the symbolic pass may keep its bitmap rows' bitmaps in
+// (above: the bits are set again)
 constexpr size_t kStoredBitmapBudget = size_t(1) << 30;
-constexpr size_t kSpillBudget = size_t(1) << 30;
 
-template <int MODE, int TPB>
-__global__ void __launch_bounds__(TPB, TPB <= 512 ? 2 : 1)
-spgemm_bitmap_rows(const int *list, const unsigned *nlist, int W,
+__global__ void __launch_bounds__(kSpgThreads, 2)
+spgemm_bitmap_symbolic(const int *list, const unsigned *nlist, int W,
+                       const int *__restrict__ Aptr, const int *__restrict__ Aind,
+                       const int *__restrict__ Bptr, const int *__restrict__ Bind, int *cnt,
+                       unsigned *gbm, int *bslot) {
+  constexpr int TPB = kSpgThreads;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  unsigned *bits = (unsigned *)dyn;
+  __shared__ int s_off[TPB], s_bs[TPB];
+  __shared__ float s_av[TPB];
+  __shared__ int s_wt[TPB / 32];
+  const int tid = threadIdx.x, lane = lane_id(), wi = warp_in_block();
+  for (int t = tid; t < W; t += TPB) bits[t] = 0u;
+  __syncthreads();
+  const unsigned nrows = *nlist;
+  for (unsigned r = blockIdx.x; r < nrows; r += gridDim.x) {
+    const int i = list[r];
+    // bits only: runs of consecutive products per thread measured faster
+    // here than the load-balanced search (one array of B per product)
+    for_each_product<false, true>(i, Aptr, Aind, nullptr, Bptr, Bind, nullptr, s_off, s_bs, s_av,
+                                  [&](int j, double) {
+                                    const unsigned bit = 1u << (j & 31);
+                                    if (!(bits[j >> 5] & bit)) atomicOr(bits + (j >> 5), bit);
+                                  });
+    __syncthreads();
+    int c = 0;
+    unsigned *dst = gbm ? gbm + (size_t)r * W : nullptr;
+    for (int w = tid; w < W; w += TPB) {
+      c += __popc(bits[w]);
+      if (dst) __stcg(dst + w, bits[w]);
+      bits[w] = 0u;
+    }
+    if (gbm && tid == 0) bslot[i] = (int)r;
+    c = warp_sum(c);
+    if (lane == 0) s_wt[wi] = c;
+    __syncthreads();
+    if (tid == 0) {
+      int tot = 0;
+      for (int k = 0; k < TPB / 32; ++k) tot += s_wt[k];
+      cnt[i] = tot;
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kSpgThreads, 2)
+spgemm_bitmap_rows(const int *list, const unsigned *nlist, int W, int claim_words,
                    const int *__restrict__ Aptr, const int *__restrict__ Aind,
                    const float *__restrict__ Aval, const int *__restrict__ Bptr,
-                   const int *__restrict__ Bind, const float *__restrict__ Bval, int *cnt,
-                   const int *Cptr, int *Cind, float *Cval, int scap, unsigned *gbm,
-                   int *bslot, const long long *prod, int *sp_pos, double *sp_val, int sp_cap) {
+                   const int *__restrict__ Bind, const float *__restrict__ Bval,
+                   const int *__restrict__ Cptr, int *Cind, float *Cval, const unsigned *gbm,
+                   const int *bslot, double *scratch) {
+  constexpr int TPB = kSpgThreads;
   extern __shared__ __align__(16) unsigned char dyn[];
   unsigned *bits = (unsigned *)dyn;
   int *woff = (int *)(bits + W);
-  double *stage = (double *)(dyn + (size_t)8 * ((W + 1) & ~1));
+  unsigned *claim = (unsigned *)(woff + W);
   __shared__ int s_off[TPB], s_bs[TPB];
   __shared__ float s_av[TPB];
   __shared__ int s_wt[33];
   const int tid = threadIdx.x, lane = lane_id(), wi = warp_in_block();
   constexpr int nw = TPB / 32;
-  for (int t = tid; t < W; t += TPB) bits[t] = 0u;
-  if (MODE == 1)
-    for (int t = tid; t < scap; t += TPB) stage[t] = 0.0;
-  __syncthreads();
+  double *row = scratch + (size_t)blockIdx.x * claim_words * 32;
   // warp wi scans words [ws, we)
   const int seg = ((W + nw - 1) / nw + 31) & ~31;
   const int ws = min(W, wi * seg), we = min(W, ws + seg);
   const unsigned nrows = *nlist;
   for (unsigned r = blockIdx.x; r < nrows; r += gridDim.x) {
     const int i = list[r];
-    if (MODE == 1 && gbm) {
-      // the symbolic pass's bitmap of this row
-      const unsigned *src = gbm + (size_t)bslot[i] * W;
-      for (int w = tid; w < W; w += TPB) bits[w] = __ldcg(src + w);
-    } else {
-      // bits only: runs of consecutive products per thread measured faster
-      // here than the load-balanced search (one array of B per product)
+    const int base = __ldg(Cptr + i);
+    // the row's length from the symbolic phase bounds every position (it
+    // equals the popcount unless A or B changed structure in between)
+    const int len = min(__ldg(Cptr + i + 1) - base, claim_words * 32);
+    const unsigned *src = gbm ? gbm + (size_t)bslot[i] * W : nullptr;
+    for (int w = tid; w < W; w += TPB) bits[w] = src ? __ldcg(src + w) : 0u;
+    for (int w = tid; w < claim_words; w += TPB) claim[w] = 0u;
+    __syncthreads();
+    if (!src) {
       for_each_product<false, true>(i, Aptr, Aind, nullptr, Bptr, Bind, nullptr, s_off, s_bs,
                                     s_av, [&](int j, double) {
                                       const unsigned bit = 1u << (j & 31);
                                       if (!(bits[j >> 5] & bit)) atomicOr(bits + (j >> 5), bit);
                                     });
-    }
-    __syncthreads();
-    if (MODE == 0) {
-      int c = 0;
-      unsigned *dst = gbm ? gbm + (size_t)r * W : nullptr;
-      for (int w = tid; w < W; w += TPB) {
-        c += __popc(bits[w]);
-        if (dst) __stcg(dst + w, bits[w]);
-        bits[w] = 0u;
-      }
-      if (gbm && tid == 0) bslot[i] = (int)r;
-      c = warp_sum(c);
-      if (lane == 0) s_wt[wi] = c;
       __syncthreads();
-      if (tid == 0) {
-        int tot = 0;
-        for (int k = 0; k < nw; ++k) tot += s_wt[k];
-        cnt[i] = tot;
-      }
-      __syncthreads();
-      continue;
     }
     int carry = 0;
     for (int w0 = ws; w0 < we; w0 += 32) {
@@ -1163,54 +1204,38 @@ spgemm_bitmap_rows(const int *list, const unsigned *nlist, int W,
     const int add = s_wt[wi];
     for (int w = ws + lane; w < we; w += 32) woff[w] += add;
     __syncthreads();
-    // the row's length from the symbolic phase bounds every position (it
-    // equals the popcount unless A or B changed structure in between)
-    const int base = Cptr[i];
-    const int len = Cptr[i + 1] - base;
-    const int np = (int)prod[i];
-    // later windows stream the first window's spilled (position, value) list
-    const bool spill = sp_pos != nullptr && len > scap && np <= sp_cap;
-    int *my_pos = spill ? sp_pos + (size_t)blockIdx.x * sp_cap : nullptr;
-    double *my_val = spill ? sp_val + (size_t)blockIdx.x * sp_cap : nullptr;
-    for (int p0 = 0; p0 < len; p0 += scap) {
-      const int p1 = min(len, p0 + scap);
-      if (p0 == 0 || !spill) {
-        for_each_product_lbs<TPB>(i, Aptr, Aind, Aval, Bptr, Bind, Bval, s_off, s_bs, s_av,
-                                  [&](int j, double v, int q) {
-                                    const int w = j >> 5;
-                                    const int pos =
-                                        woff[w] + __popc(bits[w] & ((1u << (j & 31)) - 1u));
-                                    if (spill && q < np) {
-                                      __stcg(my_pos + q, pos);
-                                      __stcg(my_val + q, v);
-                                    }
-                                    if (pos >= p0 && pos < p1) atomicAdd(stage + (pos - p0), v);
-                                  });
-      } else {
-        for (int q = tid; q < np; q += TPB) {
-          const int pos = __ldcg(my_pos + q);
-          if (pos >= p0 && pos < p1) atomicAdd(stage + (pos - p0), __ldcg(my_val + q));
-        }
-      }
-      __syncthreads();
-      for (int w = tid; w < W; w += TPB) {
-        unsigned b = bits[w];
-        int k = woff[w];
-        if (!b || k >= p1 || k + __popc(b) <= p0) continue;
-        while (b && k < p1) {
-          const int t = __ffs(b) - 1;
-          b &= b - 1;
-          if (k >= p0) {
-            Cind[base + k] = w * 32 + t;
-            Cval[base + k] = (float)stage[k - p0];
-            stage[k - p0] = 0.0;
+    int late[kLbsPer];
+    double lv[kLbsPer];
+#pragma unroll
+    for (int h = 0; h < kLbsPer; ++h) late[h] = -1;
+    for_each_product_window<TPB, kLbsPer>(
+        i, Aptr, Aind, Aval, Bptr, Bind, Bval, s_off, s_bs, s_av,
+        [&](int j, double v, int, int h) {
+          const int w = j >> 5;
+          const int pos = woff[w] + __popc(bits[w] & ((1u << (j & 31)) - 1u));
+          if (pos >= len) return;
+          const unsigned bit = 1u << (pos & 31);
+          if (atomicOr(claim + (pos >> 5), bit) & bit) {
+            late[h] = pos;
+            lv[h] = v;
+          } else {
+            __stcg(row + pos, 0.0 + v);
           }
-          ++k;
-        }
+        },
+        [&](int h) {
+          if (late[h] >= 0) atomicAdd(row + late[h], lv[h]);
+          late[h] = -1;
+        });
+    __syncthreads();
+    for (int k = tid; k < len; k += TPB) Cval[base + k] = (float)__ldcg(row + k);
+    for (int w = tid; w < W; w += TPB) {
+      unsigned b = bits[w];
+      int k = woff[w];
+      while (b && k < len) {
+        Cind[base + k++] = w * 32 + __ffs(b) - 1;
+        b &= b - 1;
       }
-      __syncthreads();
     }
-    for (int w = tid; w < W; w += TPB) bits[w] = 0u;
     __syncthreads();
   }
 }
@@ -1235,13 +1260,9 @@ __global__ void rebin_rows(int m, int *lists, SpgState *st, const int *cnt, bool
                   : c <= lim.n1   ? kBinN1
                   : c <= lim.n2 ? kBinN2
                   : c <= lim.n3 ? kBinN3
-                  : (!bitmap || c <= kStageSmem) ? kBinN4
-                                                 : kBinN5;
+                                : kBinN4;
     lists[(size_t)b * m + warp_bin_slot(st->n, b)] = i;
-    if (b == kBinN5) {
-      atomicMax(&st->maxc, (unsigned)c);
-      if (c > kStageBig) atomicMax(&st->maxp, (unsigned)prod[i]);
-    }
+    if (b == kBinN4 && bitmap) atomicMax(&st->maxc, (unsigned)c);
   }
 }
 
@@ -1325,8 +1346,8 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   const size_t dyn_sym = sizeof(int) * kBlockTable;
   cudaFuncSetAttribute(spgemm_block_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)dyn_sym);
-  cudaFuncSetAttribute(spgemm_bitmap_rows<0, kSpgThreads>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * kBitmapMaxWords));
+  cudaFuncSetAttribute(spgemm_bitmap_symbolic, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(4 * kBitmapMaxWords));
   cudaFuncSetAttribute(spgemm_mid_rows<false, 256, 13>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)mid_smem<256, 13, false>());
@@ -1381,10 +1402,9 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
     ++launches;
   }
   if (hb.n[kBinBlock] && bitmap) {
-    spgemm_bitmap_rows<0, kSpgThreads><<<gridsz(ctx, hb.n[kBinBlock], 1, 4), kSpgThreads,
-                                         (size_t)4 * bwords, st>>>(
-        L(kBinBlock), nb + kBinBlock, bwords, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
-        nullptr, cnt, nullptr, nullptr, nullptr, 0, gbm, bslot, prod, nullptr, nullptr, 0);
+    spgemm_bitmap_symbolic<<<gridsz(ctx, hb.n[kBinBlock], 1, 4), kSpgThreads, (size_t)4 * bwords,
+                             st>>>(L(kBinBlock), nb + kBinBlock, bwords, A->d_ptr, A->d_ind,
+                                   B->d_ptr, B->d_ind, cnt, gbm, bslot);
     ++launches;
   } else if (hb.n[kBinBlock]) {
     spgemm_block_rows<false><<<gridsz(ctx, hb.n[kBinBlock], 1, 4), kSpgThreads, dyn_sym, st>>>(
@@ -1446,7 +1466,6 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   ctx->spgemm_plan_n = n;
   for (int b = 0; b < kNumBins; ++b) ctx->spgemm_plan_bins[b] = hs.n[b];
   ctx->spgemm_plan_bins[kNumBins] = hs.maxc;
-  ctx->spgemm_plan_bins[kNumBins + 1] = hs.maxp;
   ctx->spgemm_plan_gbm = gbm;
   ctx->spgemm_plan_bslot = bslot;
   ctx->spgemm_plan_words = bitmap ? bwords : 0;
@@ -1482,11 +1501,8 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
                        (int)sort_smem<512>());
   cudaFuncSetAttribute(spgemm_block_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)dyn_num);
-  cudaFuncSetAttribute(spgemm_bitmap_rows<1, kSpgThreads>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(8 * kBitmapMaxWords + 8 * kStageSmem + 16));
-  cudaFuncSetAttribute(spgemm_bitmap_rows<1, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(8 * kBitmapMaxWords + 8 * kStageBig + 16));
+  cudaFuncSetAttribute(spgemm_bitmap_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(12 * kBitmapMaxWords));
   cudaFuncSetAttribute(spgemm_mid_rows<true, 256, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)mid_smem<256, 12, true>());
   const unsigned nd = hn[kBinDense];
@@ -1543,43 +1559,26 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
     ++launches;
   }
   if (hn[kBinN4] && bwords) {
-    spgemm_bitmap_rows<1, kSpgThreads><<<gridsz(ctx, hn[kBinN4], 1, 2), kSpgThreads,
-                                         (size_t)8 * ((bwords + 1) & ~1) + 8 * kStageSmem, st>>>(
-        L(kBinN4), nb + kBinN4, bwords, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
-        B->d_val, cnt, Cptr, Cind, Cval, kStageSmem, nullptr, nullptr, prod, nullptr, nullptr,
-        0);
+    // a scratch row of doubles per block, at most 2 MB each; fewer blocks when
+    // the memory for all of them cannot be had
+    const int claim = (maxc + 31) / 32;
+    int g4 = gridsz(ctx, hn[kBinN4], 1, 2);
+    double *scratch = nullptr;
+    for (;; g4 /= 2) {
+      scratch = (double *)workspace(ctx, kSlotSpgScratch,
+                                    sizeof(double) * 32 * (size_t)claim * g4);
+      if (scratch || g4 == 1) break;
+    }
+    if (!scratch) return APSPIE_ERR_OOM;
+    spgemm_bitmap_rows<<<g4, kSpgThreads, (size_t)8 * bwords + 4 * (size_t)claim, st>>>(
+        L(kBinN4), nb + kBinN4, bwords, claim, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
+        B->d_val, Cptr, Cind, Cval, (const unsigned *)ctx->spgemm_plan_gbm,
+        (const int *)ctx->spgemm_plan_bslot, scratch);
     ++launches;
   } else if (hn[kBinN4]) {
     spgemm_block_rows<true><<<gridsz(ctx, hn[kBinN4], 1, 1), kSpgThreads, dyn_num, st>>>(
         L(kBinN4), nb + kBinN4, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
         B->d_val, cnt, Cptr, Cind, Cval, n, load);
-    ++launches;
-  }
-  if (hn[kBinN5]) {
-    // rows longer than kStageSmem: 1024 threads, windows of kStageBig, the
-    // symbolic pass's bitmaps when it kept them; rows longer than one window
-    // spill their products' positions and values in the first window's pass
-    const int scap = std::min(kStageBig, std::max(maxc, 1));
-    const int g5 = gridsz(ctx, hn[kBinN5], 1, 1);
-    const unsigned maxp = hn[kNumBins + 1];
-    int *sp_pos = nullptr;
-    double *sp_val = nullptr;
-    int sp_cap = 0;
-    if (maxp > 0 && (size_t)g5 * maxp * (sizeof(int) + sizeof(double)) <= kSpillBudget) {
-      sp_pos = (int *)workspace(ctx, kSlotSpgSpillPos, sizeof(int) * (size_t)g5 * maxp);
-      sp_val = (double *)workspace(ctx, kSlotSpgSpillVal, sizeof(double) * (size_t)g5 * maxp);
-      if (sp_pos && sp_val) {
-        sp_cap = (int)maxp;
-      } else {  // not spilled: every window gathers the products again
-        sp_pos = nullptr;
-        sp_val = nullptr;
-      }
-    }
-    spgemm_bitmap_rows<1, 1024><<<g5, 1024,
-                                  (size_t)8 * ((bwords + 1) & ~1) + 8 * (size_t)scap, st>>>(
-        L(kBinN5), nb + kBinN5, bwords, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
-        B->d_val, cnt, Cptr, Cind, Cval, scap, (unsigned *)ctx->spgemm_plan_gbm,
-        (int *)ctx->spgemm_plan_bslot, prod, sp_pos, sp_val, sp_cap);
     ++launches;
   }
   if (nd) {

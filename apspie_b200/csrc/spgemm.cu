@@ -162,8 +162,14 @@ enum {
   kBinS1,
   kBinS2,
   kBinS3,
-  kNumBins
+  kNumBins,
+  // counts only: the shorter rows of the bitmap bins, listed from the end of
+  // the bin's list, so that the long ones are handed out first
+  kTailBlock = kNumBins,
+  kTailN4,
+  kNumCounts
 };
+constexpr long long kLongRow = 16384;  // products
 constexpr int kMid1MaxProd = 1024;
 constexpr int kMid2MaxProd = 4096;
 constexpr int kN1MaxNnz = 512, kN2MaxNnz = 1024, kN3MaxNnz = 2048;
@@ -187,10 +193,16 @@ BinLimits bin_limits(int load, int warp_max_prod) {
 
 // Device-side counters of one SpGEMM, read back by the host in one copy.
 struct SpgState {
-  unsigned n[kNumBins];
+  unsigned n[kNumCounts];
+  unsigned grab[kNumBins];  // rows handed out past the first of each block
   unsigned maxc;  // largest output row of bin kBinN4 over the bitmap
   long long total;  // nnz(C)
 };
+
+// Rows of a block kernel: the first by block, then on demand from the bin's
+// counter (grab).  A row's work varies with its products, and fixed shares in
+// list order left some blocks with 1.2 to 1.3 times the mean of a bin of
+// sorted rows and 2.5 times that of the bitmap rows (2^18 power-law A*A).
 
 // Slot of this lane's row in bin b: one atomic per distinct bin of the
 // active lanes (the bins' counters are few and hot).
@@ -216,8 +228,16 @@ __global__ void bin_rows(int m, const long long *prod, int *lists, SpgState *st,
             : p <= lim.mid2 ? kBinMid2
             : (bitmap || p <= lim.block) ? kBinBlock
                                          : kBinDense;
-    lists[(size_t)b * m + warp_bin_slot(st->n, b)] = i;
+    const bool tail = b == kBinBlock && bitmap && p <= kLongRow;
+    const unsigned at = warp_bin_slot(st->n, tail ? kTailBlock : b);
+    lists[(size_t)b * m + (tail ? (unsigned)m - 1u - at : at)] = i;
   }
+}
+
+// Row r of a bin whose list has nfront entries at its front and the rest at
+// its end (m entries in all).
+__device__ __forceinline__ int row_at(const int *list, int m, unsigned nfront, unsigned r) {
+  return r < nfront ? list[r] : list[(unsigned)m - 1u - (r - nfront)];
 }
 
 // Deals the products of row i over `nthreads` threads of a group (a warp or
@@ -770,7 +790,7 @@ constexpr size_t sort_smem() {
 
 template <int TPB>
 __global__ void __launch_bounds__(TPB, 1024 / TPB)
-spgemm_sort_rows(const int *list, const unsigned *nlist, const long long *prod,
+spgemm_sort_rows(const int *list, const unsigned *nlist, unsigned *grab, const long long *prod,
                  const int *__restrict__ Aptr, const int *__restrict__ Aind,
                  const float *__restrict__ Aval, const int *__restrict__ Bptr,
                  const int *__restrict__ Bind, const float *__restrict__ Bval,
@@ -784,7 +804,10 @@ spgemm_sort_rows(const int *list, const unsigned *nlist, const long long *prod,
   __shared__ float s_av[TPB];
   __shared__ int sw[33];
   const unsigned nrows = *nlist;
-  for (unsigned r = blockIdx.x; r < nrows; r += gridDim.x) {
+  __shared__ unsigned s_next[2];
+  unsigned r = blockIdx.x;
+  for (int turn = 0; r < nrows; r = s_next[turn & 1], ++turn) {
+    if (threadIdx.x == 0) s_next[turn & 1] = gridDim.x + atomicAdd(grab, 1u);
     const int i = __ldg(list + r);
     const int base = __ldg(Cptr + i), n = __ldg(Cptr + i + 1) - base;
     const int np = min((int)prod[i], CAP);
@@ -805,7 +828,7 @@ constexpr int kBucketMax = 128;        // fuller buckets: bitonic sort instead
 
 template <bool NUMERIC>
 __global__ void __launch_bounds__(kSpgThreads)
-spgemm_block_rows(const int *list, const unsigned *nlist, const long long *prod,
+spgemm_block_rows(const int *list, const unsigned *nlist, unsigned *grab, const long long *prod,
                   const int *__restrict__ Aptr, const int *__restrict__ Aind,
                   const float *__restrict__ Aval, const int *__restrict__ Bptr,
                   const int *__restrict__ Bind, const float *__restrict__ Bval, int *cnt,
@@ -819,7 +842,10 @@ spgemm_block_rows(const int *list, const unsigned *nlist, const long long *prod,
   const unsigned nrows = *nlist;
   // column buckets of 2^bshift columns, at most kBuckets of them
   const int bshift = bucket_shift(ncols, kBuckets);
-  for (unsigned r = blockIdx.x; r < nrows; r += gridDim.x) {
+  __shared__ unsigned s_next[2];
+  unsigned r = blockIdx.x;
+  for (int turn = 0; r < nrows; r = s_next[turn & 1], ++turn) {
+    if (threadIdx.x == 0) s_next[turn & 1] = gridDim.x + atomicAdd(grab, 1u);
     int i = list[r];
     int bits = table_bits(prod[i], 14, load);
     int T = 1 << bits;
@@ -918,7 +944,7 @@ constexpr size_t mid_smem() {
 
 template <bool NUMERIC, int TPB, int TBITS>
 __global__ void __launch_bounds__(TPB)
-spgemm_mid_rows(const int *list, const unsigned *nlist, const long long *prod,
+spgemm_mid_rows(const int *list, const unsigned *nlist, unsigned *grab, const long long *prod,
                 const int *__restrict__ Aptr, const int *__restrict__ Aind,
                 const float *__restrict__ Aval, const int *__restrict__ Bptr,
                 const int *__restrict__ Bind, const float *__restrict__ Bval, int *cnt,
@@ -939,7 +965,10 @@ spgemm_mid_rows(const int *list, const unsigned *nlist, const long long *prod,
   // column buckets of 2^bshift columns, at most TPB of them (a shift per
   // key instead of a 64-bit division)
   const int bshift = bucket_shift(ncols, TPB);
-  for (unsigned r = blockIdx.x; r < nrows; r += gridDim.x) {
+  __shared__ unsigned s_next[2];
+  unsigned r = blockIdx.x;
+  for (int turn = 0; r < nrows; r = s_next[turn & 1], ++turn) {
+    if (threadIdx.x == 0) s_next[turn & 1] = gridDim.x + atomicAdd(grab, 1u);
     const int i = list[r];
     const int base = NUMERIC ? Cptr[i] : 0;
     const int n = NUMERIC ? Cptr[i + 1] - base : 0;
@@ -1101,7 +1130,8 @@ constexpr int kBitmapMaxWords = 8192;
 constexpr size_t kStoredBitmapBudget = size_t(1) << 30;
 
 __global__ void __launch_bounds__(kSpgThreads, 2)
-spgemm_bitmap_symbolic(const int *list, const unsigned *nlist, int W,
+spgemm_bitmap_symbolic(const int *list, const unsigned *nlist, const unsigned *ntail,
+                       unsigned *grab, int m, int W,
                        const int *__restrict__ Aptr, const int *__restrict__ Aind,
                        const int *__restrict__ Bptr, const int *__restrict__ Bind, int *cnt,
                        unsigned *gbm, int *bslot) {
@@ -1114,9 +1144,12 @@ spgemm_bitmap_symbolic(const int *list, const unsigned *nlist, int W,
   const int tid = threadIdx.x, lane = lane_id(), wi = warp_in_block();
   for (int t = tid; t < W; t += TPB) bits[t] = 0u;
   __syncthreads();
-  const unsigned nrows = *nlist;
-  for (unsigned r = blockIdx.x; r < nrows; r += gridDim.x) {
-    const int i = list[r];
+  const unsigned nfront = *nlist, nrows = nfront + *ntail;
+  __shared__ unsigned s_next[2];
+  unsigned r = blockIdx.x;
+  for (int turn = 0; r < nrows; r = s_next[turn & 1], ++turn) {
+    if (threadIdx.x == 0) s_next[turn & 1] = gridDim.x + atomicAdd(grab, 1u);
+    const int i = row_at(list, m, nfront, r);
     // bits only: runs of consecutive products per thread measured faster
     // here than the load-balanced search (one array of B per product)
     for_each_product<false, true>(i, Aptr, Aind, nullptr, Bptr, Bind, nullptr, s_off, s_bs, s_av,
@@ -1146,7 +1179,8 @@ spgemm_bitmap_symbolic(const int *list, const unsigned *nlist, int W,
 }
 
 __global__ void __launch_bounds__(kSpgThreads, 2)
-spgemm_bitmap_rows(const int *list, const unsigned *nlist, int W, int claim_words,
+spgemm_bitmap_rows(const int *list, const unsigned *nlist, const unsigned *ntail, unsigned *grab,
+                   int m, int W, int claim_words,
                    const int *__restrict__ Aptr, const int *__restrict__ Aind,
                    const float *__restrict__ Aval, const int *__restrict__ Bptr,
                    const int *__restrict__ Bind, const float *__restrict__ Bval,
@@ -1166,9 +1200,12 @@ spgemm_bitmap_rows(const int *list, const unsigned *nlist, int W, int claim_word
   // warp wi scans words [ws, we)
   const int seg = ((W + nw - 1) / nw + 31) & ~31;
   const int ws = min(W, wi * seg), we = min(W, ws + seg);
-  const unsigned nrows = *nlist;
-  for (unsigned r = blockIdx.x; r < nrows; r += gridDim.x) {
-    const int i = list[r];
+  const unsigned nfront = *nlist, nrows = nfront + *ntail;
+  __shared__ unsigned s_next[2];
+  unsigned r = blockIdx.x;
+  for (int turn = 0; r < nrows; r = s_next[turn & 1], ++turn) {
+    if (threadIdx.x == 0) s_next[turn & 1] = gridDim.x + atomicAdd(grab, 1u);
+    const int i = row_at(list, m, nfront, r);
     const int base = __ldg(Cptr + i);
     // the row's length from the symbolic phase bounds every position (it
     // equals the popcount unless A or B changed structure in between)
@@ -1245,11 +1282,12 @@ spgemm_bitmap_rows(const int *list, const unsigned *nlist, int W, int claim_word
 __global__ void rebin_rows(int m, int *lists, SpgState *st, const int *cnt, bool bitmap,
                            BinLimits lim, const long long *prod) {
   const unsigned n1 = st->n[kBinMid1], n2 = st->n[kBinMid2], n3 = st->n[kBinBlock];
-  const unsigned n = n1 + n2 + n3;
+  const unsigned n = n1 + n2 + n3 + st->n[kTailBlock];
   for (unsigned r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
     const int src = r < n1 ? kBinMid1 : (r < n1 + n2 ? kBinMid2 : kBinBlock);
     const unsigned k = r < n1 ? r : (r < n1 + n2 ? r - n1 : r - n1 - n2);
-    const int i = lists[(size_t)src * m + k];
+    const int *list = lists + (size_t)src * m;
+    const int i = src == kBinBlock ? row_at(list, m, n3, k) : list[k];
     const int c = cnt[i];
     const long long p = prod[i];
     // sorted when the products fit a block and are not mostly repeats (a
@@ -1261,7 +1299,9 @@ __global__ void rebin_rows(int m, int *lists, SpgState *st, const int *cnt, bool
                   : c <= lim.n2 ? kBinN2
                   : c <= lim.n3 ? kBinN3
                                 : kBinN4;
-    lists[(size_t)b * m + warp_bin_slot(st->n, b)] = i;
+    const bool tail = b == kBinN4 && bitmap && p <= kLongRow;
+    const unsigned at = warp_bin_slot(st->n, tail ? kTailN4 : b);
+    lists[(size_t)b * m + (tail ? (unsigned)m - 1u - at : at)] = i;
     if (b == kBinN4 && bitmap) atomicMax(&st->maxc, (unsigned)c);
   }
 }
@@ -1343,6 +1383,7 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
     if (rc) return rc;
     hb = *h;
   }
+  const unsigned nblock = hb.n[kBinBlock] + hb.n[kTailBlock];
   const size_t dyn_sym = sizeof(int) * kBlockTable;
   cudaFuncSetAttribute(spgemm_block_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)dyn_sym);
@@ -1368,10 +1409,10 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   // the bitmap rows keep their bitmaps for the numeric phase when they fit
   unsigned *gbm = nullptr;
   int *bslot = nullptr;
-  if (bitmap && hb.n[kBinBlock] > 0 &&
-      (size_t)hb.n[kBinBlock] * bwords * sizeof(unsigned) <= kStoredBitmapBudget) {
+  if (bitmap && nblock > 0 &&
+      (size_t)nblock * bwords * sizeof(unsigned) <= kStoredBitmapBudget) {
     gbm = (unsigned *)workspace(ctx, kSlotSpgStoredBits,
-                                (size_t)hb.n[kBinBlock] * bwords * sizeof(unsigned));
+                                (size_t)nblock * bwords * sizeof(unsigned));
     bslot = (int *)workspace(ctx, kSlotSpgBitmapSlot, sizeof(int) * ((size_t)m + 1));
     if (!gbm || !bslot) {  // not kept: the numeric phase sets the bits again
       gbm = nullptr;
@@ -1380,6 +1421,7 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   }
   // ---- symbolic ----
   const unsigned *nb = sst->n;
+  unsigned *grab = sst->grab;
   int launches = 0;
   if (hb.n[kBinWarp]) {
     spgemm_warp_rows<<<gridsz(ctx, hb.n[kBinWarp], kWarpsPerBlockSmall, 64),
@@ -1390,25 +1432,25 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   if (hb.n[kBinMid1]) {
     spgemm_mid_rows<false, 128, 11><<<gridsz(ctx, hb.n[kBinMid1], 1, 16), 128,
                                       mid_smem<128, 11, false>(), st>>>(
-        L(kBinMid1), nb + kBinMid1, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
+        L(kBinMid1), nb + kBinMid1, grab + kBinMid1, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
         nullptr, cnt, nullptr, nullptr, nullptr, n, load);
     ++launches;
   }
   if (hb.n[kBinMid2]) {
     spgemm_mid_rows<false, 256, 13><<<gridsz(ctx, hb.n[kBinMid2], 1, 6), 256,
                                       mid_smem<256, 13, false>(), st>>>(
-        L(kBinMid2), nb + kBinMid2, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
+        L(kBinMid2), nb + kBinMid2, grab + kBinMid2, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
         nullptr, cnt, nullptr, nullptr, nullptr, n, load);
     ++launches;
   }
-  if (hb.n[kBinBlock] && bitmap) {
-    spgemm_bitmap_symbolic<<<gridsz(ctx, hb.n[kBinBlock], 1, 4), kSpgThreads, (size_t)4 * bwords,
-                             st>>>(L(kBinBlock), nb + kBinBlock, bwords, A->d_ptr, A->d_ind,
-                                   B->d_ptr, B->d_ind, cnt, gbm, bslot);
+  if (nblock && bitmap) {
+    spgemm_bitmap_symbolic<<<gridsz(ctx, nblock, 1, 4), kSpgThreads, (size_t)4 * bwords,
+                             st>>>(L(kBinBlock), nb + kBinBlock, nb + kTailBlock, grab + kBinBlock,
+                                   m, bwords, A->d_ptr, A->d_ind, B->d_ptr, B->d_ind, cnt, gbm, bslot);
     ++launches;
-  } else if (hb.n[kBinBlock]) {
-    spgemm_block_rows<false><<<gridsz(ctx, hb.n[kBinBlock], 1, 4), kSpgThreads, dyn_sym, st>>>(
-        L(kBinBlock), nb + kBinBlock, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
+  } else if (nblock) {
+    spgemm_block_rows<false><<<gridsz(ctx, nblock, 1, 4), kSpgThreads, dyn_sym, st>>>(
+        L(kBinBlock), nb + kBinBlock, grab + kBinBlock, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
         nullptr, cnt, nullptr, nullptr, nullptr, n, load);
     ++launches;
   }
@@ -1428,7 +1470,7 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
     rc = device_exclusive_scan<long long>(ctx, offs, offs, m, d_total);
     if (rc) return rc;
   }
-  const unsigned nre = hb.n[kBinMid1] + hb.n[kBinMid2] + hb.n[kBinBlock];
+  const unsigned nre = hb.n[kBinMid1] + hb.n[kBinMid2] + nblock;
   if (nre) {
     rebin_rows<<<gridsz(ctx, nre, 256), 256, 0, st>>>(m, lists, sst, cnt, bitmap, lim, prod);
     rc = check_launch(ctx, "rebin_rows");
@@ -1464,8 +1506,10 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   ctx->spgemm_plan_B = B->d_ptr;
   ctx->spgemm_plan_m = m;
   ctx->spgemm_plan_n = n;
-  for (int b = 0; b < kNumBins; ++b) ctx->spgemm_plan_bins[b] = hs.n[b];
-  ctx->spgemm_plan_bins[kNumBins] = hs.maxc;
+  static_assert(kNumCounts < (int)(sizeof(ctx->spgemm_plan_bins) / sizeof(unsigned)),
+                "the plan keeps every count and maxc");
+  for (int b = 0; b < kNumCounts; ++b) ctx->spgemm_plan_bins[b] = hs.n[b];
+  ctx->spgemm_plan_bins[kNumCounts] = hs.maxc;
   ctx->spgemm_plan_gbm = gbm;
   ctx->spgemm_plan_bslot = bslot;
   ctx->spgemm_plan_words = bitmap ? bwords : 0;
@@ -1484,7 +1528,7 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
   const int m = A->m, n = B->n;
   cudaStream_t st = ctx->stream;
   const unsigned *hn = ctx->spgemm_plan_bins;
-  const int maxc = (int)hn[kNumBins];
+  const int maxc = (int)hn[kNumCounts];
   const int bwords = ctx->spgemm_plan_words;
   const int load = ctx->spgemm_plan_load;
   // the symbolic phase's buffers (own slots, same sizes: no reallocation;
@@ -1496,6 +1540,8 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
   if (!prod || !lists || !cnt || !sst) return APSPIE_ERR_OOM;
   auto L = [&](int b) { return lists + (size_t)b * m; };
   const unsigned *nb = sst->n;
+  unsigned *grab = sst->grab;
+  cudaMemsetAsync(grab, 0, sizeof(sst->grab), st);
   const size_t dyn_num = sizeof(double) * kBlockTable + sizeof(int) * kBlockTable;
   cudaFuncSetAttribute(spgemm_sort_rows<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sort_smem<512>());
@@ -1530,7 +1576,7 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
     constexpr int TPB = decltype(tpb)::value;
     if (!hn[bin]) return;
     spgemm_sort_rows<TPB><<<gridsz(ctx, hn[bin], 1, per_sm), TPB, sort_smem<TPB>(), st>>>(
-        L(bin), nb + bin, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind, B->d_val, Cptr,
+        L(bin), nb + bin, grab + bin, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind, B->d_val, Cptr,
         Cind, Cval);
     ++launches;
   };
@@ -1540,29 +1586,30 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
   if (hn[kBinN1]) {
     spgemm_mid_rows<true, 128, 10><<<gridsz(ctx, hn[kBinN1], 1, 12), 128,
                                      mid_smem<128, 10, true>(), st>>>(
-        L(kBinN1), nb + kBinN1, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
+        L(kBinN1), nb + kBinN1, grab + kBinN1, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
         B->d_val, cnt, Cptr, Cind, Cval, n, load);
     ++launches;
   }
   if (hn[kBinN2]) {
     spgemm_mid_rows<true, 128, 11><<<gridsz(ctx, hn[kBinN2], 1, 6), 128,
                                      mid_smem<128, 11, true>(), st>>>(
-        L(kBinN2), nb + kBinN2, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
+        L(kBinN2), nb + kBinN2, grab + kBinN2, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
         B->d_val, cnt, Cptr, Cind, Cval, n, load);
     ++launches;
   }
   if (hn[kBinN3]) {
     spgemm_mid_rows<true, 256, 12><<<gridsz(ctx, hn[kBinN3], 1, 3), 256,
                                      mid_smem<256, 12, true>(), st>>>(
-        L(kBinN3), nb + kBinN3, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
+        L(kBinN3), nb + kBinN3, grab + kBinN3, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
         B->d_val, cnt, Cptr, Cind, Cval, n, load);
     ++launches;
   }
-  if (hn[kBinN4] && bwords) {
+  const unsigned n4 = hn[kBinN4] + hn[kTailN4];
+  if (n4 && bwords) {
     // a scratch row of doubles per block, at most 2 MB each; fewer blocks when
     // the memory for all of them cannot be had
     const int claim = (maxc + 31) / 32;
-    int g4 = gridsz(ctx, hn[kBinN4], 1, 2);
+    int g4 = gridsz(ctx, n4, 1, 2);
     double *scratch = nullptr;
     for (;; g4 /= 2) {
       scratch = (double *)workspace(ctx, kSlotSpgScratch,
@@ -1571,13 +1618,13 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
     }
     if (!scratch) return APSPIE_ERR_OOM;
     spgemm_bitmap_rows<<<g4, kSpgThreads, (size_t)8 * bwords + 4 * (size_t)claim, st>>>(
-        L(kBinN4), nb + kBinN4, bwords, claim, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
+        L(kBinN4), nb + kBinN4, nb + kTailN4, grab + kBinN4, m, bwords, claim, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
         B->d_val, Cptr, Cind, Cval, (const unsigned *)ctx->spgemm_plan_gbm,
         (const int *)ctx->spgemm_plan_bslot, scratch);
     ++launches;
-  } else if (hn[kBinN4]) {
-    spgemm_block_rows<true><<<gridsz(ctx, hn[kBinN4], 1, 1), kSpgThreads, dyn_num, st>>>(
-        L(kBinN4), nb + kBinN4, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
+  } else if (n4) {
+    spgemm_block_rows<true><<<gridsz(ctx, n4, 1, 1), kSpgThreads, dyn_num, st>>>(
+        L(kBinN4), nb + kBinN4, grab + kBinN4, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
         B->d_val, cnt, Cptr, Cind, Cval, n, load);
     ++launches;
   }

@@ -17,8 +17,10 @@ constexpr int kEdgeThreads = 256;
 constexpr int kEdgeItems = 8;                          // entries per thread
 constexpr int kEdgeTile = kEdgeThreads * kEdgeItems;  // entries per tile
 
-// Largest r with ptr[r] <= k, given ptr[m] > k.  Warp-collective.
-__device__ __forceinline__ int row_of_entry(const int *__restrict__ ptr, int m, int k) {
+// Largest r with ptr[r] <= k, given ptr[m] > k.  Warp-collective.  (P: int, or
+// long long for offsets whose total has been checked to fit an int.)
+template <typename P>
+__device__ __forceinline__ int row_of_entry(const P *__restrict__ ptr, int m, int k) {
   const int lane = lane_id();
   int lo = 0, hi = m;  // ptr[lo] <= k < ptr[hi]
   while (hi - lo > 1) {
@@ -36,7 +38,8 @@ __device__ __forceinline__ int row_of_entry(const int *__restrict__ ptr, int m, 
 
 // s_row[t] = row of entry k0 + t for t in [0, n), n <= kEdgeTile.  Called by
 // all kEdgeThreads threads; s_row is ready when it returns.
-__device__ __forceinline__ void edge_tile_rows(const int *__restrict__ ptr, int m, int k0, int n,
+template <typename P>
+__device__ __forceinline__ void edge_tile_rows(const P *__restrict__ ptr, int m, int k0, int n,
                                                int *s_row) {
   __shared__ int s_warp[kEdgeThreads / 32];
   __shared__ int s_r0;
@@ -50,7 +53,7 @@ __device__ __forceinline__ void edge_tile_rows(const int *__restrict__ ptr, int 
   const int r0 = s_r0;
   // empty rows start where the next non-empty one does: the largest id wins
   for (unsigned r = (unsigned)(r0 + 1 + t); r < (unsigned)m; r += kEdgeThreads) {
-    const int at = __ldg(ptr + r) - k0;
+    const int at = (int)__ldg(ptr + r) - k0;
     if (at >= n) break;
     atomicMax(s_row + at, (int)r);
   }

@@ -6,24 +6,32 @@
 // reference gathers column segments with four IntervalGathers and an
 // IntervalExpand, multiplies, cub-radix-sorts all (row, value) pairs on 32
 // key bits and reduces by key.  Here:
-//   * sort path (sparse output): one expand kernel writes (row, x (x) a)
-//     pairs at their scanned offsets (warp scan-based gather, big columns in a
-//     block-strided second kernel), the pairs are radix-sorted on only
-//     ceil(log2 m) key bits, and a segmented reduce emits sorted y;
-//   * bitmap path (dense frontier): products are combined with atomics into a
-//     dense accumulator and a touched bitmap, and y is compacted from the
-//     bitmap in index order -- no sort at all.
-// The path is chosen from the expanded size E against m (threshold settable,
-// picked by the autotuner).  Both give y sorted by row with one entry per
-// touched row; PLUS_TIMES accumulates in double and rounds once.
+// the frontier's columns are laid end to end by a scan of their lengths and
+// walked in tiles of equal size (edges.cuh), so a hub column costs no more
+// than its entries.
+//   * bitmap path: products are combined with atomics into a dense
+//     accumulator and a touched bitmap, and y is compacted from the bitmap in
+//     index order -- no sort, and nothing that the host has to know before
+//     the end, so the call waits for the device once;
+//   * sort path: the tiles write (row, x (x) a) pairs, the pairs are
+//     radix-sorted on only ceil(log2 m) key bits, and a segmented reduce emits
+//     sorted y.
+// The sort path is for frontiers that are sparse against a long y: its cost
+// grows with the expanded size E, the bitmap path's with m (clearing and
+// reading the accumulator, about 5 us per 2^20 rows), and the sort's launches
+// alone outlast that up to kBitmapRows rows.  Beyond, E * factor is compared
+// with m (threshold settable, picked by the autotuner; 0 always sorts).  Both
+// give y sorted by row with one entry per touched row; PLUS_TIMES accumulates
+// in double and rounds once.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 
 #include "common.cuh"
 #include "context.h"
-#include "frontier.cuh"
+#include "edges.cuh"
 #include "primitives.cuh"
 
 namespace apspie {
@@ -33,17 +41,12 @@ constexpr int kPlusTimes = 0, kMinPlus = 1, kMaxTimes = 2, kOrAnd = 3;
 
 struct SpmspvSmall {  // device-side scalars of one call
   long long total;    // expanded size E
-  unsigned nbig;      // columns of more than kBigDeg edges (a warp each)
   int ynnz;           // nnz(y)
   unsigned cnt;       // frontier size of the dense form
-  unsigned nhub;      // chunks of the columns of more than kHubDeg edges
 };
 
-// Columns longer than this are cut into kHubChunk-edge chunks, a warp each;
-// between kBigDeg and this a warp takes one column
-constexpr int kHubDeg = 1024;
-constexpr int kHubChunk = 2048;
-constexpr int kExpandThreads = 256;
+// up to this many rows of y the bitmap path is taken at any frontier density
+constexpr int kBitmapRows = 1 << 22;
 
 __device__ __forceinline__ float sr_term(int sr, float a, float x) {
   switch (sr) {
@@ -53,101 +56,77 @@ __device__ __forceinline__ float sr_term(int sr, float a, float x) {
   }
 }
 
-// ---- expansion into (row, term) pairs at scanned offsets ----
-__global__ void frontier_degrees(int xnnz, const int *__restrict__ xind, const int *__restrict__ ptr,
-                                 long long *deg) {
+// ---- the frontier's columns ----
+// Lengths, and (first entry, x value) side by side for the tiles.
+__global__ void frontier_columns(int xnnz, const int *__restrict__ xind,
+                                 const float *__restrict__ xval, const int *__restrict__ ptr,
+                                 long long *deg, int2 *col) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < xnnz; j += gridDim.x * blockDim.x) {
-    int c = xind[j];
-    deg[j] = (long long)(__ldg(ptr + c + 1) - __ldg(ptr + c));
+    const int c = xind[j];
+    const int s = __ldg(ptr + c);
+    deg[j] = (long long)(__ldg(ptr + c + 1) - s);
+    col[j] = make_int2(s, __float_as_int(xval ? xval[j] : 1.0f));
   }
 }
 
-__global__ void __launch_bounds__(kExpandThreads)
-expand_pairs(int sr, int xnnz, const int *__restrict__ xind, const float *__restrict__ xval,
-             const int *__restrict__ ptr, const int *__restrict__ ind,
-             const float *__restrict__ val, const long long *__restrict__ offs, int *keys,
-             float *vals, int *big, unsigned *nbig, int2 *hub, unsigned *nhub) {
-  const int lane = lane_id();
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int base = gwarp * 32; base < xnnz; base += nwarps * 32) {
-    int j = base + lane;
-    int s = 0, d = 0;
-    float xv = 0.f;
-    bool isbig = false;
-    if (j < xnnz) {
-      int c = xind[j];
-      s = __ldg(ptr + c);
-      d = __ldg(ptr + c + 1) - s;
-      xv = xval ? xval[j] : 1.0f;
-      if (d > kBigDeg) isbig = true;
+// Calls f(e[], row[], term[], on[]) for the entries e of the frontier's columns
+// laid end to end (offs: their exclusive scan, offs[xnnz] = *total), each
+// thread's kEdgeItems of a tile in flight together.  Blocks stride the tiles.
+// Nothing is done when the total does not fit an int (the caller reports it).
+template <typename F>
+__device__ __forceinline__ void for_each_entry(int sr, int xnnz, const long long *__restrict__ offs,
+                                               const long long *total,
+                                               const int2 *__restrict__ col,
+                                               const int *__restrict__ ind,
+                                               const float *__restrict__ val, F f) {
+  __shared__ __align__(16) int s_row[kEdgeTile];
+  const long long E = __ldcg(total);
+  if (E >= (long long)INT_MAX) return;
+  const unsigned tiles = (unsigned)((E + kEdgeTile - 1) / kEdgeTile);
+  for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int k0 = (int)(tile * kEdgeTile);
+    const int n = (int)min((long long)kEdgeTile, E - k0);
+    edge_tile_rows(offs, xnnz, k0, n, s_row);
+    int e[kEdgeItems], row[kEdgeItems];
+    float term[kEdgeItems], x[kEdgeItems];
+    bool on[kEdgeItems];
+    int k[kEdgeItems];
+#pragma unroll
+    for (int q = 0; q < kEdgeItems; ++q) {
+      const int t = (int)threadIdx.x + q * kEdgeThreads;
+      on[q] = t < n;
+      e[q] = k0 + t;
+      const int j = on[q] ? s_row[t] : 0;
+      const int2 c = __ldg(col + j);
+      k[q] = c.x + (int)(e[q] - __ldg(offs + j));
+      x[q] = __int_as_float(c.y);
     }
-    const bool ishub = isbig && d > kHubDeg;
-    const bool ismid = isbig && !ishub;
-    unsigned slot = warp_append(ismid, nbig);
-    if (ismid) big[slot] = j;
-    if (ishub) {
-      const int nc = (d + kHubChunk - 1) / kHubChunk;
-      const unsigned at = atomicAdd(nhub, (unsigned)nc);
-      for (int c = 0; c < nc; ++c) hub[at + c] = make_int2(j, c);
+#pragma unroll
+    for (int q = 0; q < kEdgeItems; ++q) {
+      row[q] = on[q] ? __ldg(ind + k[q]) : 0;
+      term[q] = on[q] && val ? __ldg(val + k[q]) : 1.0f;
     }
-    if (isbig) d = 0;
-    int incl = warp_incl_scan(d);
-    int excl = incl - d;
-    int total = __shfl_sync(kFull, incl, 31);
-    for (int e0 = 0; e0 < total; e0 += 32) {
-      int e = e0 + lane;
-      int owner = warp_owner(excl, e);
-      int so = __shfl_sync(kFull, s, owner);
-      int eo = __shfl_sync(kFull, excl, owner);
-      float xo = __shfl_sync(kFull, xv, owner);
-      int jo = __shfl_sync(kFull, j, owner);
-      if (e < total) {
-        int k = so + (e - eo);
-        long long pos = offs[jo] + (e - eo);
-        keys[pos] = __ldg(ind + k);
-        vals[pos] = sr_term(sr, val ? __ldg(val + k) : 1.0f, xo);
-      }
-    }
+#pragma unroll
+    for (int q = 0; q < kEdgeItems; ++q) term[q] = sr_term(sr, term[q], x[q]);
+    f(e, row, term, on);
+    __syncthreads();
   }
 }
 
-// The listed columns: a warp per column of the medium list, then a warp per
-// hub chunk (a hub's edges spread over all SMs).
-__global__ void expand_big(int sr, const int *__restrict__ xind, const float *__restrict__ xval,
-                           const int *__restrict__ ptr, const int *__restrict__ ind,
-                           const float *__restrict__ val, const long long *__restrict__ offs,
-                           const int *big, const unsigned *nbig, const int2 *hub,
-                           const unsigned *nhub, int *keys, float *vals) {
-  const int lane = lane_id();
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  const unsigned nb = *nbig;
-  for (unsigned b = gwarp; b < nb; b += nwarps) {
-    const int j = big[b];
-    const int c = xind[j];
-    const int s = __ldg(ptr + c), e = __ldg(ptr + c + 1);
-    const float xv = xval ? xval[j] : 1.0f;
-    const long long o = offs[j] - s;
-    for (int k = s + lane; k < e; k += 32) {
-      keys[o + k] = __ldg(ind + k);
-      vals[o + k] = sr_term(sr, val ? __ldg(val + k) : 1.0f, xv);
-    }
-  }
-  const unsigned nh = *nhub;
-  for (unsigned b = gwarp; b < nh; b += nwarps) {
-    const int2 hc = hub[b];
-    const int j = hc.x;
-    const int c = xind[j];
-    const int s0 = __ldg(ptr + c);
-    const int s = s0 + hc.y * kHubChunk, e = min(__ldg(ptr + c + 1), s + kHubChunk);
-    const float xv = xval ? xval[j] : 1.0f;
-    const long long o = offs[j] - s0;
-    for (int k = s + lane; k < e; k += 32) {
-      keys[o + k] = __ldg(ind + k);
-      vals[o + k] = sr_term(sr, val ? __ldg(val + k) : 1.0f, xv);
-    }
-  }
+__global__ void __launch_bounds__(kEdgeThreads)
+expand_pairs(int sr, int xnnz, const long long *__restrict__ offs, const long long *total,
+             const int2 *__restrict__ col, const int *__restrict__ ind,
+             const float *__restrict__ val, int *keys, float *vals) {
+  for_each_entry(sr, xnnz, offs, total, col, ind, val,
+                 [&](const int (&e)[kEdgeItems], const int (&row)[kEdgeItems],
+                     const float (&term)[kEdgeItems], const bool (&on)[kEdgeItems]) {
+#pragma unroll
+                   for (int q = 0; q < kEdgeItems; ++q)
+                     if (on[q]) {
+                       keys[e[q]] = row[q];
+                       vals[e[q]] = term[q];
+                     }
+                 });
 }
 
 // ---- segmented reduce of sorted pairs ----
@@ -185,180 +164,100 @@ __global__ void reduce_segments(int sr, const int *keys, const float *vals, long
 }
 
 // ---- bitmap path ----
-__global__ void acc_init(int sr, int m, double *acc, unsigned *bits) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    double idv = 0.0;
-    if (sr == kMinPlus) idv = (double)FLT_MAX * 2.0;  // above any float
-    if (sr == kMaxTimes) idv = -(double)FLT_MAX * 2.0;
-    acc[i] = idv;
-    if ((i & 31) == 0) bits[i >> 5] = 0u;
+// MIN_PLUS and MAX_TIMES reduce floats: one 32-bit word per row that orders as
+// the float does, so that the atomics are native (a double needs a
+// compare-and-swap loop).  NaN terms are left out, as a comparison does; a
+// row that only such terms or infinities touch keeps the identity.
+__device__ __forceinline__ unsigned ordered_bits(float f) {
+  const unsigned b = __float_as_uint(f);
+  return (b >> 31) ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float ordered_float(unsigned u) {
+  return __uint_as_float((u >> 31) ? u & 0x7fffffffu : ~u);
+}
+
+// Clears the accumulator (doubles for PLUS_TIMES, ordered words for MIN_PLUS
+// and MAX_TIMES) and the bitmap.
+__global__ void acc_init(int sr, int m, void *acc, unsigned *bits) {
+  const unsigned idw = sr == kMinPlus ? ordered_bits(INFINITY) : ordered_bits(-INFINITY);
+  const unsigned stride = gridDim.x * blockDim.x;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)m; i += stride) {
+    if (sr == kPlusTimes) ((double *)acc)[i] = 0.0;
+    else if (sr != kOrAnd) ((unsigned *)acc)[i] = idw;
+    if ((i & 31u) == 0u) bits[i >> 5] = 0u;
   }
 }
 
-__device__ __forceinline__ void atomic_min_double(double *p, double v) {
-  unsigned long long *a = (unsigned long long *)p;
-  unsigned long long old = *a;
-  while (__longlong_as_double(old) > v) {
-    unsigned long long prev = atomicCAS(a, old, __double_as_longlong(v));
-    if (prev == old) break;
-    old = prev;
-  }
-}
-__device__ __forceinline__ void atomic_max_double(double *p, double v) {
-  unsigned long long *a = (unsigned long long *)p;
-  unsigned long long old = *a;
-  while (__longlong_as_double(old) < v) {
-    unsigned long long prev = atomicCAS(a, old, __double_as_longlong(v));
-    if (prev == old) break;
-    old = prev;
-  }
-}
-
-// Bitmap path expansion.  32 consecutive frontier entries per warp: their
-// edges are dealt over the lanes by an inclusive warp scan of the degrees
-// (coalesced over each column, no lane idles on a short column).  Columns
-// of more than kBigDeg edges are listed instead: up to kHubDeg edges a warp
-// takes one in expand_accumulate_big, longer ones (hubs) are cut into
-// kHubChunk-edge chunks that warps take one by one.  Each product is folded into acc[row] with the
-// semiring's atomic and marks the row's bit.
-__device__ __forceinline__ void accumulate_one(int sr, int r, float t, double *acc,
-                                               unsigned *bits) {
-  switch (sr) {
-    case kPlusTimes: atomicAdd(acc + r, (double)t); break;
-    case kMinPlus: atomic_min_double(acc + r, (double)t); break;
-    case kMaxTimes: atomic_max_double(acc + r, (double)t); break;
-    default: break;
-  }
-  const unsigned bit = 1u << (r & 31);
-  if (!(__ldcg(bits + (r >> 5)) & bit)) atomicOr(bits + (r >> 5), bit);
-}
-
-__global__ void __launch_bounds__(kExpandThreads)
-expand_accumulate(int sr, int xnnz, const int *__restrict__ xind, const float *__restrict__ xval,
-                  const int *__restrict__ ptr, const int *__restrict__ ind,
-                  const float *__restrict__ val, double *acc, unsigned *bits, int *big,
-                  unsigned *nbig, int2 *hub, unsigned *nhub) {
-  const int lane = lane_id();
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int base = gwarp * 32; base < xnnz; base += nwarps * 32) {
-    const int j = base + lane;
-    int s = 0, d = 0;
-    float xv = 0.f;
-    bool isbig = false;
-    if (j < xnnz) {
-      const int c = xind[j];
-      s = __ldg(ptr + c);
-      d = __ldg(ptr + c + 1) - s;
-      xv = xval ? xval[j] : 1.0f;
-      if (d > kBigDeg) isbig = true;
-    }
-    const bool ishub = isbig && d > kHubDeg;
-    const bool ismid = isbig && !ishub;
-    unsigned slot = warp_append(ismid, nbig);
-    if (ismid) big[slot] = j;
-    if (ishub) {
-      const int nc = (d + kHubChunk - 1) / kHubChunk;
-      const unsigned at = atomicAdd(nhub, (unsigned)nc);
-      for (int c = 0; c < nc; ++c) hub[at + c] = make_int2(j, c);
-    }
-    if (isbig) d = 0;
-    const int incl = warp_incl_scan(d);
-    const int excl = incl - d;
-    const int total = __shfl_sync(kFull, incl, 31);
-    for (int e0 = 0; e0 < total; e0 += 32) {
-      const int e = e0 + lane;
-      const int owner = warp_owner(excl, e);
-      const int so = __shfl_sync(kFull, s, owner);
-      const int eo = __shfl_sync(kFull, excl, owner);
-      const float xo = __shfl_sync(kFull, xv, owner);
-      if (e < total) {
-        const int k = so + (e - eo);
-        accumulate_one(sr, __ldg(ind + k), sr_term(sr, val ? __ldg(val + k) : 1.0f, xo), acc,
-                       bits);
-      }
-    }
-  }
-}
-
-// The listed long columns: a warp per column of the medium list, then a warp
-// per hub chunk (a hub's edges spread over all SMs).
-__global__ void __launch_bounds__(kExpandThreads)
-expand_accumulate_big(int sr, const int *__restrict__ xind, const float *__restrict__ xval,
-                      const int *__restrict__ ptr, const int *__restrict__ ind,
-                      const float *__restrict__ val, const int *big, const unsigned *nbig,
-                      const int2 *hub, const unsigned *nhub, double *acc, unsigned *bits) {
-  const int lane = lane_id();
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
-  const unsigned nb = *nbig;
-  for (unsigned b = gwarp; b < nb; b += nwarps) {
-    const int j = big[b];
-    const int c = xind[j];
-    const int s = __ldg(ptr + c), e = __ldg(ptr + c + 1);
-    const float xv = xval ? xval[j] : 1.0f;
-    // four index / value loads in flight per lane before their atomics
-    int k = s + lane;
-    for (; k + 96 < e; k += 128) {
-      int r[4];
-      float a[4];
+__global__ void __launch_bounds__(kEdgeThreads)
+expand_accumulate(int sr, int xnnz, const long long *__restrict__ offs, const long long *total,
+                  const int2 *__restrict__ col, const int *__restrict__ ind,
+                  const float *__restrict__ val, void *acc, unsigned *bits) {
+  for_each_entry(sr, xnnz, offs, total, col, ind, val,
+                 [&](const int (&)[kEdgeItems], const int (&row)[kEdgeItems],
+                     const float (&term)[kEdgeItems], const bool (&on)[kEdgeItems]) {
+                   unsigned have[kEdgeItems];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        r[q] = __ldg(ind + k + 32 * q);
-        a[q] = val ? __ldg(val + k + 32 * q) : 1.0f;
-      }
+                   for (int q = 0; q < kEdgeItems; ++q)
+                     have[q] = on[q] ? __ldcg(bits + (row[q] >> 5)) : ~0u;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) accumulate_one(sr, r[q], sr_term(sr, a[q], xv), acc, bits);
-    }
-    for (; k < e; k += 32)
-      accumulate_one(sr, __ldg(ind + k), sr_term(sr, val ? __ldg(val + k) : 1.0f, xv), acc,
-                     bits);
-  }
-  const unsigned nh = *nhub;
-  for (unsigned b = gwarp; b < nh; b += nwarps) {
-    const int2 hc = hub[b];
-    const int j = hc.x;
-    const int c = xind[j];
-    const int s = __ldg(ptr + c) + hc.y * kHubChunk;
-    const int e = min(__ldg(ptr + c + 1), s + kHubChunk);
-    const float xv = xval ? xval[j] : 1.0f;
-    int k = s + lane;
-    for (; k + 96 < e; k += 128) {
-      int r[4];
-      float a[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        r[q] = __ldg(ind + k + 32 * q);
-        a[q] = val ? __ldg(val + k + 32 * q) : 1.0f;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) accumulate_one(sr, r[q], sr_term(sr, a[q], xv), acc, bits);
-    }
-    for (; k < e; k += 32)
-      accumulate_one(sr, __ldg(ind + k), sr_term(sr, val ? __ldg(val + k) : 1.0f, xv), acc,
-                     bits);
-  }
+                   for (int q = 0; q < kEdgeItems; ++q) {
+                     if (!on[q]) continue;
+                     if (sr == kPlusTimes) {
+                       atomicAdd((double *)acc + row[q], (double)term[q]);
+                     } else if (sr != kOrAnd && term[q] == term[q]) {
+                       const unsigned o = ordered_bits(term[q]);
+                       if (sr == kMinPlus) atomicMin((unsigned *)acc + row[q], o);
+                       else atomicMax((unsigned *)acc + row[q], o);
+                     }
+                     const unsigned bit = 1u << (row[q] & 31);
+                     if (!(have[q] & bit)) atomicOr(bits + (row[q] >> 5), bit);
+                   }
+                 });
 }
 
-__global__ void bitmap_counts(const unsigned *bits, int words, unsigned *cnt) {
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += gridDim.x * blockDim.x)
-    cnt[w] = __popc(bits[w]);
+// y from the bitmap, in two launches: the bits of every block's words are
+// counted (sums), then each block adds up the counts before its own and
+// writes its rows in order; the last one leaves nnz(y).
+constexpr int kEmitThreads = 256;
+constexpr int kEmitBlocks = 2048;  // at most
+
+__global__ void __launch_bounds__(kEmitThreads)
+bitmap_counts(const unsigned *__restrict__ bits, int words, int per_block, unsigned *sums) {
+  __shared__ unsigned sw[33];
+  const int w0 = blockIdx.x * per_block, w1 = min(words, w0 + per_block);
+  unsigned c = 0;
+  for (int w = w0 + (int)threadIdx.x; w < w1; w += kEmitThreads) c += __popc(bits[w]);
+  unsigned tot;
+  block_excl_scan(c, sw, &tot);
+  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
-__global__ void bitmap_emit(int sr, const unsigned *bits, int words, const unsigned *offs,
-                            const double *acc, int *yind, float *yval) {
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += gridDim.x * blockDim.x) {
-    unsigned b = bits[w];
-    unsigned o = offs[w];
+__global__ void __launch_bounds__(kEmitThreads)
+bitmap_emit(int sr, const unsigned *__restrict__ bits, int words, int per_block,
+            const unsigned *__restrict__ sums, const void *__restrict__ acc, int *yind,
+            float *yval, int *ynnz) {
+  __shared__ unsigned sw[33];
+  unsigned before = 0, tot;
+  for (unsigned i = threadIdx.x; i < blockIdx.x; i += kEmitThreads) before += sums[i];
+  block_excl_scan(before, sw, &tot);
+  before = tot;
+  const int w0 = blockIdx.x * per_block, w1 = min(words, w0 + per_block);
+  for (int base = w0; base < w1; base += kEmitThreads) {
+    const int w = base + (int)threadIdx.x;
+    unsigned b = w < w1 ? bits[w] : 0u;
+    unsigned o = before + block_excl_scan((unsigned)__popc(b), sw, &tot);
+    before += tot;
     while (b) {
-      int t = __ffs(b) - 1;
+      const int r = w * 32 + __ffs(b) - 1;
       b &= b - 1;
-      int r = w * 32 + t;
       yind[o] = r;
-      yval[o] = sr == kOrAnd ? 1.0f : (float)acc[r];
+      yval[o] = sr == kOrAnd ? 1.0f
+                : sr == kPlusTimes ? (float)((const double *)acc)[r]
+                                   : ordered_float(((const unsigned *)acc)[r]);
       ++o;
     }
   }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *ynnz = (int)before;
 }
 
 // ---- dense in / dense out helpers (mXv dense form) ----
@@ -400,90 +299,72 @@ int grid_for(apspie_context *ctx, long long n, int threads) {
   return (int)std::max(1ll, std::min(g, (long long)ctx->num_sms * 16));
 }
 
-// Core sparse SpMSpV.  On return *d_ynnz (device) holds nnz(y); *h_total
-// the expanded size E (host, after a sync).
+// Core sparse SpMSpV.  On return sm->ynnz (device) holds nnz(y) and sm->total
+// the expanded size E; the caller reads both back and passes E to
+// spmspv_overflow.
 int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *ind,
                 const float *val, int xnnz, const int *xind, const float *xval, int *yind,
-                float *yval, int *d_ynnz, long long *h_total) {
+                float *yval, SpmspvSmall *sm) {
   cudaStream_t st = ctx->stream;
-  long long *offs = (long long *)workspace(ctx, kSlotMisc0, sizeof(long long) * (size_t)(xnnz + 1));
-  auto *sm = (SpmspvSmall *)workspace(ctx, kSlotSmall, sizeof(SpmspvSmall));
-  if (!offs || !sm) return APSPIE_ERR_OOM;
-  long long *d_tot = &sm->total;
+  const double factor = ctx->spmspv_sort_factor;
+  if (xnnz == 0)
+    return check_cuda(ctx, cudaMemsetAsync(sm, 0, sizeof(SpmspvSmall), st), "spmspv empty");
+  auto *offs = (long long *)workspace(ctx, kSlotMisc0, sizeof(long long) * (size_t)(xnnz + 1));
+  auto *col = (int2 *)workspace(ctx, kSlotMisc2, sizeof(int2) * (size_t)xnnz);
+  if (!offs || !col) return APSPIE_ERR_OOM;
+  frontier_columns<<<grid_for(ctx, xnnz, 256), 256, 0, st>>>(xnnz, xind, xval, ptr, offs, col);
+  int rc = check_launch(ctx, "frontier_columns");
+  if (rc) return rc;
+  bool bitmap = m <= kBitmapRows && factor > 0.0;
   long long E = 0;
-  if (xnnz > 0) {
-    frontier_degrees<<<grid_for(ctx, xnnz, 256), 256, 0, st>>>(xnnz, xind, ptr, offs);
-    int rc = check_launch(ctx, "frontier_degrees");
-    if (rc) return rc;
-    rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, d_tot);
+  if (!bitmap) {
+    rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, &sm->total);
     if (rc) return rc;
     long long *h = (long long *)pinned(ctx, sizeof(long long));
     if (!h) return APSPIE_ERR_OOM;
-    rc = check_cuda(ctx, cudaMemcpyAsync(h, d_tot, sizeof(long long), cudaMemcpyDeviceToHost, st),
-                    "spmspv total");
+    rc = check_cuda(ctx, cudaMemcpyAsync(h, &sm->total, sizeof(long long), cudaMemcpyDeviceToHost,
+                                         st), "spmspv total");
     if (rc) return rc;
     rc = check_cuda(ctx, cudaStreamSynchronize(st), "spmspv total");
     if (rc) return rc;
     E = *h;
+    if (E == 0)
+      return check_cuda(ctx, cudaMemsetAsync(&sm->ynnz, 0, sizeof(int), st), "spmspv empty");
+    if (E >= (long long)INT32_MAX)
+      return set_error(ctx, APSPIE_ERR_OVERFLOW, "spmspv: %lld expanded pairs", E);
+    bitmap = (double)E * factor > (double)m;
   }
-  if (h_total) *h_total = E;
-  if (E == 0) {
-    return check_cuda(ctx, cudaMemsetAsync(d_ynnz, 0, sizeof(int), st), "spmspv empty");
-  }
-  if (E >= (long long)INT32_MAX)
-    return set_error(ctx, APSPIE_ERR_OVERFLOW, "spmspv: %lld expanded pairs", E);
-  bool bitmap = (double)E * ctx->spmspv_sort_factor > (double)m;
+  const int egrid = ctx->num_sms * 6;  // resident blocks; they stride the tiles
   if (bitmap) {
-    int words = (m + 31) / 32;
-    double *acc = (double *)workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
-    unsigned *bits = (unsigned *)workspace(ctx, kSlotBitmap, sizeof(unsigned) * (size_t)(2 * words + 2));
+    const int words = (int)(((long long)m + 31) / 32);
+    void *acc = workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
+    unsigned *bits = (unsigned *)workspace(ctx, kSlotBitmap,
+                                           sizeof(unsigned) * ((size_t)words + kEmitBlocks));
     if (!acc || !bits) return APSPIE_ERR_OOM;
-    unsigned *woffs = bits + words + 1;
-    const size_t nbig_cap = ((size_t)xnnz + 2) & ~size_t(1);  // keeps the chunk list 8-aligned
-    int *big = (int *)workspace(ctx, kSlotMisc2,
-                                sizeof(int) * nbig_cap +
-                                    sizeof(int2) * ((size_t)E / kHubChunk + (size_t)xnnz + 1));
-    if (!big) return APSPIE_ERR_OOM;
-    int2 *hub = (int2 *)(big + nbig_cap);
-    int rc = check_cuda(ctx, cudaMemsetAsync(&sm->nbig, 0, sizeof(unsigned), st), "spmspv nbig");
-    if (rc) return rc;
-    rc = check_cuda(ctx, cudaMemsetAsync(&sm->nhub, 0, sizeof(unsigned), st), "spmspv nhub");
-    if (rc) return rc;
+    unsigned *sums = bits + words;
+    if (E == 0) {  // not scanned yet
+      rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, &sm->total);
+      if (rc) return rc;
+    }
     acc_init<<<grid_for(ctx, m, 256), 256, 0, st>>>(sr, m, acc, bits);
-    expand_accumulate<<<grid_for(ctx, (long long)xnnz * 32, kExpandThreads), kExpandThreads, 0,
-                        st>>>(sr, xnnz, xind, xval, ptr, ind, val, acc, bits, big, &sm->nbig,
-                              hub, &sm->nhub);
-    expand_accumulate_big<<<ctx->num_sms * 4, kExpandThreads, 0, st>>>(
-        sr, xind, xval, ptr, ind, val, big, &sm->nbig, hub, &sm->nhub, acc, bits);
-    bitmap_counts<<<grid_for(ctx, words, 256), 256, 0, st>>>(bits, words, woffs);
-    rc = check_launch(ctx, "spmspv bitmap", 4);
-    if (rc) return rc;
-    rc = device_exclusive_scan<unsigned>(ctx, woffs, woffs, words, (unsigned *)d_ynnz);
-    if (rc) return rc;
-    bitmap_emit<<<grid_for(ctx, words, 256), 256, 0, st>>>(sr, bits, words, woffs, acc, yind, yval);
-    return check_launch(ctx, "bitmap_emit");
+    expand_accumulate<<<egrid, kEdgeThreads, 0, st>>>(sr, xnnz, offs, &sm->total, col, ind, val,
+                                                      acc, bits);
+    const int per_block = std::max(kEmitThreads, (words + kEmitBlocks - 1) / kEmitBlocks);
+    const int eblocks = (words + per_block - 1) / per_block;
+    bitmap_counts<<<eblocks, kEmitThreads, 0, st>>>(bits, words, per_block, sums);
+    bitmap_emit<<<eblocks, kEmitThreads, 0, st>>>(sr, bits, words, per_block, sums, acc, yind,
+                                                  yval, &sm->ynnz);
+    return check_launch(ctx, "spmspv bitmap", 4);
   }
   // sort path
   int *ka = (int *)workspace(ctx, kSlotSortKeysA, sizeof(int) * (size_t)E);
   int *kb = (int *)workspace(ctx, kSlotSortKeysB, sizeof(int) * (size_t)E);
   float *va = (float *)workspace(ctx, kSlotSortValsA, sizeof(float) * (size_t)E);
   float *vb = (float *)workspace(ctx, kSlotSortValsB, sizeof(float) * (size_t)E);
-  const size_t nbig_cap = ((size_t)xnnz + 2) & ~size_t(1);  // keeps the chunk list 8-aligned
-  int *big = (int *)workspace(ctx, kSlotMisc2,
-                              sizeof(int) * nbig_cap +
-                                  sizeof(int2) * ((size_t)E / kHubChunk + (size_t)xnnz + 1));
-  unsigned *nbig = &sm->nbig;
-  if (!ka || !kb || !va || !vb || !big) return APSPIE_ERR_OOM;
-  int2 *hub = (int2 *)(big + nbig_cap);
-  int rc = check_cuda(ctx, cudaMemsetAsync(nbig, 0, sizeof(unsigned), st), "spmspv nbig");
-  if (rc) return rc;
-  rc = check_cuda(ctx, cudaMemsetAsync(&sm->nhub, 0, sizeof(unsigned), st), "spmspv nhub");
-  if (rc) return rc;
-  expand_pairs<<<grid_for(ctx, (long long)xnnz * 32, kExpandThreads), kExpandThreads, 0, st>>>(
-      sr, xnnz, xind, xval, ptr, ind, val, offs, ka, va, big, nbig, hub, &sm->nhub);
-  expand_big<<<ctx->num_sms * 4, kExpandThreads, 0, st>>>(sr, xind, xval, ptr, ind, val, offs,
-                                                          big, nbig, hub, &sm->nhub, ka, va);
-  rc = check_launch(ctx, "expand_pairs", 2);
+  if (!ka || !kb || !va || !vb) return APSPIE_ERR_OOM;
+  expand_pairs<<<(unsigned)std::min<long long>(edge_tiles(E), egrid), kEdgeThreads, 0, st>>>(
+      sr, xnnz, offs, &sm->total, col, ind, val, ka, va);
+  rc = check_launch(ctx, "expand_pairs");
   if (rc) return rc;
   bool in_b = false;
   rc = device_radix_sort<int, float>(ctx, ka, va, kb, vb, E, bits_for(m), &in_b);
@@ -495,10 +376,18 @@ int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *i
   head_flags<<<grid_for(ctx, E, 256), 256, 0, st>>>(ks, E, flags);
   rc = check_launch(ctx, "head_flags");
   if (rc) return rc;
-  rc = device_exclusive_scan<unsigned>(ctx, flags, flags, E, (unsigned *)d_ynnz);
+  rc = device_exclusive_scan<unsigned>(ctx, flags, flags, E, (unsigned *)&sm->ynnz);
   if (rc) return rc;
   reduce_segments<<<grid_for(ctx, E, 256), 256, 0, st>>>(sr, ks, vs, E, flags, yind, yval, m);
   return check_launch(ctx, "reduce_segments");
+}
+
+// The expanded size read back at the end of a call: the kernels do nothing
+// with one that does not fit the int32 layout.
+int spmspv_overflow(apspie_context *ctx, long long E) {
+  return E < (long long)INT32_MAX
+             ? APSPIE_OK
+             : set_error(ctx, APSPIE_ERR_OVERFLOW, "spmspv: %lld expanded pairs", E);
 }
 
 }  // namespace
@@ -518,29 +407,33 @@ int apspie_spmspv(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int *d
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_spmspv: bad arguments");
   auto *sm = (SpmspvSmall *)workspace(ctx, kSlotSmall, sizeof(SpmspvSmall));
   if (!sm) return APSPIE_ERR_OOM;
-  int *d_ynnz = &sm->ynnz;
-  long long E = 0;
   int rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, d_xind, d_xval, d_yind, d_yval,
-                       d_ynnz, &E);
+                       sm);
   if (rc) return rc;
-  int *h = (int *)pinned(ctx, sizeof(long long));
+  struct Back {
+    SpmspvSmall s;
+    int sort_err;
+  };
+  auto *h = (Back *)pinned(ctx, sizeof(Back));
   int *sort_err = radix_sort_err(ctx);
   if (!h || !sort_err) return APSPIE_ERR_OOM;
-  rc = check_cuda(ctx, cudaMemcpyAsync(h, d_ynnz, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream),
-                  "apspie_spmspv");
+  rc = check_cuda(ctx, cudaMemcpyAsync(&h->s, sm, sizeof(SpmspvSmall), cudaMemcpyDeviceToHost,
+                                       ctx->stream), "apspie_spmspv");
   if (rc) return rc;
-  rc = check_cuda(ctx, cudaMemcpyAsync(h + 1, sort_err, sizeof(int), cudaMemcpyDeviceToHost,
+  rc = check_cuda(ctx, cudaMemcpyAsync(&h->sort_err, sort_err, sizeof(int), cudaMemcpyDeviceToHost,
                                        ctx->stream), "apspie_spmspv");
   if (rc) return rc;
   rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "apspie_spmspv");
   if (rc) return rc;
-  if (h[1]) {  // the sort path's look-back gave up: the output is not sorted
+  if (h->sort_err) {  // the sort path's look-back gave up: the output is not sorted
     rc = check_cuda(ctx, cudaMemsetAsync(sort_err, 0, sizeof(int), ctx->stream), "apspie_spmspv");
     if (rc) return rc;
     return set_error(ctx, APSPIE_ERR_TIMEOUT, "apspie_spmspv: radix sort look-back gave up");
   }
-  *h_ynnz = *h;
-  if (h_expanded) *h_expanded = E;
+  rc = spmspv_overflow(ctx, h->s.total);
+  if (rc) return rc;
+  *h_ynnz = h->s.ynnz;
+  if (h_expanded) *h_expanded = h->s.total;
   return APSPIE_OK;
 }
 
@@ -583,15 +476,22 @@ int apspie_mxv_dense(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int
   // y reset to the semiring's empty value, as preprocessFlag does
   // (0 for mXv, src/mXv.cuh:45; 1.70141e38 for SSSP, src/spmspvSssp.cuh:26)
   float empty = semiring == kMinPlus ? 1.70141e+38f : 0.0f;
-  int *d_ynnz = &sm->ynnz;
-  long long E = 0;
-  rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, fx, fv, yi, yv, d_ynnz, &E);
+  rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, fx, fv, yi, yv, sm);
   if (rc) return rc;
   dense_fill<<<grid_for(ctx, m, 256), 256, 0, st>>>(m, empty, d_y);
-  dense_scatter<<<grid_for(ctx, m, 256), 256, 0, st>>>(d_ynnz, yi, yv, d_y);
+  dense_scatter<<<grid_for(ctx, m, 256), 256, 0, st>>>(&sm->ynnz, yi, yv, d_y);
   rc = check_launch(ctx, "dense_scatter", 2);
   if (rc) return rc;
-  if (h_expanded) *h_expanded = E;
+  auto *hs = (SpmspvSmall *)pinned(ctx, sizeof(SpmspvSmall));
+  if (!hs) return APSPIE_ERR_OOM;
+  rc = check_cuda(ctx, cudaMemcpyAsync(hs, sm, sizeof(SpmspvSmall), cudaMemcpyDeviceToHost, st),
+                  "apspie_mxv_dense");
+  if (rc) return rc;
+  rc = check_cuda(ctx, cudaStreamSynchronize(st), "apspie_mxv_dense");
+  if (rc) return rc;
+  rc = spmspv_overflow(ctx, hs->total);
+  if (rc) return rc;
+  if (h_expanded) *h_expanded = hs->total;
   return APSPIE_OK;
 }
 

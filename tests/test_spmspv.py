@@ -147,3 +147,62 @@ def test_dense_spmv_all_rows(ctx, semiring):
         else:
             ref = 1.0 if np.any((a != 0) & (xs != 0)) else 0.0
             assert y[r] == ref, (r, y[r], ref)
+
+
+@pytest.mark.parametrize("sr", [0, 1, 2, 3])
+@pytest.mark.parametrize("path", ["sort", "bitmap"])
+@pytest.mark.parametrize("total", [1, 2047, 2048, 2049, 40961])
+def test_spmspv_tile_edges(ctx, sr, path, total):
+    """Expanded sizes at and around a tile of 2,048 entries, half of them in
+    one column that spans tiles, between runs of empty columns; a repeated
+    frontier vertex counts twice."""
+    import torch
+    import apspie_b200 as ap
+    rng = np.random.default_rng(total)
+    m = 3001
+    xind = np.sort(rng.choice(m, size=200, replace=False)).astype(np.int32)
+    deg = np.zeros(m, np.int64)
+    np.add.at(deg, rng.choice(xind[100:140], size=total - total // 2), 1)
+    deg[xind[60]] += total // 2
+    ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    ind = rng.integers(0, m, size=total).astype(np.int32)
+    vals = rng.uniform(0.5, 2, size=total).astype(np.float32)
+    if total > 1:
+        xind = np.append(xind, xind[110]).astype(np.int32)
+    xval = rng.uniform(0.5, 2, size=len(xind)).astype(np.float32)
+    h = ap.HostGraph(m, ptr, ind)
+    g = h.to_device(with_transpose=False)
+    ap.spmspv_set_params(ctx, 0.0 if path == "sort" else 1e12)
+    try:
+        yi, yv, e = ap.spmspv(ctx, sr, g, torch.from_numpy(xind).cuda(),
+                              torch.from_numpy(xval).cuda(), torch.from_numpy(vals).cuda())
+    finally:
+        ap.spmspv_set_params(ctx)
+    ri, rv = oracle.spmspv(sr, m, ptr, ind, vals, xind, xval)
+    assert e == int(deg[xind].sum())
+    np.testing.assert_array_equal(yi.cpu().numpy(), ri)
+    np.testing.assert_allclose(yv.cpu().numpy(), rv, rtol=1e-6)
+
+
+def test_spmspv_bitmap_extreme_terms(ctx):
+    """Negative, zero, infinite and not-a-number terms in the minimum and the
+    maximum: a row that only infinities of the identity's sign or NaN terms
+    touch is in y with the identity."""
+    import torch
+    import apspie_b200 as ap
+    inf, nan = np.inf, np.nan
+    # column 0 -> rows 0..6, column 1 -> the same rows
+    terms0 = np.array([-1.5, 0.0, inf, -inf, nan, 3.0, nan], np.float32)
+    terms1 = np.array([2.5, -2.0, inf, 7.0, nan, nan, -4.0], np.float32)
+    ptr = np.array([0, 7, 14] + [14] * 6, np.int32)
+    ind = np.tile(np.arange(7), 2).astype(np.int32)
+    val = torch.from_numpy(np.concatenate([terms0, terms1])).cuda()
+    g = ap.HostGraph(8, ptr, ind).to_device(with_transpose=False)
+    xi = torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    zero, one = torch.zeros(2, device="cuda"), torch.ones(2, device="cuda")
+    yi, yv, _ = ap.spmspv(ctx, 1, g, xi, zero, val)
+    assert yi.tolist() == list(range(7))
+    assert yv.tolist() == [-1.5, -2.0, inf, -inf, inf, 3.0, -4.0]
+    yi, yv, _ = ap.spmspv(ctx, 2, g, xi, one, val)
+    assert yi.tolist() == list(range(7))
+    assert yv.tolist() == [2.5, 0.0, inf, 7.0, -inf, 3.0, -4.0]

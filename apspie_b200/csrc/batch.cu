@@ -1038,11 +1038,6 @@ int run_deep_sources(apspie_context *ctx, int njobs, const apspie_job *jobs,
   const int K = std::max(1, std::min(nsrc, ctx->batch_deep_subs));
   int rc = ensure_subs(ctx, K);
   if (rc) return rc;
-  if (!ctx->aux_done &&
-      cudaEventCreateWithFlags(&ctx->aux_done, cudaEventDisableTiming) != cudaSuccess)
-    return check_cuda(ctx, cudaGetLastError(), "apspie_batch_run: event");
-  // the sub-streams start after everything queued so far (inputs, uploads)
-  cudaEventRecord(ctx->aux_done, ctx->stream);
   const int grid = std::max(1, budget / K);
   for (int k = 0; k < K; ++k) {
     apspie_context *sub = ctx->subs[k];
@@ -1053,26 +1048,41 @@ int run_deep_sources(apspie_context *ctx, int njobs, const apspie_job *jobs,
     sub->bfs_mode = ctx->bfs_mode;
     sub->sssp_delta_u32 = ctx->sssp_delta_u32 ? ctx->sssp_delta_u32 : kDeepDelta;
   }
-  std::vector<double> load(K, 0.0);
-  for (int pass = 0; pass < 2; ++pass)  // SSSP sources first, then BFS
-    for (int i = 0; i < njobs; ++i) {
-      const apspie_job &J = jobs[i];
-      const bool bfs = J.type == APSPIE_JOB_BFS;
-      if (!deep_job[i] || bfs != (pass == 1)) continue;
-      const int *tp = J.d_tptr ? J.d_tptr : (J.symmetric ? J.d_ptr : nullptr);
-      const int *ti = J.d_tptr ? J.d_tind : (J.symmetric ? J.d_ind : nullptr);
-      for (int s = 0; s < J.nsrc; ++s) {
-        const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        load[k] += 1.0;
-        apspie_context *sub = ctx->subs[k];
-        int32_t *out = J.d_out + (size_t)s * J.m;
-        rc = bfs ? apspie_bfs(sub, J.h_src[s], J.nnz, J.m, J.d_ptr, J.d_ind, tp, ti, out, 0)
-                 : apspie_sssp_u32(sub, J.h_src[s], J.nnz, J.m, J.d_ptr, J.d_ind, J.d_w,
+  // SSSP sources first (they take longest), then BFS, dealt over the
+  // sub-contexts in turn, K sources at a time
+  struct Source {
+    const apspie_job *job;
+    int s;
+  };
+  std::vector<Source> order;
+  for (int pass = 0; pass < 2; ++pass)
+    for (int i = 0; i < njobs; ++i)
+      if (deep_job[i] && (jobs[i].type == APSPIE_JOB_BFS) == (pass == 1))
+        for (int s = 0; s < jobs[i].nsrc; ++s) order.push_back(Source{jobs + i, s});
+  // A BFS is a chain of launches, and a launch that waits for its
+  // predecessor holds up those queued behind it on the same hardware queue
+  // (there are fewer queues than sub-streams): the first parts of the K
+  // sources are queued before the last ones.
+  auto launch = [&](const Source &x, apspie_context *sub, BfsPart part) -> int {
+    const apspie_job &J = *x.job;
+    int32_t *out = J.d_out + (size_t)x.s * J.m;
+    if (J.type != APSPIE_JOB_BFS)
+      return part == BfsPart::kMain
+                 ? APSPIE_OK
+                 : apspie_sssp_u32(sub, J.h_src[x.s], J.nnz, J.m, J.d_ptr, J.d_ind, J.d_w,
                                    reinterpret_cast<uint32_t *>(out), 0);
+    const int *tp = J.d_tptr ? J.d_tptr : (J.symmetric ? J.d_ptr : nullptr);
+    const int *ti = J.d_tptr ? J.d_tind : (J.symmetric ? J.d_ind : nullptr);
+    return bfs_enqueue(sub, J.h_src[x.s], J.nnz, J.m, J.d_ptr, J.d_ind, tp, ti, out, 0, part);
+  };
+  for (size_t first = 0; first < order.size(); first += (size_t)K)
+    for (BfsPart part : {BfsPart::kFirst, BfsPart::kMain})
+      for (size_t i = first; i < std::min(order.size(), first + (size_t)K); ++i) {
+        apspie_context *sub = ctx->subs[i - first];
+        rc = launch(order[i], sub, part);
         if (rc) return set_error(ctx, rc, "apspie_batch_run: deep source: %s",
                                  sub->last_error.c_str());
       }
-    }
   for (int k = 0; k < K; ++k) {
     ctx->launches += ctx->subs[k]->launches;
     ctx->subs[k]->launches = 0;
@@ -1155,6 +1165,20 @@ int apspie_batch_run(apspie_ctx ctx, int njobs, const apspie_job *jobs, int max_
     int rc = APSPIE_OK;
     ctx->batch_state = nullptr;
     ctx->batch_subs_used = 0;
+    // The deep sources' streams start when the multi-source launch does: not
+    // after it, and not before, or their blocks would keep a cooperative
+    // launch from fitting until they are done.
+    auto release_deep = [&]() -> int {
+      if (ndeep_src == 0) return APSPIE_OK;
+      if (!ctx->aux_done &&
+          cudaEventCreateWithFlags(&ctx->aux_done, cudaEventDisableTiming) != cudaSuccess)
+        return check_cuda(ctx, cudaGetLastError(), "apspie_batch_run: event");
+      return check_cuda(ctx, cudaEventRecord(ctx->aux_done, st), "apspie_batch_run: event");
+    };
+    if (nparts == 0) {
+      rc = release_deep();
+      if (rc) return rc;
+    }
     if (nparts > 0) {
       // workspace layout per device job
       std::vector<size_t> off(nparts + 1, 0);
@@ -1261,6 +1285,8 @@ int apspie_batch_run(apspie_ctx ctx, int njobs, const apspie_job *jobs, int max_
       if (rc) return rc;
       int n1 = nparts;
       void *args1[] = {&djobs, &n1, &dstate, &max_steps};
+      rc = release_deep();
+      if (rc) return rc;
       cudaError_t e = cudaLaunchCooperativeKernel((const void *)batch_persistent, dim3(grid1),
                                                   dim3(kBatchThreads), args1, 0, st);
       if (e != cudaSuccess) return check_cuda(ctx, e, "batch_persistent");

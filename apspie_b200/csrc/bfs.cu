@@ -749,11 +749,12 @@ int thin_blocks(int device) {
 
 using namespace apspie;
 
-extern "C" {
-
-int apspie_bfs(apspie_ctx ctx, int src, int64_t nnz, int m, const int *d_ptr,
-               const int *d_ind, const int *d_tptr, const int *d_tind, int32_t *d_depth,
-               int max_levels) {
+// The launches of a traversal: all of them, or (for callers that queue many
+// traversals on different streams) only those before the persistent kernel,
+// or only that one.
+int apspie::bfs_enqueue(apspie_context *ctx, int src, int64_t nnz, int m, const int *d_ptr,
+                        const int *d_ind, const int *d_tptr, const int *d_tind, int32_t *d_depth,
+                        int max_levels, BfsPart part) {
   APSPIE_CHECK_CTX(ctx);
   if (m <= 0 || src < 0 || src >= m)
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_bfs: src %d outside [0,%d)", src, m);
@@ -786,8 +787,11 @@ int apspie_bfs(apspie_ctx ctx, int src, int64_t nnz, int m, const int *d_ptr,
   long long nnz_ll = (long long)nnz;
   int alpha = ctx->bfs_alpha, beta = ctx->bfs_beta, mode = ctx->bfs_mode;
   if (!d_tptr) mode = 1;  // no in-adjacency: push only
-  const int thin = (long long)nnz <= kThinMeanDegree * m && mode != 2 ? thin_blocks(ctx->device) : 0;
-  if (thin) {
+  int thin = (long long)nnz <= kThinMeanDegree * m && mode != 2 ? thin_blocks(ctx->device) : 0;
+  // beside other launches (a share of the grid) half the cluster finds a place
+  // sooner, and several fit
+  if (ctx->max_grid > 0) thin = std::min(thin, kThinBlocks / 2);
+  if (thin && part != BfsPart::kMain) {
     bfs_init<<<std::min((m + 255) / 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
         m, src, d_depth, d_ptr, qa, ca, st);
     cudaLaunchAttribute at{};
@@ -806,6 +810,7 @@ int apspie_bfs(apspie_ctx ctx, int src, int64_t nnz, int m, const int *d_ptr,
     int rc = check_launch(ctx, "bfs_thin", 2);
     if (rc) return rc;
   }
+  if (part == BfsPart::kFirst) return APSPIE_OK;
   int par = thin ? -1 : ctx->bfs_par;
   void *args[] = {&m,  &nnz_ll, (void *)&d_ptr, (void *)&d_ind, (void *)&d_tptr, (void *)&d_tind,
                   &d_depth, &qa, &qb, &ca, &cb, &st, &max_levels, &alpha, &beta, &mode,
@@ -816,6 +821,15 @@ int apspie_bfs(apspie_ctx ctx, int src, int64_t nnz, int m, const int *d_ptr,
   if (!thin) ctx->bfs_par ^= 1;
   ctx->launches += 1;
   return APSPIE_OK;
+}
+
+extern "C" {
+
+int apspie_bfs(apspie_ctx ctx, int src, int64_t nnz, int m, const int *d_ptr,
+               const int *d_ind, const int *d_tptr, const int *d_tind, int32_t *d_depth,
+               int max_levels) {
+  return bfs_enqueue(ctx, src, nnz, m, d_ptr, d_ind, d_tptr, d_tind, d_depth, max_levels,
+                     BfsPart::kAll);
 }
 
 int apspie_bfs_get_stats(apspie_ctx ctx, apspie_bfs_stats *out) {

@@ -236,6 +236,12 @@ uint64_t graph_fingerprint(apspie_context *ctx, int m, int64_t nnz, const int *d
 // d_out[i] = d_ptr[m * i / 64] for i = 0..64 (one small launch)
 int gather_offsets(apspie_context *ctx, const int *d_ptr, int m, int *d_out);
 
+// The launches of a BFS, or part of them (bfs.cu).
+enum class BfsPart { kAll, kFirst, kMain };
+int bfs_enqueue(apspie_context *ctx, int src, int64_t nnz, int m, const int *d_ptr,
+                const int *d_ind, const int *d_tptr, const int *d_tind, int32_t *d_depth,
+                int max_levels, BfsPart part);
+
 // Blocks of `kernel` (threads per block, no dynamic shared memory) that fit
 // on the context's device at once: the occupancy times the SM count, cached
 // per (kernel, device) under a lock (contexts may be used from several

@@ -460,8 +460,8 @@ __device__ void msbfs_pull(BatchJob *j, int L, int unit, unsigned long long *s_a
     const int myrank = __popc(U & ((1u << lane) - 1u));
     if (mine) s_rank[myrank] = lane;
     __syncwarp();
-    const int per = 32 / k, extra = 32 % k;
-    const int jr = lane % k, slot = lane / k;
+    const int per = div32(32, k), extra = 32 - per * k;
+    const int slot = div32(lane, k), jr = lane - slot * k;
     const int nl = per + (jr < extra ? 1 : 0);
     const int owner = s_rank[jr];
     const int so = __shfl_sync(kFull, s, owner);

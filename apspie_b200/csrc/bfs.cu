@@ -561,7 +561,11 @@ bfs_persistent(int m, long long nnz, const int *__restrict__ ptr, const int *__r
       // of them unresolved, vertex of rank j gets lanes j, j+k, j+2k, ... and
       // each of those lanes probes kProbe in-neighbours (all index loads, then
       // all depth loads), so every round keeps 32 x kProbe probes in flight and
-      // a vertex leaves as soon as one probe hits.  Discoveries are counted,
+      // a vertex leaves as soon as one probe hits.  While more than half of
+      // the lanes are unresolved each probes for itself: the sharing would
+      // add less than one probe per vertex and costs most of a round's
+      // instructions (the first pull level of R-MAT 22 issued in 53 % of the
+      // cycles).  Discoveries are counted,
       // not queued: the next frontier is depth == L + 1.
       unsigned cnt = 0;
       unsigned long long edg = 0;
@@ -614,11 +618,20 @@ bfs_persistent(int m, long long nnz, const int *__restrict__ ptr, const int *__r
         while (U) {
           const int k = __popc(U);
           const bool mine = (U >> lane) & 1u;
+          if (k > 16) {
+            // most lanes are unresolved: each probes for its own vertex
+            const int nb = mine ? __ldg(tind + s) : 0;
+            const int dn = mine ? __ldcg(depth + nb) : -1;
+            found |= mine && dn == L;
+            s += mine ? 1 : 0;
+            U = __ballot_sync(kFull, mine && !found && s < e);
+            continue;
+          }
           const int myrank = __popc(U & ((1u << lane) - 1u));
           if (mine) s_rank[warp][myrank] = lane;
           __syncwarp();
-          const int per = 32 / k, extra = 32 % k;
-          const int j = lane % k, slot = lane / k;
+          const int per = div32(32, k), extra = 32 - per * k;
+          const int slot = div32(lane, k), j = lane - slot * k;
           const int nl = per + (j < extra ? 1 : 0);
           const int owner = s_rank[warp][j];
           const int so = __shfl_sync(kFull, s, owner);
@@ -636,7 +649,7 @@ bfs_persistent(int m, long long nnz, const int *__restrict__ ptr, const int *__r
           __syncwarp();
           const unsigned fm = *(volatile unsigned *)&s_found[warp];
           if (mine) s += (per + (myrank < extra ? 1 : 0)) * kProbe;
-          found = (fm >> lane) & 1u;
+          found |= (fm >> lane) & 1u;
           U = __ballot_sync(kFull, mine && !found && s < e);
         }
         if (found) depth[v] = next;

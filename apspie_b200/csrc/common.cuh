@@ -49,6 +49,15 @@ __device__ __forceinline__ int warp_owner(int excl, int e) {
   return lo;
 }
 
+// n / k for 0 <= n <= 32 and 1 <= k <= 32, by a reciprocal from constant
+// memory (k is the same for the whole warp): a division is 20 to 30
+// instructions, and the pull loops divide twice per round.
+static __constant__ unsigned kInverse[33] = {
+    0,    65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192, 7282, 6554,
+    5958, 5462,  5042,  4682,  4370,  4096,  3856,  3641, 3450, 3277, 3121,
+    2979, 2850,  2731,  2622,  2521,  2428,  2341,  2260, 2185, 2115, 2048};
+__device__ __forceinline__ int div32(int n, int k) { return (int)(((unsigned)n * kInverse[k]) >> 16); }
+
 // Warp-aggregated append of the lanes with pred set: one atomicAdd per warp.
 // Returns this lane's slot (undefined where pred is false).
 __device__ __forceinline__ unsigned warp_append(bool pred, unsigned *counter) {

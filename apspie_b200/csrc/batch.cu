@@ -516,19 +516,27 @@ __device__ __forceinline__ unsigned sat_add(unsigned d, unsigned w) {
 
 // Edges per batch of a job with row width sw: kSsspSlots rounds of 32 / sw
 // edges, at most 32 (one per loading lane).
-__device__ __forceinline__ int mssp_batch(int sw) { return min(32, kSsspSlots * (32 / sw)); }
+// (sw is a power of two: shifts, not divisions -- the relaxation is bound by
+// its instructions).
+__device__ __forceinline__ int width_log2(int sw) { return 31 - __clz(sw); }
+__device__ __forceinline__ int mssp_batch(int sw) {
+  return min(32, kSsspSlots * (32 >> width_log2(sw)));
+}
 
 // Relaxes the batch of edges held by lanes 0..nb-1 (ue: target, we: weight,
 // ve: tail, me: the tail's active-source mask; me == 0 for no edge), for every
 // active source.  Lane l of a round works on edge (round * 32/sw + l / sw)
 // and source l % sw.  Returns, on the loading lanes, whether that edge's
-// target entered the next frontier.
+// target entered the next frontier.  kOneTail: every edge has the tail ve,
+// whose distance to source l % sw the caller passes as dv (one load for a
+// hub's chunk instead of one per edge).
+template <bool kOneTail = false>
 __device__ __forceinline__ bool mssp_relax(BatchJob *j, int ue, unsigned we, int ve, unsigned me,
-                                           unsigned long long *Fn) {
+                                           unsigned long long *Fn, unsigned dv = 0u) {
   const int lane = lane_id();
-  const int sw = j->sw;
-  const int per = 32 / sw;                 // edges per round
-  const int src = lane & (sw - 1), eo = lane / sw;
+  const int sw = j->sw, lg = width_log2(sw);
+  const int per = 32 >> lg;                // edges per round
+  const int src = lane & (sw - 1), eo = lane >> lg;
   const unsigned grp = sw == 32 ? 0xffffffffu : ((1u << sw) - 1u);
   unsigned *dist = reinterpret_cast<unsigned *>(j->out);
   unsigned nd[kSsspSlots], cur[kSsspSlots];
@@ -539,13 +547,15 @@ __device__ __forceinline__ bool mssp_relax(BatchJob *j, int ue, unsigned we, int
     const int el = i * per + eo;           // the edge's loading lane
     const bool in = el < 32;
     const unsigned mi = __shfl_sync(kFull, me, el & 31);
-    const int vi = __shfl_sync(kFull, ve, el & 31);
+    const int vi = kOneTail ? ve : __shfl_sync(kFull, ve, el & 31);
     const unsigned wi = __shfl_sync(kFull, we, el & 31);
     uu[i] = __shfl_sync(kFull, ue, el & 31);
     act[i] = in && ((mi >> src) & 1u);
     // the tail's distance is read from L2 (it dropped in the last round)
-    nd[i] = act[i] ? sat_add(__ldcg(dist + (size_t)vi * sw + src), wi) : 0u;
-    cur[i] = act[i] ? __ldcg(dist + (size_t)uu[i] * sw + src) : 0u;
+    const unsigned di =
+        kOneTail ? dv : (act[i] ? __ldcg(dist + ((size_t)vi << lg) + src) : 0u);
+    cur[i] = act[i] ? __ldcg(dist + ((size_t)uu[i] << lg) + src) : 0u;
+    nd[i] = sat_add(di, wi);
   }
   // the slots' minima, issued without waiting for their old values: a
   // (target, source) whose distance read this step is above nd drops this
@@ -554,7 +564,7 @@ __device__ __forceinline__ bool mssp_relax(BatchJob *j, int ue, unsigned we, int
   // and the ballots need not wait for the atomics
 #pragma unroll
   for (int i = 0; i < kSsspSlots; ++i)
-    min_if(act[i] && nd[i] < cur[i], dist + (size_t)uu[i] * sw + src, nd[i]);
+    min_if(act[i] && nd[i] < cur[i], dist + ((size_t)uu[i] << lg) + src, nd[i]);
   unsigned mybal = 0;
 #pragma unroll
   for (int i = 0; i < kSsspSlots; ++i) {
@@ -562,7 +572,7 @@ __device__ __forceinline__ bool mssp_relax(BatchJob *j, int ue, unsigned we, int
     const unsigned b = __ballot_sync(kFull, imp);
     // loading lane i * per + g takes the bits of its edge's group g
     const int g = lane - i * per;
-    if (g >= 0 && g < per) mybal = (b >> (g * sw)) & grp;
+    if (g >= 0 && g < per) mybal = (b >> (g << lg)) & grp;
   }
   bool first = false;
   if (mybal) first = atomicOr(Fn + ue, (unsigned long long)mybal) == 0ull;
@@ -618,6 +628,10 @@ __device__ void mssp_chunk(BatchJob *j, int L, int unit, const AppendCtx &ac) {
   const int e = min(s + kSsspChunk, __ldg(j->ptr + v + 1));
   const unsigned mv = (unsigned)__ldcg(Fc + v);
   const int nb = mssp_batch(j->sw);
+  // the tail's distances, one per source; one that drops while the chunk runs
+  // queues the tail again
+  const unsigned dv = __ldcg(reinterpret_cast<unsigned *>(j->out) +
+                             ((size_t)v << width_log2(j->sw)) + (lane & (j->sw - 1)));
   for (int k0 = s; k0 < e; k0 += nb) {
     const int k = k0 + lane;
     int ue = 0;
@@ -627,7 +641,7 @@ __device__ void mssp_chunk(BatchJob *j, int L, int unit, const AppendCtx &ac) {
       we = __ldg(j->w + k);
       me = mv;
     }
-    bool f[1] = {mssp_relax(j, ue, we, v, me, Fn)};
+    bool f[1] = {mssp_relax<true>(j, ue, we, v, me, Fn, dv)};
     int u1[1] = {ue}, dg[1] = {0};
     if (f[0]) dg[0] = __ldg(j->ptr + ue + 1) - __ldg(j->ptr + ue);
     append_n<1>(j, f, u1, dg, ac);
@@ -656,8 +670,8 @@ __global__ void batch_hub_chunks(BatchJob *jobs, int jid) {
 __device__ __forceinline__ unsigned mssp_pull_min(const BatchJob *j, int a0, int a1,
                                                   const unsigned long long *Fc) {
   const int lane = lane_id();
-  const int sw = j->sw, per = 32 / sw;
-  const int src = lane & (sw - 1), eo = lane / sw;
+  const int sw = j->sw, per = 32 >> width_log2(sw);
+  const int src = lane & (sw - 1), eo = lane >> width_log2(sw);
   const unsigned *dist = reinterpret_cast<const unsigned *>(j->out);
   unsigned best = 0xffffffffu;
   // four in-edges per lane in flight: their indices, then their frontier

@@ -410,7 +410,7 @@ bfs_persistent(int m, long long nnz, const int *__restrict__ ptr, const int *__r
                int beta, int mode, unsigned *gmask, int src, int init_par) {
   const int lane = lane_id();
   const int warp = warp_in_block();
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int gwarp = spread_warp();
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
   __shared__ unsigned s_q, s_chunks, s_nbig, s_nimpl;
   __shared__ unsigned long long s_edges;

@@ -18,6 +18,14 @@ constexpr unsigned kFull = 0xffffffffu;
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_in_block() { return threadIdx.x >> 5; }
 
+// Number of this warp among the grid's, neighbours in different blocks: the
+// first n units of a small round are then n SMs' work, where block by block
+// they would be the sixteen warps of a few blocks, whose scattered accesses
+// queue in those few SMs (one per 4.5 cycles and SM).
+__device__ __forceinline__ int spread_warp() {
+  return (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
+}
+
 // Inclusive warp scan (Kogge-Stone over shuffles).
 template <typename T>
 __device__ __forceinline__ T warp_incl_scan(T v) {

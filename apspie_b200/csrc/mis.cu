@@ -80,7 +80,7 @@ mis_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
                unsigned long long *word, int32_t *out, int2 *qa, int2 *qb, MisState *st,
                double delta, int max_rounds) {
   const int lane = lane_id();
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int gwarp = spread_warp();
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
   __shared__ unsigned s_q;
   int r = 0;

@@ -243,7 +243,7 @@ sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
                 int *far1, int *far2, unsigned delta, long long nnz, const int *__restrict__ tptr,
                 const int *__restrict__ tind, const W *__restrict__ tw, const int2 *hubc,
                 int alpha, unsigned long long *xw) {
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int gwarp = spread_warp();
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
   const int lane = lane_id();
   __shared__ unsigned s_q, s_chunks, s_nbig, s_far;

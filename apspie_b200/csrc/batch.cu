@@ -758,7 +758,7 @@ __device__ void mssp_pull(BatchJob *j, int L, int unit, const AppendCtx &ac) {
 // ---------------------------------------------------------------- kernel ---
 __global__ void __launch_bounds__(kBatchThreads, 2)
 batch_persistent(BatchJob *jobs, int njobs, BatchState *st, int max_steps) {
-  const int gwarp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int gwarp = spread_warp();
   const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
   const int warp = warp_in_block();
   __shared__ unsigned s_q[kMaxJobs], s_ch[kMaxJobs];

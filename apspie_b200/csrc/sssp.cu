@@ -125,9 +125,9 @@ struct Arith<float> {
 // improved target below the threshold joins the next frontier (class 1,
 // once per round by the stamp); one at or above it goes to the far list
 // (class 2, once per phase by the far stamp).
-template <typename W>
+template <typename W, bool FAR>
 struct SsspVisit {
-  static constexpr bool kTwoWay = true;
+  static constexpr bool kTwoWay = FAR;
   const W *__restrict__ w;
   unsigned *dist;
   int *stamp;
@@ -138,7 +138,7 @@ struct SsspVisit {
   unsigned *far_count;
   unsigned *far_min;
   // far lists only exist under a finite threshold (near-far schedule)
-  __device__ __forceinline__ bool two_way() const { return thresh != Arith<W>::kInf; }
+  __device__ __forceinline__ bool two_way() const { return FAR && thresh != Arith<W>::kInf; }
   __device__ __forceinline__ bool check(bool on, unsigned du, int k, int u, unsigned &nd) const {
     // selected, not branched around: the batch's loads are in flight together
     const W wk = on ? __ldg(w + k) : W(0);
@@ -164,12 +164,16 @@ struct SsspVisit {
     int prev[N];
 #pragma unroll
     for (int r = 0; r < N; ++r) {
-      const bool near = nd[r] < thresh;
+      const bool near = !FAR || nd[r] < thresh;
       prev[r] = exch_if(ok[r], (near ? stamp : fstamp) + u[r], near ? round : phase, 0);
     }
 #pragma unroll
     for (int r = 0; r < N; ++r) {
       cls[r] = 0;
+      if (!FAR) {
+        cls[r] = ok[r] && prev[r] != round ? 1 : 0;
+        continue;
+      }
       if (ok[r]) cls[r] = nd[r] < thresh ? (prev[r] != round ? 1 : 0)
                                          : (prev[r] != phase ? 2 : 3);  // 3: far, already listed
     }
@@ -231,12 +235,17 @@ __global__ void sssp_hub_chunks(int m, const int *__restrict__ tptr, int2 *hubc,
   }
 }
 
-// MINB blocks per SM: 2 for the push-only entry points; 3 when pull rounds
-// are possible (their loops carry no atomics and gain from the extra warps:
-// R-MAT 22 push/pull 4.0 vs 4.7 ms per source, while push-only ran 12 %
-// slower at 3 blocks, which costs spills at 40 registers; measured).
-template <typename W, int MINB>
-__global__ void __launch_bounds__(kSsspThreads, MINB)
+// What a launch can do: push rounds alone, push rounds under the near-far
+// schedule, or push and pull rounds.  Each is a kernel of its own: the plain
+// rounds have no spills at 64 registers without the others' code (R-MAT 20
+// u32 617 -> 583 us).  Two blocks per SM where rounds push (three, at 40
+// registers with spills: 656 us); three for the pull kind, whose pull loops
+// carry no atomics and gain from the extra warps.
+enum SsspKind { kPlain, kNearFar, kPull };
+constexpr int sssp_blocks(SsspKind k) { return k == kPull ? 3 : 2; }
+
+template <typename W, SsspKind KIND>
+__global__ void __launch_bounds__(kSsspThreads, sssp_blocks(KIND))
 sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
                 const W *__restrict__ w, unsigned *dist, int *stamp, int *qa, int *qb, int2 *ca,
                 int2 *cb, SsspState *st, int max_rounds, int *fstamp, unsigned *xd, int *far0,
@@ -251,7 +260,7 @@ sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
   __shared__ unsigned s_best[kSsspThreads / 32][32];
   // T = infinity without near-far; else the first phase covers [0, delta)
   if (blockIdx.x == 0 && threadIdx.x == 0) st->t_start = globaltimer();
-  unsigned thresh = delta ? delta : Arith<W>::kInf;
+  unsigned thresh = KIND == kNearFar ? delta : Arith<W>::kInf;
   int phase = 0;
   int r = 0;
   for (;; ++r) {
@@ -264,7 +273,7 @@ sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
       s_chunks = bc_chunks(bc);
       s_nbig = bc_big(bc);
       s_edges = __ldcg(&cur->edges);
-      s_far = __ldcg(&st->far_count[phase % 3]);
+      s_far = KIND == kNearFar ? __ldcg(&st->far_count[phase % 3]) : 0u;
       if (blockIdx.x == 0) *clr = LevelCounters{0ull, 0, 0, 0ull};
     }
     __syncthreads();
@@ -276,7 +285,7 @@ sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
       // near frontier empty: done, or open the next phase by splitting the
       // far list of this one into the next near frontier and the next far list
       const unsigned nfar = s_far;
-      if (nfar == 0) break;
+      if (KIND != kNearFar || nfar == 0) break;
       int *fin = phase % 3 == 0 ? far0 : (phase % 3 == 1 ? far1 : far2);
       // the next threshold: one step up, or one step above the least far
       // distance when that is higher (skips empty ranges); it always grows
@@ -314,8 +323,7 @@ sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
       if (!grid_barrier(st->bar, &st->err)) return;
       continue;
     }
-    if (tptr && delta == 0u && r > 0 && alpha > 0 &&
-        (long long)s_edges * alpha > nnz) {
+    if (KIND == kPull && r > 0 && (long long)s_edges * alpha > nnz) {
       // ---- pull round: every vertex takes the least d[u] + w over its
       // in-neighbours in the frontier; hub chunks and 32-vertex groups are
       // handed out by the round's counter ----
@@ -411,7 +419,7 @@ sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
     int *qin = (r & 1) ? qb : qa;
     int2 *cin = (r & 1) ? cb : ca;
     int *fout = phase % 3 == 0 ? far0 : (phase % 3 == 1 ? far1 : far2);
-    SsspVisit<W> vis{w,    dist,   stamp, fstamp, r, phase, thresh, fout, &st->far_count[phase % 3],
+    SsspVisit<W, KIND == kNearFar> vis{w,    dist,   stamp, fstamp, r, phase, thresh, fout, &st->far_count[phase % 3],
                      &st->far_min[phase % 3]};
     // A queued vertex whose distance still equals the one it was last
     // expanded with (it improved again in the round that expanded it, so it
@@ -490,9 +498,11 @@ sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
   }
 }
 
-template <typename W, int MINB>
-int sssp_grid(apspie_context *ctx) {
-  return occupancy_grid(ctx, (const void *)sssp_persistent<W, MINB>, kSsspThreads);
+template <typename W>
+const void *sssp_kernel(SsspKind kind) {
+  return kind == kNearFar ? (const void *)sssp_persistent<W, kNearFar>
+         : kind == kPull  ? (const void *)sssp_persistent<W, kPull>
+                          : (const void *)sssp_persistent<W, kPlain>;
 }
 
 template <typename W>
@@ -507,9 +517,9 @@ int sssp_run(apspie_context *ctx, int src, int64_t nnz, int m, const int *d_ptr,
   if (!d_ptr || !d_dist || (nnz > 0 && (!d_ind || !d_w)) ||
       (d_tptr && nnz > 0 && (!d_tind || !d_tw)))
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_sssp: null pointer");
-  // without a pull switch no round pulls: the in-adjacency is not needed
-  // and the push-only kernel (two blocks per SM, more registers) runs
-  if (ctx->sssp_pull_alpha == 0) {
+  // without a pull switch, or under near-far, no round pulls: the in-adjacency
+  // is not needed
+  if (ctx->sssp_pull_alpha == 0 || delta) {
     d_tptr = nullptr;
     d_tind = nullptr;
     d_tw = nullptr;
@@ -531,8 +541,8 @@ int sssp_run(apspie_context *ctx, int src, int64_t nnz, int m, const int *d_ptr,
   int *fstamp = nf, *far0 = nf + 2 * mm, *far1 = nf + 3 * mm, *far2 = nf + 4 * mm;
   unsigned *xd = (unsigned *)(nf + mm);
   ctx->sssp_state = st;
-  const bool pull3 = d_tptr != nullptr;
-  int grid = persistent_grid(ctx, pull3 ? sssp_grid<W, 3>(ctx) : sssp_grid<W, 2>(ctx),
+  const void *kern = sssp_kernel<W>(delta ? kNearFar : (d_tptr ? kPull : kPlain));
+  int grid = persistent_grid(ctx, occupancy_grid(ctx, kern, kSsspThreads),
                              ctx->sssp_blocks_per_sm);
   if (grid <= 0) return set_error(ctx, APSPIE_ERR_CUDA, "apspie_sssp: occupancy query failed");
   int init_grid = std::min((m + 255) / 256, ctx->num_sms * 8);
@@ -555,8 +565,6 @@ int sssp_run(apspie_context *ctx, int src, int64_t nnz, int m, const int *d_ptr,
                   &qa, &qb,            &ca,            &cb,           &st,     &max_rounds,
                   &fstamp, &xd, &far0, &far1, &far2, &delta, &nnz_ll, (void *)&d_tptr,
                   (void *)&d_tind, (void *)&d_tw, &hubc, &alpha, &xw};
-  const void *kern =
-      pull3 ? (const void *)sssp_persistent<W, 3> : (const void *)sssp_persistent<W, 2>;
   cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(grid),
                                               dim3(kSsspThreads), args, 0, ctx->stream);
   if (e != cudaSuccess) return check_cuda(ctx, e, "sssp_persistent");

@@ -203,17 +203,17 @@ constexpr int kMaxPasses = 8;
 // Status words.  32 bits for sorts of fewer than 2^27 keys: flag 2 bits, pass
 // tag 3 bits, count 27 bits; else 64 bits (flag 2, tag 22, count 40).  The
 // tag tells a pass's words from those an earlier pass left, so all passes
-// share one zeroed array.  A tile loads kWindow predecessors' words at once:
-// the look-back moves on by that many tiles per L2 round trip (about 0.35 us),
-// which bounds the tiles finished per microsecond -- with 4 words a pass over
-// 16 M pairs took 170 us whether the pairs had 8 or 12 bytes.
+// share one zeroed array.  A tile loads kWindow predecessors' words at once,
+// so the look-back moves on by that many tiles per L2 round trip (about
+// 0.35 us).  It does not bound a pass: windows of 4 and of 16 words take the
+// same time (and the wider one spills registers).
 template <typename S>
 struct SortStatus;
 template <>
 struct SortStatus<unsigned> {
   static constexpr unsigned kAgg = 1u << 30, kIncl = 2u << 30, kFlags = 3u << 30;
   static constexpr unsigned kTag = 7u << 27, kCount = (1u << 27) - 1u;
-  static constexpr int kWindow = 16;
+  static constexpr int kWindow = 4;
   __device__ __forceinline__ static unsigned tag(int pass) { return (unsigned)pass << 27; }
   __device__ __forceinline__ static unsigned load(const unsigned *p) {
     unsigned v;
@@ -225,7 +225,7 @@ template <>
 struct SortStatus<unsigned long long> {
   static constexpr unsigned long long kAgg = 1ull << 62, kIncl = 2ull << 62, kFlags = 3ull << 62;
   static constexpr unsigned long long kTag = 0x3FFFFFull << 40, kCount = (1ull << 40) - 1ull;
-  static constexpr int kWindow = 8;
+  static constexpr int kWindow = 4;
   __device__ __forceinline__ static unsigned long long tag(int pass) {
     return (unsigned long long)pass << 40;
   }
@@ -284,6 +284,16 @@ __global__ void radix_digit_offsets(unsigned long long *ghist, int npass) {
 // publishes within microseconds; about half a second with the back-off).
 constexpr unsigned kLookbackSpinLimit = 1u << 20;
 
+// A pass over 16 M pairs of 4-byte keys and values takes 151 us, 1.7 TB/s of
+// the 256 MB it reads and writes: its bound is the instructions of ranking
+// and placing a key (issue slots 43 % busy, the rest mostly waits for shared
+// memory, three blocks of 80 registers per SM), not the bytes -- 12-byte
+// pairs took as long.  So such pairs go through shared memory side by side:
+// one store, one load and one look-up of the digit's run per pair (keys and
+// values apart: 167 us).
+template <typename K, typename V>
+constexpr bool kSortPairs = sizeof(K) == 4 && sizeof(V) == 4;
+
 template <typename K, typename V, typename S>
 __global__ void __launch_bounds__(kSortThreads, 3)
 radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, long long n,
@@ -291,11 +301,12 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
                unsigned *tile_counter, int *err, int *gaveup) {
   constexpr int kWarps = kSortThreads / 32;
   static_assert(sizeof(V) <= sizeof(K), "values are staged in the keys' shared array");
-  // the tile in digit order (keys, then values), each key's digit, per-warp
-  // digit counts, and per digit the output position of the tile's run minus
-  // its start within the tile
-  __shared__ __align__(16) K skeys[kSortTile];
-  __shared__ unsigned char sdig[kSortTile];
+  constexpr bool kPair = kSortPairs<K, V>;
+  // the tile in digit order (pairs, or keys and then values), each key's
+  // digit, per-warp digit counts, and per digit the output position of the
+  // tile's run minus its start within the tile
+  __shared__ __align__(16) K skeys[kPair ? 2 * kSortTile : kSortTile];
+  __shared__ unsigned char sdig[kPair ? 1 : kSortTile];
   __shared__ unsigned whist[kWarps][kRadix];
   __shared__ unsigned long long gbase[kRadix];
   __shared__ unsigned s_scan[33];
@@ -425,6 +436,7 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
   }
   gbase[d] = goff[pass * kRadix + d] + (unsigned long long)excl - loc;
   for (int ww = 0; ww < kWarps; ++ww) whist[ww][d] += loc;
+  if (kPair && vdone > 0) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
   // tile position of every key: its digit's start + the warps before it + its rank
 #pragma unroll
@@ -432,32 +444,53 @@ radix_onesweep(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, lon
     if (wofs + i * 32 + lane < tlen) {
       const unsigned dd = (unsigned)(kv[i] >> shift) & (kRadix - 1);
       pos[i] += whist[w][dd];
-      skeys[pos[i]] = kv[i];
-      sdig[pos[i]] = (unsigned char)dd;
+      if constexpr (kPair) {
+        union { V v; unsigned u; } bits;
+        const int t = wofs + i * 32 + lane;
+        bits.v = t < vdone ? svin[t] : (vals_in ? vals_in[tbase + t] : (V)(tbase + t));
+        reinterpret_cast<uint2 *>(skeys)[pos[i]] = make_uint2((unsigned)kv[i], bits.u);
+      } else {
+        skeys[pos[i]] = kv[i];
+        sdig[pos[i]] = (unsigned char)dd;
+      }
     }
   }
   __syncthreads();
-  // the bound holds for every sorted pass; it guards a pass after a
+  // The bound (at < n) holds for every sorted pass; it guards a pass after a
   // look-back give-up, whose input then holds keys the histograms did not
-  // count
-  for (int t = threadIdx.x; t < tlen; t += kSortThreads) {
-    const unsigned long long at = gbase[sdig[t]] + t;
-    if (at < (unsigned long long)n) keys_out[at] = skeys[t];
-  }
-  if (vals_out) {  // keys-only sorts pass no values
-    if (vdone > 0) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-    V *svals = reinterpret_cast<V *>(skeys);
-#pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-      const int t = wofs + i * 32 + lane;
-      if (t < tlen)
-        svals[pos[i]] = t < vdone ? svin[t] : (vals_in ? vals_in[tbase + t] : (V)(tbase + t));
+  // count.
+  if constexpr (kPair) {
+#pragma unroll 4
+    for (int t = threadIdx.x; t < tlen; t += kSortThreads) {
+      const uint2 x = reinterpret_cast<const uint2 *>(skeys)[t];
+      const unsigned long long at = gbase[(x.x >> shift) & (kRadix - 1)] + t;
+      if (at < (unsigned long long)n) {
+        union { unsigned u; V v; } bits;
+        bits.u = x.y;
+        keys_out[at] = (K)x.x;
+        if (vals_out) vals_out[at] = bits.v;
+      }
     }
-    __syncthreads();
+  } else {
     for (int t = threadIdx.x; t < tlen; t += kSortThreads) {
       const unsigned long long at = gbase[sdig[t]] + t;
-      if (at < (unsigned long long)n) vals_out[at] = svals[t];
+      if (at < (unsigned long long)n) keys_out[at] = skeys[t];
+    }
+    if (vals_out) {  // keys-only sorts pass no values
+      if (vdone > 0) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      __syncthreads();
+      V *svals = reinterpret_cast<V *>(skeys);
+#pragma unroll
+      for (int i = 0; i < kSortItems; ++i) {
+        const int t = wofs + i * 32 + lane;
+        if (t < tlen)
+          svals[pos[i]] = t < vdone ? svin[t] : (vals_in ? vals_in[tbase + t] : (V)(tbase + t));
+      }
+      __syncthreads();
+      for (int t = threadIdx.x; t < tlen; t += kSortThreads) {
+        const unsigned long long at = gbase[sdig[t]] + t;
+        if (at < (unsigned long long)n) vals_out[at] = svals[t];
+      }
     }
   }
 }

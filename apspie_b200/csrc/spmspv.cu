@@ -10,15 +10,15 @@
 // walked in tiles of equal size (edges.cuh), so a hub column costs no more
 // than its entries.
 //   * bitmap path: products are combined with atomics into a dense
-//     accumulator and a touched bitmap, and y is compacted from the bitmap in
-//     index order -- no sort, and nothing that the host has to know before
+//     accumulator, and the touched rows' bitmap, then y, are compacted from it
+//     in index order -- no sort, and nothing that the host has to know before
 //     the end, so the call waits for the device once;
 //   * sort path: the tiles write (row, x (x) a) pairs, the pairs are
 //     radix-sorted on only ceil(log2 m) key bits, and a segmented reduce emits
 //     sorted y.
 // The sort path is for frontiers that are sparse against a long y: its cost
 // grows with the expanded size E, the bitmap path's with m (clearing and
-// reading the accumulator, about 5 us per 2^20 rows), and the sort's launches
+// reading the accumulator, about 7 us per 2^20 rows), and the sort's launches
 // alone outlast that up to kBitmapRows rows.  Beyond, E * factor is compared
 // with m (threshold settable, picked by the autotuner; 0 always sorts).  Both
 // give y sorted by row with one entry per touched row; PLUS_TIMES accumulates
@@ -164,10 +164,17 @@ __global__ void reduce_segments(int sr, const int *keys, const float *vals, long
 }
 
 // ---- bitmap path ----
-// MIN_PLUS and MAX_TIMES reduce floats: one 32-bit word per row that orders as
-// the float does, so that the atomics are native (a double needs a
-// compare-and-swap loop).  NaN terms are left out, as a comparison does; a
-// row that only such terms or infinities touch keeps the identity.
+// One accumulator word per row, which also tells whether the row was touched:
+// a bitmap beside it costs a second random L2 access per product (the expansion
+// of 6.3 M products, 1 M rows: 73 us with one, 44 us without).
+//   PLUS_TIMES  a double that starts at -0.0, which no sum reaches: a term of
+//               -0.0 is added as +0.0, and x + -x is +0.0
+//   MIN_PLUS,   32 bits that order as the float does, so that the atomics are
+//   MAX_TIMES   native; they start beyond every float's word, and a NaN's word
+//               loses to every number's (fminf and fmaxf leave NaN out)
+//   OR_AND      0, then 1
+constexpr unsigned long long kNoSum = 0x8000000000000000ull;
+
 __device__ __forceinline__ unsigned ordered_bits(float f) {
   const unsigned b = __float_as_uint(f);
   return (b >> 31) ? ~b : b | 0x80000000u;
@@ -175,87 +182,112 @@ __device__ __forceinline__ unsigned ordered_bits(float f) {
 __device__ __forceinline__ float ordered_float(unsigned u) {
   return __uint_as_float((u >> 31) ? u & 0x7fffffffu : ~u);
 }
+__device__ __forceinline__ unsigned untouched_word(int sr) { return sr == kMinPlus ? ~0u : 0u; }
+__device__ __forceinline__ unsigned nan_word(int sr) { return sr == kMinPlus ? ~1u : 1u; }
 
-// Clears the accumulator (doubles for PLUS_TIMES, ordered words for MIN_PLUS
-// and MAX_TIMES) and the bitmap.
-__global__ void acc_init(int sr, int m, void *acc, unsigned *bits) {
-  const unsigned idw = sr == kMinPlus ? ordered_bits(INFINITY) : ordered_bits(-INFINITY);
+__global__ void acc_init(int sr, int m, unsigned long long *acc) {
+  const unsigned w = untouched_word(sr);
+  const unsigned long long v = sr == kPlusTimes ? kNoSum : (unsigned long long)w << 32 | w;
+  const unsigned n = sr == kPlusTimes ? (unsigned)m : ((unsigned)m + 1u) / 2u;
   const unsigned stride = gridDim.x * blockDim.x;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)m; i += stride) {
-    if (sr == kPlusTimes) ((double *)acc)[i] = 0.0;
-    else if (sr != kOrAnd) ((unsigned *)acc)[i] = idw;
-    if ((i & 31u) == 0u) bits[i >> 5] = 0u;
-  }
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) acc[i] = v;
 }
 
 __global__ void __launch_bounds__(kEdgeThreads)
 expand_accumulate(int sr, int xnnz, const long long *__restrict__ offs, const long long *total,
                   const int2 *__restrict__ col, const int *__restrict__ ind,
-                  const float *__restrict__ val, void *acc, unsigned *bits) {
+                  const float *__restrict__ val, void *acc) {
   for_each_entry(sr, xnnz, offs, total, col, ind, val,
                  [&](const int (&)[kEdgeItems], const int (&row)[kEdgeItems],
                      const float (&term)[kEdgeItems], const bool (&on)[kEdgeItems]) {
-                   unsigned have[kEdgeItems];
-#pragma unroll
-                   for (int q = 0; q < kEdgeItems; ++q)
-                     have[q] = on[q] ? __ldcg(bits + (row[q] >> 5)) : ~0u;
 #pragma unroll
                    for (int q = 0; q < kEdgeItems; ++q) {
                      if (!on[q]) continue;
                      if (sr == kPlusTimes) {
-                       atomicAdd((double *)acc + row[q], (double)term[q]);
-                     } else if (sr != kOrAnd && term[q] == term[q]) {
-                       const unsigned o = ordered_bits(term[q]);
-                       if (sr == kMinPlus) atomicMin((unsigned *)acc + row[q], o);
-                       else atomicMax((unsigned *)acc + row[q], o);
+                       atomicAdd((double *)acc + row[q], (double)__fadd_rn(term[q], 0.0f));
+                       continue;
                      }
-                     const unsigned bit = 1u << (row[q] & 31);
-                     if (!(have[q] & bit)) atomicOr(bits + (row[q] >> 5), bit);
+                     unsigned *a = (unsigned *)acc + row[q];
+                     const unsigned o = term[q] == term[q] ? ordered_bits(term[q]) : nan_word(sr);
+                     if (sr == kMinPlus) atomicMin(a, o);
+                     else if (sr == kMaxTimes) atomicMax(a, o);
+                     else __stcg(a, 1u);
                    }
                  });
 }
 
-// y from the bitmap, in two launches: the bits of every block's words are
-// counted (sums), then each block adds up the counts before its own and
-// writes its rows in order; the last one leaves nnz(y).
+// y from the accumulator, in two launches: the touched rows become a bitmap
+// and every block's are counted (sums), then each block adds up the counts
+// before its own and writes its rows in order, a warp per 32 of them; the last
+// one leaves nnz(y).
 constexpr int kEmitThreads = 256;
 constexpr int kEmitBlocks = 2048;  // at most
+constexpr int kEmitWords = 64;     // bitmap words per block, at least
 
 __global__ void __launch_bounds__(kEmitThreads)
-bitmap_counts(const unsigned *__restrict__ bits, int words, int per_block, unsigned *sums) {
+touched_rows(int sr, int m, const void *__restrict__ acc, int words, int per_block,
+             unsigned *bits, unsigned *sums) {
   __shared__ unsigned sw[33];
   const int w0 = blockIdx.x * per_block, w1 = min(words, w0 + per_block);
+  const unsigned none = untouched_word(sr);
   unsigned c = 0;
-  for (int w = w0 + (int)threadIdx.x; w < w1; w += kEmitThreads) c += __popc(bits[w]);
+#pragma unroll 4
+  for (int w = w0 + warp_in_block(); w < w1; w += kEmitThreads / 32) {
+    const unsigned r = (unsigned)w * 32u + lane_id();
+    bool on = r < (unsigned)m;
+    if (on)
+      on = sr == kPlusTimes ? __ldcg((const unsigned long long *)acc + r) != kNoSum
+                            : __ldcg((const unsigned *)acc + r) != none;
+    const unsigned b = __ballot_sync(kFull, on);
+    if (lane_id() == 0) {
+      bits[w] = b;
+      c += __popc(b);
+    }
+  }
   unsigned tot;
   block_excl_scan(c, sw, &tot);
   if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
+// A row of NaN terms only is NaN for a frontier that the sort path's threshold
+// calls sparse (E * factor <= m: the sorted reduction has it so), else the
+// infinity that the reduction starts from.
 __global__ void __launch_bounds__(kEmitThreads)
-bitmap_emit(int sr, const unsigned *__restrict__ bits, int words, int per_block,
-            const unsigned *__restrict__ sums, const void *__restrict__ acc, int *yind,
-            float *yval, int *ynnz) {
+touched_emit(int sr, int m, const unsigned *__restrict__ bits, int words, int per_block,
+             const unsigned *__restrict__ sums, const void *__restrict__ acc,
+             const long long *total, double factor, int *yind, float *yval, int *ynnz) {
   __shared__ unsigned sw[33];
+  __shared__ unsigned s_bits[kEmitThreads], s_off[kEmitThreads];
   unsigned before = 0, tot;
   for (unsigned i = threadIdx.x; i < blockIdx.x; i += kEmitThreads) before += sums[i];
   block_excl_scan(before, sw, &tot);
   before = tot;
   const int w0 = blockIdx.x * per_block, w1 = min(words, w0 + per_block);
   for (int base = w0; base < w1; base += kEmitThreads) {
-    const int w = base + (int)threadIdx.x;
-    unsigned b = w < w1 ? bits[w] : 0u;
-    unsigned o = before + block_excl_scan((unsigned)__popc(b), sw, &tot);
+    const int n = min(kEmitThreads, w1 - base);
+    const unsigned mine = (int)threadIdx.x < n ? bits[base + threadIdx.x] : 0u;
+    s_bits[threadIdx.x] = mine;
+    s_off[threadIdx.x] = before + block_excl_scan((unsigned)__popc(mine), sw, &tot);
     before += tot;
-    while (b) {
-      const int r = w * 32 + __ffs(b) - 1;
-      b &= b - 1;
-      yind[o] = r;
-      yval[o] = sr == kOrAnd ? 1.0f
-                : sr == kPlusTimes ? (float)((const double *)acc)[r]
-                                   : ordered_float(((const unsigned *)acc)[r]);
-      ++o;
+    __syncthreads();
+#pragma unroll 4
+    for (int w = warp_in_block(); w < n; w += kEmitThreads / 32) {
+      const unsigned b = s_bits[w];
+      if (!(b >> lane_id() & 1u)) continue;
+      const unsigned r = (unsigned)(base + w) * 32u + lane_id();
+      const unsigned o = s_off[w] + __popc(b & ((1u << lane_id()) - 1u));
+      float v = 1.0f;
+      if (sr == kPlusTimes) v = (float)__ldcg((const double *)acc + r);
+      else if (sr != kOrAnd) {
+        const unsigned u = __ldcg((const unsigned *)acc + r);
+        v = ordered_float(u);
+        if (u == nan_word(sr) && (double)__ldcg(total) * factor > (double)m)
+          v = sr == kMinPlus ? INFINITY : -INFINITY;
+      }
+      yind[o] = (int)r;
+      yval[o] = v;
     }
+    __syncthreads();
   }
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *ynnz = (int)before;
 }
@@ -346,14 +378,14 @@ int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *i
       rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, &sm->total);
       if (rc) return rc;
     }
-    acc_init<<<grid_for(ctx, m, 256), 256, 0, st>>>(sr, m, acc, bits);
+    acc_init<<<grid_for(ctx, m, 256), 256, 0, st>>>(sr, m, (unsigned long long *)acc);
     expand_accumulate<<<egrid, kEdgeThreads, 0, st>>>(sr, xnnz, offs, &sm->total, col, ind, val,
-                                                      acc, bits);
-    const int per_block = std::max(kEmitThreads, (words + kEmitBlocks - 1) / kEmitBlocks);
+                                                      acc);
+    const int per_block = std::max(kEmitWords, (words + kEmitBlocks - 1) / kEmitBlocks);
     const int eblocks = (words + per_block - 1) / per_block;
-    bitmap_counts<<<eblocks, kEmitThreads, 0, st>>>(bits, words, per_block, sums);
-    bitmap_emit<<<eblocks, kEmitThreads, 0, st>>>(sr, bits, words, per_block, sums, acc, yind,
-                                                  yval, &sm->ynnz);
+    touched_rows<<<eblocks, kEmitThreads, 0, st>>>(sr, m, acc, words, per_block, bits, sums);
+    touched_emit<<<eblocks, kEmitThreads, 0, st>>>(sr, m, bits, words, per_block, sums, acc,
+                                                   &sm->total, factor, yind, yval, &sm->ynnz);
     return check_launch(ctx, "spmspv bitmap", 4);
   }
   // sort path

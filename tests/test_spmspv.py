@@ -206,3 +206,52 @@ def test_spmspv_bitmap_extreme_terms(ctx):
     yi, yv, _ = ap.spmspv(ctx, 2, g, xi, one, val)
     assert yi.tolist() == list(range(7))
     assert yv.tolist() == [2.5, 0.0, inf, 7.0, -inf, 3.0, -4.0]
+
+
+@pytest.mark.parametrize("sr", [1, 2])
+@pytest.mark.parametrize("m", [55, 56, 57])
+def test_spmspv_nan_rows_below_the_threshold(ctx, sr, m):
+    """14 products at the default factor of 4: up to 55 rows a row of NaN
+    terms keeps the identity, from 56 on it is NaN, as the sort path has it."""
+    import torch
+    import apspie_b200 as ap
+    inf, nan = np.inf, np.nan
+    terms = np.array([-1.5, 0.0, inf, -inf, nan, 3.0, nan,
+                      2.5, -2.0, inf, 7.0, nan, nan, -4.0], np.float32)
+    ptr = np.array([0, 7] + [14] * (m - 1), np.int32)
+    ind = np.tile(np.arange(7), 2).astype(np.int32)
+    g = ap.HostGraph(m, ptr, ind).to_device(with_transpose=False)
+    xi = torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    xv = torch.full((2,), 0.0 if sr == 1 else 1.0, device="cuda")
+    val = torch.from_numpy(terms).cuda()
+    yi, yv, _ = ap.spmspv(ctx, sr, g, xi, xv, val)
+    ap.spmspv_set_params(ctx, 0.0)
+    try:
+        si, sv, _ = ap.spmspv(ctx, sr, g, xi, xv, val)
+    finally:
+        ap.spmspv_set_params(ctx)
+    assert yi.tolist() == si.tolist() == list(range(7))
+    expect = sv.cpu().numpy()
+    assert np.isnan(expect[4])
+    if m < 56:
+        expect[4] = inf if sr == 1 else -inf
+    np.testing.assert_array_equal(yv.cpu().numpy(), expect)
+
+
+@pytest.mark.parametrize("m", [31, 32, 33, 2049])
+def test_spmspv_zero_sums(ctx, m):
+    """PLUS_TIMES rows whose terms are zeros of either sign or cancel are in y
+    with +0.0, at the ends of the accumulator too."""
+    import torch
+    import apspie_b200 as ap
+    rows = np.array([0, 1, m - 2, m - 1], np.int32)
+    ptr = np.array([0, 4, 8] + [8] * (m - 2), np.int32)
+    ind = np.tile(rows, 2).astype(np.int32)
+    val = np.array([-0.0, 1.5, 0.0, -0.0, -0.0, -1.5, -0.0, 2.0], np.float32)
+    g = ap.HostGraph(m, ptr, ind).to_device(with_transpose=False)
+    xi = torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    yi, yv, _ = ap.spmspv(ctx, 0, g, xi, torch.ones(2, device="cuda"),
+                          torch.from_numpy(val).cuda())
+    assert yi.tolist() == rows.tolist()
+    assert yv.tolist() == [0.0, 0.0, 0.0, 2.0]
+    assert not np.signbit(yv.cpu().numpy()).any()

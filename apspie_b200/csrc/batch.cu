@@ -46,6 +46,7 @@
 #include "common.cuh"
 #include "context.h"
 #include "frontier.cuh"
+#include "primitives.cuh"
 
 namespace apspie {
 namespace {
@@ -94,8 +95,27 @@ struct BatchJob {
   const uint32_t *stw;
   int2 *hubc;
   unsigned nhc, pad2;
+  int32_t *rows;  // the caller's source-major rows
   JobCounters c[3];
 };
+
+// The blocks of one launch over every job: job k has blocks [first[k],
+// first[k + 1]).  One launch per step of the set-up instead of one per job: a
+// launch of a few microseconds each (20 us for a seed) adds up over the jobs
+// (28 BFS and 13 SSSP sources over three small graphs: 1,054 us for the whole
+// call, 920 us so).
+struct JobBlocks {
+  int first[kMaxJobs + 1];
+};
+__device__ __forceinline__ int job_of_block(const JobBlocks &b, int njobs) {
+  int lo = 0, hi = njobs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (b.first[mid] <= (int)blockIdx.x) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
 
 struct BatchState {
   alignas(8) unsigned bar[2];  // grid-barrier arrival counter (64-bit)
@@ -119,84 +139,66 @@ __device__ __forceinline__ unsigned long long srcmask(int nsrc) {
 }
 
 // ------------------------------------------------------------------ init ---
-// Queues the distinct sources of job j as its level-0 frontier (one thread).
-__device__ void seed_queue(BatchJob *j) {
-  for (int i = 0; i < 3; ++i) j->c[i] = JobCounters{0ull, 0, 0, 0ull};
-  unsigned q = 0, nch_total = 0;
-  for (int s = 0; s < j->nsrc; ++s) {
-    int v = j->src[s];
-    bool first = true;
-    for (int t = 0; t < s; ++t)
-      if (j->src[t] == v) first = false;
-    if (!first) continue;
-    int deg = __ldg(j->ptr + v + 1) - __ldg(j->ptr + v);
-    if (deg > j->big_deg) {
-      int nch = (deg + j->chunk - 1) / j->chunk;
-      for (int c = 0; c < nch; ++c) j->c0[nch_total + c] = make_int2(v, c);
-      nch_total += (unsigned)nch;
-      j->c[0].nbig += 1;
-    } else {
-      j->q0[q++] = v;
-    }
-    j->c[0].edges += (unsigned long long)deg;
-  }
-  j->c[0].qc = ((unsigned long long)nch_total << 32) | q;
+constexpr int kInitThreads = 256;
+
+// Results to "unreached" (-1, also the SSSP identity 0xFFFFFFFF), masks to 0:
+// they lie one after the other from the first to F2, with padding, so both
+// regions are filled 16 bytes at a time.
+__global__ void __launch_bounds__(kInitThreads)
+batch_init(const BatchJob *jobs, int njobs, const __grid_constant__ JobBlocks blocks) {
+  const int jid = job_of_block(blocks, njobs);
+  const BatchJob *j = jobs + jid;
+  const size_t at = (size_t)((int)blockIdx.x - blocks.first[jid]) * kInitThreads + threadIdx.x;
+  const size_t step = (size_t)(blocks.first[jid + 1] - blocks.first[jid]) * kInitThreads;
+  const size_t m = (size_t)j->m;
+  int4 *out = reinterpret_cast<int4 *>(j->out);
+  unsigned long long *first = j->type == kJobBfs ? j->visited : j->F0;
+  int4 *masks = reinterpret_cast<int4 *>(first);
+  const size_t nout = (m * j->sw + 3) / 4, nmask = ((size_t)(j->F2 - first) + m + 1) / 2;
+  for (size_t i = at; i < nout; i += step) out[i] = make_int4(-1, -1, -1, -1);
+  for (size_t i = at; i < nmask; i += step) masks[i] = make_int4(0, 0, 0, 0);
 }
 
-__global__ void batch_init_bfs(BatchJob *jobs, int jid) {
-  BatchJob *j = jobs + jid;
-  const int m = j->m;
-  const size_t n64 = (size_t)m * j->sw;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n64;
-       i += (size_t)gridDim.x * blockDim.x)
-    j->out[i] = -1;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x) {
-    j->visited[v] = 0ull;
-    j->F0[v] = 0ull;
-    j->F1[v] = 0ull;
-    j->F2[v] = 0ull;
-  }
-}
+// One block per job, one thread per source: visited / frontier bits and
+// result 0, then the distinct sources as the level-0 frontier, the hubs'
+// chunks written by the whole block.
+constexpr int kSeedThreads = 128;
 
-// sources: set visited / frontier bits and depth 0, queue each distinct source
-__global__ void batch_seed_bfs(BatchJob *jobs, int jid) {
-  BatchJob *j = jobs + jid;
-  if (blockIdx.x != 0) return;
-  for (int s = threadIdx.x; s < j->nsrc; s += blockDim.x) {
-    int v = j->src[s];
-    atomicOr(j->visited + v, 1ull << s);
+__global__ void __launch_bounds__(kSeedThreads) batch_seed(BatchJob *jobs) {
+  BatchJob *j = jobs + blockIdx.x;
+  __shared__ int s_src[kMsbfsWidth];
+  __shared__ unsigned s_off[kMsbfsWidth], s_nch[kMsbfsWidth];
+  __shared__ unsigned long long sw[33];
+  const int s = threadIdx.x, nsrc = j->nsrc;
+  int v = 0, deg = 0;
+  if (s < nsrc) {
+    v = j->src[s];
+    s_src[s] = v;
+    deg = __ldg(j->ptr + v + 1) - __ldg(j->ptr + v);
+    if (j->type == kJobBfs) atomicOr(j->visited + v, 1ull << s);
     atomicOr(j->F0 + v, 1ull << s);
     j->out[(size_t)v * j->sw + s] = 0;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    seed_queue(j);
+  bool mine = s < nsrc;
+  for (int t = 0; t < s && mine; ++t) mine = s_src[t] != v;
+  const bool big = mine && deg > j->big_deg;
+  const unsigned nch = big ? (unsigned)((deg + j->chunk - 1) / j->chunk) : 0u;
+  unsigned long long qc, edges;
+  const unsigned long long off =
+      block_excl_scan((unsigned long long)nch << 32 | (mine && !big ? 1ull : 0ull), sw, &qc);
+  block_excl_scan(mine ? (unsigned long long)deg : 0ull, sw, &edges);
+  const int nbig = __syncthreads_count(big);
+  if (s < nsrc) {
+    s_off[s] = (unsigned)(off >> 32);
+    s_nch[s] = nch;
+    if (mine && !big) j->q0[(unsigned)off] = v;
   }
-}
-
-__global__ void batch_init_sssp(BatchJob *jobs, int jid) {
-  BatchJob *j = jobs + jid;
-  const size_t n = (size_t)j->m * j->sw;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    j->out[i] = -1;  // 0xFFFFFFFF: unreached
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < j->m; v += gridDim.x * blockDim.x) {
-    j->F0[v] = 0ull;
-    j->F1[v] = 0ull;
-    j->F2[v] = 0ull;
-  }
-}
-
-__global__ void batch_seed_sssp(BatchJob *jobs, int jid) {
-  BatchJob *j = jobs + jid;
-  if (blockIdx.x != 0) return;
-  for (int s = threadIdx.x; s < j->nsrc; s += blockDim.x) {
-    int v = j->src[s];
-    j->out[(size_t)v * j->sw + s] = 0;
-    atomicOr(j->F0 + v, 1ull << s);
-  }
+  if (s < 3) j->c[s] = s == 0 ? JobCounters{qc, (unsigned)nbig, 0, edges} : JobCounters{0ull, 0, 0, 0ull};
   __syncthreads();
-  if (threadIdx.x == 0) seed_queue(j);
+  for (int t = 0; t < nsrc; ++t)
+    for (unsigned c = threadIdx.x; c < s_nch[t]; c += kSeedThreads)
+      j->c0[s_off[t] + c] = make_int2(s_src[t], (int)c);
 }
 
 // --------------------------------------------------------- append helper ---
@@ -651,14 +653,18 @@ __device__ void mssp_chunk(BatchJob *j, int L, int unit, const AppendCtx &ac) {
 // ------------------------------------------------------- SSSP pull steps ---
 // Lists the (vertex, chunk) pull units of an SSSP job's vertices with more
 // than kMsHubIn in-edges (after the job table upload, which zeroes nhc).
-__global__ void batch_hub_chunks(BatchJob *jobs, int jid) {
+__global__ void __launch_bounds__(kInitThreads)
+batch_hub_chunks(BatchJob *jobs, int njobs, const __grid_constant__ JobBlocks blocks) {
+  const int jid = job_of_block(blocks, njobs);
   BatchJob *j = jobs + jid;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < j->m; v += gridDim.x * blockDim.x) {
+  const int step = (blocks.first[jid + 1] - blocks.first[jid]) * kInitThreads;
+  for (long long v = ((int)blockIdx.x - blocks.first[jid]) * kInitThreads + (int)threadIdx.x;
+       v < j->m; v += step) {
     const int d = __ldg(j->stptr + v + 1) - __ldg(j->stptr + v);
     if (d > kMsHubIn) {
       const unsigned nc = (unsigned)((d + kMsPullChunk - 1) / kMsPullChunk);
       const unsigned at = atomicAdd(&j->nhc, nc);
-      for (unsigned c = 0; c < nc; ++c) j->hubc[at + c] = make_int2(v, (int)c);
+      for (unsigned c = 0; c < nc; ++c) j->hubc[at + c] = make_int2((int)v, (int)c);
     }
   }
 }
@@ -913,18 +919,24 @@ batch_persistent(BatchJob *jobs, int njobs, BatchState *st, int max_steps) {
   if (blockIdx.x == 0 && threadIdx.x == 0) st->steps = step;
 }
 
-// vertex-major results [m][width] -> source-major out[s][m] for s < nsrc
-// (width 64 or 32)
-__global__ void batch_transpose(const int32_t *vm, int m, int width, int nsrc, int32_t *out) {
+// vertex-major results [m][sw] -> the caller's source-major rows, 32 vertices
+// per block
+__global__ void __launch_bounds__(kInitThreads)
+batch_transpose(const BatchJob *jobs, int njobs, const __grid_constant__ JobBlocks blocks) {
   __shared__ int32_t tile[32][65];
-  const int v0 = blockIdx.x * 32;
-  for (int t = threadIdx.x; t < 32 * width; t += blockDim.x) {
-    int vv = t / width, s = t % width;
-    tile[vv][s] = (v0 + vv < m) ? vm[(size_t)(v0 + vv) * width + s] : -1;
+  const int jid = job_of_block(blocks, njobs);
+  const BatchJob *j = jobs + jid;
+  const int v0 = ((int)blockIdx.x - blocks.first[jid]) * 32, m = j->m, nsrc = j->nsrc;
+  const int width = j->sw, lg = width_log2(width);
+  const int32_t *vm = j->out;
+  int32_t *out = j->rows;
+  for (int t = threadIdx.x; t < 32 * width; t += kInitThreads) {
+    const int vv = t >> lg, s = t & (width - 1);
+    tile[vv][s] = v0 + vv < m ? vm[(size_t)(v0 + vv) * width + s] : -1;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < 32 * width; t += blockDim.x) {
-    int s = t / 32, vv = t % 32;
+  for (int t = threadIdx.x; t < 32 * width; t += kInitThreads) {
+    const int s = t / 32, vv = t % 32;
     if (s < nsrc && v0 + vv < m) out[(size_t)s * m + v0 + vv] = tile[vv][s];
   }
 }
@@ -1262,6 +1274,7 @@ int apspie_batch_run(apspie_ctx ctx, int njobs, const apspie_job *jobs, int max_
         B.c0 = (int2 *)b; b += align_up(8 * cap);
         B.c1 = (int2 *)b; b += align_up(8 * cap);
         B.c2 = (int2 *)b; b += align_up(8 * cap);
+        B.rows = J.d_out + (size_t)parts[p].first * J.m;
         B.out = (int32_t *)b;  // vertex-major; transposed into the caller's array after
         b += align_up(4 * m * B.sw);
         if (!bfs && J.d_stptr) {
@@ -1279,23 +1292,23 @@ int apspie_batch_run(apspie_ctx ctx, int njobs, const apspie_job *jobs, int max_
       cudaMemsetAsync(dstate, 0, align_up(sizeof(BatchState)), st);
       rc = check_cuda(ctx, cudaGetLastError(), "apspie_batch_run upload");
       if (rc) return rc;
-      int nhub_launches = 0;
+      JobBlocks binit{}, bhub{}, brows{};
       for (int p = 0; p < nparts; ++p) {
-        const long long m = jobs[parts[p].job].m;
-        int g = (int)std::max(1ll, std::min((m * hjobs[p].sw + 255) / 256, (long long)ctx->num_sms * 8));
-        if (hjobs[p].type == kJobBfs) {
-          batch_init_bfs<<<g, 256, 0, st>>>(djobs, p);
-          batch_seed_bfs<<<1, 64, 0, st>>>(djobs, p);
-        } else {
-          batch_init_sssp<<<g, 256, 0, st>>>(djobs, p);
-          batch_seed_sssp<<<1, 32, 0, st>>>(djobs, p);
-          if (hjobs[p].stptr) {
-            batch_hub_chunks<<<std::min(g, ctx->num_sms * 4), 256, 0, st>>>(djobs, p);
-            ++nhub_launches;
-          }
-        }
+        const BatchJob &B = hjobs[p];
+        const long long most = (long long)ctx->num_sms * 8;
+        const int g = (int)std::max(1ll, std::min(((long long)B.m * B.sw / 4 + kInitThreads - 1) /
+                                                      kInitThreads, most));
+        const bool hubs = B.type == kJobSssp && B.stptr && B.salpha > 0;
+        binit.first[p + 1] = binit.first[p] + g;
+        bhub.first[p + 1] =
+            bhub.first[p] + (hubs ? std::min((B.m + kInitThreads - 1) / kInitThreads, (int)most) : 0);
+        brows.first[p + 1] = brows.first[p] + (B.m + 31) / 32;
       }
-      rc = check_launch(ctx, "batch init", 2 * nparts + nhub_launches);
+      batch_init<<<binit.first[nparts], kInitThreads, 0, st>>>(djobs, nparts, binit);
+      batch_seed<<<nparts, kSeedThreads, 0, st>>>(djobs);
+      if (bhub.first[nparts] > 0)
+        batch_hub_chunks<<<bhub.first[nparts], kInitThreads, 0, st>>>(djobs, nparts, bhub);
+      rc = check_launch(ctx, "batch init", bhub.first[nparts] > 0 ? 3 : 2);
       if (rc) return rc;
       int n1 = nparts;
       void *args1[] = {&djobs, &n1, &dstate, &max_steps};
@@ -1305,12 +1318,8 @@ int apspie_batch_run(apspie_ctx ctx, int njobs, const apspie_job *jobs, int max_
                                                   dim3(kBatchThreads), args1, 0, st);
       if (e != cudaSuccess) return check_cuda(ctx, e, "batch_persistent");
       ctx->launches += 1;
-      for (int p = 0; p < nparts; ++p) {
-        const apspie_job &J = jobs[parts[p].job];
-        batch_transpose<<<(J.m + 31) / 32, 256, 0, st>>>(
-            hjobs[p].out, J.m, hjobs[p].sw, parts[p].n, J.d_out + (size_t)parts[p].first * J.m);
-      }
-      rc = check_launch(ctx, "batch_transpose", nparts);
+      batch_transpose<<<brows.first[nparts], kInitThreads, 0, st>>>(djobs, nparts, brows);
+      rc = check_launch(ctx, "batch_transpose");
       if (rc) return rc;
       ctx->batch_state = dstate;
     }

@@ -590,8 +590,12 @@ radix_small(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, int n,
 // callers that never synchronise (apspie_bfs_prepare, apspie_csr_transpose)
 // leave it to the next call on the context that reads it back (the device
 // graph build, apspie_tc_prepare, apspie_spmspv).
+// kSortErrWords words (give-up, test hook, two unused); the rest of the slot's
+// kSortErrBytes is a caller's that wants to read them back with its own.
+constexpr int kSortErrWords = 4;
+constexpr size_t kSortErrBytes = 64;
 inline int *radix_sort_err(apspie_context *ctx) {
-  auto *e = (int *)workspace(ctx, kSlotSortErr, 16);
+  auto *e = (int *)workspace(ctx, kSlotSortErr, kSortErrBytes);
   if (e && ctx->sort_err_zeroed != e) {
     cudaMemsetAsync(e, 0, 16, ctx->stream);
     ctx->sort_err_zeroed = e;

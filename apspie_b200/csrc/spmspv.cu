@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <cstddef>
 
 #include "common.cuh"
 #include "context.h"
@@ -56,17 +57,54 @@ __device__ __forceinline__ float sr_term(int sr, float a, float x) {
   }
 }
 
+// ---- the accumulator of the bitmap path ----
+// One accumulator word per row, which also tells whether the row was touched:
+// a bitmap beside it costs a second random L2 access per product (the expansion
+// of 6.3 M products, 1 M rows: 73 us with one, 44 us without).
+//   PLUS_TIMES  a double that starts at -0.0, which no sum reaches: a term of
+//               -0.0 is added as +0.0, and x + -x is +0.0
+//   MIN_PLUS,   32 bits that order as the float does, so that the atomics are
+//   MAX_TIMES   native; they start beyond every float's word, and a NaN's word
+//               loses to every number's (fminf and fmaxf leave NaN out)
+//   OR_AND      0, then 1
+constexpr unsigned long long kNoSum = 0x8000000000000000ull;
+
+__device__ __forceinline__ unsigned ordered_bits(float f) {
+  const unsigned b = __float_as_uint(f);
+  return (b >> 31) ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float ordered_float(unsigned u) {
+  return __uint_as_float((u >> 31) ? u & 0x7fffffffu : ~u);
+}
+__device__ __forceinline__ unsigned untouched_word(int sr) { return sr == kMinPlus ? ~0u : 0u; }
+__device__ __forceinline__ unsigned nan_word(int sr) { return sr == kMinPlus ? ~1u : 1u; }
+
+__device__ __forceinline__ void clear_acc(int sr, int m, unsigned long long *acc) {
+  const unsigned w = untouched_word(sr);
+  const unsigned long long v = sr == kPlusTimes ? kNoSum : (unsigned long long)w << 32 | w;
+  const unsigned n = sr == kPlusTimes ? (unsigned)m : ((unsigned)m + 1u) / 2u;
+  const unsigned stride = gridDim.x * blockDim.x;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) acc[i] = v;
+}
+
+__global__ void acc_init(int sr, int m, unsigned long long *acc) { clear_acc(sr, m, acc); }
+
 // ---- the frontier's columns ----
-// Lengths, and (first entry, x value) side by side for the tiles.
+// Lengths, and (first entry, x value) side by side for the tiles.  With acc,
+// the accumulator of the bitmap path is cleared in the same launch, and the
+// call's scalars are read back in one copy: a launch and a copy less took 16,384
+// columns of a 1 M-row graph from 119 to 112 us.
 __global__ void frontier_columns(int xnnz, const int *__restrict__ xind,
                                  const float *__restrict__ xval, const int *__restrict__ ptr,
-                                 long long *deg, int2 *col) {
+                                 long long *deg, int2 *col, int sr, int m,
+                                 unsigned long long *acc) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < xnnz; j += gridDim.x * blockDim.x) {
     const int c = xind[j];
     const int s = __ldg(ptr + c);
     deg[j] = (long long)(__ldg(ptr + c + 1) - s);
     col[j] = make_int2(s, __float_as_int(xval ? xval[j] : 1.0f));
   }
+  if (acc) clear_acc(sr, m, acc);
 }
 
 // Calls f(e[], row[], term[], on[]) for the entries e of the frontier's columns
@@ -164,35 +202,6 @@ __global__ void reduce_segments(int sr, const int *keys, const float *vals, long
 }
 
 // ---- bitmap path ----
-// One accumulator word per row, which also tells whether the row was touched:
-// a bitmap beside it costs a second random L2 access per product (the expansion
-// of 6.3 M products, 1 M rows: 73 us with one, 44 us without).
-//   PLUS_TIMES  a double that starts at -0.0, which no sum reaches: a term of
-//               -0.0 is added as +0.0, and x + -x is +0.0
-//   MIN_PLUS,   32 bits that order as the float does, so that the atomics are
-//   MAX_TIMES   native; they start beyond every float's word, and a NaN's word
-//               loses to every number's (fminf and fmaxf leave NaN out)
-//   OR_AND      0, then 1
-constexpr unsigned long long kNoSum = 0x8000000000000000ull;
-
-__device__ __forceinline__ unsigned ordered_bits(float f) {
-  const unsigned b = __float_as_uint(f);
-  return (b >> 31) ? ~b : b | 0x80000000u;
-}
-__device__ __forceinline__ float ordered_float(unsigned u) {
-  return __uint_as_float((u >> 31) ? u & 0x7fffffffu : ~u);
-}
-__device__ __forceinline__ unsigned untouched_word(int sr) { return sr == kMinPlus ? ~0u : 0u; }
-__device__ __forceinline__ unsigned nan_word(int sr) { return sr == kMinPlus ? ~1u : 1u; }
-
-__global__ void acc_init(int sr, int m, unsigned long long *acc) {
-  const unsigned w = untouched_word(sr);
-  const unsigned long long v = sr == kPlusTimes ? kNoSum : (unsigned long long)w << 32 | w;
-  const unsigned n = sr == kPlusTimes ? (unsigned)m : ((unsigned)m + 1u) / 2u;
-  const unsigned stride = gridDim.x * blockDim.x;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) acc[i] = v;
-}
-
 __global__ void __launch_bounds__(kEdgeThreads)
 expand_accumulate(int sr, int xnnz, const long long *__restrict__ offs, const long long *total,
                   const int2 *__restrict__ col, const int *__restrict__ ind,
@@ -344,10 +353,16 @@ int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *i
   auto *offs = (long long *)workspace(ctx, kSlotMisc0, sizeof(long long) * (size_t)(xnnz + 1));
   auto *col = (int2 *)workspace(ctx, kSlotMisc2, sizeof(int2) * (size_t)xnnz);
   if (!offs || !col) return APSPIE_ERR_OOM;
-  frontier_columns<<<grid_for(ctx, xnnz, 256), 256, 0, st>>>(xnnz, xind, xval, ptr, offs, col);
+  bool bitmap = m <= kBitmapRows && factor > 0.0;
+  void *acc = nullptr;
+  if (bitmap) {
+    acc = workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
+    if (!acc) return APSPIE_ERR_OOM;
+  }
+  frontier_columns<<<grid_for(ctx, bitmap ? std::max(xnnz, m) : xnnz, 256), 256, 0, st>>>(
+      xnnz, xind, xval, ptr, offs, col, sr, m, (unsigned long long *)acc);
   int rc = check_launch(ctx, "frontier_columns");
   if (rc) return rc;
-  bool bitmap = m <= kBitmapRows && factor > 0.0;
   long long E = 0;
   if (!bitmap) {
     rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, &sm->total);
@@ -369,16 +384,20 @@ int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *i
   const int egrid = ctx->num_sms * 6;  // resident blocks; they stride the tiles
   if (bitmap) {
     const int words = (int)(((long long)m + 31) / 32);
-    void *acc = workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
     unsigned *bits = (unsigned *)workspace(ctx, kSlotBitmap,
                                            sizeof(unsigned) * ((size_t)words + kEmitBlocks));
-    if (!acc || !bits) return APSPIE_ERR_OOM;
+    if (!bits) return APSPIE_ERR_OOM;
     unsigned *sums = bits + words;
-    if (E == 0) {  // not scanned yet
+    if (acc) {  // cleared, and the lengths not scanned yet
       rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, &sm->total);
       if (rc) return rc;
+    } else {
+      acc = workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
+      if (!acc) return APSPIE_ERR_OOM;
+      acc_init<<<grid_for(ctx, m, 256), 256, 0, st>>>(sr, m, (unsigned long long *)acc);
+      rc = check_launch(ctx, "acc_init");
+      if (rc) return rc;
     }
-    acc_init<<<grid_for(ctx, m, 256), 256, 0, st>>>(sr, m, (unsigned long long *)acc);
     expand_accumulate<<<egrid, kEdgeThreads, 0, st>>>(sr, xnnz, offs, &sm->total, col, ind, val,
                                                       acc);
     const int per_block = std::max(kEmitWords, (words + kEmitBlocks - 1) / kEmitBlocks);
@@ -386,7 +405,7 @@ int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *i
     touched_rows<<<eblocks, kEmitThreads, 0, st>>>(sr, m, acc, words, per_block, bits, sums);
     touched_emit<<<eblocks, kEmitThreads, 0, st>>>(sr, m, bits, words, per_block, sums, acc,
                                                    &sm->total, factor, yind, yval, &sm->ynnz);
-    return check_launch(ctx, "spmspv bitmap", 4);
+    return check_launch(ctx, "spmspv bitmap", 3);
   }
   // sort path
   int *ka = (int *)workspace(ctx, kSlotSortKeysA, sizeof(int) * (size_t)E);
@@ -437,22 +456,22 @@ int apspie_spmspv(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int *d
   if (semiring < 0 || semiring > 3 || m <= 0 || nnz < 0 || xnnz < 0 || xnnz > m || !d_ptr ||
       (nnz > 0 && !d_ind) || (xnnz > 0 && !d_xind) || !d_yind || !d_yval || !h_ynnz)
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_spmspv: bad arguments");
-  auto *sm = (SpmspvSmall *)workspace(ctx, kSlotSmall, sizeof(SpmspvSmall));
-  if (!sm) return APSPIE_ERR_OOM;
+  // the call's scalars lie behind the sort's give-up word: one copy reads both
+  struct Back {
+    int sort_err, pad[3];
+    SpmspvSmall s;
+  };
+  static_assert(offsetof(Back, s) == kSortErrWords * sizeof(int) &&
+                    sizeof(Back) <= kSortErrBytes, "read back in one copy");
+  int *sort_err = radix_sort_err(ctx);
+  if (!sort_err) return APSPIE_ERR_OOM;
+  auto *sm = (SpmspvSmall *)(sort_err + kSortErrWords);
   int rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, d_xind, d_xval, d_yind, d_yval,
                        sm);
   if (rc) return rc;
-  struct Back {
-    SpmspvSmall s;
-    int sort_err;
-  };
   auto *h = (Back *)pinned(ctx, sizeof(Back));
-  int *sort_err = radix_sort_err(ctx);
-  if (!h || !sort_err) return APSPIE_ERR_OOM;
-  rc = check_cuda(ctx, cudaMemcpyAsync(&h->s, sm, sizeof(SpmspvSmall), cudaMemcpyDeviceToHost,
-                                       ctx->stream), "apspie_spmspv");
-  if (rc) return rc;
-  rc = check_cuda(ctx, cudaMemcpyAsync(&h->sort_err, sort_err, sizeof(int), cudaMemcpyDeviceToHost,
+  if (!h) return APSPIE_ERR_OOM;
+  rc = check_cuda(ctx, cudaMemcpyAsync(h, sort_err, sizeof(Back), cudaMemcpyDeviceToHost,
                                        ctx->stream), "apspie_spmspv");
   if (rc) return rc;
   rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "apspie_spmspv");

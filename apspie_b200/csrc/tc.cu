@@ -17,8 +17,9 @@
 // entries of its end, or by a warp for itself.
 //
 // tc_prepare relabels vertices by ascending (degree, id) with the stable
-// radix sort, keeps the edges with new(col) < new(row), sorts them by
-// (row, col) with one radix sort on the packed key and builds L's offsets.
+// radix sort and lists the edges with new(col) < new(row) grouped by ascending
+// column, so that one stable sort on the row bits leaves every row of L
+// ascending; L's offsets come from the row lengths.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -537,8 +537,10 @@ int apspie_mxv_dense(apspie_ctx ctx, int semiring, int m, int64_t nnz,
                      const int *d_ptr, const int *d_ind, const float *d_val,
                      const float *d_x, float *d_y, int64_t *h_expanded);
 
-/* SpMSpV path choice: the bitmap (dense accumulator) path is used when
- * products * sort_factor > m, else the radix-sort path.  Default 4. */
+/* SpMSpV path choice.  sort_factor 0 always takes the radix-sort path.
+ * Otherwise the bitmap (dense accumulator) path is used up to 2^22 rows, where
+ * it is faster at any density, and beyond when products * sort_factor > m.
+ * Default 4. */
 int apspie_spmspv_set_params(apspie_ctx ctx, double sort_factor);
 
 /* ------------------------------------------------------------- SpGEMM ---

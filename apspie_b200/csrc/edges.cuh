@@ -17,8 +17,13 @@ constexpr int kEdgeThreads = 256;
 constexpr int kEdgeItems = 8;                          // entries per thread
 constexpr int kEdgeTile = kEdgeThreads * kEdgeItems;  // entries per tile
 
-// Largest r with ptr[r] <= k, given ptr[m] > k.  Warp-collective.  (P: int, or
-// long long for offsets whose total has been checked to fit an int.)
+// A kernel's tiles cover the entries [ptr[0], ptr[m]), whatever count the
+// caller gave: offsets may start anywhere in the arrays they index (a slice of
+// a larger matrix's rows).
+
+// Largest r with ptr[r] <= k, given ptr[0] <= k < ptr[m] (else some row of the
+// matrix).  Warp-collective.  (P: int, or long long for offsets whose total has
+// been checked to fit an int.)
 template <typename P>
 __device__ __forceinline__ int row_of_entry(const P *__restrict__ ptr, int m, int k) {
   const int lane = lane_id();
@@ -26,7 +31,8 @@ __device__ __forceinline__ int row_of_entry(const P *__restrict__ ptr, int m, in
   while (hi - lo > 1) {
     const long long span = hi - lo;
     const int piv = lo + (int)(span * lane / 32);
-    const unsigned b = __ballot_sync(kFull, __ldg(ptr + piv) <= k);  // lane 0 always
+    // lane 0 counts as below: the search stays inside [lo, hi] whatever k is
+    const unsigned b = __ballot_sync(kFull, lane == 0 || __ldg(ptr + piv) <= k);
     const int last = 31 - __clz(b);
     const int nlo = lo + (int)(span * last / 32);
     const int nhi = last == 31 ? hi : lo + (int)(span * (last + 1) / 32);
@@ -36,8 +42,18 @@ __device__ __forceinline__ int row_of_entry(const P *__restrict__ ptr, int m, in
   return lo;
 }
 
+// Entries of tile number `tile` (0: none left); *k0: the first of them.
+template <typename P>
+__device__ __forceinline__ int edge_tile(const P *__restrict__ ptr, int m, unsigned tile, int *k0) {
+  const long long first = (long long)__ldg(ptr) + (long long)tile * kEdgeTile;
+  const long long left = (long long)__ldg(ptr + m) - first;
+  *k0 = (int)first;
+  return left <= 0 ? 0 : (int)min((long long)kEdgeTile, left);
+}
+
 // s_row[t] = row of entry k0 + t for t in [0, n), n <= kEdgeTile.  Called by
-// all kEdgeThreads threads; s_row is ready when it returns.
+// all kEdgeThreads threads; s_row is ready when it returns, and must have been
+// read by all of them before the next call.
 template <typename P>
 __device__ __forceinline__ void edge_tile_rows(const P *__restrict__ ptr, int m, int k0, int n,
                                                int *s_row) {
@@ -101,8 +117,10 @@ __device__ __forceinline__ unsigned row_peers(int row, int *leader) {
   return below_next & ~((1u << *leader) - 1u);
 }
 
+// Blocks for nnz entries, at least one.  Kernels that call edge_tile stride
+// their tiles by it, so a count below the offsets' leaves no entry out.
 inline unsigned edge_tiles(long long nnz) {
-  return (unsigned)((nnz + kEdgeTile - 1) / kEdgeTile);
+  return (unsigned)(nnz > kEdgeTile ? (nnz + kEdgeTile - 1) / kEdgeTile : 1);
 }
 
 }  // namespace apspie

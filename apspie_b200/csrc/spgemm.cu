@@ -106,38 +106,42 @@ __device__ __forceinline__ int table_insert(int *keys, int bits, int j, bool *fr
 // atomic.  (Eight lanes per row waited for the rows of thousands of entries:
 // 97 us for 4.2 M entries.)
 __global__ void __launch_bounds__(kEdgeThreads)
-row_products(int m, int nnz, const int *__restrict__ Aptr, const int *__restrict__ Aind,
+row_products(int m, const int *__restrict__ Aptr, const int *__restrict__ Aind,
              const int *__restrict__ Bptr, unsigned long long *prod) {
   __shared__ __align__(16) int s_row[kEdgeTile];
-  const int k0 = (int)blockIdx.x * kEdgeTile;
-  const int n = min(kEdgeTile, min(nnz, __ldg(Aptr + m)) - k0);
-  if (n <= 0) return;
-  edge_tile_rows(Aptr, m, k0, n, s_row);
   const int lane = lane_id();
   constexpr int kFly = 4;  // entries per thread in flight
-  for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kFly * kEdgeThreads) {
-    int k[kFly], d[kFly], row[kFly];
+  for (unsigned tile = blockIdx.x;; tile += gridDim.x) {
+    int k0;
+    const int n = edge_tile(Aptr, m, tile, &k0);
+    if (n == 0) break;
+    edge_tile_rows(Aptr, m, k0, n, s_row);
+    for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kFly * kEdgeThreads) {
+      int k[kFly], d[kFly], row[kFly];
 #pragma unroll
-    for (int q = 0; q < kFly; ++q) {
-      const int t = t0 + q * kEdgeThreads;
-      row[q] = t < n ? s_row[t] : -1;
-      k[q] = t < n ? __ldg(Aind + k0 + t) : -1;
-    }
-#pragma unroll
-    for (int q = 0; q < kFly; ++q) d[q] = k[q] >= 0 ? __ldg(Bptr + k[q] + 1) - __ldg(Bptr + k[q]) : 0;
-#pragma unroll
-    for (int q = 0; q < kFly; ++q) {
-      int leader;
-      const unsigned peers = row_peers(row[q], &leader);
-      unsigned long long sum = (unsigned long long)d[q];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long y = __shfl_up_sync(kFull, sum, o);
-        if (lane - o >= leader) sum += y;
+      for (int q = 0; q < kFly; ++q) {
+        const int t = t0 + q * kEdgeThreads;
+        row[q] = t < n ? s_row[t] : -1;
+        k[q] = t < n ? __ldg(Aind + k0 + t) : -1;
       }
-      const int last = 31 - __clz(peers);
-      if (lane == last && row[q] >= 0 && sum) atomicAdd(prod + row[q], sum);
+#pragma unroll
+      for (int q = 0; q < kFly; ++q)
+        d[q] = k[q] >= 0 ? __ldg(Bptr + k[q] + 1) - __ldg(Bptr + k[q]) : 0;
+#pragma unroll
+      for (int q = 0; q < kFly; ++q) {
+        int leader;
+        const unsigned peers = row_peers(row[q], &leader);
+        unsigned long long sum = (unsigned long long)d[q];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long y = __shfl_up_sync(kFull, sum, o);
+          if (lane - o >= leader) sum += y;
+        }
+        const int last = 31 - __clz(peers);
+        if (lane == last && row[q] >= 0 && sum) atomicAdd(prod + row[q], sum);
+      }
     }
+    __syncthreads();
   }
 }
 
@@ -1366,10 +1370,9 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   if (rc0) return rc0;
   if (m > 0) {
     cudaMemsetAsync(prod, 0, sizeof(long long) * (size_t)m, st);
-    if (A->nnz > 0)
-      row_products<<<edge_tiles(A->nnz), kEdgeThreads, 0, st>>>(
-          m, (int)std::min<int64_t>(A->nnz, INT_MAX), A->d_ptr, A->d_ind, B->d_ptr,
-          (unsigned long long *)prod);
+    // the rows' offsets say what A's entries are, not its nnz
+    row_products<<<edge_tiles(std::min<int64_t>(A->nnz, INT_MAX)), kEdgeThreads, 0, st>>>(
+        m, A->d_ptr, A->d_ind, B->d_ptr, (unsigned long long *)prod);
     bin_rows<<<gridsz(ctx, m, 256), 256, 0, st>>>(m, prod, lists, sst, cnt, bitmap, lim);
     int rc = check_launch(ctx, "spgemm bin", 2);
     if (rc) return rc;

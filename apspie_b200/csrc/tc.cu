@@ -88,16 +88,17 @@ struct TcBins {
 constexpr int kTcRankItems = 4;
 
 __global__ void __launch_bounds__(kTcThreads)
-tc_col_ranks(int lnnz, const int *__restrict__ end, const int *__restrict__ Li, int *cnt,
+tc_col_ranks(int m, int lnnz, const int *__restrict__ Lp, const int *__restrict__ Li, int *cnt,
              int *rank) {
-  const int n = min(lnnz, __ldg(end));  // end: Lp + m
+  const int *first = Li + __ldg(Lp);
+  const int n = min(lnnz, __ldg(Lp + m) - __ldg(Lp));  // rank holds lnnz entries
   constexpr long long kStep = (long long)kTcThreads * kTcRankItems;
   for (long long b = blockIdx.x * kStep; b < n; b += gridDim.x * kStep) {
     int c[kTcRankItems], r[kTcRankItems];
 #pragma unroll
     for (int q = 0; q < kTcRankItems; ++q) {
       const long long k = b + q * kTcThreads + threadIdx.x;
-      c[q] = k < n ? __ldg(Li + k) : -1;
+      c[q] = k < n ? __ldg(first + k) : -1;
     }
 #pragma unroll
     for (int q = 0; q < kTcRankItems; ++q) r[q] = add_if(c[q] >= 0, cnt + c[q], 1, 0);
@@ -142,8 +143,9 @@ __global__ void __launch_bounds__(kEdgeThreads)
 tc_scatter(int m, int lnnz, const int *__restrict__ Lp, const int *__restrict__ Li,
            const int *__restrict__ Up, const int *__restrict__ rank, int *Ui) {
   __shared__ __align__(16) int s_row[kEdgeTile];
-  const int k0 = (int)blockIdx.x * kEdgeTile;
-  const int n = min(kEdgeTile, min(lnnz, __ldg(Lp + m)) - k0);
+  const int *erank = rank - __ldg(Lp);  // by entry
+  int k0;
+  const int n = min(edge_tile(Lp, m, blockIdx.x, &k0), lnnz - (int)blockIdx.x * kEdgeTile);
   if (n <= 0) return;
   edge_tile_rows(Lp, m, k0, n, s_row);
   int c[kEdgeItems], at[kEdgeItems];
@@ -153,8 +155,10 @@ tc_scatter(int m, int lnnz, const int *__restrict__ Lp, const int *__restrict__ 
     c[q] = t < n ? __ldg(Li + k0 + t) : -1;
   }
 #pragma unroll
-  for (int q = 0; q < kEdgeItems; ++q)
-    at[q] = c[q] >= 0 ? __ldg(Up + c[q]) + __ldg(rank + k0 + (int)threadIdx.x + q * kEdgeThreads) : 0;
+  for (int q = 0; q < kEdgeItems; ++q) {
+    const int t = (int)threadIdx.x + q * kEdgeThreads;
+    at[q] = c[q] >= 0 ? __ldg(Up + c[q]) + __ldg(erank + k0 + t) : 0;
+  }
 #pragma unroll
   for (int q = 0; q < kEdgeItems; ++q)
     if (c[q] >= 0) Ui[at[q]] = s_row[threadIdx.x + q * kEdgeThreads];
@@ -384,44 +388,47 @@ constexpr int kSplit = 4;  // entries per thread in flight in the two passes ove
 // symmetric -- exactly when the multisets of hashed pairs agree, which the two
 // sums confirm up to a 2^-64 chance.
 __global__ void __launch_bounds__(kEdgeThreads)
-split_counts(int m, int nnz, const int *__restrict__ ptr, const int *__restrict__ ind,
+split_counts(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
              const int *__restrict__ perm, int *lcnt, int *ucnt, unsigned long long *hsum) {
   __shared__ __align__(16) int s_row[kEdgeTile];
-  const int k0 = (int)blockIdx.x * kEdgeTile;
-  const int n = min(kEdgeTile, min(nnz, __ldg(ptr + m)) - k0);
-  if (n <= 0) return;
-  edge_tile_rows(ptr, m, k0, n, s_row);
   const int lane = lane_id();
   unsigned long long h_fwd = 0, h_rev = 0;
-  for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kSplit * kEdgeThreads) {
-    int v[kSplit], u[kSplit], r[kSplit], pu[kSplit];
+  for (unsigned tile = blockIdx.x;; tile += gridDim.x) {
+    int k0;
+    const int n = edge_tile(ptr, m, tile, &k0);
+    if (n == 0) break;
+    edge_tile_rows(ptr, m, k0, n, s_row);
+    for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kSplit * kEdgeThreads) {
+      int v[kSplit], u[kSplit], r[kSplit], pu[kSplit];
 #pragma unroll
-    for (int q = 0; q < kSplit; ++q) {
-      const int t = t0 + q * kEdgeThreads;
-      v[q] = t < n ? s_row[t] : -1;
-      u[q] = t < n ? __ldg(ind + k0 + t) : 0;
-    }
-#pragma unroll
-    for (int q = 0; q < kSplit; ++q) {
-      r[q] = v[q] >= 0 ? __ldg(perm + v[q]) : 0;
-      pu[q] = v[q] >= 0 ? __ldg(perm + u[q]) : 0;
-    }
-#pragma unroll
-    for (int q = 0; q < kSplit; ++q) {
-      if (v[q] >= 0) {
-        h_fwd += apspie_gen::mix64(((unsigned long long)(unsigned)v[q] << 32) | (unsigned)u[q]);
-        h_rev += apspie_gen::mix64(((unsigned long long)(unsigned)u[q] << 32) | (unsigned)v[q]);
+      for (int q = 0; q < kSplit; ++q) {
+        const int t = t0 + q * kEdgeThreads;
+        v[q] = t < n ? s_row[t] : -1;
+        u[q] = t < n ? __ldg(ind + k0 + t) : 0;
       }
-      const unsigned below = __ballot_sync(kFull, pu[q] < r[q]);
-      const unsigned above = __ballot_sync(kFull, pu[q] > r[q]);
-      int leader;
-      const unsigned peers = row_peers(v[q], &leader);
-      if (lane == leader && v[q] >= 0) {
-        const int lo = __popc(below & peers), hi = __popc(above & peers);
-        if (lo) atomicAdd(lcnt + r[q], lo);
-        if (hi) atomicAdd(ucnt + r[q], hi);
+#pragma unroll
+      for (int q = 0; q < kSplit; ++q) {
+        r[q] = v[q] >= 0 ? __ldg(perm + v[q]) : 0;
+        pu[q] = v[q] >= 0 ? __ldg(perm + u[q]) : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < kSplit; ++q) {
+        if (v[q] >= 0) {
+          h_fwd += apspie_gen::mix64(((unsigned long long)(unsigned)v[q] << 32) | (unsigned)u[q]);
+          h_rev += apspie_gen::mix64(((unsigned long long)(unsigned)u[q] << 32) | (unsigned)v[q]);
+        }
+        const unsigned below = __ballot_sync(kFull, pu[q] < r[q]);
+        const unsigned above = __ballot_sync(kFull, pu[q] > r[q]);
+        int leader;
+        const unsigned peers = row_peers(v[q], &leader);
+        if (lane == leader && v[q] >= 0) {
+          const int lo = __popc(below & peers), hi = __popc(above & peers);
+          if (lo) atomicAdd(lcnt + r[q], lo);
+          if (hi) atomicAdd(ucnt + r[q], hi);
+        }
       }
     }
+    __syncthreads();
   }
   h_fwd = warp_sum(h_fwd);
   h_rev = warp_sum(h_rev);
@@ -438,42 +445,45 @@ split_counts(int m, int nnz, const int *__restrict__ ptr, const int *__restrict_
 // (equal pairs are the same pair), so a warp reserves its places in a
 // column with one add.
 __global__ void __launch_bounds__(kEdgeThreads)
-upper_pairs(int m, int nnz, const int *__restrict__ ptr, const int *__restrict__ ind,
+upper_pairs(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
             const int *__restrict__ perm, int *uoff, unsigned *rows, int *cols) {
   __shared__ __align__(16) int s_row[kEdgeTile];
-  const int k0 = (int)blockIdx.x * kEdgeTile;
-  const int n = min(kEdgeTile, min(nnz, __ldg(ptr + m)) - k0);
-  if (n <= 0) return;
-  edge_tile_rows(ptr, m, k0, n, s_row);
   const int lane = lane_id();
-  for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kSplit * kEdgeThreads) {
-    int v[kSplit], u[kSplit], r[kSplit], pu[kSplit], base[kSplit], leader[kSplit];
-    unsigned mine[kSplit];
+  for (unsigned tile = blockIdx.x;; tile += gridDim.x) {
+    int k0;
+    const int n = edge_tile(ptr, m, tile, &k0);
+    if (n == 0) break;
+    edge_tile_rows(ptr, m, k0, n, s_row);
+    for (int t0 = (int)threadIdx.x; t0 - lane < n; t0 += kSplit * kEdgeThreads) {
+      int v[kSplit], u[kSplit], r[kSplit], pu[kSplit], base[kSplit], leader[kSplit];
+      unsigned mine[kSplit];
 #pragma unroll
-    for (int q = 0; q < kSplit; ++q) {
-      const int t = t0 + q * kEdgeThreads;
-      v[q] = t < n ? s_row[t] : -1;
-      u[q] = t < n ? __ldg(ind + k0 + t) : 0;
-    }
+      for (int q = 0; q < kSplit; ++q) {
+        const int t = t0 + q * kEdgeThreads;
+        v[q] = t < n ? s_row[t] : -1;
+        u[q] = t < n ? __ldg(ind + k0 + t) : 0;
+      }
 #pragma unroll
-    for (int q = 0; q < kSplit; ++q) {
-      r[q] = v[q] >= 0 ? __ldg(perm + v[q]) : 0;
-      pu[q] = v[q] >= 0 ? __ldg(perm + u[q]) : 0;
-    }
+      for (int q = 0; q < kSplit; ++q) {
+        r[q] = v[q] >= 0 ? __ldg(perm + v[q]) : 0;
+        pu[q] = v[q] >= 0 ? __ldg(perm + u[q]) : 0;
+      }
 #pragma unroll
-    for (int q = 0; q < kSplit; ++q) {
-      mine[q] = row_peers(v[q], &leader[q]) & __ballot_sync(kFull, pu[q] > r[q]);
-      base[q] = add_if(lane == leader[q] && mine[q] != 0u, uoff + r[q], __popc(mine[q]), 0);
-    }
+      for (int q = 0; q < kSplit; ++q) {
+        mine[q] = row_peers(v[q], &leader[q]) & __ballot_sync(kFull, pu[q] > r[q]);
+        base[q] = add_if(lane == leader[q] && mine[q] != 0u, uoff + r[q], __popc(mine[q]), 0);
+      }
 #pragma unroll
-    for (int q = 0; q < kSplit; ++q) {
-      base[q] = __shfl_sync(kFull, base[q], leader[q]);
-      if (pu[q] > r[q]) {
-        const int at = base[q] + __popc(mine[q] & ((1u << lane) - 1u));
-        rows[at] = (unsigned)pu[q];
-        cols[at] = r[q];
+      for (int q = 0; q < kSplit; ++q) {
+        base[q] = __shfl_sync(kFull, base[q], leader[q]);
+        if (pu[q] > r[q]) {
+          const int at = base[q] + __popc(mine[q] & ((1u << lane) - 1u));
+          rows[at] = (unsigned)pu[q];
+          cols[at] = r[q];
+        }
       }
     }
+    __syncthreads();
   }
 }
 
@@ -531,8 +541,7 @@ int apspie_tc_prepare(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr, cons
   // small[0]: the largest degree; small + 8 bytes .. + 24: the two edge hashes
   auto *hsum = reinterpret_cast<unsigned long long *>(small) + 1;
   if (nnz > 0) {
-    split_counts<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, (int)nnz, d_ptr, d_ind, d_perm,
-                                                           lcnt, uoff, hsum);
+    split_counts<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, d_ptr, d_ind, d_perm, lcnt, uoff, hsum);
     rc = check_launch(ctx, "split_counts");
     if (rc) return rc;
   }
@@ -568,8 +577,7 @@ int apspie_tc_prepare(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr, cons
     auto *kb = (unsigned *)workspace(ctx, kSlotMisc2, sizeof(unsigned) * (size_t)lnnz);
     auto *va = (int *)workspace(ctx, kSlotMisc3, sizeof(int) * (size_t)lnnz);
     if (!ka || !kb || !va) return APSPIE_ERR_OOM;
-    upper_pairs<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, (int)nnz, d_ptr, d_ind, d_perm,
-                                                          uoff, ka, va);
+    upper_pairs<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, d_ptr, d_ind, d_perm, uoff, ka, va);
     rc = check_launch(ctx, "upper_pairs");
     if (rc) return rc;
     in_b = false;
@@ -614,7 +622,7 @@ int apspie_tc(apspie_ctx ctx, int m, int64_t lnnz, const int *d_Lptr, const int 
   if (!lists || !units || !Up || !rank || !col || !Ui || !bins) return APSPIE_ERR_OOM;
   cudaMemsetAsync(bins, 0, sizeof(TcBins) + sizeof(int) * ((size_t)m + 1), st);
   tc_col_ranks<<<tgrid(ctx, (lnnz + kTcRankItems - 1) / kTcRankItems, kTcThreads), kTcThreads, 0,
-                 st>>>((int)lnnz, d_Lptr + m, d_Lind, Up, rank);
+                 st>>>(m, (int)lnnz, d_Lptr, d_Lind, Up, rank);
   int rc = check_launch(ctx, "tc_col_ranks");
   if (rc) return rc;
   rc = device_exclusive_scan<int>(ctx, Up, Up, (long long)m + 1, nullptr);

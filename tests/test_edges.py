@@ -1,0 +1,88 @@
+"""The passes over a CSR's entries in tiles (edges.cuh): row offsets that
+index a part of larger arrays, and counts that the offsets correct."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _t(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _csr(m, n, nnz, seed):
+    rng = np.random.default_rng(seed)
+    deg = np.bincount(rng.integers(0, m, nnz), minlength=m)
+    ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    ind = np.concatenate([np.sort(rng.choice(n, d, replace=False)) for d in deg]).astype(np.int32)
+    return ptr, ind, rng.uniform(-1, 1, nnz).astype(np.float32)
+
+
+@pytest.mark.parametrize("rows", [(1, 400), (37, 38), (200, 395), (399, 400)])
+def test_spgemm_of_a_slice_of_rows(ctx, rows):
+    """A's offsets taken from the middle of a larger matrix, its entries'
+    arrays left whole: C is the product of those rows."""
+    import apspie_b200 as ap
+    m, n = 400, 300
+    ptr, ind, val = _csr(m, n, 20000, 1)
+    bptr, bind, bval = _csr(n, n, 3000, 2)
+    r0, r1 = rows
+    d_ptr, d_ind, d_val = _t(ptr), _t(ind), _t(val)
+    B = (n, n, _t(bptr), _t(bind), _t(bval))
+    got = ap.spgemm(ctx, (r1 - r0, n, d_ptr[r0:r1 + 1], d_ind, d_val), B)
+    lo, hi = ptr[r0], ptr[r1]
+    own = (r1 - r0, n, _t(ptr[r0:r1 + 1] - lo), _t(ind[lo:hi]), _t(val[lo:hi]))
+    ref = ap.spgemm(ctx, own, B)
+    rp, ri, _ = oracle.spgemm(r1 - r0, n, ptr[r0:r1 + 1] - lo, ind[lo:hi], val[lo:hi], bptr, bind,
+                              bval)
+    np.testing.assert_array_equal(got[0].cpu().numpy(), rp)
+    np.testing.assert_array_equal(got[1].cpu().numpy(), ri)
+    # the same rows through the same kernels: sums of two or more products may
+    # differ in the last bit of their rounding only
+    np.testing.assert_allclose(got[2].cpu().numpy(), ref[2].cpu().numpy(), rtol=2.0**-22,
+                               atol=2.0**-40)
+
+
+@pytest.mark.parametrize("nnz", [0, 1, 2048, 19999])
+def test_spgemm_reads_the_offsets_not_the_count(ctx, nnz):
+    """apspie_csr's nnz below what its offsets hold leaves no entry out."""
+    import torch
+    from apspie_b200._native import Csr, check, lib
+    m = n = 400
+    ptr, ind, _ = _csr(m, n, 20000, 3)
+    bptr, bind, _ = _csr(n, n, 3000, 4)
+    t = [_t(a) for a in (ptr, ind, bptr, bind)]
+    p = [C.c_void_p(x.data_ptr()) for x in t]
+    A, B = Csr(m, n, nnz, p[0], p[1], None), Csr(n, n, len(bind), p[2], p[3], None)
+    out, total = torch.empty(m + 1, dtype=torch.int32, device="cuda"), C.c_int64(0)
+    check(lib.apspie_spgemm_symbolic(ctx.handle, C.byref(A), C.byref(B),
+                                     C.c_void_p(out.data_ptr()), C.byref(total)), ctx.handle)
+    rp, _, _ = oracle.spgemm(m, n, ptr, ind, None, bptr, bind, None)
+    np.testing.assert_array_equal(out.cpu().numpy(), rp)
+    assert total.value == rp[-1]
+
+
+def test_triangles_of_graphs_packed_in_one_array(ctx):
+    """Graphs whose rows lie one after the other in one index array, each with
+    its part of the offsets, and an L placed behind other entries."""
+    import torch
+    import apspie_b200 as ap
+    hs = [ap.gen_rmat(11, 16, seed=1), ap.gen_er(3000, 20, seed=2), ap.gen_rmat(9, 8, seed=3)]
+    base = np.concatenate([[0], np.cumsum([h.nnz for h in hs])])
+    ind = _t(np.concatenate([h.ind for h in hs]))
+    for h, b in zip(hs, base):
+        g = ap.HostGraph(h.m, h.ptr, h.ind, symmetric=True).to_device()
+        perm, lp, li = ap.tc_prepare(ctx, g)
+        _, olp, oli = oracle.tc_build_lower(h.m, h.ptr, h.ind)
+        want = oracle.tc_lower(h.m, olp, oli)
+        assert ap.triangle_count(ctx, h.m, lp, li) == want
+        g.ptr, g.ind = _t(h.ptr + np.int32(b)), ind
+        perm2, lp2, li2 = ap.tc_prepare(ctx, g)
+        assert torch.equal(perm, perm2) and torch.equal(lp, lp2) and torch.equal(li, li2)
+        behind = torch.cat([torch.zeros(5000, dtype=torch.int32, device="cuda"), li])
+        assert ap.triangle_count(ctx, h.m, lp + 5000, behind) == want

@@ -329,10 +329,14 @@ __global__ void dense_fill(int m, float v, float *y) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) y[i] = v;
 }
 
-__global__ void dense_scatter(const int *nnz, const int *yind, const float *yval, float *y) {
-  int n = *nnz;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    y[yind[i]] = yval[i];
+// (a sort that gave up, which the caller reports, may leave any length and any
+// row: both are bounds-checked)
+__global__ void dense_scatter(const int *nnz, int m, const int *yind, const float *yval, float *y) {
+  const int n = min(*nnz, m);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int r = yind[i];
+    if ((unsigned)r < (unsigned)m) y[r] = yval[i];
+  }
 }
 
 int grid_for(apspie_context *ctx, long long n, int threads) {
@@ -433,12 +437,40 @@ int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *i
   return check_launch(ctx, "reduce_segments");
 }
 
-// The expanded size read back at the end of a call: the kernels do nothing
-// with one that does not fit the int32 layout.
-int spmspv_overflow(apspie_context *ctx, long long E) {
-  return E < (long long)INT32_MAX
-             ? APSPIE_OK
-             : set_error(ctx, APSPIE_ERR_OVERFLOW, "spmspv: %lld expanded pairs", E);
+// A call's scalars lie behind the radix sort's give-up word: one copy reads both.
+struct SpmspvBack {
+  int sort_err, pad[3];
+  SpmspvSmall s;
+};
+static_assert(offsetof(SpmspvBack, s) == kSortErrWords * sizeof(int) &&
+                  sizeof(SpmspvBack) <= kSortErrBytes, "read back in one copy");
+
+SpmspvSmall *spmspv_scalars(apspie_context *ctx) {
+  int *sort_err = radix_sort_err(ctx);
+  return sort_err ? (SpmspvSmall *)(sort_err + kSortErrWords) : nullptr;
+}
+
+// Waits for a call and reads its scalars back.  A status when the sort path's
+// look-back gave up (y is not sorted), or when the expanded size does not fit
+// the int32 layout (the kernels did nothing).
+int spmspv_read_back(apspie_context *ctx, const char *what, SpmspvSmall *out) {
+  int *sort_err = radix_sort_err(ctx);
+  auto *h = (SpmspvBack *)pinned(ctx, sizeof(SpmspvBack));
+  if (!sort_err || !h) return APSPIE_ERR_OOM;
+  int rc = check_cuda(ctx, cudaMemcpyAsync(h, sort_err, sizeof(SpmspvBack), cudaMemcpyDeviceToHost,
+                                           ctx->stream), what);
+  if (rc) return rc;
+  rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), what);
+  if (rc) return rc;
+  if (h->sort_err) {
+    rc = check_cuda(ctx, cudaMemsetAsync(sort_err, 0, sizeof(int), ctx->stream), what);
+    if (rc) return rc;
+    return set_error(ctx, APSPIE_ERR_TIMEOUT, "%s: radix sort look-back gave up", what);
+  }
+  if (h->s.total >= (long long)INT32_MAX)
+    return set_error(ctx, APSPIE_ERR_OVERFLOW, "%s: %lld expanded pairs", what, h->s.total);
+  *out = h->s;
+  return APSPIE_OK;
 }
 
 }  // namespace
@@ -456,35 +488,16 @@ int apspie_spmspv(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int *d
   if (semiring < 0 || semiring > 3 || m <= 0 || nnz < 0 || xnnz < 0 || xnnz > m || !d_ptr ||
       (nnz > 0 && !d_ind) || (xnnz > 0 && !d_xind) || !d_yind || !d_yval || !h_ynnz)
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_spmspv: bad arguments");
-  // the call's scalars lie behind the sort's give-up word: one copy reads both
-  struct Back {
-    int sort_err, pad[3];
-    SpmspvSmall s;
-  };
-  static_assert(offsetof(Back, s) == kSortErrWords * sizeof(int) &&
-                    sizeof(Back) <= kSortErrBytes, "read back in one copy");
-  int *sort_err = radix_sort_err(ctx);
-  if (!sort_err) return APSPIE_ERR_OOM;
-  auto *sm = (SpmspvSmall *)(sort_err + kSortErrWords);
+  auto *sm = spmspv_scalars(ctx);
+  if (!sm) return APSPIE_ERR_OOM;
   int rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, d_xind, d_xval, d_yind, d_yval,
                        sm);
   if (rc) return rc;
-  auto *h = (Back *)pinned(ctx, sizeof(Back));
-  if (!h) return APSPIE_ERR_OOM;
-  rc = check_cuda(ctx, cudaMemcpyAsync(h, sort_err, sizeof(Back), cudaMemcpyDeviceToHost,
-                                       ctx->stream), "apspie_spmspv");
+  SpmspvSmall back;
+  rc = spmspv_read_back(ctx, "apspie_spmspv", &back);
   if (rc) return rc;
-  rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "apspie_spmspv");
-  if (rc) return rc;
-  if (h->sort_err) {  // the sort path's look-back gave up: the output is not sorted
-    rc = check_cuda(ctx, cudaMemsetAsync(sort_err, 0, sizeof(int), ctx->stream), "apspie_spmspv");
-    if (rc) return rc;
-    return set_error(ctx, APSPIE_ERR_TIMEOUT, "apspie_spmspv: radix sort look-back gave up");
-  }
-  rc = spmspv_overflow(ctx, h->s.total);
-  if (rc) return rc;
-  *h_ynnz = h->s.ynnz;
-  if (h_expanded) *h_expanded = h->s.total;
+  *h_ynnz = back.ynnz;
+  if (h_expanded) *h_expanded = back.total;
   return APSPIE_OK;
 }
 
@@ -504,7 +517,7 @@ int apspie_mxv_dense(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int
   float *fv = (float *)(buf + (m + 1));
   int *yi = buf + 2 * (m + 1);
   float *yv = (float *)(buf + 3 * (m + 1));
-  auto *sm = (SpmspvSmall *)workspace(ctx, kSlotSmall, sizeof(SpmspvSmall));
+  auto *sm = spmspv_scalars(ctx);
   if (!sm) return APSPIE_ERR_OOM;
   unsigned *d_cnt = &sm->cnt;
   dense_frontier_flags<<<grid_for(ctx, m, 256), 256, 0, st>>>(semiring, m, d_x, flags);
@@ -530,19 +543,13 @@ int apspie_mxv_dense(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int
   rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, fx, fv, yi, yv, sm);
   if (rc) return rc;
   dense_fill<<<grid_for(ctx, m, 256), 256, 0, st>>>(m, empty, d_y);
-  dense_scatter<<<grid_for(ctx, m, 256), 256, 0, st>>>(&sm->ynnz, yi, yv, d_y);
+  dense_scatter<<<grid_for(ctx, m, 256), 256, 0, st>>>(&sm->ynnz, m, yi, yv, d_y);
   rc = check_launch(ctx, "dense_scatter", 2);
   if (rc) return rc;
-  auto *hs = (SpmspvSmall *)pinned(ctx, sizeof(SpmspvSmall));
-  if (!hs) return APSPIE_ERR_OOM;
-  rc = check_cuda(ctx, cudaMemcpyAsync(hs, sm, sizeof(SpmspvSmall), cudaMemcpyDeviceToHost, st),
-                  "apspie_mxv_dense");
+  SpmspvSmall back;
+  rc = spmspv_read_back(ctx, "apspie_mxv_dense", &back);
   if (rc) return rc;
-  rc = check_cuda(ctx, cudaStreamSynchronize(st), "apspie_mxv_dense");
-  if (rc) return rc;
-  rc = spmspv_overflow(ctx, hs->total);
-  if (rc) return rc;
-  if (h_expanded) *h_expanded = hs->total;
+  if (h_expanded) *h_expanded = back.total;
   return APSPIE_OK;
 }
 

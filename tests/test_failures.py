@@ -65,6 +65,35 @@ def test_sort_lookback_timeout_is_reported_by_spmspv():
         np.testing.assert_allclose(yv.cpu().numpy(), ryv, rtol=1e-6)
 
 
+@pytest.mark.parametrize("sr", [0, 1])
+def test_sort_lookback_timeout_is_reported_by_mxv_dense(sr):
+    """The call that met the failure reports it, and y's stores stay inside y:
+    the words around it keep their value."""
+    import torch
+    import apspie_b200 as ap
+    from apspie_b200._native import lib
+    h = ap.gen_rmat(14, 16, seed=4, symmetric=False)
+    g = h.to_device()
+    val = torch.ones(h.nnz, dtype=torch.float32, device="cuda")
+    x = torch.full((h.m,), 1.70141e38, device="cuda")
+    x[::3] = 1.0
+    if sr == 0:
+        x[x > 2] = 0.0
+    around = torch.full((3 * h.m,), -7.0, device="cuda")
+    y = around[h.m:2 * h.m]
+    with ap.Context(0) as ctx:
+        ap.spmspv_set_params(ctx, 0.0)         # always the radix-sort path
+        ref, total = ap.mxv_dense(ctx, sr, g, x, val)
+        assert lib.apspie_debug_inject(ctx.handle, INJECT_SORT_LOOKBACK) == 0
+        with pytest.raises(ap.ApspieError) as e:
+            ap.mxv_dense(ctx, sr, g, x, val, y)
+        assert e.value.status == APSPIE_ERR_TIMEOUT
+        assert (around[:h.m] == -7).all() and (around[2 * h.m:] == -7).all()
+        # cleared: the next call sorts again, correctly
+        got, again = ap.mxv_dense(ctx, sr, g, x, val, y)
+        assert torch.equal(got, ref) and again == total
+
+
 def test_allocation_failure_is_a_status():
     import apspie_b200 as ap
     from apspie_b200._native import lib

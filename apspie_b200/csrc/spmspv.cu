@@ -345,15 +345,19 @@ int grid_for(apspie_context *ctx, long long n, int threads) {
 }
 
 // Core sparse SpMSpV.  On return sm->ynnz (device) holds nnz(y) and sm->total
-// the expanded size E; the caller reads both back and passes E to
-// spmspv_overflow.
+// the expanded size E, which spmspv_read_back brings to the host.  *h_total is
+// E where the call had to wait for it and nothing is left to be checked (no
+// sort, or one of a single tile, which waits for nothing), else -1.
 int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *ind,
                 const float *val, int xnnz, const int *xind, const float *xval, int *yind,
-                float *yval, SpmspvSmall *sm) {
+                float *yval, SpmspvSmall *sm, long long *h_total) {
   cudaStream_t st = ctx->stream;
+  *h_total = -1;
   const double factor = ctx->spmspv_sort_factor;
-  if (xnnz == 0)
+  if (xnnz == 0) {
+    *h_total = 0;
     return check_cuda(ctx, cudaMemsetAsync(sm, 0, sizeof(SpmspvSmall), st), "spmspv empty");
+  }
   auto *offs = (long long *)workspace(ctx, kSlotMisc0, sizeof(long long) * (size_t)(xnnz + 1));
   auto *col = (int2 *)workspace(ctx, kSlotMisc2, sizeof(int2) * (size_t)xnnz);
   if (!offs || !col) return APSPIE_ERR_OOM;
@@ -379,11 +383,13 @@ int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *i
     rc = check_cuda(ctx, cudaStreamSynchronize(st), "spmspv total");
     if (rc) return rc;
     E = *h;
+    if (E <= kSortTile) *h_total = E;
     if (E == 0)
       return check_cuda(ctx, cudaMemsetAsync(&sm->ynnz, 0, sizeof(int), st), "spmspv empty");
     if (E >= (long long)INT32_MAX)
       return set_error(ctx, APSPIE_ERR_OVERFLOW, "spmspv: %lld expanded pairs", E);
     bitmap = (double)E * factor > (double)m;
+    if (bitmap) *h_total = E;
   }
   const int egrid = ctx->num_sms * 6;  // resident blocks; they stride the tiles
   if (bitmap) {
@@ -490,8 +496,9 @@ int apspie_spmspv(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int *d
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_spmspv: bad arguments");
   auto *sm = spmspv_scalars(ctx);
   if (!sm) return APSPIE_ERR_OOM;
+  long long total;
   int rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, d_xind, d_xval, d_yind, d_yval,
-                       sm);
+                       sm, &total);
   if (rc) return rc;
   SpmspvSmall back;
   rc = spmspv_read_back(ctx, "apspie_spmspv", &back);
@@ -540,16 +547,22 @@ int apspie_mxv_dense(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int
   // y reset to the semiring's empty value, as preprocessFlag does
   // (0 for mXv, src/mXv.cuh:45; 1.70141e38 for SSSP, src/spmspvSssp.cuh:26)
   float empty = semiring == kMinPlus ? 1.70141e+38f : 0.0f;
-  rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, fx, fv, yi, yv, sm);
+  long long total;
+  rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, fx, fv, yi, yv, sm, &total);
   if (rc) return rc;
+  // the result's status before y is written: a call that fails leaves it, and
+  // the wait for E is the last one
+  if (total < 0) {
+    SpmspvSmall back;
+    rc = spmspv_read_back(ctx, "apspie_mxv_dense", &back);
+    if (rc) return rc;
+    total = back.total;
+  }
   dense_fill<<<grid_for(ctx, m, 256), 256, 0, st>>>(m, empty, d_y);
   dense_scatter<<<grid_for(ctx, m, 256), 256, 0, st>>>(&sm->ynnz, m, yi, yv, d_y);
   rc = check_launch(ctx, "dense_scatter", 2);
   if (rc) return rc;
-  SpmspvSmall back;
-  rc = spmspv_read_back(ctx, "apspie_mxv_dense", &back);
-  if (rc) return rc;
-  if (h_expanded) *h_expanded = back.total;
+  if (h_expanded) *h_expanded = total;
   return APSPIE_OK;
 }
 

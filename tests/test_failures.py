@@ -94,6 +94,25 @@ def test_sort_lookback_timeout_is_reported_by_mxv_dense(sr):
         assert torch.equal(got, ref) and again == total
 
 
+def test_failed_mxv_dense_leaves_y():
+    """y is written when the call's status is known, not before."""
+    import torch
+    import apspie_b200 as ap
+    from apspie_b200._native import lib
+    h = ap.gen_rmat(14, 16, seed=4, symmetric=False)
+    g = h.to_device()
+    x = torch.zeros(h.m, device="cuda")
+    x[::3] = 1.0
+    y = torch.full((h.m,), -7.0, device="cuda")
+    with ap.Context(0) as ctx:
+        ap.spmspv_set_params(ctx, 0.0)         # always the radix-sort path
+        assert lib.apspie_debug_inject(ctx.handle, INJECT_SORT_LOOKBACK) == 0
+        with pytest.raises(ap.ApspieError) as e:
+            ap.mxv_dense(ctx, 0, g, x, None, y)
+        assert e.value.status == APSPIE_ERR_TIMEOUT
+        assert (y == -7).all()
+
+
 def test_allocation_failure_is_a_status():
     import apspie_b200 as ap
     from apspie_b200._native import lib

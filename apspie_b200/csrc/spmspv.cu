@@ -46,8 +46,26 @@ struct SpmspvSmall {  // device-side scalars of one call
   unsigned cnt;       // frontier size of the dense form
 };
 
-// up to this many rows of y the bitmap path is taken at any frontier density
+// Path rule.  PLUS_TIMES: the bitmap path when E * factor > m, else the sort
+// path, whose sums run in the frontier's order and have the same bits in every
+// run (the bitmap path's double atomics add in any order).  The other semirings'
+// results do not depend on the order: up to kBitmapRows rows of y they take the
+// bitmap path at any density (8 entries a column, 2^22 rows: 63 us against 69
+// sorted at 32 products, 75 against 132 at 65,536; 2^20 rows: 51 against 67).
+//
+// Up to kBitmapRows rows the bitmap path starts before the host knows E (the
+// expansion checks the rule for PLUS_TIMES; frontiers that turn out sparse are
+// sorted after the read-back): for PLUS_TIMES when the frontier has at least
+// 1 / kDenseGuess of the entries that the rule asks for at the mean column
+// length.  A frontier of longer columns that was guessed sparse costs a wait,
+// 10 us; one guessed dense that is sparse costs 10 us at 2^20 rows and 25 at
+// 2^22 (launches and the cleared accumulator).
 constexpr int kBitmapRows = 1 << 22;
+constexpr double kDenseGuess = 1.25;
+
+__host__ __device__ __forceinline__ bool spmspv_dense(long long E, double factor, int m) {
+  return (double)E * factor > (double)m;
+}
 
 __device__ __forceinline__ float sr_term(int sr, float a, float x) {
   switch (sr) {
@@ -203,9 +221,11 @@ __global__ void reduce_segments(int sr, const int *keys, const float *vals, long
 
 // ---- bitmap path ----
 __global__ void __launch_bounds__(kEdgeThreads)
-expand_accumulate(int sr, int xnnz, const long long *__restrict__ offs, const long long *total,
-                  const int2 *__restrict__ col, const int *__restrict__ ind,
-                  const float *__restrict__ val, void *acc) {
+expand_accumulate(int sr, int m, double factor, int xnnz, const long long *__restrict__ offs,
+                  const long long *total, const int2 *__restrict__ col,
+                  const int *__restrict__ ind, const float *__restrict__ val, void *acc) {
+  // a sparse PLUS_TIMES frontier is sorted: no row is touched here
+  if (sr == kPlusTimes && !spmspv_dense(__ldcg(total), factor, m)) return;
   for_each_entry(sr, xnnz, offs, total, col, ind, val,
                  [&](const int (&)[kEdgeItems], const int (&row)[kEdgeItems],
                      const float (&term)[kEdgeItems], const bool (&on)[kEdgeItems]) {
@@ -258,8 +278,8 @@ touched_rows(int sr, int m, const void *__restrict__ acc, int words, int per_blo
   if (threadIdx.x == 0) sums[blockIdx.x] = tot;
 }
 
-// A row of NaN terms only is NaN for a frontier that the sort path's threshold
-// calls sparse (E * factor <= m: the sorted reduction has it so), else the
+// MIN_PLUS and MAX_TIMES: a row of NaN terms only is NaN for a frontier below
+// the threshold (E * factor <= m), as the sorted reduction has it, else the
 // infinity that the reduction starts from.
 __global__ void __launch_bounds__(kEmitThreads)
 touched_emit(int sr, int m, const unsigned *__restrict__ bits, int words, int per_block,
@@ -344,103 +364,8 @@ int grid_for(apspie_context *ctx, long long n, int threads) {
   return (int)std::max(1ll, std::min(g, (long long)ctx->num_sms * 16));
 }
 
-// Core sparse SpMSpV.  On return sm->ynnz (device) holds nnz(y) and sm->total
-// the expanded size E, which spmspv_read_back brings to the host.  *h_total is
-// E where the call had to wait for it and nothing is left to be checked (no
-// sort, or one of a single tile, which waits for nothing), else -1.
-int spmspv_core(apspie_context *ctx, int sr, int m, const int *ptr, const int *ind,
-                const float *val, int xnnz, const int *xind, const float *xval, int *yind,
-                float *yval, SpmspvSmall *sm, long long *h_total) {
-  cudaStream_t st = ctx->stream;
-  *h_total = -1;
-  const double factor = ctx->spmspv_sort_factor;
-  if (xnnz == 0) {
-    *h_total = 0;
-    return check_cuda(ctx, cudaMemsetAsync(sm, 0, sizeof(SpmspvSmall), st), "spmspv empty");
-  }
-  auto *offs = (long long *)workspace(ctx, kSlotMisc0, sizeof(long long) * (size_t)(xnnz + 1));
-  auto *col = (int2 *)workspace(ctx, kSlotMisc2, sizeof(int2) * (size_t)xnnz);
-  if (!offs || !col) return APSPIE_ERR_OOM;
-  bool bitmap = m <= kBitmapRows && factor > 0.0;
-  void *acc = nullptr;
-  if (bitmap) {
-    acc = workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
-    if (!acc) return APSPIE_ERR_OOM;
-  }
-  frontier_columns<<<grid_for(ctx, bitmap ? std::max(xnnz, m) : xnnz, 256), 256, 0, st>>>(
-      xnnz, xind, xval, ptr, offs, col, sr, m, (unsigned long long *)acc);
-  int rc = check_launch(ctx, "frontier_columns");
-  if (rc) return rc;
-  long long E = 0;
-  if (!bitmap) {
-    rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, &sm->total);
-    if (rc) return rc;
-    long long *h = (long long *)pinned(ctx, sizeof(long long));
-    if (!h) return APSPIE_ERR_OOM;
-    rc = check_cuda(ctx, cudaMemcpyAsync(h, &sm->total, sizeof(long long), cudaMemcpyDeviceToHost,
-                                         st), "spmspv total");
-    if (rc) return rc;
-    rc = check_cuda(ctx, cudaStreamSynchronize(st), "spmspv total");
-    if (rc) return rc;
-    E = *h;
-    if (E <= kSortTile) *h_total = E;
-    if (E == 0)
-      return check_cuda(ctx, cudaMemsetAsync(&sm->ynnz, 0, sizeof(int), st), "spmspv empty");
-    if (E >= (long long)INT32_MAX)
-      return set_error(ctx, APSPIE_ERR_OVERFLOW, "spmspv: %lld expanded pairs", E);
-    bitmap = (double)E * factor > (double)m;
-    if (bitmap) *h_total = E;
-  }
-  const int egrid = ctx->num_sms * 6;  // resident blocks; they stride the tiles
-  if (bitmap) {
-    const int words = (int)(((long long)m + 31) / 32);
-    unsigned *bits = (unsigned *)workspace(ctx, kSlotBitmap,
-                                           sizeof(unsigned) * ((size_t)words + kEmitBlocks));
-    if (!bits) return APSPIE_ERR_OOM;
-    unsigned *sums = bits + words;
-    if (acc) {  // cleared, and the lengths not scanned yet
-      rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, &sm->total);
-      if (rc) return rc;
-    } else {
-      acc = workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
-      if (!acc) return APSPIE_ERR_OOM;
-      acc_init<<<grid_for(ctx, m, 256), 256, 0, st>>>(sr, m, (unsigned long long *)acc);
-      rc = check_launch(ctx, "acc_init");
-      if (rc) return rc;
-    }
-    expand_accumulate<<<egrid, kEdgeThreads, 0, st>>>(sr, xnnz, offs, &sm->total, col, ind, val,
-                                                      acc);
-    const int per_block = std::max(kEmitWords, (words + kEmitBlocks - 1) / kEmitBlocks);
-    const int eblocks = (words + per_block - 1) / per_block;
-    touched_rows<<<eblocks, kEmitThreads, 0, st>>>(sr, m, acc, words, per_block, bits, sums);
-    touched_emit<<<eblocks, kEmitThreads, 0, st>>>(sr, m, bits, words, per_block, sums, acc,
-                                                   &sm->total, factor, yind, yval, &sm->ynnz);
-    return check_launch(ctx, "spmspv bitmap", 3);
-  }
-  // sort path
-  int *ka = (int *)workspace(ctx, kSlotSortKeysA, sizeof(int) * (size_t)E);
-  int *kb = (int *)workspace(ctx, kSlotSortKeysB, sizeof(int) * (size_t)E);
-  float *va = (float *)workspace(ctx, kSlotSortValsA, sizeof(float) * (size_t)E);
-  float *vb = (float *)workspace(ctx, kSlotSortValsB, sizeof(float) * (size_t)E);
-  if (!ka || !kb || !va || !vb) return APSPIE_ERR_OOM;
-  expand_pairs<<<(unsigned)std::min<long long>(edge_tiles(E), egrid), kEdgeThreads, 0, st>>>(
-      sr, xnnz, offs, &sm->total, col, ind, val, ka, va);
-  rc = check_launch(ctx, "expand_pairs");
-  if (rc) return rc;
-  bool in_b = false;
-  rc = device_radix_sort<int, float>(ctx, ka, va, kb, vb, E, bits_for(m), &in_b);
-  if (rc) return rc;
-  int *ks = in_b ? kb : ka;
-  float *vs = in_b ? vb : va;
-  unsigned *flags = (unsigned *)workspace(ctx, kSlotMisc3, sizeof(unsigned) * (size_t)E);
-  if (!flags) return APSPIE_ERR_OOM;
-  head_flags<<<grid_for(ctx, E, 256), 256, 0, st>>>(ks, E, flags);
-  rc = check_launch(ctx, "head_flags");
-  if (rc) return rc;
-  rc = device_exclusive_scan<unsigned>(ctx, flags, flags, E, (unsigned *)&sm->ynnz);
-  if (rc) return rc;
-  reduce_segments<<<grid_for(ctx, E, 256), 256, 0, st>>>(sr, ks, vs, E, flags, yind, yval, m);
-  return check_launch(ctx, "reduce_segments");
+int expand_grid(apspie_context *ctx) {
+  return ctx->num_sms * 6;  // resident blocks; they stride the tiles
 }
 
 // A call's scalars lie behind the radix sort's give-up word: one copy reads both.
@@ -479,6 +404,119 @@ int spmspv_read_back(apspie_context *ctx, const char *what, SpmspvSmall *out) {
   return APSPIE_OK;
 }
 
+// The sort path from the scanned column lengths on.
+int spmspv_sorted(apspie_context *ctx, int sr, int m, const int *ind, const float *val, int xnnz,
+                  const long long *offs, const int2 *col, long long E, int *yind, float *yval,
+                  SpmspvSmall *sm) {
+  cudaStream_t st = ctx->stream;
+  int *ka = (int *)workspace(ctx, kSlotSortKeysA, sizeof(int) * (size_t)E);
+  int *kb = (int *)workspace(ctx, kSlotSortKeysB, sizeof(int) * (size_t)E);
+  float *va = (float *)workspace(ctx, kSlotSortValsA, sizeof(float) * (size_t)E);
+  float *vb = (float *)workspace(ctx, kSlotSortValsB, sizeof(float) * (size_t)E);
+  unsigned *flags = (unsigned *)workspace(ctx, kSlotMisc3, sizeof(unsigned) * (size_t)E);
+  if (!ka || !kb || !va || !vb || !flags) return APSPIE_ERR_OOM;
+  expand_pairs<<<(unsigned)std::min<long long>(edge_tiles(E), expand_grid(ctx)), kEdgeThreads, 0,
+                 st>>>(sr, xnnz, offs, &sm->total, col, ind, val, ka, va);
+  int rc = check_launch(ctx, "expand_pairs");
+  if (rc) return rc;
+  bool in_b = false;
+  rc = device_radix_sort<int, float>(ctx, ka, va, kb, vb, E, bits_for(m), &in_b);
+  if (rc) return rc;
+  int *ks = in_b ? kb : ka;
+  float *vs = in_b ? vb : va;
+  head_flags<<<grid_for(ctx, E, 256), 256, 0, st>>>(ks, E, flags);
+  rc = check_launch(ctx, "head_flags");
+  if (rc) return rc;
+  rc = device_exclusive_scan<unsigned>(ctx, flags, flags, E, (unsigned *)&sm->ynnz);
+  if (rc) return rc;
+  reduce_segments<<<grid_for(ctx, E, 256), 256, 0, st>>>(sr, ks, vs, E, flags, yind, yval, m);
+  return check_launch(ctx, "reduce_segments");
+}
+
+// Sparse SpMSpV.  On return y and sm->ynnz (device) are written and *out holds
+// the call's scalars: the expanded size, and nnz(y) where the host had to read
+// it (out->ynnz -1: it did not; want_ynnz asks for it).  A status when the
+// sort path's look-back gave up or E does not fit the int32 layout.
+int spmspv_run(apspie_context *ctx, const char *what, int sr, int m, int64_t nnz, const int *ptr,
+               const int *ind, const float *val, int xnnz, const int *xind, const float *xval,
+               int *yind, float *yval, SpmspvSmall *sm, bool want_ynnz, SpmspvSmall *out) {
+  cudaStream_t st = ctx->stream;
+  const double factor = ctx->spmspv_sort_factor;
+  out->total = 0;
+  out->ynnz = -1;
+  int rc = APSPIE_OK;
+  if (xnnz == 0) {
+    rc = check_cuda(ctx, cudaMemsetAsync(sm, 0, sizeof(SpmspvSmall), st), what);
+    return rc || !want_ynnz ? rc : spmspv_read_back(ctx, what, out);
+  }
+  auto *offs = (long long *)workspace(ctx, kSlotMisc0, sizeof(long long) * (size_t)(xnnz + 1));
+  auto *col = (int2 *)workspace(ctx, kSlotMisc2, sizeof(int2) * (size_t)xnnz);
+  if (!offs || !col) return APSPIE_ERR_OOM;
+  // the bitmap path before E is known
+  const bool ahead = m <= kBitmapRows && factor > 0.0 &&
+                     (sr != kPlusTimes || (double)xnnz * (double)nnz * factor * kDenseGuess >=
+                                              (double)m * (double)m);
+  void *acc = nullptr;
+  if (ahead) {
+    acc = workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
+    if (!acc) return APSPIE_ERR_OOM;
+  }
+  frontier_columns<<<grid_for(ctx, ahead ? std::max(xnnz, m) : xnnz, 256), 256, 0, st>>>(
+      xnnz, xind, xval, ptr, offs, col, sr, m, (unsigned long long *)acc);
+  rc = check_launch(ctx, "frontier_columns");
+  if (rc) return rc;
+  rc = device_exclusive_scan<long long>(ctx, offs, offs, xnnz, &sm->total);
+  if (rc) return rc;
+  bool bitmap = ahead;
+  if (!ahead) {
+    long long *h = (long long *)pinned(ctx, sizeof(long long));
+    if (!h) return APSPIE_ERR_OOM;
+    rc = check_cuda(ctx, cudaMemcpyAsync(h, &sm->total, sizeof(long long), cudaMemcpyDeviceToHost,
+                                         st), what);
+    if (rc) return rc;
+    rc = check_cuda(ctx, cudaStreamSynchronize(st), what);
+    if (rc) return rc;
+    out->total = *h;
+    if (out->total >= (long long)INT32_MAX)
+      return set_error(ctx, APSPIE_ERR_OVERFLOW, "%s: %lld expanded pairs", what, out->total);
+    if (out->total == 0) {
+      rc = check_cuda(ctx, cudaMemsetAsync(&sm->ynnz, 0, sizeof(int), st), what);
+      return rc || !want_ynnz ? rc : spmspv_read_back(ctx, what, out);
+    }
+    bitmap = spmspv_dense(out->total, factor, m);
+  }
+  if (bitmap) {
+    const int words = (int)(((long long)m + 31) / 32);
+    unsigned *bits = (unsigned *)workspace(ctx, kSlotBitmap,
+                                           sizeof(unsigned) * ((size_t)words + kEmitBlocks));
+    if (!bits) return APSPIE_ERR_OOM;
+    unsigned *sums = bits + words;
+    if (!acc) {  // not cleared with the columns
+      acc = workspace(ctx, kSlotDense, sizeof(double) * (size_t)m);
+      if (!acc) return APSPIE_ERR_OOM;
+      acc_init<<<grid_for(ctx, m, 256), 256, 0, st>>>(sr, m, (unsigned long long *)acc);
+      rc = check_launch(ctx, "acc_init");
+      if (rc) return rc;
+    }
+    expand_accumulate<<<expand_grid(ctx), kEdgeThreads, 0, st>>>(sr, m, factor, xnnz, offs,
+                                                                 &sm->total, col, ind, val, acc);
+    const int per_block = std::max(kEmitWords, (words + kEmitBlocks - 1) / kEmitBlocks);
+    const int eblocks = (words + per_block - 1) / per_block;
+    touched_rows<<<eblocks, kEmitThreads, 0, st>>>(sr, m, acc, words, per_block, bits, sums);
+    touched_emit<<<eblocks, kEmitThreads, 0, st>>>(sr, m, bits, words, per_block, sums, acc,
+                                                   &sm->total, factor, yind, yval, &sm->ynnz);
+    rc = check_launch(ctx, "spmspv bitmap", 3);
+    if (rc) return rc;
+    if (ahead || want_ynnz) rc = spmspv_read_back(ctx, what, out);
+    if (rc || sr != kPlusTimes || out->total == 0 || spmspv_dense(out->total, factor, m)) return rc;
+  }
+  const long long E = out->total;
+  rc = spmspv_sorted(ctx, sr, m, ind, val, xnnz, offs, col, E, yind, yval, sm);
+  if (rc) return rc;
+  // a sort of one tile waits for no other: nothing to check
+  return want_ynnz || E > kSortTile ? spmspv_read_back(ctx, what, out) : APSPIE_OK;
+}
+
 }  // namespace
 }  // namespace apspie
 
@@ -496,12 +534,9 @@ int apspie_spmspv(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int *d
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_spmspv: bad arguments");
   auto *sm = spmspv_scalars(ctx);
   if (!sm) return APSPIE_ERR_OOM;
-  long long total;
-  int rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, d_xind, d_xval, d_yind, d_yval,
-                       sm, &total);
-  if (rc) return rc;
   SpmspvSmall back;
-  rc = spmspv_read_back(ctx, "apspie_spmspv", &back);
+  const int rc = spmspv_run(ctx, "apspie_spmspv", semiring, m, nnz, d_ptr, d_ind, d_val, xnnz,
+                            d_xind, d_xval, d_yind, d_yval, sm, true, &back);
   if (rc) return rc;
   *h_ynnz = back.ynnz;
   if (h_expanded) *h_expanded = back.total;
@@ -547,22 +582,16 @@ int apspie_mxv_dense(apspie_ctx ctx, int semiring, int m, int64_t nnz, const int
   // y reset to the semiring's empty value, as preprocessFlag does
   // (0 for mXv, src/mXv.cuh:45; 1.70141e38 for SSSP, src/spmspvSssp.cuh:26)
   float empty = semiring == kMinPlus ? 1.70141e+38f : 0.0f;
-  long long total;
-  rc = spmspv_core(ctx, semiring, m, d_ptr, d_ind, d_val, xnnz, fx, fv, yi, yv, sm, &total);
+  // y is written when the call's status is known: one that fails leaves it
+  SpmspvSmall back;
+  rc = spmspv_run(ctx, "apspie_mxv_dense", semiring, m, nnz, d_ptr, d_ind, d_val, xnnz, fx, fv,
+                  yi, yv, sm, false, &back);
   if (rc) return rc;
-  // the result's status before y is written: a call that fails leaves it, and
-  // the wait for E is the last one
-  if (total < 0) {
-    SpmspvSmall back;
-    rc = spmspv_read_back(ctx, "apspie_mxv_dense", &back);
-    if (rc) return rc;
-    total = back.total;
-  }
   dense_fill<<<grid_for(ctx, m, 256), 256, 0, st>>>(m, empty, d_y);
   dense_scatter<<<grid_for(ctx, m, 256), 256, 0, st>>>(&sm->ynnz, m, yi, yv, d_y);
   rc = check_launch(ctx, "dense_scatter", 2);
   if (rc) return rc;
-  if (h_expanded) *h_expanded = total;
+  if (h_expanded) *h_expanded = back.total;
   return APSPIE_OK;
 }
 

@@ -437,8 +437,8 @@ int apspie_autotune_bfs(apspie_ctx ctx, int nsrc, const int *h_src, int64_t nnz,
                         int32_t *d_depth_scratch, int *alpha_out, int *beta_out,
                         float *ms_out);
 /* Finds the frontier density at which the SpMSpV bitmap path beats the
- * radix-sort path on this matrix and sets the context's sort factor (see
- * apspie_spmspv_set_params).  Scratch: m ints (x), m ints + m floats (y);
+ * radix-sort path on this matrix, under PLUS_TIMES, and sets the context's
+ * sort factor (see apspie_spmspv_set_params).  Scratch: m ints (x), m ints + m floats (y);
  * the frontiers are timed with unit values, so d_xval_scratch is not
  * written and may be NULL. */
 int apspie_autotune_spmspv(apspie_ctx ctx, int m, int64_t nnz, const int *d_ptr,
@@ -537,10 +537,15 @@ int apspie_mxv_dense(apspie_ctx ctx, int semiring, int m, int64_t nnz,
                      const int *d_ptr, const int *d_ind, const float *d_val,
                      const float *d_x, float *d_y, int64_t *h_expanded);
 
-/* SpMSpV path choice.  sort_factor 0 always takes the radix-sort path.
- * Otherwise the bitmap (dense accumulator) path is used up to 2^22 rows, where
- * it is faster at any density, and beyond when products * sort_factor > m.
- * Default 4. */
+/* SpMSpV path choice, by the number of products.  sort_factor 0 always takes
+ * the radix-sort path.  Otherwise PLUS_TIMES takes the bitmap (dense
+ * accumulator) path when products * sort_factor > m, and the sort path for
+ * sparser frontiers: their sums run in the frontier's order and have the same
+ * bits in every run, where the bitmap path's double sums are formed in any
+ * order.  The other semirings give the same result either way and take the
+ * bitmap path at any density up to 2^22 rows, beyond by the same rule.  A row
+ * that only NaN terms touch is NaN under MIN_PLUS / MAX_TIMES when
+ * products * sort_factor <= m, else +inf / -inf.  Default 4. */
 int apspie_spmspv_set_params(apspie_ctx ctx, double sort_factor);
 
 /* ------------------------------------------------------------- SpGEMM ---

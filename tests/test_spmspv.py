@@ -255,3 +255,87 @@ def test_spmspv_zero_sums(ctx, m):
     assert yi.tolist() == rows.tolist()
     assert yv.tolist() == [0.0, 0.0, 0.0, 2.0]
     assert not np.signbit(yv.cpu().numpy()).any()
+
+
+@pytest.mark.parametrize("guess", ["sparse", "dense"])
+def test_spmspv_sparse_sums_run_in_the_frontiers_order(ctx, guess):
+    """PLUS_TIMES with products * factor <= m: every row's terms are added in
+    the order of the frontier's columns, in double, whatever the mean column
+    length makes of the frontier; one row less and the sum is only close."""
+    import torch
+    import apspie_b200 as ap
+    m, cols, rows = 1 << 16, 512, 32       # 16,384 products: 4 * 16,384 = m
+    rng = np.random.default_rng(5)
+    xind = np.sort(rng.choice(m, cols, replace=False)).astype(np.int32)
+    deg = np.zeros(m, np.int64)
+    if guess == "dense":
+        deg[:] = 30
+    deg[xind] = rows
+    ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    ind = rng.integers(0, m, int(ptr[-1])).astype(np.int32)
+    val = rng.uniform(1, 2, ind.size).astype(np.float32)
+    target = np.arange(rows, dtype=np.int32) * 1000
+    # small terms among huge ones that cancel: which of the small ones are left
+    # depends on the order of the additions
+    huge = np.concatenate([np.full(cols // 4, 2.0**60), np.full(cols // 4, -2.0**60),
+                           np.zeros(cols // 2)])
+    order = np.stack([rng.permutation(huge) for _ in range(rows)], axis=1)
+    for k, c in enumerate(xind):
+        ind[ptr[c]:ptr[c + 1]] = target
+        row = val[ptr[c]:ptr[c + 1]]
+        row[order[k] != 0] = order[k][order[k] != 0]
+    ref = np.zeros(rows)
+    for c in xind:
+        ref += val[ptr[c]:ptr[c + 1]].astype(np.float64)
+    t = lambda a: torch.from_numpy(a).cuda()
+    g = ap.HostGraph(m, ptr, ind).to_device(with_transpose=False)
+    for _ in range(3):
+        yi, yv, e = ap.spmspv(ctx, 0, g, t(xind), None, t(val))
+        assert e == cols * rows and yi.tolist() == target.tolist()
+        np.testing.assert_array_equal(yv.cpu().numpy(), ref.astype(np.float32))
+    x = np.zeros(m, np.float32)
+    x[xind] = 1.0
+    y, e = ap.mxv_dense(ctx, 0, g, t(x), t(val))
+    assert e == cols * rows
+    np.testing.assert_array_equal(y.cpu().numpy()[target], ref.astype(np.float32))
+    # one more product: the bitmap path
+    ptr[xind[-1] + 1:] += 1
+    ind = np.insert(ind, ptr[xind[-1]] + rows, 0).astype(np.int32)
+    val = np.insert(val, ptr[xind[-1]] + rows, 0.0).astype(np.float32)
+    g = ap.HostGraph(m, ptr, ind).to_device(with_transpose=False)
+    yi, yv, e = ap.spmspv(ctx, 0, g, t(xind), None, t(val))
+    assert e == cols * rows + 1 and yi.tolist() == target.tolist()
+    mag = np.zeros(rows)
+    for c in xind:
+        mag += np.abs(val[ptr[c]:ptr[c] + rows].astype(np.float64))
+    # 512 double additions and one rounding to float
+    assert np.all(np.abs(yv.cpu().numpy() - ref) <= 512 * 2.0**-52 * mag + 2.0**-23 * np.abs(ref))
+
+
+@pytest.mark.parametrize("sr", SEMIRINGS)
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("m", [1 << 22, (1 << 22) + 1])
+def test_spmspv_both_sides_of_the_row_limit(ctx, sr, dense, m):
+    """The rows up to which the bitmap path starts by itself, with products
+    on either side of m / factor, against the oracle."""
+    import torch
+    import apspie_b200 as ap
+    rng = np.random.default_rng(m + dense)
+    cols = 3000
+    xind = np.sort(rng.choice(m, cols, replace=False)).astype(np.int32)
+    deg = np.zeros(m, np.int64)
+    deg[xind] = rng.integers(0, 900 if dense else 20, cols)
+    total = int(deg.sum())
+    assert (total * 4 > m) == dense
+    ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    ind = (rng.integers(0, m, total) // 3 * 3).astype(np.int32)
+    ind[::7] = m - 1
+    val = rng.uniform(0.5, 2, total).astype(np.float32)
+    xval = rng.uniform(0.5, 2, cols).astype(np.float32)
+    g = ap.HostGraph(m, ptr, ind).to_device(with_transpose=False)
+    yi, yv, e = ap.spmspv(ctx, sr, g, torch.from_numpy(xind).cuda(), torch.from_numpy(xval).cuda(),
+                          torch.from_numpy(val).cuda())
+    ri, rv = oracle.spmspv(sr, m, ptr, ind, val, xind, xval)
+    assert e == total
+    np.testing.assert_array_equal(yi.cpu().numpy(), ri)
+    np.testing.assert_allclose(yv.cpu().numpy(), rv, rtol=1e-6)

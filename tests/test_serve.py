@@ -164,3 +164,26 @@ def test_server_device_results_and_replay(ctx):
         lat_p, wall_p = srv.replay(q, plain=True)
     assert (lat > 0).all() and (lat_p > 0).all()
     assert wall >= q["t_us"][-1] / 1e3 and wall_p >= q["t_us"][-1] / 1e3
+
+
+def test_server_counts_what_an_mis_query_holds():
+    """The state admitted for an MIS query covers its result row, its
+    priorities and what the call takes of a context's workspace."""
+    import torch
+    import apspie_b200 as ap
+    h = ap.gen_grid(1500, 1500)
+    d = h.to_device()
+    prio = torch.from_numpy(ap.mt19937(1, h.m).view(np.int32)).cuda()
+    with ap.Context(0) as own:
+        ap.mis(own, d, prio)
+        own.sync()
+        scratch = own.workspace_bytes
+    with ap.Server(budget_bytes=4 << 30) as srv:
+        gid = srv.add_graph(d)
+        rid = srv.submit(2, gid, 0, seed=77)     # its priorities are made first: tens of ms
+        held, end = 0, time.perf_counter() + 10
+        while held == 0 and time.perf_counter() < end:
+            held = srv.stats()["in_flight_bytes"]
+        srv.wait(rid)
+    # a slot's size is rounded up to 256 bytes
+    assert held >= 4 * h.m + 4 * h.m + scratch - 4096

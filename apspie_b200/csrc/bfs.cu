@@ -804,6 +804,14 @@ int apspie::bfs_enqueue(apspie_context *ctx, int src, int64_t nnz, int m, const 
   // beside other launches (a share of the grid) half the cluster finds a place
   // sooner, and several fit
   if (ctx->max_grid > 0) thin = std::min(thin, kThinBlocks / 2);
+  // more than eight blocks need the attribute in the CUDA context of the
+  // launch, which may be a new one since thin_blocks asked (cudaDeviceReset)
+  if (thin > 8 &&
+      cudaFuncSetAttribute(bfs_thin, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    thin = 8;
+  }
   if (thin && part != BfsPart::kMain) {
     bfs_init<<<std::min((m + 255) / 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(
         m, src, d_depth, d_ptr, qa, ca, st);

@@ -224,3 +224,43 @@ def test_bfs_thin_levels(ctx, edges, mode):
                 np.testing.assert_array_equal(d, np.where(ref < lim, ref, -1))
     finally:
         ap.bfs_set_params(ctx)
+
+
+_RESET_CHILD = """
+import ctypes as C, glob, sys
+import numpy as np
+import nvidia.cuda_runtime
+import apspie_b200 as ap
+from apspie_b200._native import lib
+rt = C.CDLL(glob.glob(list(nvidia.cuda_runtime.__path__)[0] + "/lib/libcudart.so*")[0])
+h = ap.gen_grid(200, 300)
+for turn in range(2):
+    ctx, dev = C.c_void_p(), []
+    assert lib.apspie_ctx_create(0, None, C.byref(ctx)) == 0
+    for a in (h.ptr, h.ind, np.zeros(h.m, np.int32)):
+        p = C.c_void_p()
+        assert rt.cudaMalloc(C.byref(p), C.c_size_t(a.nbytes)) == 0
+        assert rt.cudaMemcpy(p, C.c_void_p(a.ctypes.data), C.c_size_t(a.nbytes), 1) == 0
+        dev.append(p)
+    rc = lib.apspie_bfs(ctx, 0, C.c_int64(h.nnz), h.m, dev[0], dev[1], dev[0], dev[1], dev[2], 0)
+    assert rc == 0, (turn, rc, lib.apspie_last_error(ctx))
+    assert lib.apspie_ctx_sync(ctx) == 0
+    out = np.empty(h.m, np.int32)
+    assert rt.cudaMemcpy(C.c_void_p(out.ctypes.data), dev[2], C.c_size_t(out.nbytes), 2) == 0
+    r, c = np.divmod(np.arange(h.m), 300)
+    np.testing.assert_array_equal(out, r + c)
+    lib.apspie_ctx_destroy(ctx)
+    assert rt.cudaDeviceReset() == 0
+print("both turns")
+"""
+
+
+def test_sparse_bfs_after_the_device_was_reset():
+    """A process that resets its device (its own CUDA context) and goes on
+    with a new context, in a process of its own."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    res = subprocess.run([sys.executable, "-c", _RESET_CHILD], capture_output=True, text=True,
+                         timeout=300, cwd=Path(__file__).resolve().parents[1])
+    assert res.returncode == 0 and "both turns" in res.stdout, res.stdout + res.stderr[-2000:]

@@ -800,7 +800,8 @@ int apspie::bfs_enqueue(apspie_context *ctx, int src, int64_t nnz, int m, const 
   long long nnz_ll = (long long)nnz;
   int alpha = ctx->bfs_alpha, beta = ctx->bfs_beta, mode = ctx->bfs_mode;
   if (!d_tptr) mode = 1;  // no in-adjacency: push only
-  int thin = (long long)nnz <= kThinMeanDegree * m && mode != 2 ? thin_blocks(ctx->device) : 0;
+  int thin = (long long)nnz <= kThinMeanDegree * m && mode != 2 && !ctx->bfs_inject
+                 ? thin_blocks(ctx->device) : 0;
   // beside other launches (a share of the grid) half the cluster finds a place
   // sooner, and several fit
   if (ctx->max_grid > 0) thin = std::min(thin, kThinBlocks / 2);
@@ -840,6 +841,7 @@ int apspie::bfs_enqueue(apspie_context *ctx, int src, int64_t nnz, int m, const 
                                               dim3(kBfsThreads), args, 0, ctx->stream);
   if (e != cudaSuccess) return check_cuda(ctx, e, "bfs_persistent");
   if (!thin) ctx->bfs_par ^= 1;
+  ctx->bfs_inject = false;
   ctx->launches += 1;
   return APSPIE_OK;
 }
@@ -1098,6 +1100,7 @@ int bfs_inject(apspie_context *ctx) {
       ctx->bfs_par = 0;
     }
     stream = ctx->stream;
+    ctx->bfs_inject = true;
   } else {
     int dev = 0, grid = 0;
     unsigned char *base = nullptr;

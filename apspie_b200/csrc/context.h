@@ -47,6 +47,9 @@ struct apspie_context {
   int up_next = 0;
   // test hook (apspie_debug_inject): the next workspace growth fails
   bool fail_next_alloc = false;
+  // test hook: the next BFS launch's persistent kernel runs every level, so
+  // that it meets the barrier that the hook makes run out
+  bool bfs_inject = false;
 
   // at most this many blocks per persistent launch (0: as many as fit), so
   // that two persistent kernels can share the GPU

@@ -41,6 +41,28 @@ def test_bfs_barrier_timeout_is_reported_and_the_context_recovers():
             assert ap.bfs_stats(ctx)["vertices_reached"] == int((ref >= 0).sum())
 
 
+@pytest.mark.parametrize("shape", [(40, 50), (300, 400)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_bfs_barrier_timeout_is_reported_on_a_sparse_graph(shape, mode):
+    """A grid's levels are thin, and pushing alone all of them are: the
+    hook's launch meets the barrier all the same, and the context recovers."""
+    import apspie_b200 as ap
+    from apspie_b200._native import lib
+    h = ap.gen_grid(*shape)
+    g = h.to_device()
+    ref, _ = oracle.bfs(h.m, h.ptr, h.ind, 7)
+    with ap.Context(0) as ctx:
+        ap.bfs_set_params(ctx, mode=mode)
+        assert lib.apspie_debug_inject(ctx.handle, INJECT_BFS_BARRIER) == 0
+        ap.bfs(ctx, g, 7)
+        with pytest.raises(ap.ApspieError) as e:
+            ap.bfs_stats(ctx)
+        assert e.value.status == APSPIE_ERR_TIMEOUT
+        for _ in range(3):
+            np.testing.assert_array_equal(ap.bfs(ctx, g, 7).cpu().numpy(), ref)
+            assert ap.bfs_stats(ctx)["vertices_reached"] == h.m
+
+
 def test_sort_lookback_timeout_is_reported_by_spmspv():
     import torch
     import apspie_b200 as ap

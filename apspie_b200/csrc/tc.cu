@@ -16,6 +16,12 @@
 // the products of L's rows are 660 M, and a set is built once per 256
 // entries of its end, or by a warp for itself.
 //
+// Repeated edges: with M the entries of L counted by multiplicity, the result
+// is the sum of M * M over L's distinct entries, whichever end an entry belongs
+// to.  That needs column j as the set and every entry of column k as a probe, so
+// an L with repeats (tc_scatter finds them) is counted by a second kernel whose
+// entries all belong to their column's end.
+//
 // tc_prepare relabels vertices by ascending (degree, id) with the stable
 // radix sort and lists the edges with new(col) < new(row) grouped by ascending
 // column, so that one stable sort on the row bits leaves every row of L
@@ -79,7 +85,12 @@ struct TcBins {
   unsigned n[3];  // tiny ends, warp ends, units
   unsigned grab;  // units handed out
   unsigned long long count;
+  unsigned multi;  // some entry of L repeats the one before it in its row
+  unsigned pad;
 };
+
+// An entry of a column: repeats of a row's entry are stored as ~row.
+__device__ __forceinline__ int member(int x) { return x < 0 ? ~x : x; }
 
 // Lengths of L's columns, and each entry's place in its column: the atomics
 // that count the columns give it, so the scatter needs none of its own (with a
@@ -138,10 +149,11 @@ __global__ void tc_bin(int m, const int *__restrict__ Lp, const int *__restrict_
   }
 }
 
-// L's entries into their columns, in any order within a column.
+// L's entries into their columns, in any order within a column; repeats, which
+// follow each other in a row of ascending columns, are marked.
 __global__ void __launch_bounds__(kEdgeThreads)
 tc_scatter(int m, int lnnz, const int *__restrict__ Lp, const int *__restrict__ Li,
-           const int *__restrict__ Up, const int *__restrict__ rank, int *Ui) {
+           const int *__restrict__ Up, const int *__restrict__ rank, int *Ui, TcBins *bins) {
   __shared__ __align__(16) int s_row[kEdgeTile];
   const int *erank = rank - __ldg(Lp);  // by entry
   int k0;
@@ -159,15 +171,26 @@ tc_scatter(int m, int lnnz, const int *__restrict__ Lp, const int *__restrict__ 
     const int t = (int)threadIdx.x + q * kEdgeThreads;
     at[q] = c[q] >= 0 ? __ldg(Up + c[q]) + __ldg(erank + k0 + t) : 0;
   }
+  bool repeats = false;
 #pragma unroll
-  for (int q = 0; q < kEdgeItems; ++q)
-    if (c[q] >= 0) Ui[at[q]] = s_row[threadIdx.x + q * kEdgeThreads];
+  for (int q = 0; q < kEdgeItems; ++q) {
+    const int t = (int)threadIdx.x + q * kEdgeThreads;
+    int before = __shfl_up_sync(kFull, c[q], 1);
+    if (lane_id() == 0) before = t > 0 && t < n ? __ldg(Li + k0 + t - 1) : -1;
+    if (c[q] < 0) continue;
+    const int row = s_row[t];
+    bool again = before == c[q] && t > 0 && s_row[t - 1] == row;
+    if (t == 0 && __ldg(Lp + row) < k0) again = __ldg(Li + k0 - 1) == c[q];
+    repeats |= again;
+    Ui[at[q]] = again ? ~row : row;
+  }
+  if (__any_sync(kFull, repeats) && lane_id() == 0) bins->multi = 1u;
 }
 
 // Members of the set `has` among the columns (start, len) that the lanes
 // hold, one each.  Long columns one after the other with 128 entries in
 // flight, the entries of the short ones dealt flat over the lanes.
-template <typename Has>
+template <bool kMulti, typename Has>
 __device__ __forceinline__ unsigned tc_probe(int start, int len, const int *__restrict__ Ui,
                                              Has has) {
   const int lane = lane_id();
@@ -178,7 +201,10 @@ __device__ __forceinline__ unsigned tc_probe(int start, int len, const int *__re
     for (int t = lane; t < n; t += 128) {
       int x[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) x[q] = t + 32 * q < n ? __ldg(Ui + a + t + 32 * q) : -1;
+      for (int q = 0; q < 4; ++q) {
+        x[q] = t + 32 * q < n ? __ldg(Ui + a + t + 32 * q) : -1;
+        if (kMulti && t + 32 * q < n) x[q] = member(x[q]);
+      }
 #pragma unroll
       for (int q = 0; q < 4; ++q) cnt += x[q] >= 0 && has(x[q]) ? 1u : 0u;
     }
@@ -194,6 +220,7 @@ __device__ __forceinline__ unsigned tc_probe(int start, int len, const int *__re
       const int owner = warp_owner(excl, e);
       const int at = __shfl_sync(kFull, start - excl, owner) + e;
       x[q] = e < total ? __ldg(Ui + at) : -1;
+      if (kMulti && e < total) x[q] = member(x[q]);
     }
 #pragma unroll
     for (int q = 0; q < 2; ++q) cnt += x[q] >= 0 && has(x[q]) ? 1u : 0u;
@@ -203,11 +230,14 @@ __device__ __forceinline__ unsigned tc_probe(int start, int len, const int *__re
 
 // The column that this lane's entry number c of end s reads, (0, 0) when the
 // entry belongs to its other end: row entries own columns up to d, column
-// entries only shorter ones, so that equal lengths belong to one end.
+// entries only shorter ones, so that equal lengths belong to one end.  (With
+// repeats: column entries own all columns, row entries none.)
+template <bool kMulti>
 __device__ __forceinline__ int2 tc_entry(int c, int nc, int la, int ld, int us, int d,
                                          const int *__restrict__ Li, const int *__restrict__ Ui,
                                          const int2 *__restrict__ col) {
-  if (c >= nc) return make_int2(0, 0);
+  if (c >= nc || (kMulti && c < ld)) return make_int2(0, 0);
+  if (kMulti) return __ldg(col + member(__ldg(Ui + us + (c - ld))));
   const int p = c < ld ? __ldg(Li + la + c) : __ldg(Ui + us + (c - ld));
   const int2 x = __ldg(col + p);
   return x.y <= (c < ld ? d : d - 1) ? x : make_int2(0, 0);
@@ -216,6 +246,7 @@ __device__ __forceinline__ int2 tc_entry(int c, int nc, int la, int ld, int us, 
 // A tiny end per eight lanes: its column's members one per lane, an entry per
 // lane, and each member of the entry's column compared with the end's by
 // eight shuffles.
+template <bool kMulti>
 __device__ __forceinline__ unsigned tc_tiny_ends(const int *list, const TcBins *bins,
                                                 const int *__restrict__ Lp,
                                                 const int *__restrict__ Li,
@@ -236,17 +267,21 @@ __device__ __forceinline__ unsigned tc_tiny_ends(const int *list, const TcBins *
       us = c.x;
       d = c.y;
       if (l < d) mine = __ldg(Ui + us + l);
+      if (kMulti) mine = max(mine, -1);  // the set has one of each
     }
     const int nc = ld + d;
     const int most = (int)__reduce_max_sync(kFull, (unsigned)nc);
     const int dmax = (int)__reduce_max_sync(kFull, (unsigned)d);
     for (int c0 = 0; c0 < most; c0 += 8) {
-      const int2 x = tc_entry(c0 + l, nc, la, ld, us, d, Li, Ui, col);
+      const int2 x = tc_entry<kMulti>(c0 + l, nc, la, ld, us, d, Li, Ui, col);
       const int longest = (int)__reduce_max_sync(kFull, (unsigned)x.y);
       for (int t = 0; t < longest; t += 4) {
         int j[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) j[q] = t + q < x.y ? __ldg(Ui + x.x + t + q) : -2;
+        for (int q = 0; q < 4; ++q) {
+          j[q] = t + q < x.y ? __ldg(Ui + x.x + t + q) : -2;
+          if (kMulti && t + q < x.y) j[q] = member(j[q]);
+        }
         for (int e = 0; e < dmax; ++e) {
           const int other = __shfl_sync(kFull, mine, e, 8);
 #pragma unroll
@@ -261,6 +296,7 @@ __device__ __forceinline__ unsigned tc_tiny_ends(const int *list, const TcBins *
 // A warp end per warp, its set in the warp's part of the block's table.
 static_assert(kTcWarps << kTcWarpTableBits == 1 << kTcTableBits, "the warps share the table");
 
+template <bool kMulti>
 __device__ __forceinline__ unsigned long long tc_warp_ends(const int *list_end,
                                                            const TcBins *bins, int *s_keys,
                                                            const int *__restrict__ Lp,
@@ -279,12 +315,15 @@ __device__ __forceinline__ unsigned long long tc_warp_ends(const int *list_end,
     while ((1 << bits) < 2 * c.y) ++bits;
     for (int t = lane; t < (1 << bits); t += 32) keys[t] = kNone;
     __syncwarp();
-    for (int t = lane; t < c.y; t += 32) set_insert(keys, bits, __ldg(Ui + c.x + t));
+    for (int t = lane; t < c.y; t += 32) {
+      const int j = __ldg(Ui + c.x + t);
+      if (!kMulti || j >= 0) set_insert(keys, bits, j);
+    }
     __syncwarp();
     const int nc = ld + c.y;
     for (int c0 = 0; c0 < nc; c0 += 32) {
-      const int2 x = tc_entry(c0 + lane, nc, la, ld, c.x, c.y, Li, Ui, col);
-      cnt += tc_probe(x.x, x.y, Ui, [&](int j) { return set_has(keys, bits, j); });
+      const int2 x = tc_entry<kMulti>(c0 + lane, nc, la, ld, c.x, c.y, Li, Ui, col);
+      cnt += tc_probe<kMulti>(x.x, x.y, Ui, [&](int j) { return set_has(keys, bits, j); });
     }
     __syncwarp();
   }
@@ -294,6 +333,7 @@ __device__ __forceinline__ unsigned long long tc_warp_ends(const int *list_end,
 // All ends in one launch: the units first, handed out on demand, then every
 // warp its share of the warp ends and of the tiny ends, which fill the time
 // that the last units take.
+template <bool kMulti>
 __global__ void __launch_bounds__(kTcThreads, 8)
 tc_count(const int2 *units, const int *lists, TcBins *bins, int m, const int *__restrict__ Lp,
          const int *__restrict__ Li, const int2 *__restrict__ col, const int *__restrict__ Ui) {
@@ -303,6 +343,7 @@ tc_count(const int2 *units, const int *lists, TcBins *bins, int m, const int *__
   __shared__ int s_hashed;
   const int t0 = threadIdx.x, w = warp_in_block(), lane = lane_id();
   unsigned long long cnt = 0;
+  if (!kMulti && bins->multi) return;  // left to the other kernel
   const unsigned nunits = bins->n[2];
   const int top = max(0, m - kTcTop);
   for (int t = t0; t < kTcTop / 32; t += kTcThreads) s_bits[t] = 0u;
@@ -323,6 +364,7 @@ tc_count(const int2 *units, const int *lists, TcBins *bins, int m, const int *__
       const int pe = min(d, part + kTcPart);
       for (int t = part + t0; t < pe; t += kTcThreads) {
         const int j = __ldg(Ui + us + t);
+        if (kMulti && j < 0) continue;
         if (j >= top) {
           atomicOr(s_bits + ((j - top) >> 5), 1u << ((j - top) & 31));
         } else {
@@ -333,8 +375,8 @@ tc_count(const int2 *units, const int *lists, TcBins *bins, int m, const int *__
       __syncthreads();
       const bool hashed = s_hashed != 0;
       for (int c0 = c_beg + w * 32; c0 < nc; c0 += kTcThreads) {
-        const int2 x = tc_entry(c0 + lane, nc, la, ld, us, d, Li, Ui, col);
-        cnt += tc_probe(x.x, x.y, Ui, [&](int j) -> bool {
+        const int2 x = tc_entry<kMulti>(c0 + lane, nc, la, ld, us, d, Li, Ui, col);
+        cnt += tc_probe<kMulti>(x.x, x.y, Ui, [&](int j) -> bool {
           if (j >= top) return (s_bits[(j - top) >> 5] >> ((j - top) & 31)) & 1u;
           return hashed && set_has(s_keys, kTcTableBits, j);
         });
@@ -350,8 +392,8 @@ tc_count(const int2 *units, const int *lists, TcBins *bins, int m, const int *__
       __syncthreads();
     }
   }
-  cnt += tc_warp_ends(lists + (m - 1), bins, s_keys, Lp, Li, col, Ui);
-  cnt += tc_tiny_ends(lists, bins, Lp, Li, col, Ui);
+  cnt += tc_warp_ends<kMulti>(lists + (m - 1), bins, s_keys, Lp, Li, col, Ui);
+  cnt += tc_tiny_ends<kMulti>(lists, bins, Lp, Li, col, Ui);
   cnt = warp_sum(cnt);
   if (lane == 0 && cnt) atomicAdd(&bins->count, cnt);
 }
@@ -628,16 +670,24 @@ int apspie_tc(apspie_ctx ctx, int m, int64_t lnnz, const int *d_Lptr, const int 
   rc = device_exclusive_scan<int>(ctx, Up, Up, (long long)m + 1, nullptr);
   if (rc) return rc;
   tc_bin<<<tgrid(ctx, m, 256), 256, 0, st>>>(m, d_Lptr, Up, col, lists, units, bins);
-  tc_scatter<<<edge_tiles(lnnz), kEdgeThreads, 0, st>>>(m, (int)lnnz, d_Lptr, d_Lind, Up, rank, Ui);
-  tc_count<<<ctx->num_sms * 8, kTcThreads, 0, st>>>(units, lists, bins, m, d_Lptr, d_Lind, col,
-                                                    Ui);
+  tc_scatter<<<edge_tiles(lnnz), kEdgeThreads, 0, st>>>(m, (int)lnnz, d_Lptr, d_Lind, Up, rank, Ui,
+                                                        bins);
+  tc_count<false><<<ctx->num_sms * 8, kTcThreads, 0, st>>>(units, lists, bins, m, d_Lptr, d_Lind,
+                                                           col, Ui);
   rc = check_launch(ctx, "apspie_tc", 3);
   if (rc) return rc;
   auto *h = (TcBins *)pinned(ctx, sizeof(TcBins));
   if (!h) return APSPIE_ERR_OOM;
-  cudaMemcpyAsync(h, bins, sizeof(TcBins), cudaMemcpyDeviceToHost, st);
-  rc = check_cuda(ctx, cudaStreamSynchronize(st), "apspie_tc");
-  if (rc) return rc;
+  for (int pass = 0; pass < 2; ++pass) {
+    cudaMemcpyAsync(h, bins, sizeof(TcBins), cudaMemcpyDeviceToHost, st);
+    rc = check_cuda(ctx, cudaStreamSynchronize(st), "apspie_tc");
+    if (rc) return rc;
+    if (!h->multi || pass == 1) break;
+    tc_count<true><<<ctx->num_sms * 8, kTcThreads, 0, st>>>(units, lists, bins, m, d_Lptr, d_Lind,
+                                                            col, Ui);
+    rc = check_launch(ctx, "apspie_tc");
+    if (rc) return rc;
+  }
   *h_count = (int64_t)h->count;
   return APSPIE_OK;
 }

@@ -623,7 +623,9 @@ int apspie_tc_prepare(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr,
                       const int *d_ind, int *d_perm, int *d_Lptr, int *d_Lind,
                       int64_t *h_lnnz);
 /* Triangles = sum over (i, k) in L of |L(i,:) n L(k,:)|, as the masked
- * product (L * L) .* L, counted in int64.  Replaces cuSPARSE U * L
+ * product (L * L) .* L, counted in int64.  Entries of L that repeat (columns
+ * ascending in each row, as tc_prepare leaves the L of a multigraph) count
+ * once in the mask and each time in the product.  Replaces cuSPARSE U * L
  * (src/tc.cuh:63-165) + ewiseMultTc (src/tc.cuh:169-199) + the float
  * reduction of test/tc/main.cu:249.  Synchronises. */
 int apspie_tc(apspie_ctx ctx, int m, int64_t lnnz, const int *d_Lptr,

@@ -147,3 +147,40 @@ def test_empty_rows_are_not_one_blocks_work(ctx, op):
         call = lambda: ap.spmspv(ctx, 1, g, every)
         assert call()[0].tolist() == np.unique(ind).tolist()
     assert _fastest_ms(call) < 2.0
+
+
+def _symmetric(m, pairs):
+    """CSR of the undirected multigraph of the given pairs."""
+    r = np.concatenate([pairs[:, 0], pairs[:, 1]])
+    c = np.concatenate([pairs[:, 1], pairs[:, 0]])
+    order = np.lexsort((c, r))
+    return np.searchsorted(r[order], np.arange(m + 1)).astype(np.int32), c[order].astype(np.int32)
+
+
+@pytest.mark.parametrize("kind", ["tiny", "warp", "units", "parts"])
+@pytest.mark.parametrize("repeats", [0, 1, 500])
+def test_triangles_of_a_multigraph(ctx, kind, repeats):
+    """Repeated edges count once in the mask and each time in the product,
+    whatever the column lengths: columns of a quarter warp, a warp, a block and
+    a block in parts."""
+    import scipy.sparse as sp
+    import apspie_b200 as ap
+    from apspie_b200.graph import DeviceGraph
+    rng = np.random.default_rng(repeats)
+    m, clique = {"tiny": (400, 8), "warp": (400, 60), "units": (500, 300),
+                 "parts": (1500, 1300)}[kind]
+    a, b = np.triu_indices(clique, 1)
+    pairs = np.concatenate([np.stack([a, b], 1), rng.integers(0, m, (3 * m, 2))])
+    pairs = np.unique(np.sort(pairs, axis=1), axis=0)
+    pairs = pairs[pairs[:, 0] != pairs[:, 1]]
+    # some edges two or three times, those of the clique among them
+    pairs = np.concatenate([pairs, pairs[rng.integers(0, len(pairs), repeats)], pairs[:repeats]])
+    ptr, ind = _symmetric(m, pairs)
+    g = DeviceGraph(m, len(ind), _t(ptr), _t(ind), symmetric=True)
+    _, lp, li = ap.tc_prepare(ctx, g)
+    hl, hi = lp.cpu().numpy(), li.cpu().numpy()
+    M = sp.csr_matrix((np.ones(len(hi)), hi, hl), shape=(m, m))   # repeats are summed in products
+    M.sum_duplicates()
+    want = int(round((M @ M).multiply(M > 0).sum()))
+    for _ in range(2):
+        assert ap.triangle_count(ctx, m, lp, li) == want

@@ -157,10 +157,7 @@ enum SlotId : int {
   kSlotSsspNearFar,
   kSlotSsspHubs,
   kSlotSsspHubWord,
-  kSlotMisState,
-  kSlotMisQueueA,
-  kSlotMisQueueB,
-  kSlotMisWord,  // key while undecided, then the decision
+  kSlotMis,  // state, a word per vertex, two queues
   kSlotSortKeysA,
   kSlotSortKeysB,
   kSlotSortValsA,
@@ -238,6 +235,9 @@ namespace apspie {
 uint64_t graph_fingerprint(apspie_context *ctx, int m, int64_t nnz, const int *d_ptr);
 // d_out[i] = d_ptr[m * i / 64] for i = 0..64 (one small launch)
 int gather_offsets(apspie_context *ctx, const int *d_ptr, int m, int *d_out);
+
+// Workspace that an MIS of m vertices takes (mis.cu).
+size_t mis_scratch_bytes(size_t m);
 
 // The launches of a BFS, or part of them (bfs.cu).
 enum class BfsPart { kAll, kFirst, kMain };

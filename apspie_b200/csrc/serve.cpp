@@ -63,6 +63,7 @@
 #include <vector>
 
 #include "apspie.h"
+#include "context.h"
 
 namespace {
 
@@ -208,8 +209,8 @@ size_t request_bytes(const apspie_server *s, int type, int graph) {
       return 4 * m + (32 * m + 12 * m + 256 * m) / 64 + 64;
     case 1:  // SSSP: distances, stamps and two queue rows per source
       return 16 * m + 64;
-    default:  // MIS: result + priorities + two queues and a word of 8 bytes each
-      return 4 * m + 4 * m + 16 * m + 8 * m + 64;
+    default:  // MIS: result + priorities + the call's workspace
+      return 4 * m + 4 * m + apspie::mis_scratch_bytes(m);
   }
 }
 

@@ -126,3 +126,37 @@ def test_mis_scan_lengths(ctx, leaves, delta):
         np.testing.assert_array_equal(got, oracle.mis(h.m, h.ptr, h.ind, p))
     got, _, _ = _run(ctx, h, np.zeros(h.m, np.uint32), delta)
     np.testing.assert_array_equal(got, oracle.mis(h.m, h.ptr, h.ind, np.zeros(h.m, np.uint32)))
+
+
+def test_mis_first_call_allocates_once():
+    """A context's first call grows its workspace in one piece: it takes a
+    warm call and about one allocation of that size (three or four pieces:
+    three or four times as long)."""
+    import ctypes as C
+    import glob
+    import time
+    import nvidia.cuda_runtime
+    import torch
+    import apspie_b200 as ap
+    rt = C.CDLL(glob.glob(list(nvidia.cuda_runtime.__path__)[0] + "/lib/libcudart.so*")[0])
+    h = ap.gen_er(1 << 20, 8, seed=1)
+    g = h.to_device()
+    prio = torch.from_numpy(ap.mt19937(1, h.m).view(np.int32)).cuda()
+
+    def clock(call):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        call()
+        torch.cuda.synchronize()
+        return time.perf_counter() - t
+
+    first, warm, alloc = [], [], []
+    for _ in range(8):
+        with ap.Context(0) as own:
+            first.append(clock(lambda: ap.mis(own, g, prio)))
+            warm.append(clock(lambda: ap.mis(own, g, prio)))
+            size = own.workspace_bytes
+        p = C.c_void_p()
+        alloc.append(clock(lambda: rt.cudaMalloc(C.byref(p), C.c_size_t(size))))
+        rt.cudaFree(p)
+    assert min(first) < min(warm) + 2.5 * min(alloc), (first, warm, alloc)

@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(kSeedThreads) batch_seed(BatchJob *jobs) {
     s_nch[s] = nch;
     if (mine && !big) j->q0[(unsigned)off] = v;
   }
-  if (s < 3) j->c[s] = s == 0 ? JobCounters{qc, (unsigned)nbig, 0, edges} : JobCounters{0ull, 0, 0, 0ull};
+  if (s < 3)
+    j->c[s] = s == 0 ? JobCounters{qc, (unsigned)nbig, 0, edges} : JobCounters{0ull, 0, 0, 0ull};
   __syncthreads();
   for (int t = 0; t < nsrc; ++t)
     for (unsigned c = threadIdx.x; c < s_nch[t]; c += kSeedThreads)

@@ -12,8 +12,9 @@
 //     > kBigDeg are split into kChunk-edge chunks shared by all warps.
 //     Discovery is an atomicCAS on depth (the visited mask update fused into
 //     the SpMSpV, replacing addResult, src/bfs.cuh:16-24).
-//   pull (bottom-up): every unvisited vertex scans its neighbours, one warp
-//     per vertex, until one has depth L (ballot early exit).
+//   pull (bottom-up): every unvisited vertex probes its in-neighbours until one
+//     has depth L; a warp takes 32 vertices, a lane each while most of them are
+//     unresolved, then all lanes share those that are left.
 // The switch follows Beamer's rule: push->pull when the frontier's edges
 // exceed (unexplored edges)/alpha, pull->push when the frontier has fewer
 // than m/beta vertices.  Discovered vertices are appended to the next queue

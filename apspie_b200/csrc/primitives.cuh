@@ -583,13 +583,11 @@ radix_small(const K *keys_in, const V *vals_in, K *keys_out, V *vals_out, int n,
 // waited kLookbackSpinLimit polls for a predecessor (the output is then in
 // bounds but neither sorted nor a permutation of the input: some slots keep
 // stale contents).  A caller that uses sorted keys or values as indices must
-// therefore check it (radix_sort_check) before doing so; apspie_spmspv,
-// which only bounds-checks its segment writes, checks it at its end.  Sticky: zeroed when first allocated and by
-// radix_sort_check, not by each sort, so a caller that synchronises only
-// at its end still sees a give-up of any sort it ran.  Stream-ordered
-// callers that never synchronise (apspie_bfs_prepare, apspie_csr_transpose)
-// leave it to the next call on the context that reads it back (the device
-// graph build, apspie_tc_prepare, apspie_spmspv).
+// therefore check it (radix_sort_check) before doing so, or bounds-check what
+// it indexes and check the word at its end (apspie_spmspv, apspie_mxv_dense,
+// apspie_csr_transpose, which all wait for the device there).  Sticky: zeroed
+// when first allocated and by the check, not by each sort, so a caller sees a
+// give-up of any sort it ran.
 // kSortErrWords words (give-up, test hook, two unused); the rest of the slot's
 // kSortErrBytes is a caller's that wants to read them back with its own.
 constexpr int kSortErrWords = 4;

@@ -14,7 +14,7 @@
 //      table); <= 1024 / <= 4096 one block per row on a 2048 / 8192-key
 //      shared table (spgemm_mid_rows); longer rows over a shared-memory
 //      bitmap of C's columns when B has at most bitmap_max_cols columns
-//      (spgemm_bitmap_rows<0>), else a 16384-key table (<= 8192 products) or
+//      (spgemm_bitmap_symbolic), else a 16384-key table (<= 8192 products) or
 //      a dense accumulator in global memory; the distinct columns per row
 //      give nnz(C(i,:)), a scan gives C's row offsets;
 //   2. numeric rows of up to 4096 products that are not mostly repeats are
@@ -244,33 +244,27 @@ __device__ __forceinline__ int row_at(const int *list, int m, unsigned nfront, u
   return r < nfront ? list[r] : list[(unsigned)m - 1u - (r - nfront)];
 }
 
-// Deals the products of row i over `nthreads` threads of a group (a warp or
-// a block): f(j, value) is called once per product.  Group-level scan-based
-// gather over the row's A entries, up to `width` A entries per step.  RUNS
-// (blocks only): each thread takes runs of consecutive products (one owner
-// search per run; measured faster for the symbolic passes), otherwise the
-// threads stride the products (coalesced loads of B; measured faster for
-// the numeric passes, which load two arrays of B per product).
-template <bool WARP, bool RUNS = false, typename F>
-__device__ __forceinline__ void for_each_product(int i, const int *__restrict__ Aptr,
-                                                 const int *__restrict__ Aind,
-                                                 const float *__restrict__ Aval,
-                                                 const int *__restrict__ Bptr,
-                                                 const int *__restrict__ Bind,
-                                                 const float *__restrict__ Bval, int *s_off,
-                                                 int *s_bs, float *s_av, F f) {
+// Calls f(j) with the column of every product of row i, dealt over the threads
+// of a group (a warp or a block): the lengths of B's rows are scanned, `width`
+// A entries per step, and each thread finds its products' owners.  A block's
+// threads take runs of consecutive products (one owner search per run), a
+// warp's lanes stride them.
+template <bool WARP, typename F>
+__device__ __forceinline__ void for_each_column(int i, const int *__restrict__ Aptr,
+                                                const int *__restrict__ Aind,
+                                                const int *__restrict__ Bptr,
+                                                const int *__restrict__ Bind, int *s_off,
+                                                int *s_bs, F f) {
   const int a0 = __ldg(Aptr + i), a1 = __ldg(Aptr + i + 1);
   const int width = WARP ? 32 : (int)blockDim.x;
   const int tid = WARP ? lane_id() : (int)threadIdx.x;
   for (int c0 = a0; c0 < a1; c0 += width) {
     int a = c0 + tid;
     int bs = 0, d = 0;
-    float av = 0.f;
     if (a < a1) {
       int k = __ldg(Aind + a);
       bs = __ldg(Bptr + k);
       d = __ldg(Bptr + k + 1) - bs;
-      av = Aval ? __ldg(Aval + a) : 1.0f;
     }
     int excl, total;
     if (WARP) {
@@ -283,10 +277,9 @@ __device__ __forceinline__ void for_each_product(int i, const int *__restrict__ 
     }
     s_off[tid] = excl;
     s_bs[tid] = bs;
-    s_av[tid] = av;
     if (WARP) __syncwarp(); else __syncthreads();
     const int n_a = min(width, a1 - c0);
-    if (!WARP && RUNS) {
+    if (!WARP) {
       // block: each thread takes runs of vt consecutive products (vt grows
       // with the chunk's products, up to 8): one binary search for a run's
       // first owner (the largest t with s_off[t] <= p), then a linear walk
@@ -302,38 +295,31 @@ __device__ __forceinline__ void for_each_product(int i, const int *__restrict__ 
         // the run's product positions first, then all its loads, then the
         // calls: up to 8 independent loads in flight per thread
         int pos[8];
-        float av[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int p = p0 + q;
           pos[q] = -1;
-          av[q] = 0.f;
           if (p < pend) {
             while (p >= nxt) {
               ++lo;
               nxt = lo + 1 < n_a ? s_off[lo + 1] : INT_MAX;
             }
             pos[q] = s_bs[lo] + (p - s_off[lo]);
-            av[q] = s_av[lo];
           }
         }
         int jb[8];
-        float bv[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          jb[q] = pos[q] >= 0 ? __ldg(Bind + pos[q]) : -1;
-          bv[q] = (pos[q] >= 0 && Bval) ? __ldg(Bval + pos[q]) : 1.0f;
-        }
+        for (int q = 0; q < 8; ++q) jb[q] = pos[q] >= 0 ? __ldg(Bind + pos[q]) : -1;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
-          if (jb[q] >= 0) f(jb[q], (double)av[q] * (double)bv[q]);
+          if (jb[q] >= 0) f(jb[q]);
       }
       __syncthreads();
       continue;
     }
-    // strided: owner of product p, the largest t < n_a with s_off[t] <= p.
-    // A thread's p grows by `width` per step, so its owner only moves
-    // forward: gallop from the previous one
+    // warp: owner of product p, the largest t < n_a with s_off[t] <= p.
+    // A lane's p grows by 32 per step, so its owner only moves forward:
+    // gallop from the previous one
     int lo = 0;
     for (int p = tid; p < total; p += width) {
       if (lo + 1 < n_a && s_off[lo + 1] <= p) {
@@ -349,10 +335,9 @@ __device__ __forceinline__ void for_each_product(int i, const int *__restrict__ 
         }
         lo = l2;
       }
-      int b = s_bs[lo] + (p - s_off[lo]);
-      f(__ldg(Bind + b), (double)s_av[lo] * (double)(Bval ? __ldg(Bval + b) : 1.0f));
+      f(__ldg(Bind + s_bs[lo] + (p - s_off[lo])));
     }
-    if (WARP) __syncwarp(); else __syncthreads();
+    __syncwarp();
   }
 }
 
@@ -387,11 +372,11 @@ __device__ __forceinline__ int block_excl_max(int v, int *sw) {
   return res;
 }
 
-// Block version of for_each_product by load-balanced search: the chunk's
-// products are taken in windows of 2 * TPB; each A entry marks the window
+// Products with their values by load-balanced search: the products of up to
+// TPB A entries are taken in windows of PER * TPB; each A entry marks the window
 // position of its first product with its index (the entry running into the
 // window marks position 0), an inclusive max-scan turns the marks into the
-// owner of every position, and thread t handles positions t and t + TPB --
+// owner of every position, and thread t handles positions t, t + TPB, ... --
 // one shared-memory read for the owner, and the loads of B's rows coalesced.
 // f(j, value, q, h) handles product q of the row as its thread's h-th of the
 // window; g(h) is called for every h after the block barrier that ends the
@@ -513,7 +498,6 @@ spgemm_warp_rows(const int *list, const unsigned *nlist, const long long *prod,
                  const int *__restrict__ Bptr, const int *__restrict__ Bind, int *cnt, int load) {
   __shared__ int s_keys[kWarpsPerBlockSmall][kWarpTable];
   __shared__ int s_off[kWarpsPerBlockSmall][32], s_bs[kWarpsPerBlockSmall][32];
-  __shared__ float s_av[kWarpsPerBlockSmall][32];
   const int w = warp_in_block(), lane = lane_id();
   int *keys = s_keys[w];
   const unsigned nrows = *nlist;
@@ -525,12 +509,11 @@ spgemm_warp_rows(const int *list, const unsigned *nlist, const long long *prod,
     for (int t = lane; t < T; t += 32) keys[t] = kEmpty;
     __syncwarp();
     int fresh_count = 0;
-    for_each_product<true>(i, Aptr, Aind, nullptr, Bptr, Bind, nullptr, s_off[w], s_bs[w], s_av[w],
-                           [&](int j, double) {
-                             bool fresh;
-                             table_insert(keys, bits, j, &fresh);
-                             fresh_count += fresh;
-                           });
+    for_each_column<true>(i, Aptr, Aind, Bptr, Bind, s_off[w], s_bs[w], [&](int j) {
+      bool fresh;
+      table_insert(keys, bits, j, &fresh);
+      fresh_count += fresh;
+    });
     __syncwarp();
     const int c = warp_sum(fresh_count);
     if (lane == 0) cnt[i] = c;
@@ -1143,7 +1126,6 @@ spgemm_bitmap_symbolic(const int *list, const unsigned *nlist, const unsigned *n
   extern __shared__ __align__(16) unsigned char dyn[];
   unsigned *bits = (unsigned *)dyn;
   __shared__ int s_off[TPB], s_bs[TPB];
-  __shared__ float s_av[TPB];
   __shared__ int s_wt[TPB / 32];
   const int tid = threadIdx.x, lane = lane_id(), wi = warp_in_block();
   for (int t = tid; t < W; t += TPB) bits[t] = 0u;
@@ -1156,11 +1138,10 @@ spgemm_bitmap_symbolic(const int *list, const unsigned *nlist, const unsigned *n
     const int i = row_at(list, m, nfront, r);
     // bits only: runs of consecutive products per thread measured faster
     // here than the load-balanced search (one array of B per product)
-    for_each_product<false, true>(i, Aptr, Aind, nullptr, Bptr, Bind, nullptr, s_off, s_bs, s_av,
-                                  [&](int j, double) {
-                                    const unsigned bit = 1u << (j & 31);
-                                    if (!(bits[j >> 5] & bit)) atomicOr(bits + (j >> 5), bit);
-                                  });
+    for_each_column<false>(i, Aptr, Aind, Bptr, Bind, s_off, s_bs, [&](int j) {
+      const unsigned bit = 1u << (j & 31);
+      if (!(bits[j >> 5] & bit)) atomicOr(bits + (j >> 5), bit);
+    });
     __syncthreads();
     int c = 0;
     unsigned *dst = gbm ? gbm + (size_t)r * W : nullptr;
@@ -1219,11 +1200,10 @@ spgemm_bitmap_rows(const int *list, const unsigned *nlist, const unsigned *ntail
     for (int w = tid; w < claim_words; w += TPB) claim[w] = 0u;
     __syncthreads();
     if (!src) {
-      for_each_product<false, true>(i, Aptr, Aind, nullptr, Bptr, Bind, nullptr, s_off, s_bs,
-                                    s_av, [&](int j, double) {
-                                      const unsigned bit = 1u << (j & 31);
-                                      if (!(bits[j >> 5] & bit)) atomicOr(bits + (j >> 5), bit);
-                                    });
+      for_each_column<false>(i, Aptr, Aind, Bptr, Bind, s_off, s_bs, [&](int j) {
+        const unsigned bit = 1u << (j & 31);
+        if (!(bits[j >> 5] & bit)) atomicOr(bits + (j >> 5), bit);
+      });
       __syncthreads();
     }
     int carry = 0;
@@ -1435,26 +1415,27 @@ int apspie_spgemm_symbolic(apspie_ctx ctx, const apspie_csr *A, const apspie_csr
   if (hb.n[kBinMid1]) {
     spgemm_mid_rows<false, 128, 11><<<gridsz(ctx, hb.n[kBinMid1], 1, 16), 128,
                                       mid_smem<128, 11, false>(), st>>>(
-        L(kBinMid1), nb + kBinMid1, grab + kBinMid1, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
-        nullptr, cnt, nullptr, nullptr, nullptr, n, load);
+        L(kBinMid1), nb + kBinMid1, grab + kBinMid1, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr,
+        B->d_ind, nullptr, cnt, nullptr, nullptr, nullptr, n, load);
     ++launches;
   }
   if (hb.n[kBinMid2]) {
     spgemm_mid_rows<false, 256, 13><<<gridsz(ctx, hb.n[kBinMid2], 1, 6), 256,
                                       mid_smem<256, 13, false>(), st>>>(
-        L(kBinMid2), nb + kBinMid2, grab + kBinMid2, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
-        nullptr, cnt, nullptr, nullptr, nullptr, n, load);
+        L(kBinMid2), nb + kBinMid2, grab + kBinMid2, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr,
+        B->d_ind, nullptr, cnt, nullptr, nullptr, nullptr, n, load);
     ++launches;
   }
   if (nblock && bitmap) {
     spgemm_bitmap_symbolic<<<gridsz(ctx, nblock, 1, 4), kSpgThreads, (size_t)4 * bwords,
                              st>>>(L(kBinBlock), nb + kBinBlock, nb + kTailBlock, grab + kBinBlock,
-                                   m, bwords, A->d_ptr, A->d_ind, B->d_ptr, B->d_ind, cnt, gbm, bslot);
+                                   m, bwords, A->d_ptr, A->d_ind, B->d_ptr, B->d_ind, cnt, gbm,
+                                   bslot);
     ++launches;
   } else if (nblock) {
     spgemm_block_rows<false><<<gridsz(ctx, nblock, 1, 4), kSpgThreads, dyn_sym, st>>>(
-        L(kBinBlock), nb + kBinBlock, grab + kBinBlock, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr, B->d_ind,
-        nullptr, cnt, nullptr, nullptr, nullptr, n, load);
+        L(kBinBlock), nb + kBinBlock, grab + kBinBlock, prod, A->d_ptr, A->d_ind, nullptr, B->d_ptr,
+        B->d_ind, nullptr, cnt, nullptr, nullptr, nullptr, n, load);
     ++launches;
   }
   if (nd) {
@@ -1579,8 +1560,8 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
     constexpr int TPB = decltype(tpb)::value;
     if (!hn[bin]) return;
     spgemm_sort_rows<TPB><<<gridsz(ctx, hn[bin], 1, per_sm), TPB, sort_smem<TPB>(), st>>>(
-        L(bin), nb + bin, grab + bin, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind, B->d_val, Cptr,
-        Cind, Cval);
+        L(bin), nb + bin, grab + bin, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
+        B->d_val, Cptr, Cind, Cval);
     ++launches;
   };
   sort_rows(std::integral_constant<int, 512>{}, kBinS3, 4);
@@ -1589,22 +1570,22 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
   if (hn[kBinN1]) {
     spgemm_mid_rows<true, 128, 10><<<gridsz(ctx, hn[kBinN1], 1, 12), 128,
                                      mid_smem<128, 10, true>(), st>>>(
-        L(kBinN1), nb + kBinN1, grab + kBinN1, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
-        B->d_val, cnt, Cptr, Cind, Cval, n, load);
+        L(kBinN1), nb + kBinN1, grab + kBinN1, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr,
+        B->d_ind, B->d_val, cnt, Cptr, Cind, Cval, n, load);
     ++launches;
   }
   if (hn[kBinN2]) {
     spgemm_mid_rows<true, 128, 11><<<gridsz(ctx, hn[kBinN2], 1, 6), 128,
                                      mid_smem<128, 11, true>(), st>>>(
-        L(kBinN2), nb + kBinN2, grab + kBinN2, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
-        B->d_val, cnt, Cptr, Cind, Cval, n, load);
+        L(kBinN2), nb + kBinN2, grab + kBinN2, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr,
+        B->d_ind, B->d_val, cnt, Cptr, Cind, Cval, n, load);
     ++launches;
   }
   if (hn[kBinN3]) {
     spgemm_mid_rows<true, 256, 12><<<gridsz(ctx, hn[kBinN3], 1, 3), 256,
                                      mid_smem<256, 12, true>(), st>>>(
-        L(kBinN3), nb + kBinN3, grab + kBinN3, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
-        B->d_val, cnt, Cptr, Cind, Cval, n, load);
+        L(kBinN3), nb + kBinN3, grab + kBinN3, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr,
+        B->d_ind, B->d_val, cnt, Cptr, Cind, Cval, n, load);
     ++launches;
   }
   const unsigned n4 = hn[kBinN4] + hn[kTailN4];
@@ -1621,14 +1602,14 @@ int apspie_spgemm_numeric(apspie_ctx ctx, const apspie_csr *A, const apspie_csr 
     }
     if (!scratch) return APSPIE_ERR_OOM;
     spgemm_bitmap_rows<<<g4, kSpgThreads, (size_t)8 * bwords + 4 * (size_t)claim, st>>>(
-        L(kBinN4), nb + kBinN4, nb + kTailN4, grab + kBinN4, m, bwords, claim, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
-        B->d_val, Cptr, Cind, Cval, (const unsigned *)ctx->spgemm_plan_gbm,
+        L(kBinN4), nb + kBinN4, nb + kTailN4, grab + kBinN4, m, bwords, claim, A->d_ptr, A->d_ind,
+        A->d_val, B->d_ptr, B->d_ind, B->d_val, Cptr, Cind, Cval, (const unsigned *)ctx->spgemm_plan_gbm,
         (const int *)ctx->spgemm_plan_bslot, scratch);
     ++launches;
   } else if (n4) {
     spgemm_block_rows<true><<<gridsz(ctx, n4, 1, 1), kSpgThreads, dyn_num, st>>>(
-        L(kBinN4), nb + kBinN4, grab + kBinN4, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr, B->d_ind,
-        B->d_val, cnt, Cptr, Cind, Cval, n, load);
+        L(kBinN4), nb + kBinN4, grab + kBinN4, prod, A->d_ptr, A->d_ind, A->d_val, B->d_ptr,
+        B->d_ind, B->d_val, cnt, Cptr, Cind, Cval, n, load);
     ++launches;
   }
   if (nd) {

@@ -419,8 +419,9 @@ sssp_persistent(int m, const int *__restrict__ ptr, const int *__restrict__ ind,
     int *qin = (r & 1) ? qb : qa;
     int2 *cin = (r & 1) ? cb : ca;
     int *fout = phase % 3 == 0 ? far0 : (phase % 3 == 1 ? far1 : far2);
-    SsspVisit<W, KIND == kNearFar> vis{w,    dist,   stamp, fstamp, r, phase, thresh, fout, &st->far_count[phase % 3],
-                     &st->far_min[phase % 3]};
+    SsspVisit<W, KIND == kNearFar> vis{w,     dist,   stamp, fstamp,
+                                       r,     phase,  thresh, fout,
+                                       &st->far_count[phase % 3], &st->far_min[phase % 3]};
     // A queued vertex whose distance still equals the one it was last
     // expanded with (it improved again in the round that expanded it, so it
     // was queued once more) has nothing new to relax: skipped.  A hub's

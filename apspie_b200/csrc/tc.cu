@@ -119,8 +119,9 @@ tc_col_ranks(int m, int lnnz, const int *__restrict__ Lp, const int *__restrict_
   }
 }
 
-// Every vertex's column as (start, length), and its place among the tiny ends (lists from the front), the warp ends (lists from
-// the back) or its units (vertex, piece).
+// Every vertex's column as (start, length), and its place among the tiny ends
+// (lists from the front), the warp ends (lists from the back) or its units
+// (vertex, piece).
 __global__ void tc_bin(int m, const int *__restrict__ Lp, const int *__restrict__ Up,
                        int2 *col, int *lists, int2 *units, TcBins *bins) {
   const int lane = lane_id();
@@ -583,7 +584,8 @@ int apspie_tc_prepare(apspie_ctx ctx, int64_t nnz, int m, const int *d_ptr, cons
   // small[0]: the largest degree; small + 8 bytes .. + 24: the two edge hashes
   auto *hsum = reinterpret_cast<unsigned long long *>(small) + 1;
   if (nnz > 0) {
-    split_counts<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, d_ptr, d_ind, d_perm, lcnt, uoff, hsum);
+    split_counts<<<edge_tiles(nnz), kEdgeThreads, 0, st>>>(m, d_ptr, d_ind, d_perm, lcnt, uoff,
+                                                           hsum);
     rc = check_launch(ctx, "split_counts");
     if (rc) return rc;
   }

@@ -53,7 +53,8 @@ int apspie_ctx_set_stream(apspie_ctx ctx, void *stream);
 /* Caps the blocks of this context's persistent launches (BFS, SSSP, MIS,
  * batch); 0 = as many as fit (the default).  Two contexts whose caps add up
  * to at most apspie_ctx_resident_blocks can run persistent kernels at the
- * same time on different streams. */
+ * same time on different streams.  (The thin levels of a sparse graph's BFS run
+ * in a launch of their own, one cluster of 8 blocks under any cap.) */
 int apspie_ctx_set_max_grid(apspie_ctx ctx, int blocks);
 /* A cap that every persistent kernel of the library fits (2 per SM). */
 int apspie_ctx_resident_blocks(apspie_ctx ctx, int *blocks);

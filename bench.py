@@ -215,7 +215,12 @@ def run_reference(args):
         return
     import oracle
     import oracle.inputs as oi
-    kind = "reference" if oracle.have_reference() else "port"
+    if not oracle.have_reference():
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "oracle/_ref (the reference's CPU code, compiled) is not "
+                                         "here and its sources are not at hand to build it"}),
+              flush=True)
+        return
     m, ptr, ind = oi.gen_rmat(args.scale, EDGE_FACTOR, seed=SEED, symmetric=True)
     threads = os.cpu_count() or 1
     K, W = max(args.steps, 1), max(args.warmup, 0)
@@ -252,7 +257,7 @@ def run_reference(args):
         "ms_per_step": 1e3 * wall / K, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "int32", "data": "synthetic",
         "config": shared_config(args.scale, m, len(ind), world),
-        "cpu_baseline": {"value": gteps, "unit": "GTEPS", "cores": threads, "kind": kind,
+        "cpu_baseline": {"value": gteps, "unit": "GTEPS", "cores": threads, "kind": "reference",
                          "sample": f"{K} steps of {threads} concurrent single-threaded "
                                    f"SimpleReferenceBfs (src/testBfs.cpp:7-72, -O3) traversals "
                                    f"of R-MAT {args.scale}, one source each ({K * threads} "

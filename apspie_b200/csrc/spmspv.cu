@@ -63,8 +63,15 @@ struct SpmspvSmall {  // device-side scalars of one call
 constexpr int kBitmapRows = 1 << 22;
 constexpr double kDenseGuess = 1.25;
 
-__host__ __device__ __forceinline__ bool spmspv_dense(long long E, double factor, int m) {
-  return (double)E * factor > (double)m;
+bool spmspv_dense(long long E, double factor, int m) { return (double)E * factor > (double)m; }
+
+// The least E that the rule calls dense, an integer for the kernels to compare
+// with (the rule's doubles cost the expansion 1.5 us).
+long long dense_from(double factor, int m) {
+  long long E = (long long)std::min((double)m / factor, 4e18);
+  while (E > 0 && spmspv_dense(E - 1, factor, m)) --E;
+  while (E < (long long)INT_MAX && !spmspv_dense(E, factor, m)) ++E;
+  return E;
 }
 
 __device__ __forceinline__ float sr_term(int sr, float a, float x) {
@@ -128,16 +135,17 @@ __global__ void frontier_columns(int xnnz, const int *__restrict__ xind,
 // Calls f(e[], row[], term[], on[]) for the entries e of the frontier's columns
 // laid end to end (offs: their exclusive scan, offs[xnnz] = *total), each
 // thread's kEdgeItems of a tile in flight together.  Blocks stride the tiles.
-// Nothing is done when the total does not fit an int (the caller reports it).
+// Nothing is done when the total does not fit an int (the caller reports it) or
+// is below `least`.
 template <typename F>
 __device__ __forceinline__ void for_each_entry(int sr, int xnnz, const long long *__restrict__ offs,
-                                               const long long *total,
+                                               const long long *total, long long least,
                                                const int2 *__restrict__ col,
                                                const int *__restrict__ ind,
                                                const float *__restrict__ val, F f) {
   __shared__ __align__(16) int s_row[kEdgeTile];
   const long long E = __ldcg(total);
-  if (E >= (long long)INT_MAX) return;
+  if (E >= (long long)INT_MAX || E < least) return;
   const unsigned tiles = (unsigned)((E + kEdgeTile - 1) / kEdgeTile);
   for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int k0 = (int)(tile * kEdgeTile);
@@ -173,7 +181,7 @@ __global__ void __launch_bounds__(kEdgeThreads)
 expand_pairs(int sr, int xnnz, const long long *__restrict__ offs, const long long *total,
              const int2 *__restrict__ col, const int *__restrict__ ind,
              const float *__restrict__ val, int *keys, float *vals) {
-  for_each_entry(sr, xnnz, offs, total, col, ind, val,
+  for_each_entry(sr, xnnz, offs, total, 0, col, ind, val,
                  [&](const int (&e)[kEdgeItems], const int (&row)[kEdgeItems],
                      const float (&term)[kEdgeItems], const bool (&on)[kEdgeItems]) {
 #pragma unroll
@@ -221,12 +229,10 @@ __global__ void reduce_segments(int sr, const int *keys, const float *vals, long
 
 // ---- bitmap path ----
 __global__ void __launch_bounds__(kEdgeThreads)
-expand_accumulate(int sr, int m, double factor, int xnnz, const long long *__restrict__ offs,
+expand_accumulate(int sr, long long least, int xnnz, const long long *__restrict__ offs,
                   const long long *total, const int2 *__restrict__ col,
                   const int *__restrict__ ind, const float *__restrict__ val, void *acc) {
-  // a sparse PLUS_TIMES frontier is sorted: no row is touched here
-  if (sr == kPlusTimes && !spmspv_dense(__ldcg(total), factor, m)) return;
-  for_each_entry(sr, xnnz, offs, total, col, ind, val,
+  for_each_entry(sr, xnnz, offs, total, least, col, ind, val,
                  [&](const int (&)[kEdgeItems], const int (&row)[kEdgeItems],
                      const float (&term)[kEdgeItems], const bool (&on)[kEdgeItems]) {
 #pragma unroll
@@ -498,8 +504,10 @@ int spmspv_run(apspie_context *ctx, const char *what, int sr, int m, int64_t nnz
       rc = check_launch(ctx, "acc_init");
       if (rc) return rc;
     }
-    expand_accumulate<<<expand_grid(ctx), kEdgeThreads, 0, st>>>(sr, m, factor, xnnz, offs,
-                                                                 &sm->total, col, ind, val, acc);
+    // a sparse PLUS_TIMES frontier is sorted: no row is touched here
+    const long long least = sr == kPlusTimes ? dense_from(factor, m) : 0;
+    expand_accumulate<<<expand_grid(ctx), kEdgeThreads, 0, st>>>(sr, least, xnnz, offs, &sm->total,
+                                                                 col, ind, val, acc);
     const int per_block = std::max(kEmitWords, (words + kEmitBlocks - 1) / kEmitBlocks);
     const int eblocks = (words + per_block - 1) / per_block;
     touched_rows<<<eblocks, kEmitThreads, 0, st>>>(sr, m, acc, words, per_block, bits, sums);

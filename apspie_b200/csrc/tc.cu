@@ -645,12 +645,21 @@ int apspie_tc(apspie_ctx ctx, int m, int64_t lnnz, const int *d_Lptr, const int 
   APSPIE_CHECK_CTX(ctx);
   if (m <= 0 || lnnz < 0 || !d_Lptr || (lnnz > 0 && !d_Lind) || !h_count)
     return set_error(ctx, APSPIE_ERR_INVALID, "apspie_tc: bad arguments");
-  if (lnnz >= (int64_t)INT32_MAX)
-    return set_error(ctx, APSPIE_ERR_OVERFLOW, "apspie_tc: nnz(L) %lld exceeds int32 offsets",
-                     (long long)lnnz);
   *h_count = 0;
   if (lnnz == 0) return APSPIE_OK;
   cudaStream_t st = ctx->stream;
+  if (lnnz >= (int64_t)INT32_MAX) {
+    // more than int32 offsets can name (the size of a buffer, say): the
+    // offsets tell the entries
+    auto *h = (int *)pinned(ctx, 2 * sizeof(int));
+    if (!h) return APSPIE_ERR_OOM;
+    cudaMemcpyAsync(h, d_Lptr, sizeof(int), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(h + 1, d_Lptr + m, sizeof(int), cudaMemcpyDeviceToHost, st);
+    const int rc = check_cuda(ctx, cudaStreamSynchronize(st), "apspie_tc");
+    if (rc) return rc;
+    lnnz = h[1] - h[0];
+    if (lnnz <= 0) return APSPIE_OK;
+  }
   auto *lists = (int *)workspace(ctx, kSlotMisc0, sizeof(int) * (size_t)m);
   // an end with units has more than kTcWarpSet entries, or a column that is
   // longer: at most 2 lnnz / kTcWarpSet such ends, 2 lnnz / kTcUnit full units

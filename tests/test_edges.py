@@ -184,3 +184,16 @@ def test_triangles_of_a_multigraph(ctx, kind, repeats):
     want = int(round((M @ M).multiply(M > 0).sum()))
     for _ in range(2):
         assert ap.triangle_count(ctx, m, lp, li) == want
+
+
+@pytest.mark.parametrize("more", [0, 1, 1 << 33])
+def test_triangle_count_takes_a_buffers_size_for_the_entries(ctx, more):
+    """nnz(L) given as more than int32 offsets can name: the offsets tell."""
+    import apspie_b200 as ap
+    from apspie_b200._native import lib
+    h = ap.gen_rmat(10, 16, seed=1)
+    _, lp, li = ap.tc_prepare(ctx, h.to_device())
+    n = C.c_int64(-1)
+    rc = lib.apspie_tc(ctx.handle, h.m, C.c_int64(2**31 - 1 + more), C.c_void_p(lp.data_ptr()),
+                       C.c_void_p(li.data_ptr()), C.byref(n))
+    assert rc == 0 and n.value == ap.triangle_count(ctx, h.m, lp, li)
